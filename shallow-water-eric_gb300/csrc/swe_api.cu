@@ -180,6 +180,7 @@ static InstConst make_const(const swe_params& p) {
   k.fricf = (float)(k.g * k.mannings * k.mannings);
   k.lambda_sgnf = (float)k.lambda_sgn;
   k.rescale_floorf = (float)k.rescale_floor;
+  k.inv_16g = 1.0 / (16.0 * k.g);
   return k;
 }
 
@@ -274,13 +275,16 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     {   // compute_dij's norm = SQRT(c.c) and normal c/norm per entry (update.f90:309-312),
         // the same IEEE operations as a kernel would do per use
       std::vector<double> nrm(L.n_entries), nx(L.n_entries), ny(L.n_entries);
+      std::vector<float2> nf(L.n_entries);
       for (int64_t e = 0; e < L.n_entries; e++) {
         const double cx = L.cx[e], cy = L.cy[e];
         const double cc = cx * cx + cy * cy;
         nrm[e] = std::sqrt(cc);
         nx[e] = cx / nrm[e];                       // padding entries (never read): 0/0
         ny[e] = cy / nrm[e];
+        nf[e] = make_float2((float)nx[e], (float)ny[e]);
       }
+      G.cnf = upload_vec(c, nf, st);
       G.cnorm = upload_vec(c, nrm, st);
       G.cnx = upload_vec(c, nx, st);
       G.cny = upload_vec(c, ny, st);
@@ -340,6 +344,10 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     w.ovh = c->buf.alloc<double>(n, st); w.v1 = c->buf.alloc<double>(n, st); w.v2 = c->buf.alloc<double>(n, st);
     w.ent = c->buf.alloc<double>(n, st); w.alpha = c->buf.alloc<double>(n, st);
     w.sqgh = c->buf.alloc<double>(n, st);
+    w.w2 = c->buf.alloc<double>(n, st); w.eta = c->buf.alloc<double>(n, st); w.rh = c->buf.alloc<double>(n, st);
+    w.flux = c->buf.alloc<double>((size_t)2 * c->S * n, st);
+    w.nf = c->buf.alloc<float4>(n, st);
+    if (c->S == 5) w.pt = c->buf.alloc<double>(n, st);
     w.dL = c->buf.alloc<double>(ne, st); w.muL = c->buf.alloc<double>(ne, st); w.fct = c->buf.alloc<double>(ne, st);
     w.dLii = c->buf.alloc<double>(n, st); w.muLii = c->buf.alloc<double>(n, st);
     w.res = c->buf.alloc<double>(n, st); w.rminus = c->buf.alloc<double>(n, st);
@@ -636,7 +644,7 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
   }
   if (kev) cudaEventRecord(kev->ev[0], s);
   if (c->precision == SWE_PREC_FP64)
-    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w.fct, nullptr, c->d_err, c->block, s, &c->w);
+    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.fct, nullptr, c->d_err, c->block, s);
   else launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, c->tune,
                    c->tiles_ok ? &c->tiles : nullptr, s);
   if (kev) cudaEventRecord(kev->ev[1], s);
@@ -963,7 +971,10 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
   std::vector<InstState> saved;
   if ((rc = save_state(c, saved))) return rc;
   if ((rc = set_inst_state_dt(c, inst, c->params[inst].dt > 0 ? c->params[inst].dt : 1.0, 1))) return rc;
-  launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w.dL, c->w.dLii, c->d_err, c->block, c->stream);
+  StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
+  a.w.alpha = nullptr;                               // the last euler call's alpha stays readable
+  launch_node_f64(a, c->stream);
+  launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, c->stream);
   CK(cudaGetLastError());
   if ((rc = read_errors(c))) { restore_done(c, saved); return rc; }
   std::vector<double> d(c->meshes[inst].ja.size());

@@ -22,6 +22,7 @@ struct InstConst {
   float gf, htinyf, htiny_lo;      // htiny = htinyf + htiny_lo (double-float)
   float fricf;                     // g n^2 (friction)
   float lambda_sgnf, rescale_floorf;
+  double inv_16g;                  // 1 / (16 g), rounded once
 };
 
 // Per-instance time-loop state, device resident.
@@ -60,6 +61,7 @@ struct Graph {
   const double* __restrict__ cnorm;       // FP64 path, per entry: |c_ij| and c_ij/|c_ij|
   const double* __restrict__ cnx;         // (compute_dij's norm and normal, formed once)
   const double* __restrict__ cny;
+  const float2* __restrict__ cnf;         // FP64 path, per entry: the normal in FP32
   const double* __restrict__ lumped;
   const double* __restrict__ inv_lumped;
   const float* __restrict__ lumpedf;      // FP32 copies (mixed path)
@@ -260,6 +262,154 @@ __device__ __forceinline__ bool lambda_vacc(T hl, T qxl, T qyl, T ovhl, T sqghl,
   T lbdr = vr + sqr * sqrt((T(1) + tmax((ht - hr) * ovhr / T(2), T(0))) * (T(1) + tmax((ht - hr) * ovhr, T(0))));
   *lambda = tmax(tabs(lbdl), tabs(lbdr));
   return ok;
+}
+
+// ---- FP64 arithmetic on GB300: an FP64 instruction (add, multiply, compare,
+// conversion) holds an SM's FP64 unit for 16 cycles per warp, an integer or
+// FP32 one a quarter to half a cycle.  The FP64 kernels therefore compare and
+// select with integer instructions on the bits, divide by values whose
+// reciprocal is known with three FP64 instructions instead of about seven,
+// and decide in FP32, with error bounds, which of the reference's branches
+// can matter before they evaluate one in FP64.  Every result keeps the
+// reference's bits (the sign of a zero aside).
+__device__ __forceinline__ long long bits64(double x) { return __double_as_longlong(x); }
+// MAX(x, 0)
+__device__ __forceinline__ double pos_part(double x) { return bits64(x) > 0 ? x : 0.0; }
+// MAX, MIN of non-negative values
+__device__ __forceinline__ double max_nn(double a, double b) { return bits64(a) > bits64(b) ? a : b; }
+__device__ __forceinline__ double min_nn(double a, double b) { return bits64(a) < bits64(b) ? a : b; }
+// h <= t for t >= 0 and any h
+__device__ __forceinline__ bool le_nn(double h, double t) { return bits64(h) <= bits64(t); }
+// integers in the order of the doubles
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = bits64(x);
+  return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+__device__ __forceinline__ double max_any(double a, double b) { return order_key(a) > order_key(b) ? a : b; }
+__device__ __forceinline__ double min_any(double a, double b) { return order_key(a) < order_key(b) ? a : b; }
+
+// a / b correctly rounded, given y = 1/b correctly rounded: q = RN(a y) is
+// within 1.5 units in the last place of a/b, r = a - b q is exact, and
+// RN(q + r y) is RN(a / b) (Markstein, IBM J. Res. Dev. 34(1), 1990;
+// Brisebarre, Muller and Raina, IEEE Trans. Comput. 53(8), 2004) while no
+// intermediate leaves the normal range: a is 0 or within 2^+-600 and y within
+// 2^+-400, else the ordinary division.
+__host__ __device__ __forceinline__ bool div_range(unsigned hi_a, unsigned lo_a, unsigned hi_y) {
+  const unsigned ea = (hi_a >> 20) & 0x7ffu, ey = (hi_y >> 20) & 0x7ffu;
+  return (ea - 423u <= 1200u || ((hi_a << 1) | lo_a) == 0u) && ey - 623u <= 800u;
+}
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+  if (div_range((unsigned)__double2hiint(a), (unsigned)__double2loint(a), (unsigned)__double2hiint(y))) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+  }
+  return a / b;
+}
+
+// The general evaluation, out of line: the states the FP32 tests of
+// lambda_row cannot settle (thin films, depth ratios above 3.34, strong
+// compression).
+static __device__ __noinline__ double lambda_general(double hl, double qxl, double qyl, double ovhl, double sqghl,
+                                                     double hr, double qxr, double qyr, double ovhr, double sqghr,
+                                                     double nx, double ny, double g, double htiny, bool* ok) {
+  const LamConstF64<double> k = lam_const_f64(g, sqrt(2.0));
+  double lam;
+  *ok = lambda_vacc(hl, qxl, qyl, ovhl, sqghl, hr, qxr, qyr, ovhr, sqghr, nx, ny, g, htiny, k, &lam);
+  return lam;
+}
+
+// A state as compute_lambda_vacc sees it, and its FP32 shadow
+// (h, sqrt(g |h|), q one_over_h).
+struct LamState {
+  double h, q1, q2, ovh, sq;
+  float4 f;
+};
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// compute_lambda_vacc (SOURCES/condlim.f90:879-957) with the same bits and
+// about a third of the FP64 instructions (the bound of k_dt_f64 and
+// k_low_f64).  With c = sqrt(g h):
+//  * phi(x0 hmin) >= 0, the two-rarefaction branch, is certain when
+//    x0 hmin > hmax and vl - vr <= 1.888 c_min: then both terms of phi are
+//    shocks and the one of hmin alone is (x0 - 1) sqrt((1 + 1/x0) / 2) c_min =
+//    1.8884 c_min.  phi's square roots and division are not formed.
+//  * sqrt((1 + max(x/2, 0)) (1 + max(x, 0))) is 1 exactly where ht <= h.
+//  * only the larger of |lambda_l| and |lambda_r| is formed where FP32 tells
+//    them apart.
+// FP32 bounds: with M = sum |v| + 2 (c_l + c_r) the FP32 velocities, c and s
+// are within 8 roundings (5e-7 M) and the two speeds within 2e-6 M; the tests
+// use 2e-6 M and 1e-5 M.  What is not certain is evaluated in full.
+__device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r, double nx, double ny, float2 nf,
+                                           const InstConst& c, double* lambda) {
+  const float lv = nf.x * l.f.z + nf.y * l.f.w, rv = nf.x * r.f.z + nf.y * r.f.w;
+  const float M = fabsf(l.f.z) + fabsf(l.f.w) + fabsf(r.f.z) + fabsf(r.f.w) + 2.f * (l.f.y + r.f.y);
+  const float tol = 2e-6f * M;
+  const float hmin = fminf(l.f.x, r.f.x), hmax = fmaxf(l.f.x, r.f.x);
+  if (!(hmin > 1.00001f * c.htinyf && 3.3431f * hmin > hmax && (lv - rv) + tol <= 1.888f * fminf(l.f.y, r.f.y) &&
+        hmin > 1e-30f && hmax < 1e30f)) {
+    if (((bits64(l.h) | bits64(r.h)) << 1) == 0 && bits64(c.htiny) > 0) {   // two dry nodes: v = 0, c = 0
+      *lambda = 0.0;
+      return true;
+    }
+    bool ok;
+    *lambda = lambda_general(l.h, l.q1, l.q2, l.ovh, l.sq, r.h, r.q1, r.q2, r.ovh, r.sq, nx, ny, c.g, c.htiny, &ok);
+    return ok;
+  }
+  const float s = (lv - rv) + 2.f * (l.f.y + r.f.y);
+  const float i16g = 0.0625f / c.gf;
+  const float su = fmaxf(s + tol, 0.f), sm = fmaxf(s, 0.f);
+  const float hup = su * su * i16g * 1.000002f, hst = sm * sm * i16g;   // ht <= hup
+  const bool triv_l = hup <= l.f.x * 0.999998f, triv_r = hup <= r.f.x * 0.999998f;
+  const float xl = fmaxf(__fdividef(hst - l.f.x, l.f.x), 0.f), xr = fmaxf(__fdividef(hst - r.f.x, r.f.x), 0.f);
+  const float al = fabsf(lv - l.f.y * sqrt_approx((1.f + 0.5f * xl) * (1.f + xl)));
+  const float ar = fabsf(rv + r.f.y * sqrt_approx((1.f + 0.5f * xr) * (1.f + xr)));
+  const float tl = 1e-5f * M;
+  const bool need_l = !(ar > al + tl), need_r = !(al > ar + tl);
+  // the side evaluated first: l unless r is the larger for certain
+  const bool both = need_l && need_r;
+  const bool tr1 = need_l ? triv_l : triv_r;
+  const double h1 = need_l ? l.h : r.h, o1 = need_l ? l.ovh : r.ovh, c1 = need_l ? l.sq : r.sq;
+  const double v1 = __dmul_rn(__dadd_rn(__dmul_rn(need_l ? l.q1 : r.q1, nx), __dmul_rn(need_l ? l.q2 : r.q2, ny)), o1);
+  double f1 = 1.0, v2 = 0.0, ht = 0.0;
+  const bool nt = !tr1 || (both && !triv_r);
+  if (nt || both) {
+    const double o2 = need_l ? r.ovh : l.ovh;
+    v2 = __dmul_rn(__dadd_rn(__dmul_rn(need_l ? r.q1 : l.q1, nx), __dmul_rn(need_l ? r.q2 : l.q2, ny)), o2);
+  }
+  if (nt) {
+    const double vl = need_l ? v1 : v2, vr = need_l ? v2 : v1;
+    // ((vl - vr) + 2 sql) + 2 sqr, each product by 2 exact
+    const double sd = pos_part(__fma_rn(2.0, r.sq, __fma_rn(2.0, l.sq, __dsub_rn(vl, vr))));
+    ht = div_known(__dmul_rn(sd, sd), 16.0 * c.g, c.inv_16g);
+    if (!(hup < 3.3431f * hmin)) {
+      const double t0 = 2.0 * sqrt(2.0) - 1.0;
+      ht = tmin((t0 * t0) * tmin(l.h, r.h), ht);
+    }
+    if (!tr1) {
+      const double x = pos_part(__dmul_rn(__dsub_rn(ht, h1), o1));
+      f1 = sqrt(__dmul_rn(__fma_rn(x, 0.5, 1.0), __dadd_rn(1.0, x)));   // x/2 is exact
+    }
+  }
+  double cf = tr1 ? c1 : __dmul_rn(c1, f1);
+  double lam = fabs(need_l ? __dsub_rn(v1, cf) : __dadd_rn(v1, cf));
+  if (both) {
+    double f2 = f1;
+    if (bits64(l.h) != bits64(r.h)) {                     // equal depths: equal factors
+      f2 = 1.0;
+      if (!triv_r) {
+        const double x = pos_part(__dmul_rn(__dsub_rn(ht, r.h), r.ovh));
+        f2 = sqrt(__dmul_rn(__fma_rn(x, 0.5, 1.0), __dadd_rn(1.0, x)));
+      }
+    }
+    lam = max_nn(lam, fabs(__dadd_rn(v2, __dmul_rn(r.sq, f2))));
+  }
+  *lambda = lam;
+  return true;
 }
 
 }  // namespace swe

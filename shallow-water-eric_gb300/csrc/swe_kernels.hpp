@@ -28,6 +28,12 @@ struct StateMix {
 struct WorkF64 {
   double *ovh, *v1, *v2, *ent, *alpha;   // per row
   double* sqgh;                          // per row: sqrt(g |h|)
+  double* w2;                            // per row: qy one_over_h (v2 is 0 for type 13)
+  double *eta, *rh;                      // per row: h + z, 1/h
+  double* flux;                          // per row: v1 u_q, v2 u_q (component q at 2 q n_rows, (2 q + 1) n_rows)
+  double* pt;                            // per row: the SGN pressure pTilde (type 13)
+  float4* nf;                            // per row, FP32: h, sqrt(g |h|), q one_over_h
+  double* ab;                            // per entry: the row differences of the fused 'fct' kernels, or null
   double *dL, *muL, *fct;                // per off-diagonal entry
   double *dLii, *muLii;                  // per row: the diagonal of dL, muL
   double *res, *rminus;                  // per row
@@ -57,6 +63,8 @@ struct StageArgs {
   unsigned* err;
   int block;
   int entropy = 0;   // some instance uses 'entropy_visc': launch k_entropy
+  int fused = 0;     // every instance runs 'fct' with the roundoff fix: the fused row kernels
+  int S = 3;
   const double* dij_in = nullptr;   // stage 1: d_ij of k_dt on the same state (bit-identical)
   int skip_node = 0;                // stage 1: k_node already ran on this state (before k_dt)
 };
@@ -95,9 +103,10 @@ struct KernelEvents {
 };
 
 void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* kev = nullptr);
-void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, double* d_out,
-                   double* dii_out, unsigned* err, int block, cudaStream_t s, const WorkF64* node = nullptr);
-void launch_node_f64(const StageArgs& a, cudaStream_t s);   // per-node arrays of the state a.u
+// launch_node_f64: per-node arrays of the state a.u; launch_dt_f64 reads them (node)
+void launch_node_f64(const StageArgs& a, cudaStream_t s);
+void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
+                   double* d_out, double* dii_out, unsigned* err, int block, cudaStream_t s);
 void launch_step_begin(const InstConst* C, InstState* St, int n_inst, cudaStream_t s);
 void launch_step_end(InstState* St, int n_inst, cudaStream_t s);
 void launch_reset_counters(InstState* St, int n_inst, cudaStream_t s);

@@ -23,14 +23,44 @@ struct NodeF64 {        // per-row arrays of the FP64 path
   double* v1;
   double* v2;
   double* ent;
-  double* alpha;
+  double* alpha;        // or null: no alpha_i (swe_compute_dij)
   double* sqgh;         // sqrt(g |h|), the sql / sqr of compute_lambda_vacc
+  double* w2;           // qy one_over_h (v2 unless type 13)
+  double* eta;          // h + z
+  double* rh;           // 1/h
+  double* flux;         // v1 u_q and v2 u_q: (2 q + a) n_rows + r
+  double* pt;           // SGN pressure (type 13)
+  float4* nf;           // FP32: h, sqrt(g |h|), q one_over_h
 };
+static NodeF64 node_of(const WorkF64& w) {
+  return NodeF64{w.ovh, w.v1, w.v2, w.ent, w.alpha, w.sqgh, w.w2, w.eta, w.rh, w.flux, w.pt, w.nf};
+}
+
+// The state of row r as lambda_row takes it.
+__device__ __forceinline__ LamState lam_state(const StateF64& u, const NodeF64& nd, int64_t r) {
+  return LamState{u.h[r], u.q1[r], u.q2[r], nd.ovh[r], nd.sqgh[r], nd.nf[r]};
+}
+
+// SGN pressure pTilde_n and source s_n (mSGN_RHS, update.f90:505-529)
+__device__ __forceinline__ void sgn_node_f64(const InstConst& c, double m, double h, double heta,
+                                             double* pTilde, double* s) {
+  double lms = sqrt(m);
+  double pc = c.lambda_sgn * c.g / (3.0 * lms);
+  double x = heta / (h * h);
+  double psi = 12.0 * (x - 1.0);
+  double x3 = (x * x) * x, x4 = (x * x) * (x * x);
+  *pTilde = pc * ((h * h) * h) * (2.0 + 4.0 * x3 - 6.0 * x4);
+  double t = heta / h;
+  *s = 3.0 * pc * (t * t) * psi;
+}
 
 // ---------------------------------------------------------------------------
 // k_node: flux() globals (SOURCES/condlim.f90:21-77, 79-90), the entropy
-// E_i = 0.5 (g h^2 + v.q) of entropy_residual (update.f90:844-851) and the
-// smoothness indicator alpha_i of alpha_limit (update.f90:758-781).
+// E_i = 0.5 (g h^2 + v.q) of entropy_residual (update.f90:844-851), the
+// smoothness indicator alpha_i of alpha_limit (update.f90:758-781), and every
+// other quantity of one node that the entry loops would otherwise form once
+// per entry: the flux products v u_q, h + z, 1/h, the SGN pressure and the
+// FP32 shadow of lambda_row.
 // ---------------------------------------------------------------------------
 __global__ void k_node_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
                            StateF64 u, NodeF64 nd) {
@@ -41,18 +71,41 @@ __global__ void k_node_f64(Graph G, const InstConst* __restrict__ C, const InstS
   int b = G.slice_inst[r >> 5];
   if (St[b].done) return;
   const InstConst& c = C[b];
+  const int64_t n = G.n_rows;
   double h = u.h[r], qx = u.q1[r], qy = u.q2[r];
   double o = one_over_h(h, c.htiny);
   double v1 = qx * o;
-  double v2 = (c.type_test == 13) ? qy * o * 0.0 : qy * o;
+  double w2 = qy * o;
+  double v2 = (c.type_test == 13) ? w2 * 0.0 : w2;
+  const double sq = sqrt(c.g * fabs(h));
   nd.ovh[r] = o;
   nd.v1[r] = v1;
   nd.v2[r] = v2;
-  nd.sqgh[r] = sqrt(c.g * tabs(h));
+  nd.w2[r] = w2;
+  nd.sqgh[r] = sq;
+  nd.eta[r] = h + G.bath[r];
+  nd.rh[r] = 1.0 / h;
+  nd.nf[r] = make_float4((float)h, (float)sq, (float)v1, (float)w2);
+  const double f10 = v1 * h, f11 = v1 * qx, f22 = v2 * qy;
+  nd.flux[r] = f10;
+  nd.flux[2 * n + r] = f11;
+  nd.flux[4 * n + r] = v1 * qy;
+  if (c.type_test == 13) {           // v2 = 0
+    const double heta = u.q3[r];
+    nd.flux[6 * n + r] = v1 * heta;
+    nd.flux[8 * n + r] = v1 * u.q4[r];
+    double s;
+    sgn_node_f64(c, G.lumped[r], h, heta, &nd.pt[r], &s);
+  } else {
+    nd.flux[n + r] = v2 * h;
+    nd.flux[3 * n + r] = v2 * qx;
+    nd.flux[5 * n + r] = f22;
+  }
   double E = c.g * (h * h);
-  E = E + v1 * qx;
-  E = E + v2 * qy;
+  E = E + f11;
+  E = E + f22;
   nd.ent[r] = 0.5 * E;
+  if (!nd.alpha) return;
   double alpha = 1.0;
   if (c.alpha_limit && !(h <= c.htiny)) {
     const int64_t base = entry_base(G, r);
@@ -62,7 +115,7 @@ __global__ void k_node_f64(Graph G, const InstConst* __restrict__ C, const InstS
       const int k = kk - (kk > dp ? 1 : 0);
       const double hj = (kk == dp) ? h : u.h[G.col[base + 32 * k]];
       num = num + hj - h;
-      denom = denom + tabs(hj - h);
+      denom = denom + fabs(hj - h);
     }
     double a = (denom <= tabs(num)) ? 1.0 : tabs(num) / (denom);
     double a2 = a * a, a4 = a2 * a2;
@@ -99,19 +152,6 @@ __device__ __forceinline__ void source_f64(const InstConst& c, const InstState& 
     rk[3] = rk[3] + m * ui[4];
     rk[4] = rk[4] - m * s_i;
   }
-}
-
-// SGN pressure pTilde_n and source s_n (mSGN_RHS, update.f90:505-529)
-__device__ __forceinline__ void sgn_node_f64(const InstConst& c, double m, double h, double heta,
-                                             double* pTilde, double* s) {
-  double lms = sqrt(m);
-  double pc = c.lambda_sgn * c.g / (3.0 * lms);
-  double x = heta / (h * h);
-  double psi = 12.0 * (x - 1.0);
-  double x3 = (x * x) * x, x4 = (x * x) * (x * x);
-  *pTilde = pc * ((h * h) * h) * (2.0 + 4.0 * x3 - 6.0 * x4);
-  double t = heta / h;
-  *s = 3.0 * pc * (t * t) * psi;
 }
 
 // Viscosities seen by the row sums: the low-order (alpha-limited) d_ij, mu_ij,
@@ -242,8 +282,7 @@ __device__ __forceinline__ void smb_rows_f64(const Graph& G, const InstConst& c,
       const int64_t e = base + 32 * (kk - (kk > dp ? 1 : 0));
       const int j = isd ? (int)r : G.col[e];
       const double cxe = isd ? G.cxii[r] : G.cx[e], cye = isd ? G.cyii[r] : G.cy[e];
-      double pj, sj;
-      sgn_node_f64(c, G.lumped[j], u.h[j], u.q3[j], &pj, &sj);
+      const double pj = nd.pt[j];
       ax = ax - pj * cxe; ay = ay - pj * cye;
       bx = bx - pj * cxe; by = by - pj * cye;
       tx = tx - pj * cxe; ty = ty - pj * cye;
@@ -278,9 +317,9 @@ __global__ void k_low_f64(Graph G, const InstConst* __restrict__ C, const InstSt
   const InstConst& c = C[b];
   const int S = c.S;
   const double g = c.g, htiny = c.htiny, dt = st.dt;
-  const LamConstF64<double> lk = lam_const_f64(g, sqrt(2.0));
   const int64_t base = entry_base(G, r);
   const int dp = G.dpos[r];
+  const LamState li = lam_state(u, nd, r);
   double ui[5];
   ui[0] = u.h[r]; ui[1] = u.q1[r]; ui[2] = u.q2[r];
   if (S == 5) { ui[3] = u.q3[r]; ui[4] = u.q4[r]; }
@@ -301,13 +340,9 @@ __global__ void k_low_f64(Graph G, const InstConst* __restrict__ C, const InstSt
       if (dij_in) {                            // stage 1: k_dt computed this d_ij on this state
         d = dij_in[e];
       } else {
-        const double norm = G.cnorm[e], nx = G.cnx[e], ny = G.cny[e];   // sqrt(c.c), c/norm
         double lam;
-        if (!lambda_vacc(ui[0], ui[1], ui[2], ovhi, nd.sqgh[r], u.h[j], u.q1[j], u.q2[j], nd.ovh[j], nd.sqgh[j], nx,
-                         ny, g, htiny, lk,
-                         &lam))
-          delta_bad = true;
-        d = norm * lam;
+        if (!lambda_row(li, lam_state(u, nd, j), G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) delta_bad = true;
+        d = G.cnorm[e] * lam;                   // sqrt(c.c) lambda_max, normal c/sqrt(c.c)
       }
       const double sl = cxe * v1i + cye * v2i;
       // compute_muij uses q*ovh of the raw state, equal to velocity except
@@ -615,52 +650,31 @@ __global__ void k_entropy_f64(Graph G, const InstConst* __restrict__ C, const In
 // max |d_ii|/m_i (main.f90:166-174), per instance.  d_out (nullable)
 // receives every d_ij.
 // ---------------------------------------------------------------------------
-__global__ void k_dt_f64(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St, StateF64 u,
-                         const double* __restrict__ ovh, const double* __restrict__ sqgh, double* __restrict__ d_out,
-                         double* __restrict__ dii_out, unsigned* __restrict__ err) {
+__global__ void k_dt_f64(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St, StateF64 u, NodeF64 nd,
+                         double* __restrict__ d_out, double* __restrict__ dii_out, unsigned* __restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double val = 0.0;
-  int b = -1;
-  if (r < G.n_rows && G.len[r] > 0) {
-    b = G.slice_inst[r >> 5];
-    if (!St[b].done) {
-      const InstConst& c = C[b];
-      const int L = G.len[r];
-      const int64_t base = entry_base(G, r);
-      const LamConstF64<double> lk = lam_const_f64(c.g, sqrt(2.0));
-      const double hi = u.h[r], q1 = u.q1[r], q2 = u.q2[r];
-      const double ovhi = ovh ? ovh[r] : one_over_h(hi, c.htiny);
-      const double sqgi = sqgh ? sqgh[r] : sqrt(c.g * tabs(hi));
-      double s = 0.0;
-      bool bad = false;
-      for (int k = 0; k < L; k++) {
-        const int64_t e = base + 32 * k;
-        double d = 0.0;
-        {
-          const int j = G.col[e];
-          const double norm = G.cnorm[e];                                  // sqrt(c.c)
-          const double hj = u.h[j];
-          const double ovhj = ovh ? ovh[j] : one_over_h(hj, c.htiny);
-          const double sqgj = sqgh ? sqgh[j] : sqrt(c.g * tabs(hj));
-          double lam;
-          if (!lambda_vacc(hi, q1, q2, ovhi, sqgi, hj, u.q1[j], u.q2[j], ovhj, sqgj, G.cnx[e], G.cny[e], c.g,
-                           c.htiny, lk, &lam))
-            bad = true;
-          d = norm * lam;
-        }
-        if (d_out) d_out[e] = d;
-        s = s + d;
-      }
-      if (dii_out) dii_out[r] = -s;
-      val = tabs(-s) / G.lumped[r];
-      if (bad) atomicOr(err, ERRB_DELTA);
-    } else {
-      b = -1;
+  if (r < G.n_rows && G.len[r] > 0 && !St[G.slice_inst[r >> 5]].done) {
+    const InstConst& c = C[G.slice_inst[r >> 5]];
+    const int L = G.len[r];
+    const int64_t base = entry_base(G, r);
+    const LamState li = lam_state(u, nd, r);
+    double s = 0.0;
+    bool bad = false;
+    for (int k = 0; k < L; k++) {
+      const int64_t e = base + 32 * k;
+      double lam;
+      if (!lambda_row(li, lam_state(u, nd, G.col[e]), G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
+      const double d = G.cnorm[e] * lam;                                   // sqrt(c.c) lambda_max
+      if (d_out) d_out[e] = d;
+      s = s + d;
     }
+    if (dii_out) dii_out[r] = -s;
+    val = div_known(fabs(-s), G.lumped[r], G.inv_lumped[r]);
+    if (bad) atomicOr(err, ERRB_DELTA);
   }
   // warp-level max per instance: a warp covers one 32-row slice and a slice
   // never straddles two instances
-  (void)b;
   const unsigned full = 0xffffffffu;
   for (int off = 16; off > 0; off >>= 1) val = fmax(val, __shfl_down_sync(full, val, off));
   const int64_t r0 = r & ~(int64_t)31;
@@ -777,13 +791,13 @@ static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) 
 #define EV_END(k) if (kev) cudaEventRecord(kev->ev[2 * (k) + 1], s)
 
 void launch_node_f64(const StageArgs& a, cudaStream_t s) {
-  NodeF64 nd{a.w.ovh, a.w.v1, a.w.v2, a.w.ent, a.w.alpha, a.w.sqgh};
+  const NodeF64 nd = node_of(a.w);
   k_node_f64<<<nblk(a.G.n_rows, a.block), a.block, 0, s>>>(a.G, a.C, a.St, a.u, nd);
 }
 
 void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* kev) {
   const int bs = a.block;
-  NodeF64 nd{a.w.ovh, a.w.v1, a.w.v2, a.w.ent, a.w.alpha, a.w.sqgh};
+  const NodeF64 nd = node_of(a.w);
   EV_BEGIN(1);
   if (!a.skip_node) k_node_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, nd);
   EV_END(1); EV_BEGIN(2);
@@ -801,10 +815,9 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
   EV_END(4);
 }
 
-void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, double* d_out,
-                   double* dii_out, unsigned* err, int block, cudaStream_t s, const WorkF64* node) {
-  k_dt_f64<<<nblk(G.n_rows, block), block, 0, s>>>(G, C, St, u, node ? node->ovh : nullptr,
-                                                   node ? node->sqgh : nullptr, d_out, dii_out, err);
+void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
+                   double* d_out, double* dii_out, unsigned* err, int block, cudaStream_t s) {
+  k_dt_f64<<<nblk(G.n_rows, block), block, 0, s>>>(G, C, St, u, node_of(node), d_out, dii_out, err);
 }
 
 void launch_step_begin(const InstConst* C, InstState* St, int n_inst, cudaStream_t s) {

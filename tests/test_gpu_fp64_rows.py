@@ -1,0 +1,84 @@
+"""The FP64 row kernels against the oracle, bit for bit, on states chosen to
+take every branch of their wave-speed bound and of their row sums: thin films
+about htiny, two dry nodes, equal and nearly equal depths, depth ratios about
+(2 sqrt2 - 1)^2, strong compression and expansion, supercritical flow, depths
+far outside the ordinary range.  No tolerance: the kernels form the oracle's
+own roundings."""
+
+import numpy as np
+import pytest
+
+import oracle
+from swe import cases as C, mesh as M
+from swe import lib as L
+from swe.update import Update
+
+pytestmark = pytest.mark.gpu
+
+STATES = ["rest", "equal", "near_equal", "ratio", "film", "dry", "compress", "expand", "fast", "mixed", "tiny", "huge"]
+
+
+def _state(kind, n, htiny, rng):
+    h = rng.uniform(0.5, 1.5, n)
+    v = rng.normal(0.0, 0.3, (2, n))
+    if kind == "rest":
+        h[:], v[:] = 0.7, 0.0
+    elif kind == "equal":
+        h[:] = 0.7
+    elif kind == "near_equal":
+        h = 0.7 * (1.0 + rng.integers(-3, 4, n) * 2.0 ** -52)
+        v *= 1e-9
+    elif kind == "ratio":                        # about the two-rarefaction limit of the depth ratio
+        h = np.where(rng.random(n) < 0.5, 1.0, 3.3431457505 * (1.0 + rng.uniform(-2e-4, 2e-4, n)))
+    elif kind == "film":
+        h = htiny * (1.0 + rng.choice([-1e-3, -1e-6, -1e-12, 0.0, 1e-12, 1e-6, 1e-3, 2.0], n))
+        v *= 0.01
+    elif kind == "dry":
+        h = np.where(rng.random(n) < 0.6, 0.0, h)
+    elif kind in ("compress", "expand"):         # |vl - vr| about 1.888 sqrt(g h)
+        v = (1 if kind == "expand" else -1) * rng.normal(0.0, 6.0, (2, n))
+    elif kind == "fast":
+        v = np.array([[300.0], [-200.0]]) + v
+    elif kind == "mixed":
+        h = np.exp(rng.uniform(np.log(1e-3 * htiny), np.log(2.0), n)) * (rng.random(n) < 0.9)
+        v *= np.where(h < 10 * htiny, 0.01, 1.0)
+    elif kind == "tiny":
+        h = np.where(rng.random(n) < 0.5, h, 10.0 ** rng.uniform(-300, -20, n))
+    elif kind == "huge":
+        h = h * 1e30
+        v *= 1e14
+    return np.asfortranarray(np.vstack([h, h * v[0], h * v[1]]))
+
+
+def _pair(mesh, bath, p):
+    o = oracle.Oracle(mesh["jj"], mesh["rr"])
+    o.set_params(oracle.Params(*p.fields()))
+    o.set_bath(bath)
+    return o, Update(mesh, bath, p)
+
+
+def _both(f_oracle, f_gpu, codes):
+    """The oracle's result and the GPU's, or (None, None) where both refuse."""
+    try:
+        ref = f_oracle()
+    except oracle.OracleError:
+        with pytest.raises(L.SweError) as e:
+            f_gpu()
+        assert e.value.code in codes
+        return None, None
+    return ref, f_gpu()
+
+
+@pytest.mark.parametrize("n", [5, 33])
+@pytest.mark.parametrize("kind", STATES)
+def test_dij_bit_exact(kind, n):
+    rng = np.random.default_rng(STATES.index(kind) + n)
+    mesh = M.jittered_mesh(n, n, 0.0, 1.0, 0.0, 1.0, jitter=0.3, seed=4)
+    p = C.Params(max_water_h=1.0, htiny=1e-4)
+    o, upd = _pair(mesh, np.zeros(n * n), p)
+    for _ in range(4):
+        u = _state(kind, n * n, p.htiny, rng)
+        ref, got = _both(lambda: o.compute_dij(u), lambda: upd.compute_dij(u), (L.SWE_ERR_DELTA,))
+        if ref is not None:
+            np.testing.assert_array_equal(got[0], ref[0])
+            assert got[1] == ref[1]
