@@ -197,6 +197,13 @@ static bool has_entropy(const swe_ctx* c) {
   return false;
 }
 
+// every instance runs 'fct' with the roundoff fix: the FP64 path's fused row kernels
+static bool all_fct(const swe_ctx* c) {
+  for (const swe_params& p : c->params)
+    if (p.viscosity_type != SWE_VISC_FCT || !p.if_roundoff_fix) return false;
+  return true;
+}
+
 static int check_params(swe_ctx* c, const swe_params& p) {
   if (p.syst_size != 3 && p.syst_size != 5) return fail(c, SWE_ERR_ARG, "syst_size must be 3 or 5");
   if ((p.syst_size == 5) != (p.type_test == 13)) return fail(c, SWE_ERR_ARG, "syst_size 5 goes with type_test 13");
@@ -348,6 +355,8 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     w.flux = c->buf.alloc<double>((size_t)2 * c->S * n, st);
     w.nf = c->buf.alloc<float4>(n, st);
     if (c->S == 5) w.pt = c->buf.alloc<double>(n, st);
+    w.ab = c->buf.alloc<double>((size_t)2 * c->S * ne, st);
+    w.n_entries = (int64_t)ne;
     w.dL = c->buf.alloc<double>(ne, st); w.muL = c->buf.alloc<double>(ne, st); w.fct = c->buf.alloc<double>(ne, st);
     w.dLii = c->buf.alloc<double>(n, st); w.muLii = c->buf.alloc<double>(n, st);
     w.res = c->buf.alloc<double>(n, st); w.rminus = c->buf.alloc<double>(n, st);
@@ -655,6 +664,8 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
     if (c->precision == SWE_PREC_FP64) {
       StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, stage, nullptr, c->d_err, c->block};
       a.entropy = has_entropy(c);
+      a.fused = all_fct(c);
+      a.S = c->S;
       if (stage == 1) { a.dij_in = c->w.fct; a.skip_node = 1; }
       if (stage == 2) { a.u = c->B; a.out = c->Cs; }
       if (stage == 3) { a.u = c->Cs; a.out = c->A; }
@@ -805,6 +816,10 @@ SWE_API int swe_set_params(swe_ctx* c, int inst, const swe_params* p) {
   if (rc) return rc;
   if (p->syst_size != c->S || p->precision != c->precision)
     return fail(c, SWE_ERR_ARG, "syst_size and precision are fixed at creation");
+  const swe_params& was = c->params[inst];
+  if (was.viscosity_type != p->viscosity_type || was.viscous_type != p->viscous_type ||
+      was.if_roundoff_fix != p->if_roundoff_fix)
+    drop_graphs(c);                                  // the captured kernels follow the modes
   c->params[inst] = *p;
   InstConst k = make_const(*p);
   CK(cudaMemcpyAsync(c->d_C + inst, &k, sizeof(InstConst), cudaMemcpyHostToDevice, c->stream));
@@ -1002,6 +1017,8 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
   if (c->precision == SWE_PREC_FP64) {
     StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
+    a.fused = all_fct(c);
+    a.S = c->S;
     launch_stage_f64(a, c->stream);
   } else {
     StageArgsMix a{c->G, c->d_C, c->d_St, c->mA, c->mA, c->mB, c->wm, 0, c->d_err, c->block};

@@ -33,7 +33,8 @@ struct WorkF64 {
   double* flux;                          // per row: v1 u_q, v2 u_q (component q at 2 q n_rows, (2 q + 1) n_rows)
   double* pt;                            // per row: the SGN pressure pTilde (type 13)
   float4* nf;                            // per row, FP32: h, sqrt(g |h|), q one_over_h
-  double* ab;                            // per entry: the row differences of the fused 'fct' kernels, or null
+  double* ab;                            // per entry: the row differences of the 'fct' row kernels (2 S n_entries)
+  int64_t n_entries;
   double *dL, *muL, *fct;                // per off-diagonal entry
   double *dLii, *muLii;                  // per row: the diagonal of dL, muL
   double *res, *rminus;                  // per row
@@ -63,7 +64,7 @@ struct StageArgs {
   unsigned* err;
   int block;
   int entropy = 0;   // some instance uses 'entropy_visc': launch k_entropy
-  int fused = 0;     // every instance runs 'fct' with the roundoff fix: the fused row kernels
+  int fused = 0;     // every instance runs 'fct' with the roundoff fix: the 'fct' row kernels
   int S = 3;
   const double* dij_in = nullptr;   // stage 1: d_ij of k_dt on the same state (bit-identical)
   int skip_node = 0;                // stage 1: k_node already ran on this state (before k_dt)

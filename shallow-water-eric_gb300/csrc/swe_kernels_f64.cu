@@ -124,6 +124,20 @@ __global__ void k_node_f64(Graph G, const InstConst* __restrict__ C, const InstS
   nd.alpha[r] = alpha;
 }
 
+// x**gamma of the Manning friction (update.f90:436), gamma = 4/3 rounded to 64
+// bits: with c = cbrt(x), r = x - c^3 (exact products), x**(4/3) = x c + c r/3,
+// and x**(gamma - 4/3) = 1 + (gamma - 4/3) ln x.  Within 0.6 units in the last
+// place over [1e-8, 20] (CUDA's pow: 1.0), in 29 FP64 instructions against 99.
+__device__ __forceinline__ double pow_43(double x) {
+  const double c = cbrt(x), c2 = c * c, p = x * c;
+  const double r = __fma_rn(-__fma_rn(c, c, -c2), c, __fma_rn(-c2, c, x));
+  const float lx = __logf(fminf(fmaxf((float)x, 1.2e-38f), 3e38f));
+  double t = __fma_rn(x, c, -p);
+  t = __fma_rn(c * r, 1.0 / 3.0, t);
+  t = __fma_rn(p, (double)(-7.4014868308343765e-17f * lx), t);
+  return p + t;
+}
+
 // Source terms (SOURCES/update.f90:425-551) added to the undivided rk of one
 // row.  velocity is the row's own (v1, v2).
 __device__ __forceinline__ void source_f64(const InstConst& c, const InstState& st, double m, const double* ui,
@@ -131,9 +145,9 @@ __device__ __forceinline__ void source_f64(const InstConst& c, const InstState& 
                                            double s_i) {
   const int S = c.S;
   if (c.type_test == 9 || c.type_test == 10) {
-    const double gamma = 4.0 / 3.0, chi = 1.0;
+    const double chi = 1.0;
     double fric = c.g * c.mannings * c.mannings;
-    double hstar = pow(tmax(ui[0], c.htiny), gamma);
+    double hstar = pow_43(tmax(ui[0], c.htiny));
     double vel = fric * sqrt(v1 * v1 + v2 * v2);
     double hloc = chi * vel * st.dt;
     for (int k = 1; k < S; k++) rk[k] = rk[k] - m * ui[k] * vel * 2 / (hstar + tmax(hstar, hloc));
@@ -534,8 +548,8 @@ __device__ __forceinline__ void finish_row_f64(const Graph& G, const InstConst& 
   for (int q = 0; q < 5; q++) {
     if (q >= S) break;
     double v = un[q];
-    if (rk_stage == 2) v = (3 * comp_f64(u0, q, r) + v) / 4;
-    else if (rk_stage == 3) v = (comp_f64(u0, q, r) + 2 * v) / 3;
+    if (rk_stage == 2) v = (3 * comp_f64(u0, q, r) + v) * 0.25;
+    else if (rk_stage == 3) v = div_known(__fma_rn(2.0, v, comp_f64(u0, q, r)), 3.0, 1.0 / 3.0);   // 2 v is exact
     if (msk & (1u << q)) v = dirichlet_value(G, c, st, rk_stage, q, r);
     store_f64(out, q, r, v);
   }
@@ -642,6 +656,329 @@ __global__ void k_entropy_f64(Graph G, const InstConst* __restrict__ C, const In
     un[0] = tmax(ui[0] + dt * (rs.rk2[0] / m), 0.0);
     for (int q = 1; q < S; q++) un[q] = ui[q] + dt * (rs.rk2[q] / m);
   }
+  finish_row_f64(G, c, st, r, S, un, true, rk_stage, u0, out, err);
+}
+
+// ---------------------------------------------------------------------------
+// The 'fct' row kernels (every instance of the context runs 'fct' with the
+// roundoff fix; others take the general kernels above).  The FP64 unit bounds
+// them: an SM retires a warp's FP64 instruction in 16 cycles, so they spend
+// memory (idle at 1-3% of its rate in the general kernels) to form every
+// FP64 value once:
+//   * k_low_fct walks the row once (d_ij, mu_ij, both right-hand sides) and
+//     stores, per entry and component, the two row differences
+//       A_q = u_j rat_ji - u_i rat_ij,  B_q = u_j (1 - rat_ji) - u_i (1 - rat_ij)
+//     that compute_fct_matrix and apply_viscosity form again;
+//   * the diagonal contributes only -c_ii.F_i and the rounding residue of
+//     (h_i + z_i) - h_i - z_i: both are formed once per row and added at the
+//     diagonal's place in the row;
+//   * where both depths exceed htiny the two right-hand sides add the same
+//     products, and where both rats are 1 (flat bottom) B_q = 0;
+//   * the diagonals of d and mu enter nothing ('fct' multiplies them by
+//     u_i rat_ii - u_i rat_ii = 0): only swe_euler, which hands them out, forms
+//     them.
+// ---------------------------------------------------------------------------
+
+// H / h for H >= 0, h > 0 (rh = 1/h): 1 where they are equal
+__device__ __forceinline__ double rat_f64(double H, double h, double rh) {
+  if (bits64(h) <= 0) return 0.0;
+  return bits64(H) == bits64(h) ? 1.0 : div_known(H, h, rh);
+}
+
+template <int S>
+__global__ void __launch_bounds__(128, 4)
+k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St, StateF64 u, NodeF64 nd,
+          double* __restrict__ dL, double* __restrict__ muL, double* __restrict__ dLii, double* __restrict__ muLii,
+          StateF64 uL, double* __restrict__ res, double* __restrict__ ab, const double* __restrict__ dij_in,
+          int want_diag, int64_t n_entries, unsigned* __restrict__ err) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= G.n_rows) return;
+  const int L = G.len[r];
+  if (L == 0) return;
+  const int b = G.slice_inst[r >> 5];
+  if (St[b].done) return;
+  const InstConst& c = C[b];
+  const int64_t base = entry_base(G, r), nr = G.n_rows;
+  const int dp = G.dpos[r];
+  const double g = c.g, htiny = c.htiny;
+  const LamState li = lam_state(u, nd, r);
+  double ui[S];
+  ui[0] = li.h; ui[1] = li.q1; ui[2] = li.q2;
+  if (S == 5) { ui[3] = u.q3[r]; ui[4] = u.q4[r]; }
+  const double zi = G.bath[r], etai = nd.eta[r], rhi = nd.rh[r], ai = nd.alpha[r];
+  const double w1i = nd.v1[r], w2i = nd.w2[r], ghi = g * ui[0];
+  const bool wet_i = !le_nn(ui[0], htiny);
+  // the diagonal's terms: -c_ii.F_i and the topography residue
+  double Dq[S], Dfix, tdx, tdy;
+  {
+    const double cxd = G.cxii[r], cyd = G.cyii[r];
+    const double td = ghi * (etai - ui[0] - zi);
+    tdx = td * cxd; tdy = td * cyd;
+#pragma unroll
+    for (int q = 0; q < S; q++) {
+      Dq[q] = cxd * nd.flux[(int64_t)(2 * q) * nr + r];
+      if (S == 3) Dq[q] = Dq[q] + cyd * nd.flux[(int64_t)(2 * q + 1) * nr + r];
+    }
+    Dfix = cxd * w1i;
+    if (S == 3) Dfix = Dfix + cyd * w2i;
+  }
+  double fix = 0.0, rk[S], rk2[S];
+#pragma unroll
+  for (int q = 0; q < S; q++) rk[q] = rk2[q] = 0.0;
+  double emax = nd.ent[r], emin = emax, sd = 0.0, sm = 0.0;
+  bool bad = false;
+  for (int k = 0; k <= L; k++) {
+    if (k == dp) {                              // the diagonal's place in the row
+      fix = fix - Dfix;
+      rk2[0] = rk2[0] - Dq[0];
+#pragma unroll
+      for (int q = 1; q < S; q++) { rk[q] = rk[q] - Dq[q]; rk2[q] = rk2[q] - Dq[q]; }
+      rk[1] = rk[1] - tdx; rk[2] = rk[2] - tdy;
+      rk2[1] = rk2[1] - tdx; rk2[2] = rk2[2] - tdy;
+    }
+    if (k == L) break;
+    const int64_t e = base + 32 * k;
+    const int j = G.col[e];
+    const double cxe = G.cx[e], cye = G.cy[e];
+    const LamState lj = lam_state(u, nd, j);
+    // d_ij, mu_ij (compute_dij, compute_muij, MAX, alpha_limit)
+    double d;
+    if (dij_in) {
+      d = dij_in[e];
+    } else {
+      double lam;
+      if (!lambda_row(li, lj, G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
+      d = G.cnorm[e] * lam;
+    }
+    const double w1j = nd.v1[j];
+    const double sl = cxe * w1i + cye * w2i;
+    double sr = cxe * w1j, srf = sr;             // c.v_j: the viscosity's velocity, the flux's (type 13: v2 = 0)
+    sr = sr + cye * nd.w2[j];
+    if (S == 3) srf = sr;
+    double mu = max_nn(pos_part(-sl), pos_part(sr));
+    if (want_diag) { sd = sd + d; sm = sm + mu; }
+    d = max_nn(d, mu);
+    const double s = max_nn(ai, nd.alpha[j]);    // 1 without alpha_limit
+    d = d * s;
+    mu = mu * s;
+    dL[e] = d;
+    muL[e] = mu;
+    const double ej = nd.ent[j];
+    emax = max_any(emax, ej);
+    emin = min_any(emin, ej);
+    // hydrostatic reconstruction
+    const double zj = G.bath[j], etaj = nd.eta[j];
+    const double zmax = max_any(zi, zj);
+    const double Hij = pos_part(etai - zmax), Hji = pos_part(etaj - zmax);
+    const double qij = rat_f64(Hij, ui[0], rhi), qji = rat_f64(Hji, lj.h, nd.rh[j]);
+    const bool wet_j = !le_nn(lj.h, htiny);
+    const double dmu = d - mu;
+    // smb_2_roundoff mass row
+    fix = fix - mu - (wet_i ? dmu * qij : 0.0);
+    rk[0] = rk[0] + (mu - srf) * lj.h + pos_part(dmu * Hji);
+    // the momenta of both right-hand sides and the mass row of smb_2
+    double uj[S];
+    uj[0] = lj.h; uj[1] = lj.q1; uj[2] = lj.q2;
+    if (S == 5) { uj[3] = u.q3[j]; uj[4] = u.q4[j]; }
+    const bool flat = bits64(qij) == 0x3ff0000000000000ll && bits64(qji) == 0x3ff0000000000000ll;
+    const bool wet = wet_i && wet_j;
+    const double tp = ghi * (etaj - ui[0] - zi);
+    const double tx = tp * cxe, ty = tp * cye;
+    const double pij = 1.0 - qij, pji = 1.0 - qji;
+#pragma unroll
+    for (int q = 0; q < S; q++) {
+      double x2 = cxe * nd.flux[(int64_t)(2 * q) * nr + j];
+      if (S == 3) x2 = x2 + cye * nd.flux[(int64_t)(2 * q + 1) * nr + j];
+      double A, B = 0.0, mB = 0.0;
+      if (flat) {
+        A = uj[q] - ui[q];
+      } else {
+        A = uj[q] * qji - ui[q] * qij;
+        B = uj[q] * pji - ui[q] * pij;
+        mB = mu * B;
+      }
+      const double dA = d * A;
+      ab[(int64_t)(2 * q) * n_entries + e] = A;
+      ab[(int64_t)(2 * q + 1) * n_entries + e] = B;
+      rk2[q] = rk2[q] - x2 + dA;
+      if (!flat) rk2[q] = rk2[q] + mB;
+      if (q > 0) {
+        rk[q] = rk[q] - x2;
+        if (wet) {
+          rk[q] = rk[q] + dA;
+          if (!flat) rk[q] = rk[q] + mB;
+        } else {                                // rats are 0 where h <= htiny
+          const double ti = wet_i ? qij : 0.0, tj = wet_j ? qji : 0.0;
+          rk[q] = rk[q] + d * (uj[q] * tj - ui[q] * ti) + mu * (uj[q] * (1.0 - tj) - ui[q] * (1.0 - ti));
+        }
+      }
+      if (q == 1) { rk[1] = rk[1] - tx; rk2[1] = rk2[1] - tx; }
+      if (q == 2) { rk[2] = rk[2] - ty; rk2[2] = rk2[2] - ty; }
+    }
+  }
+  if (want_diag) {   // the diagonals of the viscosities (update.f90:315-323, 782-798), as k_low_f64 forms them
+    const double dii_raw = -sd, muii_raw = -sm;
+    double dii = tmax(dii_raw, muii_raw), muii = muii_raw;
+    if (c.alpha_limit) {
+      sd = sm = 0.0;
+      for (int kk = 0; kk <= L; kk++) {
+        if (kk == dp) { sm = sm + muii; continue; }
+        const int64_t e = base + 32 * (kk - (kk > dp ? 1 : 0));
+        sd = sd + dL[e];
+        sm = sm + muL[e];
+      }
+      dii = -sd;
+      muii = -sm;
+    }
+    dLii[r] = dii;
+    muLii[r] = muii;
+  }
+  const double m = G.lumped[r], im = G.inv_lumped[r], dt = St[b].dt;
+  const double v1i = w1i, v2i = nd.v2[r];
+  // source terms (:425-551), the same for both right-hand sides
+  if (S == 5) {      // mSGN_RHS subtracts pTilde_j c_ij after the loops, entry by entry
+    double p_i, s_i;
+    sgn_node_f64(c, m, ui[0], ui[3], &p_i, &s_i);
+    const double pdx = p_i * G.cxii[r], pdy = p_i * G.cyii[r];
+    for (int k = 0; k <= L; k++) {
+      if (k == dp) { rk[1] = rk[1] - pdx; rk[2] = rk[2] - pdy; rk2[1] = rk2[1] - pdx; rk2[2] = rk2[2] - pdy; }
+      if (k == L) break;
+      const int64_t e = base + 32 * k;
+      const double pj = nd.pt[G.col[e]];
+      const double px = pj * G.cx[e], py = pj * G.cy[e];
+      rk[1] = rk[1] - px; rk[2] = rk[2] - py;
+      rk2[1] = rk2[1] - px; rk2[2] = rk2[2] - py;
+    }
+    const double a3 = m * ui[S - 1], a4 = m * s_i;
+    rk[S - 2] = rk[S - 2] + a3; rk2[S - 2] = rk2[S - 2] + a3;
+    rk[S - 1] = rk[S - 1] - a4; rk2[S - 1] = rk2[S - 1] - a4;
+  } else if (c.type_test == 9 || c.type_test == 10) {
+    const double fric = c.g * c.mannings * c.mannings;
+    const double hstar = pow_43(max_any(ui[0], htiny));
+    const double vel = fric * sqrt(v1i * v1i + v2i * v2i);
+    const double den = hstar + max_nn(hstar, vel * dt), y = 1.0 / den;
+#pragma unroll
+    for (int q = 1; q < 3; q++) {
+      const double x = div_known(m * ui[q] * vel * 2.0, den, y);
+      rk[q] = rk[q] - x;
+      rk2[q] = rk2[q] - x;
+    }
+  } else if (c.type_test == 11) {
+    const double kappa = 0.2;
+#pragma unroll
+    for (int q = 1; q < 3; q++) {
+      const double x = m * kappa * ui[q];
+      rk[q] = rk[q] - x;
+      rk2[q] = rk2[q] - x;
+    }
+  } else if (c.type_test == 12) {
+    const double f = 2.0, x1 = m * f * ui[2], x2 = m * f * ui[1];
+    rk[1] = rk[1] + x1; rk2[1] = rk2[1] + x1;
+    rk[2] = rk[2] - x2; rk2[2] = rk2[2] - x2;
+  }
+  // divide_by_lumped (:801-808) and the low-order state (:202-215)
+  double ul[S];
+  ul[0] = ui[0] * (1.0 + div_known(dt * fix, m, im)) + dt * div_known(rk[0], m, im);
+#pragma unroll
+  for (int q = 1; q < S; q++) ul[q] = ui[q] + dt * div_known(rk[q], m, im);
+  uL.h[r] = ul[0]; uL.q1[r] = ul[1]; uL.q2[r] = ul[2];
+  if (S == 5) { uL.q3[r] = ul[3]; uL.q4[r] = ul[4]; }
+  if (bad) atomicOr(err, ERRB_DELTA);
+  // entropy residual (update.f90:838-868); Entprime(4:5) are 0
+  double rm[3], un_[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    rm[q] = div_known(rk2[q], m, im);
+    un_[q] = ui[q] + dt * rm[q];
+  }
+  const double on = one_over_h(un_[0], htiny);
+  const double vn1 = un_[1] * on, vn2 = un_[2] * on;
+  double En = g * (un_[0] * un_[0]);
+  En = En + vn1 * un_[1];
+  En = En + vn2 * un_[2];
+  En = 0.5 * En;
+  const double E = nd.ent[r];
+  const double Ep0 = ghi - 0.5 * (v1i * v1i) - 0.5 * (v2i * v2i);
+  double rsd = div_known(m * (En - E), dt, St[b].inv_dt);
+  rsd = rsd - m * rm[0] * Ep0;
+  rsd = rsd - m * rm[1] * v1i;
+  rsd = rsd - m * rm[2] * v2i;
+  const double rescale = __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor);   // the product is exact
+  res[r] = fabs(rsd) / rescale;
+}
+
+// f_ij and R^-_i from the stored differences: five FP64 instructions per
+// entry (the general k_fct_f64 forms the rats again: 42).
+__global__ void k_fct_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
+                          const double* __restrict__ dL, const double* __restrict__ muL, const double* __restrict__ hL,
+                          const double* __restrict__ res, const double* __restrict__ ab, double* __restrict__ fct,
+                          double* __restrict__ rminus, int64_t n_entries, unsigned* __restrict__ err) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= G.n_rows) return;
+  const int L = G.len[r];
+  if (L == 0) return;
+  const int b = G.slice_inst[r >> 5];
+  if (St[b].done) return;
+  const int64_t base = entry_base(G, r);
+  const double resi = res[r];
+  double P = -1.e-15;
+#pragma unroll 2
+  for (int k = 0; k < L; k++) {
+    const int64_t e = base + 32 * k;
+    const double rij = max_nn(resi, res[G.col[e]]);
+    const double d0 = dL[e], m0 = muL[e];
+    const double f = (min_nn(d0, rij) - d0) * ab[e] + (min_nn(m0, rij) - m0) * ab[n_entries + e];
+    fct[e] = f;
+    if (bits64(f) < 0) P = P + f;                 // -0 adds nothing
+  }
+  const double h = hL[r];
+  if (h < 0.0) atomicOr(err, ERRB_NEG_H);
+  const double scaled = div_known(G.lumped[r], St[b].dt, St[b].inv_dt) * h;
+  const double Q = 0.0 - scaled;
+  double R = tmin(Q / P, 1.0);
+  if (scaled <= C[b].htiny) R = 0.0;
+  rminus[r] = R;
+}
+
+// l_ij, the limited antidiffusion from the stored differences, and the end of
+// the stage (see k_update_f64 for rk_stage).
+template <int S>
+__global__ void k_update_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
+                             const double* __restrict__ dL, const double* __restrict__ muL, StateF64 uL,
+                             const double* __restrict__ res, const double* __restrict__ fct,
+                             const double* __restrict__ rminus, const double* __restrict__ ab, StateF64 u0,
+                             StateF64 out, int rk_stage, double* __restrict__ lij_out, int64_t n_entries,
+                             unsigned* __restrict__ err) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= G.n_rows) return;
+  const int L = G.len[r];
+  if (L == 0) return;
+  const int b = G.slice_inst[r >> 5];
+  const InstState& st = St[b];
+  if (st.done) return;
+  const InstConst& c = C[b];
+  const int64_t base = entry_base(G, r);
+  const double resi = res[r], Ri = rminus[r];
+  double xx[S];
+#pragma unroll
+  for (int q = 0; q < S; q++) xx[q] = 0.0;
+  for (int k = 0; k < L; k++) {
+    const int64_t e = base + 32 * k;
+    const int j = G.col[e];
+    const double l = (bits64(fct[e]) << 1) == 0 || bits64(fct[e]) > 0 ? rminus[j] : Ri;   // f >= 0
+    if (lij_out) lij_out[e] = l;
+    const double rij = max_nn(resi, res[j]);
+    const double d0 = dL[e], m0 = muL[e];
+    const double dd = (min_nn(d0, rij) - d0) * l;
+    const double dm = (min_nn(m0, rij) - m0) * l;
+#pragma unroll
+    for (int q = 0; q < S; q++)
+      xx[q] = xx[q] + dd * ab[(int64_t)(2 * q) * n_entries + e] + dm * ab[(int64_t)(2 * q + 1) * n_entries + e];
+  }
+  const double m = G.lumped[r], im = G.inv_lumped[r], dt = st.dt;
+  double un[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+  for (int q = 0; q < S; q++) un[q] = comp_f64(uL, q, r) + dt * div_known(xx[q], m, im);
   finish_row_f64(G, c, st, r, S, un, true, rk_stage, u0, out, err);
 }
 
@@ -801,17 +1138,39 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
   EV_BEGIN(1);
   if (!a.skip_node) k_node_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, nd);
   EV_END(1); EV_BEGIN(2);
-  k_low_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii,
-                                                a.w.uL, a.w.res, a.dij_in, a.err);
+  const unsigned nb = nblk(a.G.n_rows, bs);
+  if (a.fused) {
+    const int64_t ne = a.w.n_entries;
+    const int diag = a.rk_stage == 0;            // swe_euler_intermediates hands out the diagonals
+    if (a.S == 5)
+      k_low_fct<5><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
+                                     a.w.ab, a.dij_in, diag, ne, a.err);
+    else
+      k_low_fct<3><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
+                                     a.w.ab, a.dij_in, diag, ne, a.err);
+    EV_END(2); EV_BEGIN(3);
+    k_fct_fct<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
+                                a.err);
+    EV_END(3); EV_BEGIN(4);
+    if (a.S == 5)
+      k_update_fct<5><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
+                                        a.u0, a.out, a.rk_stage, a.lij_out, ne, a.err);
+    else
+      k_update_fct<3><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
+                                        a.u0, a.out, a.rk_stage, a.lij_out, ne, a.err);
+    EV_END(4);
+    return;
+  }
+  k_low_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res, a.dij_in,
+                              a.err);
   EV_END(2); EV_BEGIN(3);
-  k_fct_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct,
-                                                a.w.rminus, a.err);
+  k_fct_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.err);
   EV_END(3); EV_BEGIN(4);
-  k_update_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct,
-                                                   a.w.rminus, a.u0, a.out, a.rk_stage, a.lij_out, a.err);
+  k_update_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.u0, a.out,
+                                 a.rk_stage, a.lij_out, a.err);
   if (a.entropy)
-    k_entropy_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii,
-                                                      a.w.res, a.u0, a.out, a.rk_stage, a.err);
+    k_entropy_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.res, a.u0, a.out,
+                                    a.rk_stage, a.err);
   EV_END(4);
 }
 

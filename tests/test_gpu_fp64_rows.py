@@ -5,6 +5,8 @@ about htiny, two dry nodes, equal and nearly equal depths, depth ratios about
 far outside the ordinary range.  No tolerance: the kernels form the oracle's
 own roundings."""
 
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
@@ -82,3 +84,79 @@ def test_dij_bit_exact(kind, n):
         if ref is not None:
             np.testing.assert_array_equal(got[0], ref[0])
             assert got[1] == ref[1]
+
+
+DUMPS = ("dij_low", "muij_low", "alpha", "u_low", "res", "fctmat", "rminus", "lij")
+
+
+@pytest.mark.parametrize("type_test,alpha,bumpy", [(4, 1, 0), (4, 1, 1), (4, 0, 1), (11, 1, 1), (12, 1, 0)])
+@pytest.mark.parametrize("kind", STATES)
+def test_fct_stage_bit_exact(kind, type_test, alpha, bumpy):
+    """One 'fct' stage and its intermediates, over a flat and an uneven
+    bottom, with and without alpha_limit, with the linear source terms."""
+    n = 17
+    rng = np.random.default_rng(100 + STATES.index(kind))
+    mesh = M.jittered_mesh(n, n + 4, 0.0, 1.0, 0.0, 1.0, jitter=0.3, seed=5)
+    nn = mesh["rr"].shape[1]
+    z = bumpy * rng.uniform(-0.4, 0.4, nn) * (rng.random(nn) < 0.7)
+    p = C.Params(max_water_h=1.0, htiny=1e-4, type_test=type_test, if_alpha_limit=alpha)
+    o, upd = _pair(mesh, z, p)
+    for _ in range(3):
+        u = _state(kind, nn, p.htiny, rng)
+        try:
+            dt = o.compute_dij(u)[1]
+        except oracle.OracleError:
+            continue
+        pd = replace(p, dt=dt)
+        o.set_params(oracle.Params(*pd.fields()))
+        upd.set_params(pd)
+        ref, got = _both(lambda: o.euler(u, dump=True), lambda: upd.euler(u),
+                         (L.SWE_ERR_NEG_H, L.SWE_ERR_DELTA, L.SWE_ERR_NAN))
+        if ref is None:
+            continue
+        inter = upd.euler_intermediates()
+        for k in DUMPS:
+            np.testing.assert_array_equal(inter[k], ref[1][k], err_msg=k)
+        np.testing.assert_array_equal(got, ref[0])
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (33, 3), (65, 64)])
+@pytest.mark.parametrize("sgn", [0, 1])
+def test_fct_steps_bit_exact(sgn, nx, ny):
+    """RK3 steps of both system sizes at row counts about a warp, a block and
+    several, against the oracle."""
+    if sgn:
+        case = C.sgn_case(nx=max(nx, 3), ny=ny, Lx=0.01 * nx, Ly=0.01 * ny, x0=0.005 * nx, cfl=5e-4)
+    else:
+        mesh = M.jittered_mesh(nx, ny, 0.0, 10.0, 0.0, 10.0, jitter=0.3, seed=2)
+        case = C.bump_basin_case(mesh=mesh)
+        case = replace(case, params=replace(case.params, type_test=4))
+    o, upd = _pair(case.mesh, case.bath, case.params)
+    for comp, js, vals in case.dirichlet:
+        o.set_dirichlet(comp, js, vals)
+        upd.set_dirichlet(comp, js, vals)
+    u, t = case.u0.copy(order="F"), 0.0
+    for _ in range(9):
+        t = o.rk3_step(u, t)
+    upd.upload(case.u0)
+    upd.set_time(0.0, 1e30)
+    upd.rk3_steps(9)
+    np.testing.assert_array_equal(upd.download(), u)
+    assert upd.get_time()[0][0] == t
+
+
+def test_mode_changes_between_calls():
+    """A captured run follows a later change of the viscosity mode."""
+    case = C.dam_break_case(n=21, tfinal=1.0)
+    o, upd = _pair(case.mesh, case.bath, case.params)
+    u, t = case.u0.copy(order="F"), 0.0
+    upd.upload(case.u0)
+    upd.set_time(0.0, 1e30)
+    for visc in ("fct", "viscous", "entropy_visc", "fct"):
+        p = replace(case.params, viscosity_type=C.VISC[visc])
+        o.set_params(oracle.Params(*p.fields()))
+        upd.set_params(p)
+        for _ in range(3):
+            t = o.rk3_step(u, t)
+        upd.rk3_steps(3)
+        np.testing.assert_array_equal(upd.download(), u)
