@@ -331,29 +331,44 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ float one_over_h_f(float h, float htiny) {
+  const float m = fmaxf(h, htiny);
+  return __fdividef(2.f * h, h * h + m * m);
+}
+
 // compute_lambda_vacc (SOURCES/condlim.f90:879-957) with the same bits and
 // about a third of the FP64 instructions (the bound of k_dt_f64 and
-// k_low_f64).  With c = sqrt(g h):
+// k_low_fct).  With c = sqrt(g h):
+//  * a node with h = 0 makes ht = 0 in every branch and has v = c = 0 itself:
+//    lambda is the other node's |v -+ c|.
 //  * phi(x0 hmin) >= 0, the two-rarefaction branch, is certain when
-//    x0 hmin > hmax and vl - vr <= 1.888 c_min: then both terms of phi are
-//    shocks and the one of hmin alone is (x0 - 1) sqrt((1 + 1/x0) / 2) c_min =
-//    1.8884 c_min.  phi's square roots and division are not formed.
+//    x0 hmin > hmax (both terms of phi are shocks, so >= 0) and vl - vr is at
+//    most the term of hmin alone: (x0 - 1) sqrt((1 + 1/x0) / 2) c_min =
+//    1.8884 c_min for hmin >= htiny, at least (x0 - 1) / sqrt(2 x0) c_min =
+//    0.9061 c_min where only x0 hmin >= htiny.  phi's square roots and
+//    division are not formed.
 //  * sqrt((1 + max(x/2, 0)) (1 + max(x, 0))) is 1 exactly where ht <= h.
 //  * only the larger of |lambda_l| and |lambda_r| is formed where FP32 tells
 //    them apart.
-// FP32 bounds: with M = sum |v| + 2 (c_l + c_r) the FP32 velocities, c and s
-// are within 8 roundings (5e-7 M) and the two speeds within 2e-6 M; the tests
-// use 2e-6 M and 1e-5 M.  What is not certain is evaluated in full.
+// FP32 bounds: with V = sum |v| and M = V + 2 (c_l + c_r) the FP32 velocities
+// are within 5e-7 V, c and s within 5e-7 M and the two speeds within 2e-6 M;
+// the tests use 2e-6 V, 2e-6 M and 1e-5 M.  What is not certain is evaluated
+// in full.
 __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r, double nx, double ny, float2 nf,
                                            const InstConst& c, double* lambda) {
   const float lv = nf.x * l.f.z + nf.y * l.f.w, rv = nf.x * r.f.z + nf.y * r.f.w;
-  const float M = fabsf(l.f.z) + fabsf(l.f.w) + fabsf(r.f.z) + fabsf(r.f.w) + 2.f * (l.f.y + r.f.y);
+  const float V = fabsf(l.f.z) + fabsf(l.f.w) + fabsf(r.f.z) + fabsf(r.f.w);
+  const float M = V + 2.f * (l.f.y + r.f.y);
   const float tol = 2e-6f * M;
   const float hmin = fminf(l.f.x, r.f.x), hmax = fmaxf(l.f.x, r.f.x);
-  if (!(hmin > 1.00001f * c.htinyf && 3.3431f * hmin > hmax && (lv - rv) + tol <= 1.888f * fminf(l.f.y, r.f.y) &&
-        hmin > 1e-30f && hmax < 1e30f)) {
-    if (((bits64(l.h) | bits64(r.h)) << 1) == 0 && bits64(c.htiny) > 0) {   // two dry nodes: v = 0, c = 0
-      *lambda = 0.0;
+  const float kmin = hmin > 1.00001f * c.htinyf ? 1.888f : (3.3431f * hmin > 1.00001f * c.htinyf ? 0.906f : 0.f);
+  if (!(3.3431f * hmin > hmax && (lv - rv) + 2e-6f * V <= kmin * fminf(l.f.y, r.f.y) && hmin > 1e-18f &&
+        hmax < 1e18f)) {
+    const bool dry_l = (bits64(l.h) << 1) == 0, dry_r = (bits64(r.h) << 1) == 0;
+    if ((dry_l || dry_r) && bits64(l.h) >= 0 && bits64(r.h) >= 0 && bits64(c.htiny) > 0 && V < 1e30f) {
+      const double qx = dry_l ? r.q1 : l.q1, qy = dry_l ? r.q2 : l.q2, o = dry_l ? r.ovh : l.ovh;
+      const double v = __dmul_rn(__dadd_rn(__dmul_rn(qx, nx), __dmul_rn(qy, ny)), o);
+      *lambda = fabs(dry_l ? __dadd_rn(v, r.sq) : __dsub_rn(v, l.sq));
       return true;
     }
     bool ok;
@@ -365,7 +380,8 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
   const float su = fmaxf(s + tol, 0.f), sm = fmaxf(s, 0.f);
   const float hup = su * su * i16g * 1.000002f, hst = sm * sm * i16g;   // ht <= hup
   const bool triv_l = hup <= l.f.x * 0.999998f, triv_r = hup <= r.f.x * 0.999998f;
-  const float xl = fmaxf(__fdividef(hst - l.f.x, l.f.x), 0.f), xr = fmaxf(__fdividef(hst - r.f.x, r.f.x), 0.f);
+  const float xl = fmaxf((hst - l.f.x) * one_over_h_f(l.f.x, c.htinyf), 0.f);
+  const float xr = fmaxf((hst - r.f.x) * one_over_h_f(r.f.x, c.htinyf), 0.f);
   const float al = fabsf(lv - l.f.y * sqrt_approx((1.f + 0.5f * xl) * (1.f + xl)));
   const float ar = fabsf(rv + r.f.y * sqrt_approx((1.f + 0.5f * xr) * (1.f + xr)));
   const float tl = 1e-5f * M;
