@@ -78,6 +78,7 @@ struct swe_ctx {
   WorkMix wm{};
   TileCtl tiles{};                       // row tiles of the shared-memory variants
   bool tiles_ok = false;
+  bool tiles_named = false;              // a tuning description may name tile variants (without tiles they run as the others)
   double* d_mass_acc = nullptr;
   double* d_mass_part = nullptr;         // per-slice partial sums of swe_mass
   int64_t* d_inst_slice = nullptr;       // n_inst + 1 slice offsets
@@ -202,6 +203,12 @@ static bool all_fct(const swe_ctx* c) {
   for (const swe_params& p : c->params)
     if (p.viscosity_type != SWE_VISC_FCT || !p.if_roundoff_fix) return false;
   return true;
+}
+
+static bool all_fct_limited(const swe_ctx* c) {
+  for (const swe_params& p : c->params)
+    if (!p.if_alpha_limit) return false;
+  return all_fct(c);
 }
 
 static int check_params(swe_ctx* c, const swe_params& p) {
@@ -376,19 +383,34 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     }
     w.qL = c->buf.alloc<float2>(n, st);
     if (c->S == 5) { w.q3L = c->buf.alloc<float>(n, st); w.q4L = c->buf.alloc<float>(n, st); }
-    // row tiles of the shared-memory kernel variants (SWE_TILE rows, default
-    // 256; 0 disables), while the tile and its halo fit in 48 KB
+    // row tiles of the shared-memory kernel variants (SWE_TILE rows: 64,
+    // 128 or the default 256; 0 disables), while the tile, its halo and its entries leave room for
+    // two blocks per SM
     const char* ft = getenv("SWE_TILE");
-    const int tile = ft ? atoi(ft) : 256;
+    const int want = ft ? atoi(ft) : 256;
+    const int tile = want >= 256 ? 256 : want >= 128 ? 128 : want >= 64 ? 64 : 0;   // the sizes that are built
     RowTiles F;
     TileCtl probe{};
-    if (c->S == 3 && tile > 0 && build_row_tiles(L, tile, F) &&
-        (probe.tile_rows = F.tile, probe.halo_cap = F.halo_cap, tile_smem_bytes(probe, true) <= 48 * 1024)) {
+    if (c->S == 3 && tile > 0 && build_row_tiles(L, tile, F)) {
+      probe.tile_rows = F.tile;
+      probe.halo_cap = (F.halo_cap + 3) / 4 * 4;
+      probe.ent_cap = F.ent_cap;
+      c->tiles_named = 32 * (F.tile + F.halo_cap) + F.tile / 4 + F.tile <= 48 * 1024;
+    }
+    if (c->tiles_named && tile_smem_max(probe, is_split(c)) <= (size_t)kTileSmemMax) {
+      c->tiles = probe;
       c->tiles.loc = upload_vec(c, F.loc, st);
-      c->tiles.halo_ptr = upload_vec(c, F.halo_ptr, st);
-      c->tiles.halo_rows = upload_vec(c, F.halo_rows, st);
-      c->tiles.tile_rows = F.tile;
-      c->tiles.halo_cap = F.halo_cap;
+      std::vector<int4> head(F.halo_ptr.size() - 1);
+      std::vector<int> halo(head.size() * (size_t)probe.halo_cap, -1);
+      for (size_t t = 0; t < head.size(); t++) {
+        const int64_t r0 = (int64_t)t * F.tile, r1 = std::min<int64_t>(r0 + F.tile, L.n_rows);
+        const int64_t e0 = L.slice_ptr[r0 >> 5], ne = L.slice_ptr[(r1 + 31) >> 5] - e0;
+        head[t] = make_int4((int)(uint32_t)e0, (int)(uint32_t)((uint64_t)e0 >> 32), (int)ne, 0);
+        std::copy(F.halo_rows.begin() + F.halo_ptr[t], F.halo_rows.begin() + F.halo_ptr[t + 1],
+                  halo.begin() + t * (size_t)probe.halo_cap);
+      }
+      c->tiles.head = upload_vec(c, head, st);
+      c->tiles.halo_rows = upload_vec(c, halo, st);
       c->tiles_ok = true;
     }
   }
@@ -675,6 +697,7 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
       a.tiles = c->tiles_ok ? &c->tiles : nullptr;
       a.f64 = is_split(c);
       a.type1 = has_type1(c);
+      a.fct = all_fct_limited(c);
       if (stage == 2) { a.u = c->mB; a.out = c->mC; }
       if (stage == 3) { a.u = c->mC; a.out = c->mA; }
       launch_stage_mix(a, s, kev, c->tune);
@@ -818,7 +841,7 @@ SWE_API int swe_set_params(swe_ctx* c, int inst, const swe_params* p) {
     return fail(c, SWE_ERR_ARG, "syst_size and precision are fixed at creation");
   const swe_params& was = c->params[inst];
   if (was.viscosity_type != p->viscosity_type || was.viscous_type != p->viscous_type ||
-      was.if_roundoff_fix != p->if_roundoff_fix)
+      was.if_roundoff_fix != p->if_roundoff_fix || was.if_alpha_limit != p->if_alpha_limit)
     drop_graphs(c);                                  // the captured kernels follow the modes
   c->params[inst] = *p;
   InstConst k = make_const(*p);
@@ -1025,6 +1048,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
     a.tiles = c->tiles_ok ? &c->tiles : nullptr;
     a.f64 = is_split(c);
     a.type1 = has_type1(c);
+    a.fct = all_fct_limited(c);
     launch_stage_mix(a, c->stream, nullptr, c->tune);
   }
   CK(cudaGetLastError());
@@ -1250,10 +1274,6 @@ SWE_API int swe_set_time(swe_ctx* c, const double* time, const double* t_final) 
   return restore_done(c, hs);
 }
 
-// Autotuner of the mixed kernels: for every kernel kind, time each (block
-// size, entry batch) variant on the current state and keep the fastest.  The
-// variants agree to FP32 rounding, and every timed kernel is idempotent on its
-// inputs (it only rewrites its own outputs), so the state is unchanged.
 // Launch configuration from the autotuner's own description ("dt:block256/
 // batch4/resident node:... low:block128/batch2/regs64/tiled ..."), so that a
 // profiling run can reproduce the variants a timed run chose.  Kinds not
@@ -1305,7 +1325,7 @@ static bool parse_tuning(const char* spec, bool tiles, KernelTune& t) {
 // A fixed launch configuration (the autotuner's description) instead of timing
 static int apply_tuning(swe_ctx* c, const char* spec, const char* what) {
   KernelTune t;
-  if (!parse_tuning(spec, c->tiles_ok, t)) return fail(c, SWE_ERR_ARG, std::string("bad ") + what + ": " + spec);
+  if (!parse_tuning(spec, c->tiles_named, t)) return fail(c, SWE_ERR_ARG, std::string("bad ") + what + ": " + spec);
   c->tune = t;
   c->tuned = true;
   c->tuning = std::string("thread-per-row SELL-32; fixed ") + spec;
@@ -1313,10 +1333,37 @@ static int apply_tuning(swe_ctx* c, const char* spec, const char* what) {
   return SWE_OK;
 }
 
+// Launch configuration of the mixed kernels: the tile variants where the mesh
+// has tiles; else (5-component systems, tiles too large for shared memory)
+// every (block size, entry batch, grid) variant of each kernel is timed on the
+// current state and the fastest kept.  All variants give the same bits, and
+// every timed kernel is idempotent on its inputs (it only rewrites its own
+// outputs), so the state is unchanged.
 static int autotune(swe_ctx* c) {
   if (!is_mixed(c)) { c->tuned = true; return SWE_OK; }
   if (const char* spec = getenv("SWE_TUNE")) return apply_tuning(c, spec, "SWE_TUNE");
   int rc;
+  const char* tenv = getenv("SWE_TILED");   // 0 leaves the tile variants out
+  // A mesh with row tiles runs them, without timing: per RK3 step they take
+  // 44 / 46 / 72 / 105 / 1470 us at 2k / 20k / 100k / 200k / 4M nodes, the best
+  // of the global-gather variants 60 / 68 / 87 / 128 / 1780 us.  k_low runs four
+  // resident blocks per SM (64 registers, a few spilled) where an SM has more
+  // than three tiles, else three.
+  if (c->tiles_ok && !(tenv && tenv[0] == '0')) {
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
+    const int64_t n_tiles = (c->G.n_rows + c->tiles.tile_rows - 1) / c->tiles.tile_rows;
+    KernelTune t;
+    t.cap_low = n_tiles > 3 * (int64_t)sms;
+    for (int k = 0; k < 5; k++) { t.block[k] = 256; t.tiled[k] = 1; }
+    c->tune = t;
+    c->tuned = true;
+    c->tuning = std::string("thread-per-row SELL-32; autotuned dt:block256/batch1/tiled node:block256/batch1/tiled "
+                            "low:block256/batch1/") + (t.cap_low ? "regs64" : "regs85") +
+                "/tiled fct:block256/batch1/tiled update:block256/batch1/tiled";
+    drop_graphs(c);
+    return SWE_OK;
+  }
   std::vector<InstState> saved;
   if ((rc = save_state(c, saved))) return rc;
   std::vector<InstState> run = saved;
@@ -1324,11 +1371,11 @@ static int autotune(swe_ctx* c) {
   if ((rc = restore_done(c, run))) return rc;
   const cudaStream_t s = c->stream;
   StageArgsMix a{c->G, c->d_C, c->d_St, c->mA, c->mA, c->mB, c->wm, 1, c->d_err, c->block};
-  a.tiles = c->tiles_ok ? &c->tiles : nullptr;
   a.f64 = is_split(c);
   a.type1 = has_type1(c);
   KernelTune t = c->tune;
-  launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, t, a.tiles, s);   // populate every work array once
+  for (int& k : t.tiled) k = 0;
+  launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, t, nullptr, s);   // populate every work array once
   launch_stage_mix(a, s, nullptr, t);
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1341,29 +1388,23 @@ static int autotune(swe_ctx* c) {
   a_low.rk_stage = 2;
   std::string desc;
   const char* names[5] = {"dt", "node", "low", "fct", "update"};
-  // SWE_TILED=0 leaves the shared-memory variants out, SWE_TILED=1 takes them
-  const char* tenv = getenv("SWE_TILED");
   for (int kind = 0; kind < 5; kind++) {
     float best = 1e30f;
-    int bb = t.block[kind], bt = t.batch[kind], bc = t.cap_low, bg = t.grid[kind], btl = t.tiled[kind];
-    // grid modes: a thread per row, resident grid, shared-memory tiles
-    const bool tiles = a_low.tiles && kind_has_tiles(kind) && !(tenv && tenv[0] == '0');
-    const int gm0 = (tiles && tenv && tenv[0] == '1') ? 2 : 0, n_modes = tiles ? 3 : 2;
+    int bb = t.block[kind], bt = t.batch[kind], bc = t.cap_low, bg = t.grid[kind];
     for (int ib = 0; ib < 3; ib++)
       for (int it = 0; it < 4; it++)
         for (int cap = 0; cap < (kind == 2 ? 3 : 1); cap++)
-          for (int gm = gm0; gm < n_modes; gm++) {
+          for (int gm = 0; gm < 2; gm++) {   // a thread per row, resident grid
             if (kind == 2 && batches[it] > 2) continue;
             KernelTune v = t;
             v.block[kind] = blocks[ib];
             v.batch[kind] = batches[it];
             v.grid[kind] = gm == 1;
-            v.tiled[kind] = gm == 2;
             if (kind == 2) v.cap_low = cap;
             float tmin = 1e30f;
             for (int rep = 0; rep < 3; rep++) {
               cudaEventRecord(e0, s);
-              if (kind == 0) launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, v, a.tiles, s);
+              if (kind == 0) launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, v, nullptr, s);
               else launch_kernel_mix(kind, a_low, v, s);
               cudaEventRecord(e1, s);
               CK(cudaEventSynchronize(e1));
@@ -1372,19 +1413,17 @@ static int autotune(swe_ctx* c) {
               tmin = std::min(tmin, ms);
             }
             if (tmin < best) {
-              best = tmin; bb = blocks[ib]; bt = batches[it]; bg = gm == 1; btl = gm == 2;
+              best = tmin; bb = blocks[ib]; bt = batches[it]; bg = gm == 1;
               if (kind == 2) bc = cap;
             }
           }
     t.block[kind] = bb;
     t.batch[kind] = bt;
     t.grid[kind] = bg;
-    t.tiled[kind] = btl;
     if (kind == 2) t.cap_low = bc;
     char buf[96];
     snprintf(buf, sizeof buf, "%s%s:block%d/batch%d%s%s", kind ? " " : "", names[kind], bb, bt,
-             kind == 2 ? (bc == 2 ? "/regs51" : bc ? "/regs64" : "/regs85") : "",
-             bg ? "/resident" : (btl ? "/tiled" : ""));
+             kind == 2 ? (bc == 2 ? "/regs51" : bc ? "/regs64" : "/regs85") : "", bg ? "/resident" : "");
     desc += buf;
   }
   cudaEventDestroy(e0);

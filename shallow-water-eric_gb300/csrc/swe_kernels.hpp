@@ -75,12 +75,15 @@ struct StageArgs {
 // order) and first copies the node records of its rows and of its halo (the
 // rows outside the tile that its entries reference) into shared memory; the
 // entry loops then read neighbours there by tile-local position.
+// The tile's per-entry arrays (one contiguous range: its slices are
+// consecutive) are copied there too.
 struct TileCtl {
   const int16_t* loc;     // per entry: col - tile start, or tile_rows + halo index
-  const int* halo_ptr;    // n_tiles + 1
-  const int* halo_rows;   // ascending per tile
-  int tile_rows;
-  int halo_cap;           // largest halo
+  const int4* head;       // per tile: first entry (64 bits), number of entries
+  const int* halo_rows;   // halo_cap per tile, ascending, then -1
+  int tile_rows;          // 64, 128 or 256
+  int halo_cap;           // largest halo, rounded up to a multiple of 4
+  int ent_cap;            // most entries of a tile (a multiple of 32)
 };
 
 struct StageArgsMix {
@@ -95,6 +98,7 @@ struct StageArgsMix {
   const TileCtl* tiles = nullptr;  // row tiles of the shared-memory variants, or null
   bool f64 = false;                 // precision split: h^L, R^- and the depth's limited sum in FP64
   bool type1 = false;               // some instance runs 'viscous' with viscous_type 'type1'
+  bool fct = false;                 // every instance runs 'fct' with the roundoff fix and alpha_limit
 };
 
 // Optional per-kernel event timing: when non-null, ev[2k], ev[2k+1] bracket
@@ -135,8 +139,12 @@ struct KernelTune {
 };
 
 void launch_stage_mix(const StageArgsMix& a, cudaStream_t s, const KernelEvents* kev, const KernelTune& t);
-// dynamic shared memory of one tile block (d: with the FP64 R^- of the precision split)
-size_t tile_smem_bytes(const TileCtl& tc, bool d = false);
+// most dynamic shared memory of a tile block: two blocks per SM
+constexpr int kTileSmemMax = 100 * 1024;
+// dynamic shared memory of one tile block of a kernel kind (d: with the FP64
+// R^- of the precision split; lamin: k_low with k_dt's |c_ij| lambda)
+size_t tile_smem_bytes(const TileCtl& tc, int kind, bool d, bool lamin);
+size_t tile_smem_max(const TileCtl& tc, bool d);   // over the kernel kinds
 void launch_kernel_mix(int kind, const StageArgsMix& a, const KernelTune& t, cudaStream_t s);
 bool kind_has_tiles(int kind);   // kernel kinds with a shared-memory tile variant
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,

@@ -104,9 +104,9 @@ __device__ __forceinline__ Recon recon(float hi, float hj, float dz) {
   return R;
 }
 // rat_ij = H*_ij / h_i with the reference's h <= 0 test (0 there); 1 exactly
-// downhill and never above 1.
-__device__ __forceinline__ float rat_of(float H, float h, bool flat, float invh) {
-  return (h > 0.f) ? (flat ? 1.f : fminf(__fmul_rn(H, invh), 1.f)) : 0.f;
+// downhill and never above 1.  inv = 1/h and one = 1 where h > 0, else 0.
+__device__ __forceinline__ float rat_of(float H, bool flat, float inv, float one) {
+  return flat ? one : fminf(__fmul_rn(H, inv), 1.f);
 }
 __device__ __forceinline__ float inv_pos(float h) { return (h > 0.f) ? fdiv(1.0f, h) : 0.f; }
 // z_j - z_i from the node records: (eta_j - eta_i) + (h_i - h_j)
@@ -153,19 +153,33 @@ __device__ __forceinline__ float phi_f(float h, float vl, float hl, float vr, fl
 // ovh*: one_over_h of the states; sq*: sqrt(g |h|).  Returns false where the
 // reference STOPs (Delta < 0), with a relative band of 1e-5 h_min for FP32
 // rounding.
+//
+// phi(x0 hmin) only selects the branch, and its sign is mostly certain without
+// it: with x0 hmin > hmax both terms of phi are shocks, so not negative, and
+// for hmin > htiny the one of hmin alone is (x0 - 1) sqrt((1 + 1/x0) / 2)
+// sqrt(g hmin) = 1.888 sqrt(g hmin); 1.85 and 1e-6 (|vl| + |vr|) leave room for
+// the roundings of phi.  hmin = 0 gives ht = 0 in every branch.  The skipped
+// evaluation is 3 square roots, a division and about 20 other instructions of
+// 75 (k_low and k_dt are bound by instruction issue).
 __device__ __forceinline__ bool lambda_f(float hl, float hr, float vl, float vr, float ovhl, float ovhr, float sql,
                                          float sqr, const LamK& k, float* lambda) {
   const float x0 = 3.34314575f;   // (2 sqrt(2) - 1)^2
-  const bool lmin = hl <= hr;
-  const float hmin = lmin ? hl : hr, hmax = lmin ? hr : hl;
+  const float hmin = fminf(hl, hr), hmax = fmaxf(hl, hr);
+  const float hx = x0 * hmin, dv = vl - vr;
   bool ok = true;
   float ht;
-  float fh = phi_f(x0 * hmin, vl, hl, vr, hr, ovhl, ovhr, sql, sqr, k);
-  if (0.f <= fh) {
-    const float s = fmaxf(fma_(2.f, sqr, fma_(2.f, sql, vl - vr)), 0.f);
-    ht = fminf(x0 * hmin, fdiv(s * s, 16.f * k.g));
+  if (hx > hmax &&
+      fma_(1e-6f, fabsf(vl) + fabsf(vr), dv) <= (hmin > k.htiny ? 1.85f : 0.f) * fminf(sql, sqr)) {
+    const float s = fmaxf(fma_(2.f, sqr, fma_(2.f, sql, dv)), 0.f);
+    ht = fminf(hx, fdiv(s * s, 16.f * k.g));
+  } else if (hmin == 0.f) {
+    ht = 0.f;
+  } else if (0.f <= phi_f(hx, vl, hl, vr, hr, ovhl, ovhr, sql, sqr, k)) {
+    const float s = fmaxf(fma_(2.f, sqr, fma_(2.f, sql, dv)), 0.f);
+    ht = fminf(hx, fdiv(s * s, 16.f * k.g));
   } else {
-    fh = phi_f(x0 * hmax, vl, hl, vr, hr, ovhl, ovhr, sql, sqr, k);
+    const bool lmin = hl <= hr;
+    const float fh = phi_f(x0 * hmax, vl, hl, vr, hr, ovhl, ovhr, sql, sqr, k);
     const float sqrmin = (lmin ? sql : sqr) * k.rsg, sqrmax = (lmin ? sqr : sql) * k.rsg;
     if (0.f <= fh) {
       const float a = 0.353553391f;   // 1 / (2 sqrt(2))
@@ -200,108 +214,246 @@ __device__ __forceinline__ bool dlam_f(float cxe, float cye, float cvi, float cv
   return ok;
 }
 
-// Entry loops are processed in batches of B entries: every global load of a
-// batch is issued before any of them is used, so a thread keeps B loads in
-// flight (the kernels are latency-bound otherwise); the tile variants read
-// neighbours from shared memory at the point of use (no registers held for
-// them).  Sums keep the entry order, so every batch size gives the same
-// bits.  The autotuner picks B per kernel.
+// What the entry loops need of a node, in each kernel.
+struct NodeF {        // k_low (and its own row)
+  float h, q1, q2, eta, ovh, v1, v2;
+  float sq;           // sqrt(g |h|)
+  float inv, one;     // 1/h and 1 where h > 0, else 0
+  float E;            // entropy
+  float al;           // alpha
+};
+struct NodeL {        // k_dt
+  float h, v1, v2, sq, ovh;
+};
+struct NodeC {        // k_fct
+  float h, eta, res;
+};
+struct NodeU {        // k_update
+  float h, q1, q2, eta, res, R, inv, one;
+};
+
+// 0.5 (g h^2 + v1 q1 + v2 q2): the entropy of the reference's entropy_residual
+__device__ __forceinline__ float entropy_f(float g, float h, float v1, float q1, float v2, float q2) {
+  return 0.5f * fma_(v2, q2, fma_(v1, q1, (g * h) * h));
+}
+__device__ __forceinline__ NodeL node_l(float4 n, float g, float htiny) {
+  NodeL r;
+  r.h = n.x;
+  r.ovh = ovh_f(n.x, htiny);
+  r.v1 = n.y * r.ovh;
+  r.v2 = n.z * r.ovh;
+  r.sq = sqrtf(g * fabsf(n.x));
+  return r;
+}
+// sgn: flux() zeroes velocity(2) for type 13
+__device__ __forceinline__ NodeF node_f(float4 n, float al, float g, float htiny, bool sgn) {
+  const NodeL l = node_l(n, g, htiny);
+  NodeF r;
+  r.h = n.x; r.q1 = n.y; r.q2 = n.z; r.eta = n.w;
+  r.ovh = l.ovh; r.v1 = l.v1; r.v2 = l.v2; r.sq = l.sq;
+  r.inv = inv_pos(n.x);
+  r.one = n.x > 0.f ? 1.f : 0.f;
+  r.E = entropy_f(g, n.x, r.v1, n.y, sgn ? 0.f : r.v2, n.z);
+  r.al = al;
+  return r;
+}
+__device__ __forceinline__ NodeU node_u(float4 n, float res, float R) {
+  return NodeU{n.x, n.y, n.z, n.w, res, R, inv_pos(n.x), n.x > 0.f ? 1.f : 0.f};
+}
+
+// A row's place in the graph.
+struct RowHead {
+  int L, b;           // entries, instance
+  int64_t base;       // first entry
+};
+__device__ __forceinline__ RowHead row_head(const Graph& G, int64_t r) {
+  return RowHead{G.len[r], G.slice_inst[r >> 5], entry_base(G, r)};
+}
 
 // Neighbour access of the entry loops: straight from HBM by column index
 // (NbGlobal), or from the block's shared-memory copy of its tile and halo
-// nodes by tile-local position (NbTile, rows of 3-component systems only).
-// aux is the per-node scalar the loop needs besides the node record (alpha
-// in k_low, the residual in k_fct and k_update); R is R^- (k_update).
-// Entry k of a row is read at row_index(base)[32 k]: a per-row pointer and a
-// 32-bit offset.  self(r) is the row's own position in nq / aux / R (the
-// tile variants read their own rows from shared memory too), len(r) and
-// base(r) its entry count and first entry (the tile variants read them from
-// shared memory, staged with the tile).
+// nodes by tile-local position (the tile kernels, 3-component systems only),
+// where the quantities of one node are formed once per node and block instead
+// of once per entry.  Both form them with the same operations.
+//
+// The global variants process the entries in batches of B: every global load
+// of a batch is issued before any of them is used, so a thread keeps B loads
+// in flight.  Sums keep the entry order, so every batch size gives the same
+// bits.  aux is the per-node scalar the loop needs besides the node record
+// (alpha in k_low, the residual in k_fct and k_update); R is R^- (k_update).
 struct NbGlobal {
   static constexpr bool kGlobal = true;
-  const int* col;
+  const Graph& G;
   const float4* nq;
   const float* aux;
   const float* R;
   const double* R64;          // FP64 R^- (precision split), or null
-  __device__ __forceinline__ const int* row_index(int64_t base) const { return col + base; }
-  __device__ __forceinline__ int self(int64_t r) const { return (int)r; }
-  __device__ __forceinline__ int len(const Graph& G, int64_t r) const { return G.len[r]; }
-  __device__ __forceinline__ int64_t base(const Graph& G, int64_t r) const { return entry_base(G, r); }
+  struct Raw {
+    float4 n;
+    float a, R;
+  };
+  __device__ __forceinline__ const int* row_index(int64_t base) const { return G.col + base; }
+  __device__ __forceinline__ const float2* cf(int64_t base) const { return G.cf + base; }
+  __device__ __forceinline__ const float2* dm(const float2* p, int64_t base) const { return p + base; }
+  __device__ __forceinline__ const float* dl(const float* p, int64_t base) const { return p + base; }
+  __device__ __forceinline__ int self(int r) const { return r; }
+  __device__ __forceinline__ float depth(int j) const { return nq[j].x; }
+  __device__ __forceinline__ Raw raw(int j, bool a, bool r) const {
+    return Raw{nq[j], a ? aux[j] : 0.f, r ? R[j] : 1.f};
+  }
+  __device__ __forceinline__ NodeF low(const Raw& w, int, float g, float htiny, bool sgn) const {
+    return node_f(w.n, w.a, g, htiny, sgn);
+  }
+  __device__ __forceinline__ NodeL dt(const Raw& w, int, float g, float htiny) const { return node_l(w.n, g, htiny); }
+  __device__ __forceinline__ NodeC fct(const Raw& w, int) const { return NodeC{w.n.x, w.n.w, w.a}; }
+  __device__ __forceinline__ NodeU upd(const Raw& w, int) const { return node_u(w.n, w.a, w.R); }
+  __device__ __forceinline__ double r64(int j) const { return R64[j]; }
 };
+
+// ---- tile kernels: one block of T threads per tile of T rows, a row per
+// thread.  The block copies the tile's entries into shared memory (cp.async:
+// positions, c_ij or (d, mu)), reads the node records of its rows and halo,
+// forms every quantity of one node and stores it beside them.  The whole tile
+// is in flight at once, the entry loops then touch shared memory only, and
+// what they would form per entry (six times per node) is formed 1.4 times per
+// node.  The size is a template argument: with one row per thread the
+// prologue is a third of the instructions, and constant strides halve it.
 struct NbTile {
   static constexpr bool kGlobal = false;
-  const int16_t* loc;
-  const float4* nq;
-  const float* aux;
-  const float* R;
-  const double* R64;
-  int64_t t0;
-  const int64_t* sp;          // slice pointers of the tile's slices
-  const uint8_t* ln;          // entry counts of the tile's rows
-  __device__ __forceinline__ const int16_t* row_index(int64_t base) const { return loc + base; }
-  __device__ __forceinline__ int self(int64_t r) const { return (int)(r - t0); }
-  __device__ __forceinline__ int len(const Graph&, int64_t r) const { return ln[r - t0]; }
-  __device__ __forceinline__ int64_t base(const Graph&, int64_t r) const { return sp[(r - t0) >> 5] + (r & 31); }
-};
-
-// Shared-memory tile of one block: node records, aux and R^- (and the FP64
-// R^- of the precision split) of the tile's rows (positions 0 .. T-1) and of
-// its halo rows (T .. T+nh-1), then the slice pointers and entry counts of
-// the tile's rows.  Layout: nq | R64 (split only) | aux | R | sp | ln.
-struct TileSmem {
-  float4* nq;
-  double* R64;
-  float* aux;
-  float* R;
-  int64_t* sp;
-  uint8_t* ln;
-};
-template <bool D>
-__device__ __forceinline__ TileSmem tile_smem(void* base, int cap, int T) {
-  float4* nq = reinterpret_cast<float4*>(base);
-  double* r64 = reinterpret_cast<double*>(nq + cap);
-  float* aux = reinterpret_cast<float*>(D ? (void*)(r64 + cap) : (void*)(nq + cap));
-  float* R = aux + cap;
-  int64_t* sp = reinterpret_cast<int64_t*>(R + cap);   // 24 or 32 bytes per position before it: 8-byte aligned
-  return TileSmem{nq, D ? r64 : nullptr, aux, R, sp, reinterpret_cast<uint8_t*>(sp + T / 32)};
-}
-
-// Copy the tile's and the halo's node data into shared memory (coalesced for
-// the tile rows, ascending gathers for the halo); returns the tile start.
-template <bool AUX, bool RM, bool D = false>
-__device__ __forceinline__ int64_t stage_tile(const Graph& G, const TileCtl& tc, const StateMix& u,
-                                              const float* __restrict__ aux, const float* __restrict__ rminus,
-                                              const TileSmem& sm, const double* __restrict__ rminus64 = nullptr) {
-  const int T = tc.tile_rows;
-  const int64_t t0 = (int64_t)blockIdx.x * T;
-  const int h0 = tc.halo_ptr[blockIdx.x], nh = tc.halo_ptr[blockIdx.x + 1] - h0;
-  for (int i = threadIdx.x; i < T + nh; i += blockDim.x) {
-    const int64_t row = i < T ? t0 + i : (int64_t)tc.halo_rows[h0 + i - T];
-    if (row < G.n_rows) {
-      sm.nq[i] = u.nq[row];
-      if (AUX) sm.aux[i] = aux[row];
-      if (RM) sm.R[i] = rminus[row];
-      if (RM && D) sm.R64[i] = rminus64[row];
-      if (i < T) sm.ln[i] = G.len[row];
-    }
-    // slices of the tile that exist (the last tile may be partial)
-    if (i < T / 32 && t0 + 32 * (int64_t)i < G.n_rows) sm.sp[i] = G.slice_ptr[(t0 >> 5) + i];
+  const float4* a;            // k_low (h, q1, q2, eta); k_dt (h, v1, v2, sq); k_fct (h, eta, res); k_update as k_low
+  const float4* b;            // k_low (ovh, v1, v2, sq); k_update (res, R, inv, one)
+  const float4* c;            // k_low (inv, one, E, alpha)
+  const float* o;             // k_dt: ovh; k_node: h
+  const double* R64_;
+  const int16_t* loc;         // this row's positions, c_ij or (d, mu), |c_ij| lambda
+  const float2* e8;
+  const float* e4;
+  struct Raw {};
+  __device__ __forceinline__ const int16_t* row_index(int64_t) const { return loc; }
+  __device__ __forceinline__ const float2* cf(int64_t) const { return e8; }
+  __device__ __forceinline__ const float2* dm(const float2*, int64_t) const { return e8; }
+  __device__ __forceinline__ const float* dl(const float*, int64_t) const { return e4; }
+  __device__ __forceinline__ int self(int) const { return threadIdx.x; }
+  __device__ __forceinline__ float depth(int j) const { return o[j]; }
+  __device__ __forceinline__ Raw raw(int, bool, bool) const { return Raw{}; }
+  __device__ __forceinline__ NodeF low(const Raw&, int j, float, float, bool) const {
+    const float4 x = a[j], y = b[j], z = c[j];
+    return NodeF{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
   }
-  __syncthreads();
-  return t0;
+  __device__ __forceinline__ NodeL dt(const Raw&, int j, float, float) const {
+    const float4 x = a[j];
+    return NodeL{x.x, x.y, x.z, x.w, o[j]};
+  }
+  __device__ __forceinline__ NodeC fct(const Raw&, int j) const {
+    const float4 x = a[j];
+    return NodeC{x.x, x.y, x.z};
+  }
+  __device__ __forceinline__ NodeU upd(const Raw&, int j) const {
+    const float4 x = a[j], y = b[j];
+    return NodeU{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  }
+  __device__ __forceinline__ double r64(int j) const { return R64_[j]; }
+};
+
+// Shared memory of one tile block: per-node parts over the tile's rows
+// (positions 0 .. T-1) and its halo rows (T ..), then the tile's entries; each
+// part a multiple of 16 bytes.  What a kernel does not use takes no space.
+struct TileParts {
+  int a, b, c, o, r64, e8, e4;   // bytes per position / entry
+};
+__host__ __device__ constexpr TileParts tile_parts(int kind, bool d, bool lamin) {
+  return TileParts{kind == 1 ? 0 : 16,           kind == 2 || kind == 4 ? 16 : 0, kind == 2 ? 16 : 0,
+                   kind <= 1 ? 4 : 0,            kind == 4 && d ? 8 : 0,          kind == 1 ? 0 : 8,
+                   kind == 2 && lamin ? 4 : 0};
+}
+struct TileSmem {
+  float4 *a, *b, *c;
+  double* r64;
+  float2* e8;
+  float *e4, *o;
+  int16_t* loc;
+};
+template <int T, int KIND, bool D, bool LAMIN>
+__device__ __forceinline__ TileSmem tile_smem(void* base, const TileCtl& tc) {
+  constexpr TileParts P = tile_parts(KIND, D, LAMIN);
+  const int cap = T + tc.halo_cap, ec = tc.ent_cap;
+  char* p = reinterpret_cast<char*>(base);
+  TileSmem s{};
+  if (P.a) { s.a = reinterpret_cast<float4*>(p); p += P.a * cap; }
+  if (P.b) { s.b = reinterpret_cast<float4*>(p); p += P.b * cap; }
+  if (P.c) { s.c = reinterpret_cast<float4*>(p); p += P.c * cap; }
+  if (P.r64) { s.r64 = reinterpret_cast<double*>(p); p += P.r64 * cap; }
+  if (P.e8) { s.e8 = reinterpret_cast<float2*>(p); p += P.e8 * ec; }
+  if (P.e4) { s.e4 = reinterpret_cast<float*>(p); p += P.e4 * ec; }
+  if (P.o) { s.o = reinterpret_cast<float*>(p); p += P.o * cap; }
+  s.loc = reinterpret_cast<int16_t*>(p);
+  return s;
 }
 
-__device__ __forceinline__ int64_t tile_end(const Graph& G, const TileCtl& tc, int64_t t0) {
-  return t0 + tc.tile_rows < G.n_rows ? t0 + tc.tile_rows : G.n_rows;
+// a contiguous range, both ends multiples of 16 bytes, copied asynchronously
+template <int T>
+__device__ __forceinline__ void cp_range(void* dst, const void* src, int bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst) + 16 * threadIdx.x;
+  const char* g = reinterpret_cast<const char*>(src) + 16 * threadIdx.x;
+  for (int o = 0; o + 16 * (int)threadIdx.x < bytes; o += 16 * T)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + o), "l"(g + o) : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A block's tile and this thread's row.  All loads are independent of each
+// other, so one memory latency covers them.
+struct Tile {
+  int r;                  // this thread's row
+  bool live;              // it exists
+  int hr;                 // this thread's halo row (position T + threadIdx.x), or -1
+  int ne;                 // entries of the tile
+  int64_t e0;             // the first of them
+  RowHead hd;
+};
+template <int T>
+__device__ __forceinline__ Tile tile_of(const Graph& G, const TileCtl& tc) {
+  const int4 h = tc.head[blockIdx.x];
+  Tile t;
+  t.r = (int)blockIdx.x * T + (int)threadIdx.x;
+  t.live = t.r < (int)G.n_rows;
+  t.hr = (int)threadIdx.x < tc.halo_cap ? tc.halo_rows[(int)blockIdx.x * tc.halo_cap + (int)threadIdx.x] : -1;
+  t.hd = RowHead{0, 0, 0};
+  if (t.live) t.hd = row_head(G, t.r);
+  t.e0 = (int64_t)(((unsigned long long)(unsigned)h.y << 32) | (unsigned)h.x);
+  t.ne = h.z;
+  return t;
+}
+// load(row) reads a node's data, put(position, row, data) forms and stores its
+// shared-memory record; both rows of a thread are read before either is put.
+template <int T, class Load, class Put>
+__device__ __forceinline__ void stage_nodes(const TileCtl& tc, const Tile& t, Load load, Put put) {
+  const int i = threadIdx.x;
+  const int ro = t.live ? t.r : 0, rh = t.hr >= 0 ? t.hr : ro;
+  const auto x = load(ro);
+  const auto y = load(rh);
+  if (t.live) put(i, ro, x);
+  if (t.hr >= 0) put(T + i, rh, y);
+  for (int k = i + T; k < tc.halo_cap; k += T) {       // halos above T rows
+    const int row = tc.halo_rows[(int)blockIdx.x * tc.halo_cap + k];
+    if (row >= 0) put(T + k, row, load(row));
+  }
+}
+__device__ __forceinline__ NbTile nb_tile(const Tile& t, const TileSmem& sm) {
+  const int o = (int)(t.hd.base - t.e0);
+  return NbTile{sm.a, sm.b, sm.c, sm.o, sm.r64, sm.loc + o, sm.e8 + o, sm.e4 + o};
+}
+// the instance whose g and htiny a node's quantities take (rows of a tile may
+// belong to several instances; a row and its neighbours share one)
+__device__ __forceinline__ const InstConst& inst_of(const Graph& G, const InstConst* C, int row) {
+  return C[G.slice_inst[row >> 5]];
 }
 
 // L2 prefetch of a byte range with the TMA unit (cp.async.bulk.prefetch):
 // no registers or shared memory are held while the data comes in.  The range
 // is widened to the 16-byte granule the instruction requires; every array
 // passed here starts 256-byte aligned and is a multiple of 16 bytes long
-// (per-row and per-entry arrays of a multiple of 32 elements), so the
-// widened range stays inside it.
+// (per-row arrays of a multiple of 32 elements), so the widened range stays
+// inside it.
 __device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes) {
   if (bytes <= 0) return;
   const uint64_t a = reinterpret_cast<uint64_t>(p);
@@ -309,27 +461,24 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((unsigned)(hi - lo)) : "memory");
 }
 
-// The tile's per-entry arrays are one contiguous range (its slices are
-// consecutive): one thread of the block prefetches it into L2, with the
-// per-row arrays the rows read after their entry loops, while the block
-// stages its nodes.  e0/e1: the tile's first and one-past-last entry.
-struct TilePrefetch {
-  const void* ent[3];   // per-entry arrays
-  int esz[3];           // their element sizes (0: unused)
+// The per-row arrays that the rows read after their entry loops: lanes of the
+// first warp prefetch the tile's range of one array each into L2 while the
+// block stages.
+struct RowPrefetch {
   const void* row[6];   // per-row arrays
-  int rsz[6];
+  int rsz[6];           // their element sizes (0: unused)
 };
-__device__ __forceinline__ void tile_prefetch(const Graph& G, const TileCtl& tc, const TilePrefetch& pf) {
-  if (threadIdx.x != 0) return;
-  const int64_t t0 = (int64_t)blockIdx.x * tc.tile_rows;
-  const int64_t t1 = tile_end(G, tc, t0);
-  const int64_t e0 = G.slice_ptr[t0 >> 5], e1 = G.slice_ptr[(t1 + 31) >> 5];
+template <int T>
+__device__ __forceinline__ void row_prefetch(const Graph& G, const RowPrefetch& pf) {
+  if (threadIdx.x >= 6) return;
+  const void* p = pf.row[0];
+  int sz = pf.rsz[0];
 #pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (pf.esz[k]) prefetch_l2(static_cast<const char*>(pf.ent[k]) + e0 * pf.esz[k], (e1 - e0) * pf.esz[k]);
-#pragma unroll
-  for (int k = 0; k < 6; k++)
-    if (pf.rsz[k]) prefetch_l2(static_cast<const char*>(pf.row[k]) + t0 * pf.rsz[k], (t1 - t0) * pf.rsz[k]);
+  for (int k = 1; k < 6; k++)
+    if ((int)threadIdx.x == k) { p = pf.row[k]; sz = pf.rsz[k]; }
+  const int64_t t0 = (int64_t)blockIdx.x * T;
+  const int rows = G.n_rows - t0 < T ? (int)(G.n_rows - t0) : T;
+  prefetch_l2(static_cast<const char*>(p) + t0 * sz, rows * sz);
 }
 
 // alpha_i (SOURCES/update.f90:758-781) from the stencil sums of the FP32
@@ -342,20 +491,18 @@ __device__ __forceinline__ float alpha_from(float num, float denom) {
 
 // k_node_mix: alpha_i from the FP32 depth.
 template <int B, class Nb>
-__device__ __forceinline__ void node_row(int64_t r, Graph G, const InstConst* __restrict__ C,
-                                                  const InstState* __restrict__ St, StateMix u,
-                                                  float* __restrict__ alpha_out, const Nb& nb) {
-  const int L = nb.len(G, r);
+__device__ __forceinline__ void node_row(int r, const RowHead& hd, const InstConst* __restrict__ C,
+                                         const InstState* __restrict__ St, float* __restrict__ alpha_out,
+                                         const Nb& nb) {
+  const int L = hd.L;
   if (L == 0) return;
-  const int b = G.slice_inst[r >> 5];
-  if (St[b].done) return;
-  const InstConst& c = C[b];
-  const float* hs = reinterpret_cast<const float*>(nb.nq);
+  if (St[hd.b].done) return;
+  const InstConst& c = C[hd.b];
   const int me = nb.self(r);
-  const float h = hs[4 * me];
+  const float h = nb.depth(me);
   float alpha = 1.0f;
   if (c.alpha_limit && !(h <= c.htinyf)) {
-    const auto ip = nb.row_index(nb.base(G, r));
+    const auto ip = nb.row_index(hd.base);
     float num = 0.0f, denom = 0.0f;
     for (int k0 = 0; k0 < L; k0 += B) {
       int j[B];
@@ -363,7 +510,7 @@ __device__ __forceinline__ void node_row(int64_t r, Graph G, const InstConst* __
       for (int q = 0; q < B; q++) j[q] = (k0 + q < L) ? (int)ip[32 * (k0 + q)] : me;
       float hj[B];
 #pragma unroll
-      for (int q = 0; q < B; q++) hj[q] = hs[4 * (int64_t)j[q]];
+      for (int q = 0; q < B; q++) hj[q] = nb.depth(j[q]);
 #pragma unroll
       for (int q = 0; q < B; q++)
         if (k0 + q < L) {
@@ -382,42 +529,25 @@ __global__ void __launch_bounds__(256) k_node_mix(Graph G, const InstConst* __re
                                                   float* __restrict__ alpha_out) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G.col, u.nq, nullptr, nullptr, nullptr};
+  const NbGlobal nb{G, u.nq, nullptr, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
-    node_row<B>(r, G, C, St, u, alpha_out, nb);
+    node_row<B>((int)r, row_head(G, r), C, St, alpha_out, nb);
 }
 
-template <int B>
-__global__ void __launch_bounds__(256) k_node_tile(Graph G, const InstConst* __restrict__ C,
-                                                   const InstState* __restrict__ St, StateMix u,
-                                                   float* __restrict__ alpha_out, TileCtl tc) {
+template <int T>
+__global__ void __launch_bounds__(T) k_node_tile(Graph G, const InstConst* __restrict__ C,
+                                                 const InstState* __restrict__ St, StateMix u,
+                                                 float* __restrict__ alpha_out, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
-  pdl_trigger();
-  tile_prefetch(G, tc, TilePrefetch{{tc.loc, nullptr, nullptr}, {2, 0, 0}, {}, {}});
+  const Tile t = tile_of<T>(G, tc);
+  const TileSmem sm = tile_smem<T, 1, false, false>(tile_mem, tc);
+  cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
-  const TileSmem sm = tile_smem<false>(tile_mem, tc.tile_rows + tc.halo_cap, tc.tile_rows);
-  const int64_t t0 = stage_tile<false, false>(G, tc, u, nullptr, nullptr, sm);
-  const int64_t t1 = tile_end(G, tc, t0);
-  const NbTile nb{tc.loc, sm.nq, nullptr, nullptr, nullptr, t0, sm.sp, sm.ln};
-  for (int64_t r = t0 + threadIdx.x; r < t1; r += blockDim.x) node_row<B>(r, G, C, St, u, alpha_out, nb);
-}
-
-struct NodeF {   // FP32 view of one node used by the edge loop
-  float h, q1, q2, eta, ovh, v1, v2;
-};
-
-__device__ __forceinline__ NodeF node_from(const float4 a, float htiny) {
-  NodeF n;
-  n.h = a.x; n.q1 = a.y; n.q2 = a.z; n.eta = a.w;
-  n.ovh = ovh_f(n.h, htiny);
-  n.v1 = n.q1 * n.ovh;
-  n.v2 = n.q2 * n.ovh;
-  return n;
-}
-
-// 0.5 (g h^2 + v1 q1 + v2 q2): the entropy of the reference's entropy_residual
-__device__ __forceinline__ float entropy_f(float g, float h, float v1, float q1, float v2, float q2) {
-  return 0.5f * fma_(v2, q2, fma_(v1, q1, (g * h) * h));
+  stage_nodes<T>(tc, t, [&](int row) { return u.nq[row].x; }, [&](int i, int, float h) { sm.o[i] = h; });
+  cp_wait();
+  __syncthreads();
+  pdl_trigger();
+  node_row<1>(t.r, t.hd, C, St, alpha_out, nb_tile(t, sm));
 }
 
 __device__ __forceinline__ float sgn_pressure(float lambda_sgn, float g, float m, float h, float heta) {
@@ -441,50 +571,48 @@ __device__ __forceinline__ float sgn_pressure(float lambda_sgn, float g, float m
 // (N <= h_i sum d, so a N <= CFL h_i): the reference's fix h + rk_1 with
 // rat_ij h_i = H*_ij.  At rest the two sums add equal terms in the same
 // order, so P - N is exactly 0.
-template <int B, bool LAMIN, int MINB, bool D, class Nb>
-__device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __restrict__ C,
-                                                       const InstState* __restrict__ St, StateMix u,
-                                                       const float* __restrict__ alpha, float2* __restrict__ dmu,
-                                                       WorkMix w, float* __restrict__ res, unsigned* __restrict__ err,
-                                                       const Nb& nb) {
-  const int L = nb.len(G, r);
+//
+// FCT: every instance runs 'fct' with the roundoff fix and alpha_limit (the
+// usual run), so the mode tests fall away.
+template <int B, bool LAMIN, bool D, bool FCT, class Nb>
+__device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
+                                        const InstState* __restrict__ St, const StateMix& u, float2* __restrict__ dmu,
+                                        const WorkMix& w, float* __restrict__ res, unsigned* __restrict__ err,
+                                        const Nb& nb) {
+  const int L = hd.L;
   if (L == 0) return;
-  const int b = G.slice_inst[r >> 5];
-  const InstState& st = St[b];
+  const InstState& st = St[hd.b];
   if (st.done) return;
-  const InstConst& c = C[b];
+  const InstConst& c = C[hd.b];
   const int S = Nb::kGlobal ? c.S : 3;         // tiles hold 3-component systems only
   const bool sgn = Nb::kGlobal && c.type_test == 13;
-  const bool galerkin = c.visc == VISC_GALERKIN;   // every d_ij, mu_ij = 0 (update.f90:155-158)
-  const float vis = galerkin ? 0.f : 1.f;
+  const bool galerkin = !FCT && c.visc == VISC_GALERKIN;   // every d_ij, mu_ij = 0 (update.f90:155-158)
+  const bool limit = FCT || c.alpha_limit;
   const float g = c.gf, htiny = c.htinyf, dtf = st.dtf;
   const LamK lk = lam_k(g, htiny);
   // the low-order momenta: smb_2_roundoff's htiny tests, or smb_2's h <= 0
   // tests (rat = 0 already where h <= 0) when the step is not roundoff-fixed
-  const bool roundoff = c.roundoff_fix && !galerkin;
+  const bool roundoff = FCT || (c.roundoff_fix && !galerkin);
   const float hthr = roundoff ? htiny : 0.f;
-  const int64_t base = nb.base(G, r);
+  const int64_t base = hd.base;
   const int me = nb.self(r);
   const auto ip = nb.row_index(base);
-  const float2* cp = G.cf + base;
-  const float* dlp = w.dlam + base;
+  const float2* cp = nb.cf(base);
+  const float* dlp = nb.dl(w.dlam, base);
   float2* dmp = dmu + base;
-  const NodeF ni = node_from(nb.nq[me], htiny);
-  const float sqi = sqrtf(g * fabsf(ni.h));
+  const NodeF ni = nb.low(nb.raw(me, true, false), me, g, htiny, sgn);
   const float v2i_flux = sgn ? 0.f : ni.v2;          // flux() zeroes velocity(2) for type 13
-  const float ai = nb.aux[me];
   const float m = G.lumpedf[r];
   const float ghi = g * ni.h;
   const bool wet_i = !(ni.h <= hthr);
   float ui3 = 0.f, ui4 = 0.f;
   if (S == 5) { ui3 = u.q3[r]; ui4 = u.q4[r]; }
-  const float invhi = inv_pos(ni.h);
   bool delta_bad = false;
 
   float P = 0.f, N = 0.f;                                          // smb_2_roundoff mass row
   float rk1 = 0.f, rk2_ = 0.f, rk3 = 0.f, rk4 = 0.f;               // smb_2_roundoff momenta
   float g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f, g4 = 0.f;          // smb_2
-  const float Ei = entropy_f(g, ni.h, ni.v1, ni.q1, v2i_flux, ni.q2);
+  const float Ei = ni.E;
   float emax = Ei, emin = Ei;
   float ptx = 0.f, pty = 0.f;
   // diagonal: Galerkin boundary term -c_ii.v_i (fix_roundoff / smb_2);
@@ -492,20 +620,22 @@ __device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __r
   const float cxd = G.cxiif[r], cyd = G.cyiif[r];
   const float cvd = dotc(cxd, cyd, ni.v1, v2i_flux);
   g0 = -cvd * ni.h;
-  rk1 = -cvd * ni.q1; rk2_ = -cvd * ni.q2;
-  g1 = rk1; g2 = rk2_;
-  if (S == 5) { rk3 = -cvd * ui3; rk4 = -cvd * ui4; g3 = rk3; g4 = rk4; }
+  g1 = -cvd * ni.q1; g2 = -cvd * ni.q2;
+  if (S == 5) { g3 = -cvd * ui3; g4 = -cvd * ui4; }
   if (sgn) {
     const float pt = sgn_pressure(c.lambda_sgnf, g, m, ni.h, ui3);
     ptx = -pt * cxd;
     pty = -pt * cyd;
   }
+  // the momenta of the two right-hand sides are the same sums until an entry
+  // with a node at or below hthr: only then does the row carry both
+  bool fork = false;
   for (int k0 = 0; k0 < L; k0 += B) {
    int jb[B];
    float cxb[B], cyb[B], dlb[B];
 #pragma unroll
    for (int q = 0; q < B; q++) {
-     if (k0 + q < L) {
+     if (B == 1 || k0 + q < L) {
        const int off = 32 * (k0 + q);
        const float2 cc = cp[off];
        jb[q] = ip[off]; cxb[q] = cc.x; cyb[q] = cc.y;
@@ -514,49 +644,41 @@ __device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __r
        jb[q] = me; cxb[q] = 0.f; cyb[q] = 0.f; dlb[q] = 0.f;
      }
    }
-   float4 nqb[Nb::kGlobal ? B : 1];
-   float alb[Nb::kGlobal ? B : 1];
-   if constexpr (Nb::kGlobal) {
+   typename Nb::Raw rw[B];
 #pragma unroll
-     for (int q = 0; q < B; q++) { nqb[q] = nb.nq[jb[q]]; alb[q] = nb.aux[jb[q]]; }
-   }
+   for (int q = 0; q < B; q++) rw[q] = nb.raw(jb[q], true, false);
 #pragma unroll
    for (int q = 0; q < B; q++) {
-    if (k0 + q >= L) break;
+    if (B > 1 && k0 + q >= L) break;
     const int off = 32 * (k0 + q);
     const float cxe = cxb[q], cye = cyb[q];
     const int j = jb[q];
-    const NodeF nj = node_from(Nb::kGlobal ? nqb[q] : nb.nq[j], htiny);
-    const float alj = Nb::kGlobal ? alb[q] : nb.aux[j];
+    const NodeF nj = nb.low(rw[q], j, g, htiny, sgn);
     // --- viscosities: compute_dij, compute_muij, MAX, alpha_limit
     const float cvi = dotc(cxe, cye, ni.v1, ni.v2);                   // c.v_i (compute_muij)
     const float cvj = dotc(cxe, cye, nj.v1, nj.v2);                   // c.v_j
     float dlam;                                                       // |c_ij| lambda_max
     if (LAMIN) {
       dlam = dlb[q];                                                  // from k_dt_mix on this state
-    } else if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, sqi, sqrtf(g * fabsf(nj.h)), lk, &dlam)) {
+    } else if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, ni.sq, nj.sq, lk, &dlam)) {
       delta_bad = true;
     }
     float mu = fmaxf(fmaxf(-cvi, 0.f), fmaxf(cvj, 0.f));
     float d = fmaxf(dlam, mu);
-    const float s = (c.alpha_limit ? fmaxf(ai, alj) : 1.f) * vis;
+    const float s = galerkin ? 0.f : (limit ? fmaxf(ni.al, nj.al) : 1.f);
     d *= s;
     mu *= s;
     dmp[off] = make_float2(d, mu);
     // --- entropy stencil
-    const float v2j_flux = sgn ? 0.f : nj.v2;
-    const float Ej = entropy_f(g, nj.h, nj.v1, nj.q1, v2j_flux, nj.q2);
-    emax = fmaxf(emax, Ej);
-    emin = fminf(emin, Ej);
+    emax = fmaxf(emax, nj.E);
+    emin = fminf(emin, nj.E);
     // --- hydrostatic reconstruction from the free surface
     const float deta = __fsub_rn(nj.eta, ni.eta);
     const float dz = dz_of(deta, ni.h, nj.h);
     const Recon R = recon(ni.h, nj.h, dz);
-    const float rij = rat_of(R.Hij, ni.h, dz <= 0.f, invhi);          // h <= 0 tests (smb_2)
-    const float rji = rat_of(R.Hji, nj.h, dz >= 0.f, inv_pos(nj.h));
+    const float rij = rat_of(R.Hij, dz <= 0.f, ni.inv, ni.one);       // h <= 0 tests (smb_2)
+    const float rji = rat_of(R.Hji, dz >= 0.f, nj.inv, nj.one);
     const bool wet_j = !(nj.h <= hthr);
-    const float rijt = wet_i ? rij : 0.f;                             // h <= htiny tests
-    const float rjit = wet_j ? rji : 0.f;
     const float cvj_flux = sgn ? dotc(cxe, cye, nj.v1, 0.f) : cvj;   // c.velocity_j of flux()
     const float topo = ghi * deta;                                    // g h_i (eta_j - eta_i)
     const float dmu = d - mu;
@@ -571,23 +693,27 @@ __device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __r
     const float A2 = fma_(mu, nj.q2 - ni.q2, -cvj_flux * nj.q2);
     const float T1 = fma_(dmu, fma_(nj.q1, rji, -ni.q1 * rij), A1);
     const float T2 = fma_(dmu, fma_(nj.q2, rji, -ni.q2 * rij), A2);
-    g1 = fma_(-topo, cxe, g1 + T1);
-    g2 = fma_(-topo, cye, g2 + T2);
-    if (rijt == rij && rjit == rji) {                                 // both wet: same terms
-      rk1 += T1;
-      rk2_ += T2;
-    } else {
+    float uj3 = 0.f, uj4 = 0.f, A3 = 0.f, A4 = 0.f;
+    if (Nb::kGlobal && S == 5) {
+      uj3 = u.q3[j]; uj4 = u.q4[j];
+      A3 = fma_(mu, uj3 - ui3, -cvj_flux * uj3);
+      A4 = fma_(mu, uj4 - ui4, -cvj_flux * uj4);
+    }
+    if (fork || !(wet_i && wet_j)) {
+      if (!fork) { rk1 = g1; rk2_ = g2; rk3 = g3; rk4 = g4; fork = true; }
+      const float rijt = wet_i ? rij : 0.f, rjit = wet_j ? rji : 0.f;  // h <= htiny tests
       rk1 += fma_(dmu, fma_(nj.q1, rjit, -ni.q1 * rijt), A1);
       rk2_ += fma_(dmu, fma_(nj.q2, rjit, -ni.q2 * rijt), A2);
+      rk1 = fma_(-topo, cxe, rk1);
+      rk2_ = fma_(-topo, cye, rk2_);
+      if (Nb::kGlobal && S == 5) {
+        rk3 += fma_(dmu, fma_(uj3, rjit, -ui3 * rijt), A3);
+        rk4 += fma_(dmu, fma_(uj4, rjit, -ui4 * rijt), A4);
+      }
     }
-    rk1 = fma_(-topo, cxe, rk1);
-    rk2_ = fma_(-topo, cye, rk2_);
+    g1 = fma_(-topo, cxe, g1 + T1);
+    g2 = fma_(-topo, cye, g2 + T2);
     if (Nb::kGlobal && S == 5) {
-      const float uj3 = u.q3[j], uj4 = u.q4[j];
-      const float A3 = fma_(mu, uj3 - ui3, -cvj_flux * uj3);
-      const float A4 = fma_(mu, uj4 - ui4, -cvj_flux * uj4);
-      rk3 += fma_(dmu, fma_(uj3, rjit, -ui3 * rijt), A3);
-      rk4 += fma_(dmu, fma_(uj4, rjit, -ui4 * rijt), A4);
       g3 += fma_(dmu, fma_(uj3, rji, -ui3 * rij), A3);
       g4 += fma_(dmu, fma_(uj4, rji, -ui4 * rij), A4);
       if (sgn) {
@@ -598,6 +724,7 @@ __device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __r
     }
    }
   }
+  if (!fork) { rk1 = g1; rk2_ = g2; rk3 = g3; rk4 = g4; }
   // source terms (update.f90:425-551)
   if (c.type_test == 9 || c.type_test == 10) {
     const float hstar = __powf(fmaxf(ni.h, htiny), 4.0f / 3.0f);
@@ -629,7 +756,7 @@ __device__ __forceinline__ void low_row(int64_t r, Graph G, const InstConst* __r
   const float2 h = u.h[r];
   // ('entropy_visc' without the roundoff fix keeps h + dt rk unclipped: its
   // k_update adds the high-order correction before MAX(., 0))
-  const bool clip = !(c.visc == VISC_ENTROPY);
+  const bool clip = FCT || c.visc != VISC_ENTROPY;
   if (D) {
     const double hd = df_to_double(h), ad = st.dt * G.inv_lumped[r];
     double hL;
@@ -673,29 +800,40 @@ __global__ void __launch_bounds__(256, MINB) k_low_mix(Graph G, const InstConst*
                                                        WorkMix w, float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G.col, u.nq, alpha, nullptr, nullptr};
+  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
-    low_row<B, LAMIN, MINB, D>(r, G, C, St, u, alpha, dmu, w, res, err, nb);
+    low_row<B, LAMIN, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, res, err, nb);
 }
 
-template <int B, bool LAMIN, int MINB, bool D>
-__global__ void __launch_bounds__(256, MINB) k_low_tile(Graph G, const InstConst* __restrict__ C,
-                                                        const InstState* __restrict__ St, StateMix u,
-                                                        const float* __restrict__ alpha, float2* __restrict__ dmu,
-                                                        WorkMix w, float* __restrict__ res, unsigned* __restrict__ err,
-                                                        TileCtl tc) {
+template <int T, bool LAMIN, int MINB, bool D, bool FCT>
+__global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const InstConst* __restrict__ C,
+                                                                 const InstState* __restrict__ St, StateMix u,
+                                                                 const float* __restrict__ alpha,
+                                                                 float2* __restrict__ dmu, WorkMix w,
+                                                                 float* __restrict__ res, unsigned* __restrict__ err,
+                                                                 TileCtl tc) {
   extern __shared__ float4 tile_mem[];
-  pdl_trigger();
-  tile_prefetch(G, tc, TilePrefetch{{tc.loc, G.cf, nullptr}, {2, 8, 0},
-                                    {G.lumpedf, G.inv_lumpedf, G.cxiif, G.cyiif, nullptr, nullptr}, {4, 4, 4, 4, 0, 0}});
+  const Tile t = tile_of<T>(G, tc);
+  const TileSmem sm = tile_smem<T, 2, D, LAMIN>(tile_mem, tc);
+  cp_range<T>(sm.e8, G.cf + t.e0, 8 * t.ne);
+  cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
-  tile_prefetch(G, tc, TilePrefetch{{w.dlam, nullptr, nullptr}, {LAMIN ? 4 : 0, 0, 0}, {u.h}, {8}});
-  const TileSmem sm = tile_smem<false>(tile_mem, tc.tile_rows + tc.halo_cap, tc.tile_rows);
-  const int64_t t0 = stage_tile<true, false>(G, tc, u, alpha, nullptr, sm);
-  const int64_t t1 = tile_end(G, tc, t0);
-  const NbTile nb{tc.loc, sm.nq, sm.aux, nullptr, nullptr, t0, sm.sp, sm.ln};
-  for (int64_t r = t0 + threadIdx.x; r < t1; r += blockDim.x)
-    low_row<B, LAMIN, MINB, D>(r, G, C, St, u, alpha, dmu, w, res, err, nb);
+  if (LAMIN) cp_range<T>(sm.e4, w.dlam + t.e0, 4 * t.ne);
+  row_prefetch<T>(G, RowPrefetch{{G.lumpedf, G.inv_lumpedf, G.cxiif, G.cyiif, u.h, nullptr}, {4, 4, 4, 4, 8, 0}});
+  struct Node { float4 n; float al; };
+  stage_nodes<T>(
+      tc, t, [&](int row) { return Node{u.nq[row], alpha[row]}; },
+      [&](int i, int row, const Node& x) {
+        const InstConst& c = inst_of(G, C, row);
+        const NodeF n = node_f(x.n, x.al, c.gf, c.htinyf, false);
+        sm.a[i] = x.n;
+        sm.b[i] = make_float4(n.ovh, n.v1, n.v2, n.sq);
+        sm.c[i] = make_float4(n.inv, n.one, n.E, n.al);
+      });
+  cp_wait();
+  __syncthreads();
+  pdl_trigger();
+  low_row<1, LAMIN, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, res, err, nb_tile(t, sm));
 }
 
 // 'viscous' with viscous_type 'type1' (update.f90:189-201, smb_1 :366-423):
@@ -709,19 +847,16 @@ template <bool D>
 __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const InstConst& c, const InstState& st,
                                               const StateMix& u, const float* __restrict__ alpha,
                                               float2* __restrict__ dmu, const WorkMix& w, unsigned* __restrict__ err) {
-  const NbGlobal nb{G.col, u.nq, alpha, nullptr, nullptr};
-  const int L = nb.len(G, r);
+  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
+  const int L = G.len[r];
   const float g = c.gf, htiny = c.htinyf, dtf = st.dtf;
   const LamK lk = lam_k(g, htiny);
-  const int64_t base = nb.base(G, r);
+  const int64_t base = entry_base(G, r);
   const int me = nb.self(r);
   const int* ip = nb.row_index(base);
   const float2* cp = G.cf + base;
   float2* dmp = dmu + base;
-  const NodeF ni = node_from(nb.nq[me], htiny);
-  const float sqi = sqrtf(g * fabsf(ni.h));
-  const float ai = nb.aux[me];
-  const float invhi = inv_pos(ni.h);
+  const NodeF ni = node_f(nb.nq[me], nb.aux[me], g, htiny, false);
   const bool wet_i = !(ni.h <= htiny);
   // diagonal: the centred flux -c_ii.v_i u_i (rat_ii = 1 for h_i > htiny)
   const float cxd = G.cxiif[r], cyd = G.cyiif[r];
@@ -733,23 +868,23 @@ __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const I
     const int off = 32 * k;
     const float2 cc = cp[off];
     const int j = ip[off];
-    const NodeF nj = node_from(nb.nq[j], htiny);
+    const NodeF nj = node_f(nb.nq[j], nb.aux[j], g, htiny, false);
     const float cxe = cc.x, cye = cc.y;
     const float cvi = dotc(cxe, cye, ni.v1, ni.v2), cvj = dotc(cxe, cye, nj.v1, nj.v2);
     float dlam;
-    if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, sqi, sqrtf(g * fabsf(nj.h)), lk, &dlam))
+    if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, ni.sq, nj.sq, lk, &dlam))
       delta_bad = true;
     float mu = fmaxf(fmaxf(-cvi, 0.f), fmaxf(cvj, 0.f));
     float d = fmaxf(dlam, mu);
-    const float s = c.alpha_limit ? fmaxf(ai, nb.aux[j]) : 1.f;
+    const float s = c.alpha_limit ? fmaxf(ni.al, nj.al) : 1.f;
     d *= s;
     mu *= s;
     dmp[off] = make_float2(d, mu);
     const float deta = __fsub_rn(nj.eta, ni.eta);
     const float dz = dz_of(deta, ni.h, nj.h);
     const Recon R = recon(ni.h, nj.h, dz);
-    const float rij = wet_i ? rat_of(R.Hij, ni.h, dz <= 0.f, invhi) : 0.f;
-    const float rji = !(nj.h <= htiny) ? rat_of(R.Hji, nj.h, dz >= 0.f, inv_pos(nj.h)) : 0.f;
+    const float rij = wet_i ? rat_of(R.Hij, dz <= 0.f, ni.inv, ni.one) : 0.f;
+    const float rji = !(nj.h <= htiny) ? rat_of(R.Hji, dz >= 0.f, nj.inv, nj.one) : 0.f;
     const float ai_ = cvi * rij, aj = cvj * rji;          // c.v_i rat_ij, c.v_j rat_ji
     rk0 += fma_(d, fma_(nj.h, rji, -ni.h * rij), -fma_(aj, nj.h, ai_ * ni.h));
     rk1 += fma_(d, fma_(nj.q1, rji, -ni.q1 * rij), -fma_(aj, nj.q1, ai_ * ni.q1));
@@ -784,14 +919,14 @@ __global__ void __launch_bounds__(256) k_low_type1(Graph G, const InstConst* __r
                                                    float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G.col, u.nq, alpha, nullptr, nullptr};
+  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x) {
     if (G.len[r] == 0) continue;
     const int b = G.slice_inst[r >> 5];
     if (St[b].done) continue;
     const InstConst& c = C[b];
     if (c.viscous_type == 1 && c.visc == VISC_VISCOUS) low_row_type1<D>(r, G, c, St[b], u, alpha, dmu, w, err);
-    else low_row<1, false, 3, D>(r, G, C, St, u, alpha, dmu, w, res, err, nb);
+    else low_row<1, false, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, res, err, nb);
   }
 }
 
@@ -812,48 +947,43 @@ __device__ __forceinline__ float fct_entry(float d0, float m0, float rij, float 
 // k_fct_mix: f_ij and the limiter R^-_i (fct.f90:15-30): P^- = sum f^- - 1e-15,
 // Q^- = -m h^L/dt, R^- = min(Q^-/P^-, 1), 0 where m h^L/dt <= htiny.
 template <int B, bool D, class Nb>
-__device__ __forceinline__ void fct_row(int64_t r, Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St, StateMix u,
-                          const float2* __restrict__ dmu, WorkMix w, const float* __restrict__ res,
-                          unsigned* __restrict__ err, const Nb& nb) {
-  const int L = nb.len(G, r);
+__device__ __forceinline__ void fct_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
+                                        const InstState* __restrict__ St, const float2* __restrict__ dmu,
+                                        const WorkMix& w, unsigned* __restrict__ err, const Nb& nb) {
+  const int L = hd.L;
   if (L == 0) return;
-  const int b = G.slice_inst[r >> 5];
-  const InstState& st = St[b];
+  const InstState& st = St[hd.b];
   if (st.done) return;
-  const InstConst& c = C[b];
+  const InstConst& c = C[hd.b];
   if (c.visc != VISC_FCT) return;
-  const int64_t base = nb.base(G, r);
+  const int64_t base = hd.base;
   const int me = nb.self(r);
   const auto ip = nb.row_index(base);
-  const float2* dmp = dmu + base;
-  const float4 ni = nb.nq[me];
-  const float hi = ni.x, etai = ni.w, resi = nb.aux[me];
+  const float2* dmp = nb.dm(dmu, base);
+  const NodeC ni = nb.fct(nb.raw(me, true, false), me);
   float neg = 0.f;                       // f_ii = 0 adds nothing
+#pragma unroll(B == 1 ? 2 : 1)
   for (int k0 = 0; k0 < L; k0 += B) {
     int jb[B];
-    float d0b[B], m0b[B];
+    float2 vb[B];
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      if (k0 + q < L) {
+      if (B == 1 || k0 + q < L) {
         const int off = 32 * (k0 + q);
-        jb[q] = ip[off]; const float2 v = dmp[off]; d0b[q] = v.x; m0b[q] = v.y;
+        jb[q] = ip[off]; vb[q] = dmp[off];
       } else {
-        jb[q] = me; d0b[q] = 0.f; m0b[q] = 0.f;
+        jb[q] = me; vb[q] = make_float2(0.f, 0.f);
       }
     }
-    float4 njb[Nb::kGlobal ? B : 1];
-    float rsb[Nb::kGlobal ? B : 1];
-    if constexpr (Nb::kGlobal) {
+    typename Nb::Raw rw[B];
 #pragma unroll
-      for (int q = 0; q < B; q++) { njb[q] = nb.nq[jb[q]]; rsb[q] = nb.aux[jb[q]]; }
-    }
+    for (int q = 0; q < B; q++) rw[q] = nb.raw(jb[q], true, false);
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      if (k0 + q >= L) break;
-      const float4 nj = Nb::kGlobal ? njb[q] : nb.nq[jb[q]];
-      const float rsj = Nb::kGlobal ? rsb[q] : nb.aux[jb[q]];
-      const Recon R = recon(hi, nj.x, dz_of(__fsub_rn(nj.w, etai), hi, nj.x));
-      const float f = fct_entry(d0b[q], m0b[q], fmaxf(resi, rsj), hi, nj.x, R);
+      if (B > 1 && k0 + q >= L) break;
+      const NodeC nj = nb.fct(rw[q], jb[q]);
+      const Recon R = recon(ni.h, nj.h, dz_of(__fsub_rn(nj.eta, ni.eta), ni.h, nj.h));
+      const float f = fct_entry(vb[q].x, vb[q].y, fmaxf(ni.res, nj.res), ni.h, nj.h, R);
       if (f < 0.f) neg = __fadd_rn(neg, f);
     }
   }
@@ -891,27 +1021,30 @@ __global__ void __launch_bounds__(256) k_fct_mix(Graph G, const InstConst* __res
                                                  const float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G.col, u.nq, res, nullptr, nullptr};
+  const NbGlobal nb{G, u.nq, res, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
-    fct_row<B, D>(r, G, C, St, u, dmu, w, res, err, nb);
+    fct_row<B, D>((int)r, row_head(G, r), G, C, St, dmu, w, err, nb);
 }
 
-template <int B, bool D>
-__global__ void __launch_bounds__(256) k_fct_tile(Graph G, const InstConst* __restrict__ C,
-                                                  const InstState* __restrict__ St, StateMix u,
-                                                  const float2* __restrict__ dmu, WorkMix w,
-                                                  const float* __restrict__ res, unsigned* __restrict__ err, TileCtl tc) {
+template <int T, bool D>
+__global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* __restrict__ C,
+                                                const InstState* __restrict__ St, StateMix u,
+                                                const float2* __restrict__ dmu, WorkMix w,
+                                                const float* __restrict__ res, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
-  pdl_trigger();
-  tile_prefetch(G, tc, TilePrefetch{{tc.loc, nullptr, nullptr}, {2, 0, 0}, {G.lumpedf}, {4}});
+  const Tile t = tile_of<T>(G, tc);
+  const TileSmem sm = tile_smem<T, 3, D, false>(tile_mem, tc);
+  cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
-  tile_prefetch(G, tc, TilePrefetch{{dmu, nullptr, nullptr}, {8, 0, 0},
-                                    {D ? (const void*)w.hL64 : (const void*)w.hL}, {8}});
-  const TileSmem sm = tile_smem<false>(tile_mem, tc.tile_rows + tc.halo_cap, tc.tile_rows);
-  const int64_t t0 = stage_tile<true, false>(G, tc, u, res, nullptr, sm);
-  const int64_t t1 = tile_end(G, tc, t0);
-  const NbTile nb{tc.loc, sm.nq, sm.aux, nullptr, nullptr, t0, sm.sp, sm.ln};
-  for (int64_t r = t0 + threadIdx.x; r < t1; r += blockDim.x) fct_row<B, D>(r, G, C, St, u, dmu, w, res, err, nb);
+  cp_range<T>(sm.e8, dmu + t.e0, 8 * t.ne);
+  row_prefetch<T>(G, RowPrefetch{{G.lumpedf, D ? (const void*)w.hL64 : (const void*)w.hL}, {4, 8}});
+  struct Node { float4 n; float res; };
+  stage_nodes<T>(tc, t, [&](int row) { return Node{u.nq[row], res[row]}; },
+                 [&](int i, int, const Node& x) { sm.a[i] = make_float4(x.n.x, x.n.w, x.res, 0.f); });
+  cp_wait();
+  __syncthreads();
+  pdl_trigger();
+  fct_row<1, D>(t.r, t.hd, G, C, St, dmu, w, err, nb_tile(t, sm));
 }
 
 // End of a stage for one row: non-finite check, the SSP-RK combination and
@@ -964,36 +1097,36 @@ __device__ __forceinline__ void finish_mix(const Graph& G, const InstConst& c, c
 // this kernel's antidiffusion with every l_ij = 1, and the rats of the RHS
 // the stage uses (smb_2_roundoff: the htiny tests, the mass row testing
 // only h_i; smb_2: the h <= 0 tests, then MAX(h, 0)).
-template <int B, bool D, class Nb>
-__device__ __forceinline__ void update_row(int64_t r, Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                             StateMix u, const float2* __restrict__ dmu, WorkMix w,
-                             const float* __restrict__ res, StateMix u0, StateMix out, int rk_stage,
-                             unsigned* __restrict__ err, const Nb& nb) {
-  const int L = nb.len(G, r);
+//
+// FCT: every instance runs 'fct'.
+template <int B, bool D, bool FCT, class Nb>
+__device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph& G,
+                                           const InstConst* __restrict__ C, const InstState* __restrict__ St,
+                                           const StateMix& u, const float2* __restrict__ dmu, const WorkMix& w,
+                                           const StateMix& u0, const StateMix& out, int rk_stage,
+                                           unsigned* __restrict__ err, const Nb& nb) {
+  const int L = hd.L;
   if (L == 0) return;
-  const int b = G.slice_inst[r >> 5];
-  const InstState& st = St[b];
+  const InstState& st = St[hd.b];
   if (st.done) return;
-  const InstConst& c = C[b];
+  const InstConst& c = C[hd.b];
   const int S = Nb::kGlobal ? c.S : 3;
   const int me = nb.self(r);
-  const float4 ni = nb.nq[me];
-  const bool ent = c.visc == VISC_ENTROPY;
-  if (c.visc != VISC_FCT && !ent) {             // 'galerkin' / 'viscous': u^L is the result
+  const bool ent = !FCT && c.visc == VISC_ENTROPY;
+  if (!FCT && c.visc != VISC_FCT && !ent) {             // 'galerkin' / 'viscous': u^L is the result
     const float2 qL = w.qL[r];
     finish_mix(G, c, st, r, S, D ? df_from_double(w.hL64[r]) : w.hL[r], qL.x, qL.y, S == 5 ? w.q3L[r] : 0.f,
                S == 5 ? w.q4L[r] : 0.f, rk_stage, u0, out, err);
     return;
   }
-  const int64_t base = nb.base(G, r);
+  const int64_t base = hd.base;
   const auto ip = nb.row_index(base);
-  const float2* dmp = dmu + base;
-  const float hi = ni.x, etai = ni.w, resi = nb.aux[me];
-  const float invhi = inv_pos(hi);
-  const float Ri = ent ? 1.f : nb.R[me];
+  const float2* dmp = nb.dm(dmu, base);
+  const NodeU ni = nb.upd(nb.raw(me, true, !ent), me);
+  const float Ri = ent ? 1.f : ni.R;
   // entropy_visc with the roundoff fix: smb_2_roundoff's h <= htiny tests
   const float hthr = (ent && c.roundoff_fix) ? c.htinyf : 0.f;
-  const bool wet_i = !(hi <= hthr);
+  const bool wet_i = !(ni.h <= hthr);
   float ui3 = 0.f, ui4 = 0.f;
   if (S == 5) { ui3 = u.q3[r]; ui4 = u.q4[r]; }
   float neg = 0.f, pos = 0.f;            // sum_{f < 0} f_ij, sum_{f >= 0} R_j f_ij
@@ -1001,42 +1134,39 @@ __device__ __forceinline__ void update_row(int64_t r, Graph G, const InstConst* 
   float x1 = 0.f, x2 = 0.f, x3 = 0.f, x4 = 0.f;
   for (int k0 = 0; k0 < L; k0 += B) {    // the diagonal's terms vanish: u_i rat_ii - u_i rat_ii = 0
    int jb[B];
-   float d0b[B], m0b[B];
+   float2 vb[B];
 #pragma unroll
    for (int q = 0; q < B; q++) {
-     if (k0 + q < L) {
+     if (B == 1 || k0 + q < L) {
        const int off = 32 * (k0 + q);
-       jb[q] = ip[off]; const float2 v = dmp[off]; d0b[q] = v.x; m0b[q] = v.y;
+       jb[q] = ip[off]; vb[q] = dmp[off];
      } else {
-       jb[q] = me; d0b[q] = 0.f; m0b[q] = 0.f;
+       jb[q] = me; vb[q] = make_float2(0.f, 0.f);
      }
    }
-   float4 njb[Nb::kGlobal ? B : 1];
-   float rsb[Nb::kGlobal ? B : 1], Rjb[Nb::kGlobal ? B : 1];
-   if constexpr (Nb::kGlobal) {
+   typename Nb::Raw rw[B];
 #pragma unroll
-     for (int q = 0; q < B; q++) { njb[q] = nb.nq[jb[q]]; rsb[q] = nb.aux[jb[q]]; Rjb[q] = ent ? 1.f : nb.R[jb[q]]; }
-   }
+   for (int q = 0; q < B; q++) rw[q] = nb.raw(jb[q], true, !ent);
 #pragma unroll
    for (int q = 0; q < B; q++) {
-    if (k0 + q >= L) break;
-    const float4 nj = Nb::kGlobal ? njb[q] : nb.nq[jb[q]];
-    const float d0 = d0b[q], m0 = m0b[q];
-    const float rij = fmaxf(resi, Nb::kGlobal ? rsb[q] : nb.aux[jb[q]]);
+    if (B > 1 && k0 + q >= L) break;
+    const NodeU nj = nb.upd(rw[q], jb[q]);
+    const float d0 = vb[q].x, m0 = vb[q].y;
+    const float rij = fmaxf(ni.res, nj.res);
     const float ddr = fminf(d0, rij) - d0, dmr = fminf(m0, rij) - m0;
-    const float dz = dz_of(__fsub_rn(nj.w, etai), hi, nj.x);
-    Recon R = recon(hi, nj.x, dz);
-    float rij_ = rat_of(R.Hij, hi, dz <= 0.f, invhi);
-    float rji_ = rat_of(R.Hji, nj.x, dz >= 0.f, inv_pos(nj.x));
+    const float dz = dz_of(__fsub_rn(nj.eta, ni.eta), ni.h, nj.h);
+    Recon R = recon(ni.h, nj.h, dz);
+    float rij_ = rat_of(R.Hij, dz <= 0.f, ni.inv, ni.one);
+    float rji_ = rat_of(R.Hji, dz >= 0.f, nj.inv, nj.one);
     if (ent) {           // the rats and the mass row's H*_ij of the stage's RHS
       if (!wet_i) { rij_ = 0.f; R.Hij = 0.f; }
-      if (nj.x <= hthr) rji_ = 0.f;
+      if (nj.h <= hthr) rji_ = 0.f;
     }
-    const float f = fct_from(ddr, dmr, hi, nj.x, R);
+    const float f = fct_from(ddr, dmr, ni.h, nj.h, R);
     float lf = Ri;
     if (f >= 0.f) {
-      lf = ent ? 1.f : (Nb::kGlobal ? Rjb[q] : nb.R[jb[q]]);
-      if (D && !ent) pos64 = fma(nb.R64[jb[q]], (double)f, pos64);
+      lf = ent ? 1.f : nj.R;
+      if (D && !ent) pos64 = fma(nb.r64(jb[q]), (double)f, pos64);
       else pos = __fmaf_rn(lf, f, pos);
     } else {
       neg = __fadd_rn(neg, f);
@@ -1044,8 +1174,8 @@ __device__ __forceinline__ void update_row(int64_t r, Graph G, const InstConst* 
     // l (dd (u_j rat_ji - u_i rat_ij) + dm (u_j (1 - rat_ji) - u_i (1 - rat_ij)))
     // = l (dm (u_j - u_i) + (dd - dm) (u_j rat_ji - u_i rat_ij))
     const float dm = dmr * lf, dx = (ddr - dmr) * lf;
-    x1 = fma_(dx, fma_(nj.y, rji_, -ni.y * rij_), fma_(dm, nj.y - ni.y, x1));
-    x2 = fma_(dx, fma_(nj.z, rji_, -ni.z * rij_), fma_(dm, nj.z - ni.z, x2));
+    x1 = fma_(dx, fma_(nj.q1, rji_, -ni.q1 * rij_), fma_(dm, nj.q1 - ni.q1, x1));
+    x2 = fma_(dx, fma_(nj.q2, rji_, -ni.q2 * rij_), fma_(dm, nj.q2 - ni.q2, x2));
     if constexpr (Nb::kGlobal) {
       if (S == 5) {
         const int j = jb[q];
@@ -1059,7 +1189,7 @@ __device__ __forceinline__ void update_row(int64_t r, Graph G, const InstConst* 
   const float invm = G.inv_lumpedf[r], dtf = st.dtf;
   float2 hn;
   if (D) {       // u^L + dt/m sum l_ij f_ij for the depth, in FP64
-    const double sh = ent ? (double)__fadd_rn(neg, pos) : fma(nb.R64[me], (double)neg, pos64);
+    const double sh = ent ? (double)__fadd_rn(neg, pos) : fma(nb.r64(me), (double)neg, pos64);
     double h64 = fma(st.dt * G.inv_lumped[r], sh, w.hL64[r]);
     if (ent && !c.roundoff_fix && h64 < 0.0) h64 = 0.0;       // smb_2: MAX(h + dt rk, 0)
     hn = df_from_double(h64);
@@ -1084,31 +1214,39 @@ __global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* __
                                                     int rk_stage, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G.col, u.nq, res, w.rminus, w.rminus64};
+  const NbGlobal nb{G, u.nq, res, w.rminus, w.rminus64};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
-    update_row<B, D>(r, G, C, St, u, dmu, w, res, u0, out, rk_stage, err, nb);
+    update_row<B, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, u0, out, rk_stage, err, nb);
 }
 
-template <int B, bool D>
-__global__ void __launch_bounds__(256) k_update_tile(Graph G, const InstConst* __restrict__ C,
-                                                     const InstState* __restrict__ St, StateMix u,
-                                                     const float2* __restrict__ dmu, WorkMix w,
-                                                     const float* __restrict__ res, StateMix u0, StateMix out,
-                                                     int rk_stage, unsigned* __restrict__ err, TileCtl tc) {
+template <int T, bool D, bool FCT>
+__global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* __restrict__ C,
+                                                   const InstState* __restrict__ St, StateMix u,
+                                                   const float2* __restrict__ dmu, WorkMix w,
+                                                   const float* __restrict__ res, StateMix u0, StateMix out,
+                                                   int rk_stage, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
-  pdl_trigger();
-  tile_prefetch(G, tc, TilePrefetch{{tc.loc, nullptr, nullptr}, {2, 0, 0}, {G.inv_lumpedf, G.bathdf}, {4, 8}});
+  const Tile t = tile_of<T>(G, tc);
+  const TileSmem sm = tile_smem<T, 4, D, false>(tile_mem, tc);
+  cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
-  tile_prefetch(G, tc, TilePrefetch{{dmu, nullptr, nullptr}, {8, 0, 0},
-                                    {w.hL, w.qL, rk_stage >= 2 ? (const void*)u0.nq : nullptr,
-                                     rk_stage >= 2 ? (const void*)u0.h : nullptr},
-                                    {8, 8, rk_stage >= 2 ? 16 : 0, rk_stage >= 2 ? 8 : 0}});
-  const TileSmem sm = tile_smem<D>(tile_mem, tc.tile_rows + tc.halo_cap, tc.tile_rows);
-  const int64_t t0 = stage_tile<true, true, D>(G, tc, u, res, w.rminus, sm, w.rminus64);
-  const int64_t t1 = tile_end(G, tc, t0);
-  const NbTile nb{tc.loc, sm.nq, sm.aux, sm.R, sm.R64, t0, sm.sp, sm.ln};
-  for (int64_t r = t0 + threadIdx.x; r < t1; r += blockDim.x)
-    update_row<B, D>(r, G, C, St, u, dmu, w, res, u0, out, rk_stage, err, nb);
+  cp_range<T>(sm.e8, dmu + t.e0, 8 * t.ne);
+  row_prefetch<T>(G, RowPrefetch{{G.inv_lumpedf, G.bathdf, w.hL, w.qL, rk_stage >= 2 ? (const void*)u0.nq : nullptr,
+                                  rk_stage >= 2 ? (const void*)u0.h : nullptr},
+                                 {4, 8, 8, 8, rk_stage >= 2 ? 16 : 0, rk_stage >= 2 ? 8 : 0}});
+  struct Node { float4 n; float res, R; double r64; };
+  stage_nodes<T>(
+      tc, t, [&](int row) { return Node{u.nq[row], res[row], w.rminus[row], D ? w.rminus64[row] : 0.0}; },
+      [&](int i, int, const Node& x) {
+        const NodeU n = node_u(x.n, x.res, x.R);
+        sm.a[i] = x.n;
+        sm.b[i] = make_float4(n.res, n.R, n.inv, n.one);
+        if (D) sm.r64[i] = x.r64;
+      });
+  cp_wait();
+  __syncthreads();
+  pdl_trigger();
+  update_row<1, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, u0, out, rk_stage, err, nb_tile(t, sm));
 }
 
 // One row of k_dt_mix: FP32 lambda_max, |d_ii| / m_i (main.f90:166-174; 0 for
@@ -1117,49 +1255,46 @@ __global__ void __launch_bounds__(256) k_update_tile(Graph G, const InstConst* _
 // reused by stage 1's k_low_mix) and alpha_i (alpha_out, stage 1's
 // k_node_mix), when those are non-null.
 template <int B, class Nb>
-__device__ __forceinline__ float dt_row(int64_t r, const Graph& G, const InstConst* __restrict__ C,
-                                        const InstState* __restrict__ St, const StateMix& u, float* __restrict__ dlam,
+__device__ __forceinline__ float dt_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
+                                        const InstState* __restrict__ St, float* __restrict__ dlam,
                                         float* __restrict__ alpha_out, unsigned* __restrict__ err, const Nb& nb) {
-  if (r >= G.n_rows || nb.len(G, r) == 0) return 0.f;
-  const int b = G.slice_inst[r >> 5];
-  if (St[b].done) return 0.f;
-  const InstConst& c = C[b];
+  const int L = hd.L;
+  if (L == 0) return 0.f;
+  if (St[hd.b].done) return 0.f;
+  const InstConst& c = C[hd.b];
   const float g = c.gf, htiny = c.htinyf;
   const LamK lk = lam_k(g, htiny);
-  const int L = nb.len(G, r);
-  const int64_t base = nb.base(G, r);
+  const int64_t base = hd.base;
   const int me = nb.self(r);
   const auto ip = nb.row_index(base);
-  const float2* cp = G.cf + base;
-  const NodeF ni = node_from(nb.nq[me], htiny);
-  const float sqi = sqrtf(g * fabsf(ni.h));
+  const float2* cp = nb.cf(base);
+  const NodeL ni = nb.dt(nb.raw(me, false, false), me, g, htiny);
   float s = 0.f;
   float num = 0.f, denom = 0.f;          // alpha_limit stencil (as k_node_mix)
   bool bad = false;
   for (int k0 = 0; k0 < L; k0 += B) {
     int jb[B];
-    float cxb[B], cyb[B];
+    float2 cb[B];
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      if (k0 + q < L) {
+      if (B == 1 || k0 + q < L) {
         const int off = 32 * (k0 + q);
-        const float2 cc = cp[off];
-        jb[q] = ip[off]; cxb[q] = cc.x; cyb[q] = cc.y;
+        jb[q] = ip[off]; cb[q] = cp[off];
       } else {
-        jb[q] = me; cxb[q] = 1.f; cyb[q] = 0.f;
+        jb[q] = me; cb[q] = make_float2(1.f, 0.f);
       }
     }
-    float4 njb[B];
+    typename Nb::Raw rw[B];
 #pragma unroll
-    for (int q = 0; q < B; q++) njb[q] = nb.nq[jb[q]];
+    for (int q = 0; q < B; q++) rw[q] = nb.raw(jb[q], false, false);
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      if (k0 + q >= L) break;
-      const NodeF nj = node_from(njb[q], htiny);
-      const float cxe = cxb[q], cye = cyb[q];
+      if (B > 1 && k0 + q >= L) break;
+      const NodeL nj = nb.dt(rw[q], jb[q], g, htiny);
+      const float cxe = cb[q].x, cye = cb[q].y;
       float dl;
       if (!dlam_f(cxe, cye, dotc(cxe, cye, ni.v1, ni.v2), dotc(cxe, cye, nj.v1, nj.v2), ni.h, nj.h, ni.ovh, nj.ovh,
-                  sqi, sqrtf(g * fabsf(nj.h)), lk, &dl))
+                  ni.sq, nj.sq, lk, &dl))
         bad = true;
       if (dlam) dlam[base + 32 * (k0 + q)] = dl;
       s += dl;
@@ -1192,30 +1327,35 @@ __global__ void __launch_bounds__(256) k_dt_mix(Graph G, const InstConst* __rest
   pdl_wait();
   // grid-stride over block-sized row ranges: every lane of a warp runs the
   // same iterations (the warp reduction needs all 32)
-  const NbGlobal nb{G.col, u.nq, nullptr, nullptr, nullptr};
+  const NbGlobal nb{G, u.nq, nullptr, nullptr, nullptr};
   for (int64_t rb = blockIdx.x * (int64_t)blockDim.x; rb < G.n_rows; rb += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = rb + threadIdx.x;
-    dt_reduce(dt_row<B>(r, G, C, St, u, dlam, alpha_out, err, nb), r, G, St);
+    dt_reduce(r < G.n_rows ? dt_row<B>((int)r, row_head(G, r), G, C, St, dlam, alpha_out, err, nb) : 0.f, r, G, St);
   }
 }
 
-template <int B>
-__global__ void __launch_bounds__(256) k_dt_tile(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St,
-                                                 StateMix u, float* __restrict__ dlam, float* __restrict__ alpha_out,
-                                                 unsigned* __restrict__ err, TileCtl tc) {
+template <int T>
+__global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St,
+                                               StateMix u, float* __restrict__ dlam, float* __restrict__ alpha_out,
+                                               unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
-  pdl_trigger();
-  tile_prefetch(G, tc, TilePrefetch{{tc.loc, G.cf, nullptr}, {2, 8, 0}, {G.inv_lumpedf}, {4}});
+  const Tile t = tile_of<T>(G, tc);
+  const TileSmem sm = tile_smem<T, 0, false, false>(tile_mem, tc);
+  cp_range<T>(sm.e8, G.cf + t.e0, 8 * t.ne);
+  cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
-  const TileSmem sm = tile_smem<false>(tile_mem, tc.tile_rows + tc.halo_cap, tc.tile_rows);
-  const int64_t t0 = stage_tile<false, false>(G, tc, u, nullptr, nullptr, sm);
-  const NbTile nb{tc.loc, sm.nq, nullptr, nullptr, nullptr, t0, sm.sp, sm.ln};
-  // tile_rows is a multiple of 32: every lane of a warp runs the same iterations
-  for (int64_t rb = t0; rb < t0 + tc.tile_rows; rb += blockDim.x) {
-    const int64_t r = rb + threadIdx.x;
-    if (rb - t0 + (int64_t)threadIdx.x - (threadIdx.x & 31) >= tc.tile_rows) break;   // warp past the tile
-    dt_reduce(dt_row<B>(r, G, C, St, u, dlam, alpha_out, err, nb), r, G, St);
-  }
+  row_prefetch<T>(G, RowPrefetch{{G.inv_lumpedf}, {4}});
+  stage_nodes<T>(tc, t, [&](int row) { return u.nq[row]; },
+                 [&](int i, int row, float4 x) {
+                   const InstConst& c = inst_of(G, C, row);
+                   const NodeL n = node_l(x, c.gf, c.htinyf);
+                   sm.a[i] = make_float4(n.h, n.v1, n.v2, n.sq);
+                   sm.o[i] = n.ovh;
+                 });
+  cp_wait();
+  __syncthreads();
+  pdl_trigger();
+  dt_reduce(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile(t, sm)), t.r, G, St);
 }
 
 // Free surface of the packed node records after a bathymetry change
@@ -1294,37 +1434,36 @@ static unsigned row_grid(K kern, int64_t n, int block, int mode) {
     default: launch_k(KERNEL<1, D>, row_grid(KERNEL<1, D>, N, BS, MODE), BS, 0, s, __VA_ARGS__); break;        \
   }
 
-// Tile variants: one block per tile, shared memory for the tile's and the
-// halo's node records, residuals and R^- (24 B per row; 32 B with the FP64
-// R^- of the precision split)
-size_t tile_smem_bytes(const TileCtl& tc, bool d) {
-  const size_t cap = tc.tile_rows + tc.halo_cap;
-  return cap * (d ? 32 : 24) + (size_t)tc.tile_rows / 32 * 8 + tc.tile_rows;
+// Tile variants: one block per tile
+size_t tile_smem_bytes(const TileCtl& tc, int kind, bool d, bool lamin) {
+  const TileParts P = tile_parts(kind, d, lamin);
+  const size_t cap = tc.tile_rows + tc.halo_cap, ec = tc.ent_cap;
+  return cap * (P.a + P.b + P.c + P.o + P.r64) + ec * (P.e8 + P.e4 + 2);
 }
-#define SWE_DISPATCH_TILE(b, KERNEL, BS, TC, NROWS, ...)                                                \
-  do {                                                                                                \
-    const TileCtl& tc_ = (TC);                                                                        \
-    const unsigned g_ = (unsigned)(((NROWS) + tc_.tile_rows - 1) / tc_.tile_rows);                    \
-    const size_t sm_ = tile_smem_bytes(tc_);                                                          \
-    switch (b) {                                                                                      \
-      case 8: launch_k(KERNEL<8>, g_, BS, sm_, s, __VA_ARGS__); break;                                \
-      case 4: launch_k(KERNEL<4>, g_, BS, sm_, s, __VA_ARGS__); break;                                \
-      case 2: launch_k(KERNEL<2>, g_, BS, sm_, s, __VA_ARGS__); break;                                \
-      default: launch_k(KERNEL<1>, g_, BS, sm_, s, __VA_ARGS__); break;                               \
-    }                                                                                                 \
-  } while (0)
-#define SWE_DISPATCH_TILE_D(b, KERNEL, BS, TC, NROWS, D, SMEM, ...)                                     \
-  do {                                                                                                \
-    const TileCtl& tc_ = (TC);                                                                        \
-    const unsigned g_ = (unsigned)(((NROWS) + tc_.tile_rows - 1) / tc_.tile_rows);                    \
-    const size_t sm_ = (SMEM);                                                                        \
-    switch (b) {                                                                                      \
-      case 8: launch_k(KERNEL<8, D>, g_, BS, sm_, s, __VA_ARGS__); break;                             \
-      case 4: launch_k(KERNEL<4, D>, g_, BS, sm_, s, __VA_ARGS__); break;                             \
-      case 2: launch_k(KERNEL<2, D>, g_, BS, sm_, s, __VA_ARGS__); break;                             \
-      default: launch_k(KERNEL<1, D>, g_, BS, sm_, s, __VA_ARGS__); break;                            \
-    }                                                                                                 \
-  } while (0)
+size_t tile_smem_max(const TileCtl& tc, bool d) {
+  size_t m = 0;
+  for (int kind = 0; kind < 5; kind++)
+    for (int lamin = 0; lamin < 2; lamin++) {
+      const size_t b = tile_smem_bytes(tc, kind, d, lamin != 0);
+      m = b > m ? b : m;
+    }
+  return m;
+}
+template <typename... KArgs, typename... Args>
+static void launch_tile(void (*kern)(KArgs...), const TileCtl& tc, int64_t n_rows, int kind, bool d, bool lamin,
+                        cudaStream_t s, Args... args) {
+  const size_t sm = tile_smem_bytes(tc, kind, d, lamin);
+  if (sm > 48 * 1024)    // above the default limit; the attribute only ever grows a kernel's allowance
+    cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+  launch_k(kern, (unsigned)((n_rows + tc.tile_rows - 1) / tc.tile_rows), tc.tile_rows, sm, s, args..., tc);
+}
+// KERNEL<T, ...> for the tile sizes that are built
+#define SWE_TILE_T(TC, CALL)                     \
+  switch ((TC).tile_rows) {                      \
+    case 64: { constexpr int T = 64; CALL; break; }   \
+    case 128: { constexpr int T = 128; CALL; break; } \
+    default: { constexpr int T = 256; CALL; break; }  \
+  }
 
 // k_low variants: entry batch 1 or 2, lambda_max computed or taken from
 // k_dt_mix (stage 1), registers capped at 85, 64 or 51 (3, 4 or 5 resident
@@ -1332,14 +1471,13 @@ size_t tile_smem_bytes(const TileCtl& tc, bool d) {
 template <bool LAMIN, bool D>
 static void launch_low(const StageArgsMix& a, int batch, int cap, int mode, int block, bool tiled, cudaStream_t s) {
   if (tiled && a.tiles) {
-    const TileCtl& tc = *a.tiles;
-    const unsigned g = (unsigned)((a.G.n_rows + tc.tile_rows - 1) / tc.tile_rows);
-    const size_t sm = tile_smem_bytes(tc);
-#define SWE_LOWT(BB, MB) \
-    launch_k(k_low_tile<BB, LAMIN, MB, D>, g, block, sm, s, a.G, a.C, a.St, a.u, a.w.alpha, a.w.dmu, a.w, a.w.res, \
-             a.err, tc)
-    if (batch >= 2) { if (cap == 2) SWE_LOWT(2, 5); else if (cap) SWE_LOWT(2, 4); else SWE_LOWT(2, 3); }
-    else { if (cap == 2) SWE_LOWT(1, 5); else if (cap) SWE_LOWT(1, 4); else SWE_LOWT(1, 3); }
+#define SWE_LOWT(TT, MB, F)                                                                                        \
+    launch_tile(k_low_tile<TT, LAMIN, MB, D, F>, *a.tiles, a.G.n_rows, 2, D, LAMIN, s, a.G, a.C, a.St, a.u, a.w.alpha, \
+                a.w.dmu, a.w, a.w.res, a.err)
+    if (a.tiles->tile_rows == 64) SWE_LOWT(64, 3, false);
+    else if (a.tiles->tile_rows == 128) SWE_LOWT(128, 3, false);
+    else if (a.fct) { if (cap) SWE_LOWT(256, 4, true); else SWE_LOWT(256, 3, true); }
+    else { if (cap) SWE_LOWT(256, 4, false); else SWE_LOWT(256, 3, false); }
 #undef SWE_LOWT
     return;
   }
@@ -1358,7 +1496,7 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
   const int64_t n = a.G.n_rows;
   switch (kind) {
     case 1: if (t.tiled[1] && a.tiles) {
-              SWE_DISPATCH_TILE(t.batch[1], k_node_tile, t.block[1], *a.tiles, n, a.G, a.C, a.St, a.u, a.w.alpha, *a.tiles);
+              SWE_TILE_T(*a.tiles, launch_tile(k_node_tile<T>, *a.tiles, n, 1, D, false, s, a.G, a.C, a.St, a.u, a.w.alpha));
             } else {
               SWE_DISPATCH_B(t.batch[1], k_node_mix, n, t.block[1], t.grid[1], a.G, a.C, a.St, a.u, a.w.alpha)
             }
@@ -1372,16 +1510,20 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
               launch_low<false, D>(a, t.batch[2], t.cap_low, t.grid[2], t.block[2], t.tiled[2], s);
             break;
     case 3: if (t.tiled[3] && a.tiles) {
-              SWE_DISPATCH_TILE_D(t.batch[3], k_fct_tile, t.block[3], *a.tiles, n, D, tile_smem_bytes(*a.tiles), a.G, a.C, a.St, a.u, a.w.dmu, a.w,
-                                  a.w.res, a.err, *a.tiles);
+              SWE_TILE_T(*a.tiles, launch_tile(k_fct_tile<T, D>, *a.tiles, n, 3, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu,
+                                               a.w, a.w.res, a.err));
             } else {
               SWE_DISPATCH_BD(t.batch[3], k_fct_mix, D, n, t.block[3], t.grid[3], a.G, a.C, a.St, a.u, a.w.dmu, a.w,
                               a.w.res, a.err)
             }
             break;
     case 4: if (t.tiled[4] && a.tiles) {
-              SWE_DISPATCH_TILE_D(t.batch[4], k_update_tile, t.block[4], *a.tiles, n, D, tile_smem_bytes(*a.tiles, D), a.G, a.C, a.St, a.u,
-                                  a.w.dmu, a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err, *a.tiles);
+              if (a.fct && a.tiles->tile_rows == 256)
+                launch_tile(k_update_tile<256, D, true>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu, a.w,
+                            a.w.res, a.u0, a.out, a.rk_stage, a.err);
+              else
+                SWE_TILE_T(*a.tiles, launch_tile(k_update_tile<T, D, false>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St,
+                                                 a.u, a.w.dmu, a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err));
             } else {
               SWE_DISPATCH_BD(t.batch[4], k_update_mix, D, n, t.block[4], t.grid[4], a.G, a.C, a.St, a.u, a.w.dmu,
                               a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err)
@@ -1408,7 +1550,7 @@ void launch_stage_mix(const StageArgsMix& a, cudaStream_t s, const KernelEvents*
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,
                    unsigned* err, const KernelTune& t, const TileCtl* tiles, cudaStream_t s) {
   if (t.tiled[0] && tiles) {
-    SWE_DISPATCH_TILE(t.batch[0], k_dt_tile, t.block[0], *tiles, G.n_rows, G, C, St, u, dlam, alpha, err, *tiles);
+    SWE_TILE_T(*tiles, launch_tile(k_dt_tile<T>, *tiles, G.n_rows, 0, false, false, s, G, C, St, u, dlam, alpha, err));
   } else {
     SWE_DISPATCH_B(t.batch[0], k_dt_mix, G.n_rows, t.block[0], t.grid[0], G, C, St, u, dlam, alpha, err)
   }

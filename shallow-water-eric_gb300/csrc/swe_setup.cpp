@@ -285,6 +285,7 @@ bool build_row_tiles(const Layout& L, int tile, RowTiles& F) {
     std::sort(h.begin(), h.end());
     h.erase(std::unique(h.begin(), h.end()), h.end());
     if (tile + (int64_t)h.size() > 32767) ok = false;
+    if (L.slice_ptr[(r1 + 31) >> 5] - L.slice_ptr[r0 >> 5] > 65535) ok = false;
     for (int64_t r = r0; r < r1; r++) {
       const int64_t base = L.slice_ptr[r >> 5] + (r & 31);
       for (int k = 0; k < L.len[r]; k++) {
@@ -296,8 +297,10 @@ bool build_row_tiles(const Layout& L, int tile, RowTiles& F) {
     }
   }
   if (!ok) return false;
-  F.halo_cap = 0;
+  F.halo_cap = F.ent_cap = 0;
   for (int64_t t = 0; t < n_tiles; t++) {
+    const int64_t r0 = t * tile, r1 = std::min<int64_t>(r0 + tile, L.n_rows);
+    F.ent_cap = std::max(F.ent_cap, (int)(L.slice_ptr[(r1 + 31) >> 5] - L.slice_ptr[r0 >> 5]));
     F.halo_ptr[t + 1] = F.halo_ptr[t] + (int)halo[t].size();
     F.halo_cap = std::max(F.halo_cap, (int)halo[t].size());
   }

@@ -89,10 +89,12 @@ Layout build_layout(const std::vector<HostMesh>& meshes, const std::vector<std::
 // the rows outside tile t that its entries reference; loc[e] is the column's
 // position in the tile's shared-memory arrays: col - tile start for rows of
 // the tile, tile + (index in the halo list) for halo rows, 0 for padding
-// entries.  Returns false when a tile would need more than 32767 positions.
+// entries.  Returns false when a tile would need more than 32767 positions or
+// hold more than 65535 entries.
 struct RowTiles {
   int tile = 0;
   int halo_cap = 0;
+  int ent_cap = 0;                       // most entries of a tile
   std::vector<int16_t> loc;
   std::vector<int> halo_ptr, halo_rows;
 };
