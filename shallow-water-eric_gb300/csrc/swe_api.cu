@@ -73,6 +73,16 @@ struct swe_ctx {
   StateF64 A{}, B{}, Cs{};
   WorkF64 w{};
   double* d_lij = nullptr;
+  // per-call operators (swe_euler, swe_compute_dij): their own instance state,
+  // so that the time loop's is neither saved nor restored
+  InstState* d_St_call = nullptr;
+  // page-locked: the instance states and the error word that a call reads back
+  InstState* h_St = nullptr;
+  unsigned* h_err = nullptr;
+  double* d_times = nullptr;             // swe_set_time: time and t_final per instance
+  int* d_ref_pos = nullptr;              // per entry / per row: CSR position in its instance or -1 (on first use)
+  int* d_ref_pos_diag = nullptr;
+  double* d_csr = nullptr;               // one instance's entries in CSR order
   // mixed path
   StateMix mA{}, mB{}, mC{};
   WorkMix wm{};
@@ -335,6 +345,16 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
   }
   c->d_C = upload_vec(c, hc, st);
   c->d_St = upload_vec(c, hs, st);
+  c->d_St_call = upload_vec(c, hs, st);
+  c->d_times = c->buf.alloc<double>(2 * (size_t)c->n_inst, st);
+  if (st == cudaSuccess) {
+    void* h = nullptr;
+    st = cudaMallocHost(&h, sizeof(InstState) * c->n_inst + sizeof(unsigned));
+    if (st == cudaSuccess) {
+      c->h_St = static_cast<InstState*>(h);
+      c->h_err = reinterpret_cast<unsigned*>(c->h_St + c->n_inst);
+    }
+  }
   c->d_err = c->buf.alloc<unsigned>(1, st);
   // host node -> device row map, staging buffer
   c->node_off.assign(c->n_inst + 1, 0);
@@ -473,6 +493,13 @@ __global__ void k_gather_out_mix(double* __restrict__ stage, const int* __restri
 // Node ranges of the transfer chunks: k of `chunks` equal parts of [b, e).
 static inline int64_t chunk_at(int64_t b, int64_t e, int k, int chunks) { return b + (e - b) * k / chunks; }
 
+// Chunks of a transfer of nn nodes: the copy streams pay for several copy
+// engines and for the overlap of copies and permutations only above some MB;
+// below, one copy on the context's stream (two API calls instead of twenty).
+static inline int chunks_of(const swe_ctx* c, int64_t nn) {
+  return nn * c->S * (int64_t)sizeof(double) >= (int64_t)4 << 20 ? c->copy_chunks : 1;
+}
+
 // Copy streams and events on first use (SWE_COPY_CHUNKS, default 4, 1..8).
 static int copy_setup(swe_ctx* c) {
   if (c->copy_chunks) return SWE_OK;
@@ -501,21 +528,25 @@ static int to_device(swe_ctx* c, const double* un, bool device_src, int64_t node
   if (nn <= 0) return SWE_OK;
   int rc = copy_setup(c);
   if (rc) return rc;
-  const int K = nn >= 1024 ? c->copy_chunks : 1;
+  const int K = chunks_of(c, nn);
+  const cudaMemcpyKind how = device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   // chunk k: copy on copy_stream[k] (after the work already on `stream`),
   // then its permutation into the rows on `stream` once it has landed
-  CK(cudaEventRecord(c->copy_go, c->stream));
-  for (int k = 0; k < K; k++) {
+  if (K == 1) {
+    CK(cudaMemcpyAsync(c->d_stage + (size_t)c->S * node_begin, un, (size_t)c->S * nn * sizeof(double), how, c->stream));
+  } else {
+    CK(cudaEventRecord(c->copy_go, c->stream));
+  }
+  for (int k = 0; k < K && K > 1; k++) {
     const int64_t b = chunk_at(node_begin, node_end, k, K), e = chunk_at(node_begin, node_end, k + 1, K);
     CK(cudaStreamWaitEvent(c->copy_stream[k], c->copy_go, 0));
     CK(cudaMemcpyAsync(c->d_stage + (size_t)c->S * b, un + (size_t)c->S * (b - node_begin),
-                       (size_t)c->S * (e - b) * sizeof(double),
-                       device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->copy_stream[k]));
+                       (size_t)c->S * (e - b) * sizeof(double), how, c->copy_stream[k]));
     CK(cudaEventRecord(c->copy_ev[k], c->copy_stream[k]));
   }
   for (int k = 0; k < K; k++) {
     const int64_t b = chunk_at(node_begin, node_end, k, K), e = chunk_at(node_begin, node_end, k + 1, K);
-    CK(cudaStreamWaitEvent(c->stream, c->copy_ev[k], 0));
+    if (K > 1) CK(cudaStreamWaitEvent(c->stream, c->copy_ev[k], 0));
     const unsigned nb = (unsigned)((e - b + 255) / 256);
     if (nb == 0) continue;
     if (c->precision == SWE_PREC_FP64)
@@ -534,7 +565,7 @@ static int from_device_state(swe_ctx* c, double* un, bool device_dst, int64_t no
   if (nn <= 0) return SWE_OK;
   int rc = copy_setup(c);
   if (rc) return rc;
-  const int K = nn >= 1024 ? c->copy_chunks : 1;
+  const int K = chunks_of(c, nn);
   // chunk k: gathered into reference order on `stream`, then copied out on
   // copy_stream[k] while the next chunk is gathered; `stream` waits for every
   // copy, so the caller's synchronisation on it covers the transfer
@@ -548,12 +579,15 @@ static int from_device_state(swe_ctx* c, double* un, bool device_dst, int64_t no
                                                         c->wm, low_mix ? 1 : 0);
       CK(cudaGetLastError());
     }
-    CK(cudaEventRecord(c->copy_ev[k], c->stream));
-    CK(cudaStreamWaitEvent(c->copy_stream[k], c->copy_ev[k], 0));
+    if (K > 1) {
+      CK(cudaEventRecord(c->copy_ev[k], c->stream));
+      CK(cudaStreamWaitEvent(c->copy_stream[k], c->copy_ev[k], 0));
+    }
     CK(cudaMemcpyAsync(un + (size_t)c->S * (b - node_begin), stg, (size_t)c->S * (e - b) * sizeof(double),
-                       device_dst ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c->copy_stream[k]));
+                       device_dst ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                       K > 1 ? c->copy_stream[k] : c->stream));
   }
-  for (int k = 0; k < K; k++) {
+  for (int k = 0; k < K && K > 1; k++) {
     CK(cudaEventRecord(c->copy_ev[k], c->copy_stream[k]));
     CK(cudaStreamWaitEvent(c->stream, c->copy_ev[k], 0));
   }
@@ -615,10 +649,8 @@ __global__ void k_frame_fields(const int* __restrict__ row_of_node, int64_t n_no
 static int frames_wait(swe_ctx* c);
 static void free_gauges(swe_ctx* c);
 
-static int read_errors(swe_ctx* c) {
-  unsigned e = 0;
-  CK(cudaMemcpyAsync(&e, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+// The status of an error word that has been read back; clears the device's.
+static int error_status(swe_ctx* c, unsigned e) {
   if (e) CK(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
   if (e & ERRB_NAN) return fail(c, SWE_ERR_NAN, "non-finite state produced");
   if (e & ERRB_DELTA) return fail(c, SWE_ERR_DELTA, "BUG in compute_lambda_vacc: Delta < 0");
@@ -626,16 +658,35 @@ static int read_errors(swe_ctx* c) {
   return SWE_OK;
 }
 
-static int set_inst_state_dt(swe_ctx* c, int inst, double dt, int done_others) {
-  std::vector<InstState> hs(c->n_inst);
-  CK(cudaMemcpyAsync(hs.data(), c->d_St, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
+static int read_errors(swe_ctx* c) {
+  unsigned e = 0;
+  CK(cudaMemcpyAsync(&e, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  for (int b = 0; b < c->n_inst; b++) {
-    if (b == inst) { inst_set_dt(hs[b], dt); hs[b].done = 0; }
-    else if (done_others) hs[b].done = 1;
-  }
-  CK(cudaMemcpyAsync(c->d_St, hs.data(), sizeof(InstState) * c->n_inst, cudaMemcpyHostToDevice, c->stream));
-  return SWE_OK;
+  return error_status(c, e);
+}
+
+// Instance state of a per-call operator: instance inst steps with dt, the
+// others are done.
+__global__ void k_call_state(InstState* __restrict__ St, int n_inst, int inst, double dt) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n_inst) return;
+  InstState s{};
+  s.t_final = 1e300;
+  s.done = b != inst;
+  inst_set_dt(s, dt);
+  St[b] = s;
+}
+static int call_begin(swe_ctx* c, int inst, double dt) {
+  k_call_state<<<(c->n_inst + 127) / 128, 128, 0, c->stream>>>(c->d_St_call, c->n_inst, inst, dt);
+  return cuda_check(c, cudaGetLastError(), "call state");
+}
+// What a per-call operator reads back (the instance's state, the error word),
+// with the stream's one synchronisation.
+static int call_end(swe_ctx* c, int inst) {
+  CK(cudaMemcpyAsync(c->h_St + inst, c->d_St_call + inst, sizeof(InstState), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return error_status(c, *c->h_err);
 }
 
 static int restore_done(swe_ctx* c, const std::vector<InstState>& saved) {
@@ -827,11 +878,29 @@ SWE_API void swe_destroy(swe_ctx* c) {
   }
   if (c->copy_go) cudaEventDestroy(c->copy_go);
   c->buf.release();
+  if (c->h_St) cudaFreeHost(c->h_St);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
 
 SWE_API const char* swe_last_error(const swe_ctx* c) { return c ? c->err.c_str() : "null context"; }
+
+// Parameters and instance times are written by kernels on the context's
+// stream: no copy of the instance states to the host and back.
+__global__ void k_set_params(InstConst* __restrict__ C, InstConst k, InstState* __restrict__ St, double dt) {
+  *C = k;
+  inst_set_dt(*St, dt);
+}
+__global__ void k_set_time(InstState* __restrict__ St, int n_inst, const double* __restrict__ t,
+                           const double* __restrict__ tf) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n_inst) return;
+  if (t) St[b].time = t[b];
+  if (tf) St[b].t_final = tf[b];
+  St[b].done = 0;
+  St[b].steps = 0;
+  St[b].maxd_bits = 0ull;
+}
 
 SWE_API int swe_set_params(swe_ctx* c, int inst, const swe_params* p) {
   if (!c || !p || inst < 0 || inst >= c->n_inst) return fail(c, SWE_ERR_ARG, "bad instance or params");
@@ -844,12 +913,8 @@ SWE_API int swe_set_params(swe_ctx* c, int inst, const swe_params* p) {
       was.if_roundoff_fix != p->if_roundoff_fix || was.if_alpha_limit != p->if_alpha_limit)
     drop_graphs(c);                                  // the captured kernels follow the modes
   c->params[inst] = *p;
-  InstConst k = make_const(*p);
-  CK(cudaMemcpyAsync(c->d_C + inst, &k, sizeof(InstConst), cudaMemcpyHostToDevice, c->stream));
-  std::vector<InstState> hs;
-  if ((rc = save_state(c, hs))) return rc;
-  inst_set_dt(hs[inst], p->dt);
-  return restore_done(c, hs);
+  k_set_params<<<1, 1, 0, c->stream>>>(c->d_C + inst, make_const(*p), c->d_St + inst, p->dt);
+  return cuda_check(c, cudaGetLastError(), "set_params");
 }
 
 SWE_API int swe_set_bath(swe_ctx* c, int inst, const double* bath) {
@@ -965,28 +1030,52 @@ SWE_API int swe_get_matrices(swe_ctx* c, int inst, int* ia, int* ja, double* mas
   return SWE_OK;
 }
 
-// copy a per-entry device array of one instance back into CSR order; the
-// diagonal positions come from a per-row device array (or are 0 if null)
-template <typename T> static double comp_of(const T& v, int) { return (double)v; }
-static double comp_of(const float2& v, int k) { return (double)(k ? v.y : v.x); }
+template <typename T> __device__ static double comp_of(const T& v, int) { return (double)v; }
+__device__ static double comp_of(const float2& v, int k) { return (double)(k ? v.y : v.x); }
+
+// Per-entry values of one instance in CSR order: the SELL entries and the
+// rows' diagonals (0 if null) scattered on the device, one copy to the host.
+// The permutation of nnz values on one host core took three quarters of
+// swe_compute_dij at 50k nodes.
+template <typename T, typename U>
+__global__ void k_entries_to_csr(const T* __restrict__ ent, const U* __restrict__ diag, const int* __restrict__ pos,
+                                 const int* __restrict__ pos_diag, int64_t e0, int64_t e1, int64_t r0, int64_t r1,
+                                 int comp, double* __restrict__ out) {
+  const int64_t n = (e1 - e0) + (r1 - r0);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (i < e1 - e0) {
+      const int p = pos[e0 + i];
+      if (p >= 0) out[p] = comp_of(ent[e0 + i], comp);
+    } else {
+      const int64_t r = r0 + i - (e1 - e0);
+      const int p = pos_diag[r];
+      if (p >= 0) out[p] = diag ? (double)diag[r] : 0.0;
+    }
+  }
+}
 
 template <typename T, typename U = T>
 static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, const U* d_diag_rows = nullptr,
                           int comp = 0) {
   const Layout& L = c->L;
+  if (!c->d_csr) {                                   // on first use
+    std::vector<int> pos(L.ref_pos.begin(), L.ref_pos.end()), pd(L.ref_pos_diag.begin(), L.ref_pos_diag.end());
+    size_t most = 0;
+    for (const HostMesh& m : c->meshes) most = std::max(most, m.ja.size());
+    cudaError_t st = cudaSuccess;
+    c->d_ref_pos = upload_vec(c, pos, st);
+    c->d_ref_pos_diag = upload_vec(c, pd, st);
+    double* csr = c->buf.alloc<double>(most, st);
+    if (st != cudaSuccess) return cuda_check(c, st, "device allocation");
+    c->d_csr = csr;
+  }
   const int64_t s0 = L.row_off[inst] / 32, s1 = L.row_off[inst + 1] / 32;
-  const int64_t e0 = L.slice_ptr[s0], e1 = L.slice_ptr[s1];
-  std::vector<T> h(e1 - e0);
-  CK(cudaMemcpyAsync(h.data(), d_arr + e0, (e1 - e0) * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
-  const int64_t r0 = L.row_off[inst], r1 = L.row_off[inst + 1];
-  std::vector<U> hd(r1 - r0, U(0));
-  if (d_diag_rows)
-    CK(cudaMemcpyAsync(hd.data(), d_diag_rows + r0, (r1 - r0) * sizeof(U), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  for (int64_t e = e0; e < e1; e++)
-    if (L.ref_pos[e] >= 0) out[L.ref_pos[e]] = comp_of(h[e - e0], comp);
-  for (int64_t r = r0; r < r1; r++)
-    if (L.ref_pos_diag[r] >= 0) out[L.ref_pos_diag[r]] = (double)hd[r - r0];
+  const int64_t e0 = L.slice_ptr[s0], e1 = L.slice_ptr[s1], r0 = L.row_off[inst], r1 = L.row_off[inst + 1];
+  const int64_t nb = std::min<int64_t>(((e1 - e0) + (r1 - r0) + 255) / 256, 152 * 16);
+  k_entries_to_csr<T, U><<<(unsigned)nb, 256, 0, c->stream>>>(d_arr, d_diag_rows, c->d_ref_pos, c->d_ref_pos_diag, e0, e1,
+                                                              r0, r1, comp, c->d_csr);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(out, c->d_csr, c->meshes[inst].ja.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   return SWE_OK;
 }
 
@@ -1005,24 +1094,23 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
   if (!c || inst < 0 || inst >= c->n_inst || !un) return fail(c, SWE_ERR_ARG, "bad arguments");
   if (c->precision != SWE_PREC_FP64) return fail(c, SWE_ERR_ARG, "swe_compute_dij is an FP64 operator");
   int rc = to_device(c, un, false, c->node_off[inst], c->node_off[inst + 1]);
+  if (!rc) rc = call_begin(c, inst, c->params[inst].dt > 0 ? c->params[inst].dt : 1.0);
+  if (!rc) {
+    StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
+    a.w.alpha = nullptr;                             // the last euler call's alpha stays readable
+    launch_node_f64(a, c->stream);
+    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, c->stream);
+    rc = cuda_check(c, cudaGetLastError(), "compute_dij");
+  }
+  if (!rc) rc = call_end(c, inst);                   // nothing is written to the caller's arrays on an error
   if (rc) { drain(c); return rc; }
-  std::vector<InstState> saved;
-  if ((rc = save_state(c, saved))) return rc;
-  if ((rc = set_inst_state_dt(c, inst, c->params[inst].dt > 0 ? c->params[inst].dt : 1.0, 1))) return rc;
-  StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
-  a.w.alpha = nullptr;                               // the last euler call's alpha stays readable
-  launch_node_f64(a, c->stream);
-  launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, c->stream);
-  CK(cudaGetLastError());
-  if ((rc = read_errors(c))) { restore_done(c, saved); return rc; }
-  std::vector<double> d(c->meshes[inst].ja.size());
-  if ((rc = entries_to_csr(c, inst, c->w.dL, d.data(), c->w.dLii))) return rc;
-  if ((rc = restore_done(c, saved))) return rc;
-  if (dij) std::copy(d.begin(), d.end(), dij);
-  if (dt_out) {
-    const HostMesh& m = c->meshes[inst];
-    double mx = std::fabs(d[m.diag[0]]) / m.lumped[0];
-    for (int i = 1; i < m.np; i++) mx = std::max(mx, std::fabs(d[m.diag[i]]) / m.lumped[i]);
+  if (dij) {
+    if ((rc = entries_to_csr(c, inst, c->w.dL, dij, c->w.dLii))) { drain(c); return rc; }
+    CK(cudaStreamSynchronize(c->stream));
+  }
+  if (dt_out) {                                      // COMPUTE_DT: CFL / max |d_ii| / m_i, the maximum from k_dt
+    double mx;
+    std::memcpy(&mx, &c->h_St[inst].maxd_bits, sizeof mx);
     *dt_out = c->params[inst].cfl * 1 / mx;
   }
   return SWE_OK;
@@ -1033,37 +1121,32 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
   if (!c || inst < 0 || inst >= c->n_inst || !un || !unext) return fail(c, SWE_ERR_ARG, "bad arguments");
   if (!(c->params[inst].dt > 0)) return fail(c, SWE_ERR_ARG, "params.dt must be > 0 for swe_euler");
   int rc = to_device(c, un, false, c->node_off[inst], c->node_off[inst + 1]);
+  if (!rc) rc = call_begin(c, inst, c->params[inst].dt);
   if (rc) { drain(c); return rc; }
-  std::vector<InstState> saved;
-  if ((rc = save_state(c, saved))) return rc;
-  if ((rc = set_inst_state_dt(c, inst, c->params[inst].dt, 1))) return rc;
   if (c->precision == SWE_PREC_FP64) {
-    StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
+    StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
     a.fused = all_fct(c);
     a.S = c->S;
     launch_stage_f64(a, c->stream);
   } else {
-    StageArgsMix a{c->G, c->d_C, c->d_St, c->mA, c->mA, c->mB, c->wm, 0, c->d_err, c->block};
+    StageArgsMix a{c->G, c->d_C, c->d_St_call, c->mA, c->mA, c->mB, c->wm, 0, c->d_err, c->block};
     a.tiles = c->tiles_ok ? &c->tiles : nullptr;
     a.f64 = is_split(c);
     a.type1 = has_type1(c);
     a.fct = all_fct_limited(c);
     launch_stage_mix(a, c->stream, nullptr, c->tune);
   }
-  CK(cudaGetLastError());
-  int erc = read_errors(c);
-  if ((rc = restore_done(c, saved))) return rc;
-  c->euler_done = true;
-  c->euler_inst = inst;
-  if ((rc = from_device_state(c, unext, false, c->node_off[inst], c->node_off[inst + 1],
+  if ((rc = cuda_check(c, cudaGetLastError(), "euler")) ||
+      (rc = from_device_state(c, unext, false, c->node_off[inst], c->node_off[inst + 1],
                               c->precision == SWE_PREC_FP64 ? &c->B : nullptr,
                               c->precision == SWE_PREC_FP64 ? nullptr : &c->mB))) {
     drain(c);
     return rc;
   }
-  CK(cudaStreamSynchronize(c->stream));
-  return erc;
+  c->euler_done = true;
+  c->euler_inst = inst;
+  return call_end(c, inst);
 }
 
 SWE_API int swe_euler_intermediates(swe_ctx* c, int inst, double* dij_low, double* muij_low, double* alpha,
@@ -1120,7 +1203,10 @@ SWE_API int swe_fct_positivity(swe_ctx* c, int inst, const double* unext, const 
   launch_fct_positivity_f64(c->G, c->d_C, c->w.uL.h, c->w.fct, c->w.dLii, c->w.rminus, c->d_lij, c->stream);
   CK(cudaGetLastError());
   c->euler_done = false;
-  return entries_to_csr(c, inst, c->d_lij, lij, c->w.rminus);   // l_ii = R_i
+  const int rc = entries_to_csr(c, inst, c->d_lij, lij, c->w.rminus);   // l_ii = R_i
+  if (rc) { drain(c); return rc; }
+  CK(cudaStreamSynchronize(c->stream));
+  return SWE_OK;
 }
 
 SWE_API int swe_fct_generic(swe_ctx* c, int inst, double* unext, const double* maxn, const double* minn,
@@ -1261,17 +1347,16 @@ SWE_API int swe_get_time(swe_ctx* c, double* time, double* t_final, double* dt) 
 
 SWE_API int swe_set_time(swe_ctx* c, const double* time, const double* t_final) {
   if (!c) return SWE_ERR_ARG;
-  std::vector<InstState> hs;
-  int rc = save_state(c, hs);
-  if (rc) return rc;
-  for (int b = 0; b < c->n_inst; b++) {
-    if (time) hs[b].time = time[b];
-    if (t_final) hs[b].t_final = t_final[b];
-    hs[b].done = 0;
-    hs[b].steps = 0;
-    hs[b].maxd_bits = 0ull;
-  }
-  return restore_done(c, hs);
+  const size_t bytes = sizeof(double) * c->n_inst;
+  double* dt = c->d_times;
+  double* df = dt + c->n_inst;
+  if (time) CK(cudaMemcpyAsync(dt, time, bytes, cudaMemcpyHostToDevice, c->stream));
+  if (t_final) CK(cudaMemcpyAsync(df, t_final, bytes, cudaMemcpyHostToDevice, c->stream));
+  k_set_time<<<(c->n_inst + 127) / 128, 128, 0, c->stream>>>(c->d_St, c->n_inst, time ? dt : nullptr,
+                                                            t_final ? df : nullptr);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(c->stream));              // the caller's arrays are only borrowed
+  return SWE_OK;
 }
 
 // Launch configuration from the autotuner's own description ("dt:block256/
@@ -1695,9 +1780,11 @@ static int enqueue_rk3_steps(swe_ctx* c, int nsteps) {
 // The instances' clocks and the error word after everything enqueued, in one
 // synchronisation.
 static int finish_rk3_steps(swe_ctx* c, double* time_out, double* dt_out, int* steps_done) {
-  std::vector<InstState> out(c->n_inst);
-  CK(cudaMemcpyAsync(out.data(), c->d_St, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
-  const int rc = read_errors(c);
+  const InstState* out = c->h_St;
+  CK(cudaMemcpyAsync(c->h_St, c->d_St, sizeof(InstState) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  const int rc = error_status(c, *c->h_err);
   for (int b = 0; b < c->n_inst; b++) {
     if (time_out) time_out[b] = out[b].time;
     if (dt_out) dt_out[b] = out[b].dt;
