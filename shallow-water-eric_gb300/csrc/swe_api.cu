@@ -411,7 +411,8 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     const int tile = want >= 256 ? 256 : want >= 128 ? 128 : want >= 64 ? 64 : 0;   // the sizes that are built
     RowTiles F;
     TileCtl probe{};
-    if (c->S == 3 && tile > 0 && build_row_tiles(L, tile, F)) {
+    if (tile > 0 && (c->S == 3 || tile == 256) && build_row_tiles(L, tile, F)) {
+      probe.S = c->S;
       probe.tile_rows = F.tile;
       probe.halo_cap = (F.halo_cap + 3) / 4 * 4;
       probe.ent_cap = F.ent_cap;
@@ -1059,12 +1060,11 @@ static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, con
                           int comp = 0) {
   const Layout& L = c->L;
   if (!c->d_csr) {                                   // on first use
-    std::vector<int> pos(L.ref_pos.begin(), L.ref_pos.end()), pd(L.ref_pos_diag.begin(), L.ref_pos_diag.end());
     size_t most = 0;
     for (const HostMesh& m : c->meshes) most = std::max(most, m.ja.size());
     cudaError_t st = cudaSuccess;
-    c->d_ref_pos = upload_vec(c, pos, st);
-    c->d_ref_pos_diag = upload_vec(c, pd, st);
+    c->d_ref_pos = upload_vec(c, L.ref_pos, st);
+    c->d_ref_pos_diag = upload_vec(c, L.ref_pos_diag, st);
     double* csr = c->buf.alloc<double>(most, st);
     if (st != cudaSuccess) return cuda_check(c, st, "device allocation");
     c->d_csr = csr;

@@ -81,7 +81,8 @@ struct TileCtl {
   const int16_t* loc;     // per entry: col - tile start, or tile_rows + halo index
   const int4* head;       // per tile: first entry (64 bits), number of entries
   const int* halo_rows;   // halo_cap per tile, ascending, then -1
-  int tile_rows;          // 64, 128 or 256
+  int tile_rows;          // 64, 128 or 256 (5-component systems: 256)
+  int S;                  // components
   int halo_cap;           // largest halo, rounded up to a multiple of 4
   int ent_cap;            // most entries of a tile (a multiple of 32)
 };
@@ -141,10 +142,8 @@ struct KernelTune {
 void launch_stage_mix(const StageArgsMix& a, cudaStream_t s, const KernelEvents* kev, const KernelTune& t);
 // most dynamic shared memory of a tile block: two blocks per SM
 constexpr int kTileSmemMax = 100 * 1024;
-// dynamic shared memory of one tile block of a kernel kind (d: with the FP64
-// R^- of the precision split; lamin: k_low with k_dt's |c_ij| lambda)
-size_t tile_smem_bytes(const TileCtl& tc, int kind, bool d, bool lamin);
-size_t tile_smem_max(const TileCtl& tc, bool d);   // over the kernel kinds
+// dynamic shared memory of a tile block, the most over the kernel kinds (d: with the FP64 R^- of the precision split)
+size_t tile_smem_max(const TileCtl& tc, bool d);
 void launch_kernel_mix(int kind, const StageArgsMix& a, const KernelTune& t, cudaStream_t s);
 bool kind_has_tiles(int kind);   // kernel kinds with a shared-memory tile variant
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,

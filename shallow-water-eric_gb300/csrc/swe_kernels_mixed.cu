@@ -214,6 +214,12 @@ __device__ __forceinline__ bool dlam_f(float cxe, float cye, float cvi, float cv
   return ok;
 }
 
+__device__ __forceinline__ float sgn_pressure(float lambda_sgn, float g, float m, float h, float heta) {
+  const float pc = fdiv(lambda_sgn * g, 3.0f * sqrtf(m));
+  const float x = fdiv(heta, h * h);
+  return pc * h * h * h * (2.f + 4.f * x * x * x - 6.f * x * x * x * x);   // mSGN_RHS pTilde (update.f90:522)
+}
+
 // What the entry loops need of a node, in each kernel.
 struct NodeF {        // k_low (and its own row)
   float h, q1, q2, eta, ovh, v1, v2;
@@ -272,7 +278,7 @@ __device__ __forceinline__ RowHead row_head(const Graph& G, int64_t r) {
 
 // Neighbour access of the entry loops: straight from HBM by column index
 // (NbGlobal), or from the block's shared-memory copy of its tile and halo
-// nodes by tile-local position (the tile kernels, 3-component systems only),
+// nodes by tile-local position (the tile kernels),
 // where the quantities of one node are formed once per node and block instead
 // of once per entry.  Both form them with the same operations.
 //
@@ -283,7 +289,9 @@ __device__ __forceinline__ RowHead row_head(const Graph& G, int64_t r) {
 // (alpha in k_low, the residual in k_fct and k_update); R is R^- (k_update).
 struct NbGlobal {
   static constexpr bool kGlobal = true;
+  static constexpr int kS = 0;         // system size: the instance's
   const Graph& G;
+  const StateMix& u;
   const float4* nq;
   const float* aux;
   const float* R;
@@ -308,6 +316,11 @@ struct NbGlobal {
   __device__ __forceinline__ NodeC fct(const Raw& w, int) const { return NodeC{w.n.x, w.n.w, w.a}; }
   __device__ __forceinline__ NodeU upd(const Raw& w, int) const { return node_u(w.n, w.a, w.R); }
   __device__ __forceinline__ double r64(int j) const { return R64[j]; }
+  // h eta and h w, and the SGN pressure of a node (5-component systems)
+  __device__ __forceinline__ float2 q34(int j) const { return make_float2(u.q3[j], u.q4[j]); }
+  __device__ __forceinline__ float pressure(int j, const InstConst& c, float h, float q3) const {
+    return sgn_pressure(c.lambda_sgnf, c.gf, G.lumpedf[j], h, q3);
+  }
 };
 
 // ---- tile kernels: one block of T threads per tile of T rows, a row per
@@ -318,12 +331,16 @@ struct NbGlobal {
 // what they would form per entry (six times per node) is formed 1.4 times per
 // node.  The size is a template argument: with one row per thread the
 // prologue is a third of the instructions, and constant strides halve it.
+template <int S>
 struct NbTile {
   static constexpr bool kGlobal = false;
+  static constexpr int kS = S;
   const float4* a;            // k_low (h, q1, q2, eta); k_dt (h, v1, v2, sq); k_fct (h, eta, res); k_update as k_low
   const float4* b;            // k_low (ovh, v1, v2, sq); k_update (res, R, inv, one)
   const float4* c;            // k_low (inv, one, E, alpha)
   const float* o;             // k_dt: ovh; k_node: h
+  const float2* q;            // h eta, h w (5-component systems)
+  const float* p;             // k_low: SGN pressure
   const double* R64_;
   const int16_t* loc;         // this row's positions, c_ij or (d, mu), |c_ij| lambda
   const float2* e8;
@@ -353,39 +370,50 @@ struct NbTile {
     return NodeU{x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
   }
   __device__ __forceinline__ double r64(int j) const { return R64_[j]; }
+  __device__ __forceinline__ float2 q34(int j) const { return q[j]; }
+  __device__ __forceinline__ float pressure(int j, const InstConst&, float, float) const { return p[j]; }
 };
 
 // Shared memory of one tile block: per-node parts over the tile's rows
 // (positions 0 .. T-1) and its halo rows (T ..), then the tile's entries; each
 // part a multiple of 16 bytes.  What a kernel does not use takes no space.
 struct TileParts {
-  int a, b, c, o, r64, e8, e4;   // bytes per position / entry
+  int a, b, c, q, r64, e8, e4, o, p;   // bytes per position / entry
 };
-__host__ __device__ constexpr TileParts tile_parts(int kind, bool d, bool lamin) {
-  return TileParts{kind == 1 ? 0 : 16,           kind == 2 || kind == 4 ? 16 : 0, kind == 2 ? 16 : 0,
-                   kind <= 1 ? 4 : 0,            kind == 4 && d ? 8 : 0,          kind == 1 ? 0 : 8,
-                   kind == 2 && lamin ? 4 : 0};
+__host__ __device__ constexpr TileParts tile_parts(int kind, int S, bool d, bool lamin) {
+  return TileParts{kind == 1 ? 0 : 16,
+                   kind == 2 || kind == 4 ? 16 : 0,
+                   kind == 2 ? 16 : 0,
+                   S == 5 && (kind == 2 || kind == 4) ? 8 : 0,
+                   kind == 4 && d ? 8 : 0,
+                   kind == 1 ? 0 : 8,
+                   kind == 2 && lamin ? 4 : 0,
+                   kind <= 1 ? 4 : 0,
+                   S == 5 && kind == 2 ? 4 : 0};
 }
 struct TileSmem {
   float4 *a, *b, *c;
+  float2* q;
   double* r64;
   float2* e8;
-  float *e4, *o;
+  float *e4, *o, *p;
   int16_t* loc;
 };
-template <int T, int KIND, bool D, bool LAMIN>
+template <int T, int KIND, int S, bool D, bool LAMIN>
 __device__ __forceinline__ TileSmem tile_smem(void* base, const TileCtl& tc) {
-  constexpr TileParts P = tile_parts(KIND, D, LAMIN);
+  constexpr TileParts P = tile_parts(KIND, S, D, LAMIN);
   const int cap = T + tc.halo_cap, ec = tc.ent_cap;
   char* p = reinterpret_cast<char*>(base);
   TileSmem s{};
   if (P.a) { s.a = reinterpret_cast<float4*>(p); p += P.a * cap; }
   if (P.b) { s.b = reinterpret_cast<float4*>(p); p += P.b * cap; }
   if (P.c) { s.c = reinterpret_cast<float4*>(p); p += P.c * cap; }
+  if (P.q) { s.q = reinterpret_cast<float2*>(p); p += P.q * cap; }
   if (P.r64) { s.r64 = reinterpret_cast<double*>(p); p += P.r64 * cap; }
   if (P.e8) { s.e8 = reinterpret_cast<float2*>(p); p += P.e8 * ec; }
   if (P.e4) { s.e4 = reinterpret_cast<float*>(p); p += P.e4 * ec; }
   if (P.o) { s.o = reinterpret_cast<float*>(p); p += P.o * cap; }
+  if (P.p) { s.p = reinterpret_cast<float*>(p); p += P.p * cap; }
   s.loc = reinterpret_cast<int16_t*>(p);
   return s;
 }
@@ -438,9 +466,10 @@ __device__ __forceinline__ void stage_nodes(const TileCtl& tc, const Tile& t, Lo
     if (row >= 0) put(T + k, row, load(row));
   }
 }
-__device__ __forceinline__ NbTile nb_tile(const Tile& t, const TileSmem& sm) {
+template <int S>
+__device__ __forceinline__ NbTile<S> nb_tile(const Tile& t, const TileSmem& sm) {
   const int o = (int)(t.hd.base - t.e0);
-  return NbTile{sm.a, sm.b, sm.c, sm.o, sm.r64, sm.loc + o, sm.e8 + o, sm.e4 + o};
+  return NbTile<S>{sm.a, sm.b, sm.c, sm.o, sm.q, sm.p, sm.r64, sm.loc + o, sm.e8 + o, sm.e4 + o};
 }
 // the instance whose g and htiny a node's quantities take (rows of a tile may
 // belong to several instances; a row and its neighbours share one)
@@ -529,7 +558,7 @@ __global__ void __launch_bounds__(256) k_node_mix(Graph G, const InstConst* __re
                                                   float* __restrict__ alpha_out) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G, u.nq, nullptr, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, nullptr, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
     node_row<B>((int)r, row_head(G, r), C, St, alpha_out, nb);
 }
@@ -540,20 +569,14 @@ __global__ void __launch_bounds__(T) k_node_tile(Graph G, const InstConst* __res
                                                  float* __restrict__ alpha_out, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
-  const TileSmem sm = tile_smem<T, 1, false, false>(tile_mem, tc);
+  const TileSmem sm = tile_smem<T, 1, 3, false, false>(tile_mem, tc);
   cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
   stage_nodes<T>(tc, t, [&](int row) { return u.nq[row].x; }, [&](int i, int, float h) { sm.o[i] = h; });
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  node_row<1>(t.r, t.hd, C, St, alpha_out, nb_tile(t, sm));
-}
-
-__device__ __forceinline__ float sgn_pressure(float lambda_sgn, float g, float m, float h, float heta) {
-  const float pc = fdiv(lambda_sgn * g, 3.0f * sqrtf(m));
-  const float x = fdiv(heta, h * h);
-  return pc * h * h * h * (2.f + 4.f * x * x * x - 6.f * x * x * x * x);   // mSGN_RHS pTilde (update.f90:522)
+  node_row<1>(t.r, t.hd, C, St, alpha_out, nb_tile<3>(t, sm));
 }
 
 // k_low_mix: one pass over the row's entries computing d_ij (lambda_max),
@@ -584,8 +607,8 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
   const InstState& st = St[hd.b];
   if (st.done) return;
   const InstConst& c = C[hd.b];
-  const int S = Nb::kGlobal ? c.S : 3;         // tiles hold 3-component systems only
-  const bool sgn = Nb::kGlobal && c.type_test == 13;
+  const int S = Nb::kS ? Nb::kS : c.S;
+  const bool sgn = Nb::kS ? Nb::kS == 5 : c.type_test == 13;   // 5 components: type 13
   const bool galerkin = !FCT && c.visc == VISC_GALERKIN;   // every d_ij, mu_ij = 0 (update.f90:155-158)
   const bool limit = FCT || c.alpha_limit;
   const float g = c.gf, htiny = c.htinyf, dtf = st.dtf;
@@ -623,7 +646,7 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
   g1 = -cvd * ni.q1; g2 = -cvd * ni.q2;
   if (S == 5) { g3 = -cvd * ui3; g4 = -cvd * ui4; }
   if (sgn) {
-    const float pt = sgn_pressure(c.lambda_sgnf, g, m, ni.h, ui3);
+    const float pt = nb.pressure(me, c, ni.h, ui3);
     ptx = -pt * cxd;
     pty = -pt * cyd;
   }
@@ -694,8 +717,9 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
     const float T1 = fma_(dmu, fma_(nj.q1, rji, -ni.q1 * rij), A1);
     const float T2 = fma_(dmu, fma_(nj.q2, rji, -ni.q2 * rij), A2);
     float uj3 = 0.f, uj4 = 0.f, A3 = 0.f, A4 = 0.f;
-    if (Nb::kGlobal && S == 5) {
-      uj3 = u.q3[j]; uj4 = u.q4[j];
+    if (S == 5) {
+      const float2 qj = nb.q34(j);
+      uj3 = qj.x; uj4 = qj.y;
       A3 = fma_(mu, uj3 - ui3, -cvj_flux * uj3);
       A4 = fma_(mu, uj4 - ui4, -cvj_flux * uj4);
     }
@@ -706,18 +730,18 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
       rk2_ += fma_(dmu, fma_(nj.q2, rjit, -ni.q2 * rijt), A2);
       rk1 = fma_(-topo, cxe, rk1);
       rk2_ = fma_(-topo, cye, rk2_);
-      if (Nb::kGlobal && S == 5) {
+      if (S == 5) {
         rk3 += fma_(dmu, fma_(uj3, rjit, -ui3 * rijt), A3);
         rk4 += fma_(dmu, fma_(uj4, rjit, -ui4 * rijt), A4);
       }
     }
     g1 = fma_(-topo, cxe, g1 + T1);
     g2 = fma_(-topo, cye, g2 + T2);
-    if (Nb::kGlobal && S == 5) {
+    if (S == 5) {
       g3 += fma_(dmu, fma_(uj3, rji, -ui3 * rij), A3);
       g4 += fma_(dmu, fma_(uj4, rji, -ui4 * rij), A4);
       if (sgn) {
-        const float pt = sgn_pressure(c.lambda_sgnf, g, G.lumpedf[j], nj.h, uj3);
+        const float pt = nb.pressure(j, c, nj.h, uj3);
         ptx = fma_(-pt, cxe, ptx);
         pty = fma_(-pt, cye, pty);
       }
@@ -800,12 +824,12 @@ __global__ void __launch_bounds__(256, MINB) k_low_mix(Graph G, const InstConst*
                                                        WorkMix w, float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, alpha, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
     low_row<B, LAMIN, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, res, err, nb);
 }
 
-template <int T, bool LAMIN, int MINB, bool D, bool FCT>
+template <int T, int S, bool LAMIN, int MINB, bool D, bool FCT>
 __global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const InstConst* __restrict__ C,
                                                                  const InstState* __restrict__ St, StateMix u,
                                                                  const float* __restrict__ alpha,
@@ -814,18 +838,27 @@ __global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const 
                                                                  TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
-  const TileSmem sm = tile_smem<T, 2, D, LAMIN>(tile_mem, tc);
+  const TileSmem sm = tile_smem<T, 2, S, D, LAMIN>(tile_mem, tc);
   cp_range<T>(sm.e8, G.cf + t.e0, 8 * t.ne);
   cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
   if (LAMIN) cp_range<T>(sm.e4, w.dlam + t.e0, 4 * t.ne);
   row_prefetch<T>(G, RowPrefetch{{G.lumpedf, G.inv_lumpedf, G.cxiif, G.cyiif, u.h, nullptr}, {4, 4, 4, 4, 8, 0}});
-  struct Node { float4 n; float al; };
+  struct Node { float4 n; float al, q3, q4, m; };
   stage_nodes<T>(
-      tc, t, [&](int row) { return Node{u.nq[row], alpha[row]}; },
+      tc, t,
+      [&](int row) {
+        Node x{u.nq[row], alpha[row], 0.f, 0.f, 0.f};
+        if (S == 5) { x.q3 = u.q3[row]; x.q4 = u.q4[row]; x.m = G.lumpedf[row]; }
+        return x;
+      },
       [&](int i, int row, const Node& x) {
         const InstConst& c = inst_of(G, C, row);
-        const NodeF n = node_f(x.n, x.al, c.gf, c.htinyf, false);
+        const NodeF n = node_f(x.n, x.al, c.gf, c.htinyf, S == 5);
+        if (S == 5) {
+          sm.q[i] = make_float2(x.q3, x.q4);
+          sm.p[i] = sgn_pressure(c.lambda_sgnf, c.gf, x.m, n.h, x.q3);
+        }
         sm.a[i] = x.n;
         sm.b[i] = make_float4(n.ovh, n.v1, n.v2, n.sq);
         sm.c[i] = make_float4(n.inv, n.one, n.E, n.al);
@@ -833,7 +866,7 @@ __global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const 
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  low_row<1, LAMIN, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, res, err, nb_tile(t, sm));
+  low_row<1, LAMIN, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, res, err, nb_tile<S>(t, sm));
 }
 
 // 'viscous' with viscous_type 'type1' (update.f90:189-201, smb_1 :366-423):
@@ -847,7 +880,7 @@ template <bool D>
 __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const InstConst& c, const InstState& st,
                                               const StateMix& u, const float* __restrict__ alpha,
                                               float2* __restrict__ dmu, const WorkMix& w, unsigned* __restrict__ err) {
-  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, alpha, nullptr, nullptr};
   const int L = G.len[r];
   const float g = c.gf, htiny = c.htinyf, dtf = st.dtf;
   const LamK lk = lam_k(g, htiny);
@@ -919,7 +952,7 @@ __global__ void __launch_bounds__(256) k_low_type1(Graph G, const InstConst* __r
                                                    float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G, u.nq, alpha, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, alpha, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x) {
     if (G.len[r] == 0) continue;
     const int b = G.slice_inst[r >> 5];
@@ -1021,7 +1054,7 @@ __global__ void __launch_bounds__(256) k_fct_mix(Graph G, const InstConst* __res
                                                  const float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G, u.nq, res, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, res, nullptr, nullptr};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
     fct_row<B, D>((int)r, row_head(G, r), G, C, St, dmu, w, err, nb);
 }
@@ -1033,7 +1066,7 @@ __global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* __rest
                                                 const float* __restrict__ res, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
-  const TileSmem sm = tile_smem<T, 3, D, false>(tile_mem, tc);
+  const TileSmem sm = tile_smem<T, 3, 3, D, false>(tile_mem, tc);
   cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
   cp_range<T>(sm.e8, dmu + t.e0, 8 * t.ne);
@@ -1044,7 +1077,7 @@ __global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* __rest
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  fct_row<1, D>(t.r, t.hd, G, C, St, dmu, w, err, nb_tile(t, sm));
+  fct_row<1, D>(t.r, t.hd, G, C, St, dmu, w, err, nb_tile<3>(t, sm));
 }
 
 // End of a stage for one row: non-finite check, the SSP-RK combination and
@@ -1110,7 +1143,7 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
   const InstState& st = St[hd.b];
   if (st.done) return;
   const InstConst& c = C[hd.b];
-  const int S = Nb::kGlobal ? c.S : 3;
+  const int S = Nb::kS ? Nb::kS : c.S;
   const int me = nb.self(r);
   const bool ent = !FCT && c.visc == VISC_ENTROPY;
   if (!FCT && c.visc != VISC_FCT && !ent) {             // 'galerkin' / 'viscous': u^L is the result
@@ -1176,13 +1209,10 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
     const float dm = dmr * lf, dx = (ddr - dmr) * lf;
     x1 = fma_(dx, fma_(nj.q1, rji_, -ni.q1 * rij_), fma_(dm, nj.q1 - ni.q1, x1));
     x2 = fma_(dx, fma_(nj.q2, rji_, -ni.q2 * rij_), fma_(dm, nj.q2 - ni.q2, x2));
-    if constexpr (Nb::kGlobal) {
-      if (S == 5) {
-        const int j = jb[q];
-        const float uj3 = u.q3[j], uj4 = u.q4[j];
-        x3 = fma_(dx, fma_(uj3, rji_, -ui3 * rij_), fma_(dm, uj3 - ui3, x3));
-        x4 = fma_(dx, fma_(uj4, rji_, -ui4 * rij_), fma_(dm, uj4 - ui4, x4));
-      }
+    if (S == 5) {
+      const float2 qj = nb.q34(jb[q]);
+      x3 = fma_(dx, fma_(qj.x, rji_, -ui3 * rij_), fma_(dm, qj.x - ui3, x3));
+      x4 = fma_(dx, fma_(qj.y, rji_, -ui4 * rij_), fma_(dm, qj.y - ui4, x4));
     }
    }
   }
@@ -1214,12 +1244,12 @@ __global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* __
                                                     int rk_stage, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
-  const NbGlobal nb{G, u.nq, res, w.rminus, w.rminus64};
+  const NbGlobal nb{G, u, u.nq, res, w.rminus, w.rminus64};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < G.n_rows; r += (int64_t)gridDim.x * blockDim.x)
     update_row<B, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, u0, out, rk_stage, err, nb);
 }
 
-template <int T, bool D, bool FCT>
+template <int T, int S, bool D, bool FCT>
 __global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* __restrict__ C,
                                                    const InstState* __restrict__ St, StateMix u,
                                                    const float2* __restrict__ dmu, WorkMix w,
@@ -1227,26 +1257,32 @@ __global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* __r
                                                    int rk_stage, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
-  const TileSmem sm = tile_smem<T, 4, D, false>(tile_mem, tc);
+  const TileSmem sm = tile_smem<T, 4, S, D, false>(tile_mem, tc);
   cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
   cp_range<T>(sm.e8, dmu + t.e0, 8 * t.ne);
   row_prefetch<T>(G, RowPrefetch{{G.inv_lumpedf, G.bathdf, w.hL, w.qL, rk_stage >= 2 ? (const void*)u0.nq : nullptr,
                                   rk_stage >= 2 ? (const void*)u0.h : nullptr},
                                  {4, 8, 8, 8, rk_stage >= 2 ? 16 : 0, rk_stage >= 2 ? 8 : 0}});
-  struct Node { float4 n; float res, R; double r64; };
+  struct Node { float4 n; float res, R, q3, q4; double r64; };
   stage_nodes<T>(
-      tc, t, [&](int row) { return Node{u.nq[row], res[row], w.rminus[row], D ? w.rminus64[row] : 0.0}; },
+      tc, t,
+      [&](int row) {
+        Node x{u.nq[row], res[row], w.rminus[row], 0.f, 0.f, D ? w.rminus64[row] : 0.0};
+        if (S == 5) { x.q3 = u.q3[row]; x.q4 = u.q4[row]; }
+        return x;
+      },
       [&](int i, int, const Node& x) {
         const NodeU n = node_u(x.n, x.res, x.R);
         sm.a[i] = x.n;
         sm.b[i] = make_float4(n.res, n.R, n.inv, n.one);
         if (D) sm.r64[i] = x.r64;
+        if (S == 5) sm.q[i] = make_float2(x.q3, x.q4);
       });
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  update_row<1, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, u0, out, rk_stage, err, nb_tile(t, sm));
+  update_row<1, D, FCT>(t.r, t.hd, G, C, St, u, dmu, w, u0, out, rk_stage, err, nb_tile<S>(t, sm));
 }
 
 // One row of k_dt_mix: FP32 lambda_max, |d_ii| / m_i (main.f90:166-174; 0 for
@@ -1327,7 +1363,7 @@ __global__ void __launch_bounds__(256) k_dt_mix(Graph G, const InstConst* __rest
   pdl_wait();
   // grid-stride over block-sized row ranges: every lane of a warp runs the
   // same iterations (the warp reduction needs all 32)
-  const NbGlobal nb{G, u.nq, nullptr, nullptr, nullptr};
+  const NbGlobal nb{G, u, u.nq, nullptr, nullptr, nullptr};
   for (int64_t rb = blockIdx.x * (int64_t)blockDim.x; rb < G.n_rows; rb += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = rb + threadIdx.x;
     dt_reduce(r < G.n_rows ? dt_row<B>((int)r, row_head(G, r), G, C, St, dlam, alpha_out, err, nb) : 0.f, r, G, St);
@@ -1340,7 +1376,7 @@ __global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* __restr
                                                unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
-  const TileSmem sm = tile_smem<T, 0, false, false>(tile_mem, tc);
+  const TileSmem sm = tile_smem<T, 0, 3, false, false>(tile_mem, tc);
   cp_range<T>(sm.e8, G.cf + t.e0, 8 * t.ne);
   cp_range<T>(sm.loc, tc.loc + t.e0, 2 * t.ne);
   pdl_wait();
@@ -1355,7 +1391,7 @@ __global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* __restr
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  dt_reduce(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile(t, sm)), t.r, G, St);
+  dt_reduce(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile<3>(t, sm)), t.r, G, St);
 }
 
 // Free surface of the packed node records after a bathymetry change
@@ -1435,10 +1471,10 @@ static unsigned row_grid(K kern, int64_t n, int block, int mode) {
   }
 
 // Tile variants: one block per tile
-size_t tile_smem_bytes(const TileCtl& tc, int kind, bool d, bool lamin) {
-  const TileParts P = tile_parts(kind, d, lamin);
+static size_t tile_smem_bytes(const TileCtl& tc, int kind, bool d, bool lamin) {
+  const TileParts P = tile_parts(kind, tc.S, d, lamin);
   const size_t cap = tc.tile_rows + tc.halo_cap, ec = tc.ent_cap;
-  return cap * (P.a + P.b + P.c + P.o + P.r64) + ec * (P.e8 + P.e4 + 2);
+  return cap * (P.a + P.b + P.c + P.q + P.o + P.p + P.r64) + ec * (P.e8 + P.e4 + 2);
 }
 size_t tile_smem_max(const TileCtl& tc, bool d) {
   size_t m = 0;
@@ -1471,13 +1507,14 @@ static void launch_tile(void (*kern)(KArgs...), const TileCtl& tc, int64_t n_row
 template <bool LAMIN, bool D>
 static void launch_low(const StageArgsMix& a, int batch, int cap, int mode, int block, bool tiled, cudaStream_t s) {
   if (tiled && a.tiles) {
-#define SWE_LOWT(TT, MB, F)                                                                                        \
-    launch_tile(k_low_tile<TT, LAMIN, MB, D, F>, *a.tiles, a.G.n_rows, 2, D, LAMIN, s, a.G, a.C, a.St, a.u, a.w.alpha, \
-                a.w.dmu, a.w, a.w.res, a.err)
-    if (a.tiles->tile_rows == 64) SWE_LOWT(64, 3, false);
-    else if (a.tiles->tile_rows == 128) SWE_LOWT(128, 3, false);
-    else if (a.fct) { if (cap) SWE_LOWT(256, 4, true); else SWE_LOWT(256, 3, true); }
-    else { if (cap) SWE_LOWT(256, 4, false); else SWE_LOWT(256, 3, false); }
+#define SWE_LOWT(TT, SS, MB, F)                                                                                      \
+    launch_tile(k_low_tile<TT, SS, LAMIN, MB, D, F>, *a.tiles, a.G.n_rows, 2, D, LAMIN, s, a.G, a.C, a.St, a.u,      \
+                a.w.alpha, a.w.dmu, a.w, a.w.res, a.err)
+    if (a.tiles->S == 5) { if (a.fct) SWE_LOWT(256, 5, 3, true); else SWE_LOWT(256, 5, 3, false); }
+    else if (a.tiles->tile_rows == 64) SWE_LOWT(64, 3, 3, false);
+    else if (a.tiles->tile_rows == 128) SWE_LOWT(128, 3, 3, false);
+    else if (a.fct) { if (cap) SWE_LOWT(256, 3, 4, true); else SWE_LOWT(256, 3, 3, true); }
+    else { if (cap) SWE_LOWT(256, 3, 4, false); else SWE_LOWT(256, 3, 3, false); }
 #undef SWE_LOWT
     return;
   }
@@ -1518,12 +1555,14 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
             }
             break;
     case 4: if (t.tiled[4] && a.tiles) {
-              if (a.fct && a.tiles->tile_rows == 256)
-                launch_tile(k_update_tile<256, D, true>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu, a.w,
-                            a.w.res, a.u0, a.out, a.rk_stage, a.err);
-              else
-                SWE_TILE_T(*a.tiles, launch_tile(k_update_tile<T, D, false>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St,
-                                                 a.u, a.w.dmu, a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err));
+#define SWE_UPDT(TT, SS, F)                                                                                        \
+              launch_tile(k_update_tile<TT, SS, D, F>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu,   \
+                          a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err)
+              if (a.tiles->S == 5) { if (a.fct) SWE_UPDT(256, 5, true); else SWE_UPDT(256, 5, false); }
+              else if (a.tiles->tile_rows == 64) SWE_UPDT(64, 3, false);
+              else if (a.tiles->tile_rows == 128) SWE_UPDT(128, 3, false);
+              else { if (a.fct) SWE_UPDT(256, 3, true); else SWE_UPDT(256, 3, false); }
+#undef SWE_UPDT
             } else {
               SWE_DISPATCH_BD(t.batch[4], k_update_mix, D, n, t.block[4], t.grid[4], a.G, a.C, a.St, a.u, a.w.dmu,
                               a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err)

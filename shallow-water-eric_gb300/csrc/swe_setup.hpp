@@ -75,8 +75,8 @@ struct Layout {
   std::vector<int> col;                  // n_entries (padding -> own row)
   std::vector<double> cx, cy;            // n_entries (padding -> 0)
   std::vector<double> cxii, cyii;        // n_rows: diagonal c_ii
-  std::vector<int64_t> ref_pos;          // n_entries: instance-local CSR position or -1
-  std::vector<int64_t> ref_pos_diag;     // n_rows: CSR position of (i,i) or -1
+  std::vector<int> ref_pos;              // n_entries: instance-local CSR position or -1
+  std::vector<int> ref_pos_diag;         // n_rows: CSR position of (i,i) or -1
   std::vector<double> lumped, bath;      // n_rows
   std::vector<int64_t> old_of_new;       // n_rows: instance-local old index or -1
   std::vector<std::vector<int>> new_of_old;   // per instance, global row index
