@@ -27,22 +27,90 @@ using namespace swe;
 
 namespace {
 
+// Zeroed device arrays, 256-byte aligned, freed together.  Small ones share
+// slabs of 1 MB: a context has some fifty, and an allocation and a memset each
+// were most of the set-up time of a small mesh.
 struct DevBuf {
+  static constexpr size_t kSlab = 1 << 20;
   std::vector<void*> ptrs;
+  char* slab = nullptr;
+  size_t left = 0;
   template <typename T> T* alloc(size_t n, cudaError_t& st) {
-    void* p = nullptr;
     if (st != cudaSuccess) return nullptr;
-    st = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T));
-    if (st == cudaSuccess) { ptrs.push_back(p); cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)); }
-    return (T*)p;
+    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+    if (bytes > left || bytes > kSlab / 4) {
+      const bool shared = bytes <= kSlab / 4;
+      const size_t take = shared ? kSlab : bytes;
+      void* p = nullptr;
+      st = cudaMalloc(&p, take);
+      if (st != cudaSuccess) return nullptr;
+      ptrs.push_back(p);
+      st = cudaMemset(p, 0, take);
+      if (st == cudaSuccess) st = cudaStreamSynchronize(0);   // contexts run on their own non-blocking streams
+      if (st != cudaSuccess) return nullptr;
+      if (!shared) return static_cast<T*>(p);
+      slab = static_cast<char*>(p);
+      left = take;
+    }
+    char* p = slab;
+    slab += bytes;
+    left -= bytes;
+    return reinterpret_cast<T*>(p);
   }
-  void release() { for (void* p : ptrs) cudaFree(p); ptrs.clear(); }
+  void release() { for (void* p : ptrs) cudaFree(p); ptrs.clear(); slab = nullptr; left = 0; }
 };
+
+// Page-locked memory for what calls read back, in one process-wide page of
+// fixed slots (page-locking costs a millisecond): given out under a lock, freed
+// with the last slot.  Sizes above a slot are page-locked on their own.
+class PinnedSlots {
+ public:
+  void* take(size_t bytes) {
+    if (bytes <= kSlot) {
+      std::lock_guard<std::mutex> lk(mu_);
+      if (!page_ && cudaMallocHost(&page_, kSlot * kSlots) != cudaSuccess) page_ = nullptr;
+      if (page_)
+        for (size_t k = 0; k < kSlots; k++)
+          if (!used_[k]) {
+            used_[k] = true;
+            n_++;
+            return static_cast<char*>(page_) + k * kSlot;
+          }
+    }
+    void* p = nullptr;
+    return cudaMallocHost(&p, bytes) == cudaSuccess ? p : nullptr;
+  }
+  void give(void* p) {
+    if (!p) return;
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      const char* c = static_cast<char*>(p);
+      const char* b = static_cast<char*>(page_);
+      if (page_ && c >= b && c < b + kSlot * kSlots) {
+        used_[(c - b) / kSlot] = false;
+        if (--n_ == 0) {
+          cudaFreeHost(page_);
+          page_ = nullptr;
+        }
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr size_t kSlot = 1024, kSlots = 64;
+  std::mutex mu_;
+  void* page_ = nullptr;
+  bool used_[kSlots] = {};
+  size_t n_ = 0;
+};
+PinnedSlots g_pinned;
 
 }  // namespace
 
 struct swe_ctx {
-  int dev = 0;
+  int dev = 0, sms = 1;
   cudaStream_t stream = nullptr;
   // state transfers: chunks copied on their own streams (several copy engines)
   // and permuted on `stream` as each lands
@@ -60,6 +128,7 @@ struct swe_ctx {
   InstConst* d_C = nullptr;
   InstState* d_St = nullptr;
   unsigned* d_err = nullptr;
+  unsigned* d_ticket = nullptr;          // StepTurn
   int* d_row_of_node = nullptr;          // concatenated host node -> device row
   double* d_stage = nullptr;             // staging (S, total nodes), reference layout
   uint8_t* d_dir_mask = nullptr;
@@ -208,7 +277,14 @@ static bool has_entropy(const swe_ctx* c) {
   return false;
 }
 
-// every instance runs 'fct' with the roundoff fix: the FP64 path's fused row kernels
+// every instance runs 'fct', or 'viscous' 'type2', with the roundoff fix: the FP64 path's row kernels
+static bool all_fct_rows(const swe_ctx* c) {
+  for (const swe_params& p : c->params)
+    if (!p.if_roundoff_fix || p.viscous_type != 2 ||
+        (p.viscosity_type != SWE_VISC_FCT && p.viscosity_type != SWE_VISC_VISCOUS))
+      return false;
+  return true;
+}
 static bool all_fct(const swe_ctx* c) {
   for (const swe_params& p : c->params)
     if (p.viscosity_type != SWE_VISC_FCT || !p.if_roundoff_fix) return false;
@@ -348,14 +424,13 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
   c->d_St_call = upload_vec(c, hs, st);
   c->d_times = c->buf.alloc<double>(2 * (size_t)c->n_inst, st);
   if (st == cudaSuccess) {
-    void* h = nullptr;
-    st = cudaMallocHost(&h, sizeof(InstState) * c->n_inst + sizeof(unsigned));
-    if (st == cudaSuccess) {
-      c->h_St = static_cast<InstState*>(h);
-      c->h_err = reinterpret_cast<unsigned*>(c->h_St + c->n_inst);
-    }
+    void* h = g_pinned.take(sizeof(InstState) * c->n_inst + sizeof(unsigned));
+    if (!h) return fail(c, SWE_ERR_CUDA, "page-locked allocation");
+    c->h_St = static_cast<InstState*>(h);
+    c->h_err = reinterpret_cast<unsigned*>(c->h_St + c->n_inst);
   }
   c->d_err = c->buf.alloc<unsigned>(1, st);
+  c->d_ticket = c->buf.alloc<unsigned>(1, st);
   // host node -> device row map, staging buffer
   c->node_off.assign(c->n_inst + 1, 0);
   for (int b = 0; b < c->n_inst; b++) c->node_off[b + 1] = c->node_off[b] + c->meshes[b].np;
@@ -703,9 +778,18 @@ static int save_state(swe_ctx* c, std::vector<InstState>& saved) {
   return SWE_OK;
 }
 
-// One time step.  With kev/acc (profiling), every kernel is bracketed by an
-// event pair and its duration added to acc[kind] after a synchronisation.
-static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* acc = nullptr) {
+// k_dt's last block runs the turn between steps: up to four 256-row blocks per SM
+static bool turn_in_dt(const swe_ctx* c) { return c->G.n_rows <= 4 * 256 * (int64_t)c->sms; }
+
+// One time step of a sequence.  k_dt's last block closes the step before
+// (open: it is still open) and opens this one; the last step of a sequence
+// (and, for the gauges, every step) is closed by k_step_end.  With kev/acc
+// (profiling), every kernel is bracketed by an event pair and its duration
+// added to acc[kind] after a synchronisation.
+static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* kev = nullptr, double* acc = nullptr) {
+  const StepTurn own{nullptr, c->n_inst, open ? 1 : 0};
+  StepTurn turn = own;
+  if (turn_in_dt(c)) turn.ticket = c->d_ticket;
   const cudaStream_t s = c->stream;
   auto harvest = [&](int first, int last) {
     if (!kev) return;
@@ -727,18 +811,18 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
   }
   if (kev) cudaEventRecord(kev->ev[0], s);
   if (c->precision == SWE_PREC_FP64)
-    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.fct, nullptr, c->d_err, c->block, s);
+    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.fct, nullptr, c->d_err, c->block, turn, s);
   else launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, c->tune,
-                   c->tiles_ok ? &c->tiles : nullptr, s);
+                   c->tiles_ok ? &c->tiles : nullptr, turn, s);
   if (kev) cudaEventRecord(kev->ev[1], s);
+  if (!turn.ticket) launch_step_turn(own, c->d_C, c->d_St, s);
   harvest(0, 0);                                   // waits for k_dt, the later of the two
   if (c->precision == SWE_PREC_FP64) harvest(1, 1);
-  launch_step_begin(c->d_C, c->d_St, c->n_inst, s);
   for (int stage = 1; stage <= 3; stage++) {
     if (c->precision == SWE_PREC_FP64) {
       StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, stage, nullptr, c->d_err, c->block};
       a.entropy = has_entropy(c);
-      a.fused = all_fct(c);
+      a.fused = all_fct_rows(c);
       a.S = c->S;
       if (stage == 1) { a.dij_in = c->w.fct; a.skip_node = 1; }
       if (stage == 2) { a.u = c->B; a.out = c->Cs; }
@@ -756,7 +840,7 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
     }
     harvest(1, 4);
   }
-  launch_step_end(c->d_St, c->n_inst, s);
+  if (close || c->n_gauges) launch_step_end(c->d_St, c->n_inst, s);
   if (c->n_gauges)
     k_gauges<<<1, 256, 0, s>>>(c->n_gauges, c->d_gauge_inst, c->d_gauge_rows, c->d_gauge_w, c->d_St,
                                c->precision == SWE_PREC_FP64 ? 1 : 0, c->A, c->mA, c->G.bath, c->d_gauge_rec,
@@ -766,7 +850,7 @@ static void enqueue_step(swe_ctx* c, const KernelEvents* kev = nullptr, double* 
 static int capture_steps(swe_ctx* c, int steps, cudaGraphExec_t* exec) {
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < steps; k++) enqueue_step(c);
+  for (int k = 0; k < steps; k++) enqueue_step(c, k > 0 && !c->n_gauges, k == steps - 1);
   CK(cudaStreamEndCapture(c->stream, &g));
   cudaError_t e = cudaGraphInstantiate(exec, g, 0);
   cudaGraphDestroy(g);
@@ -807,6 +891,7 @@ static int create_common(swe_ctx** out, int n_inst, const int* np, const int* me
     return fail(c, SWE_ERR_CUDA, "no CUDA device: this library has no CPU path");
   }
   cudaGetDevice(&c->dev);
+  cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev);
   c->n_inst = n_inst;
   c->S = params[0].syst_size;
   c->precision = params[0].precision;
@@ -879,7 +964,7 @@ SWE_API void swe_destroy(swe_ctx* c) {
   }
   if (c->copy_go) cudaEventDestroy(c->copy_go);
   c->buf.release();
-  if (c->h_St) cudaFreeHost(c->h_St);
+  g_pinned.give(c->h_St);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -1099,7 +1184,7 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
     a.w.alpha = nullptr;                             // the last euler call's alpha stays readable
     launch_node_f64(a, c->stream);
-    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, c->stream);
+    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, StepTurn{}, c->stream);
     rc = cuda_check(c, cudaGetLastError(), "compute_dij");
   }
   if (!rc) rc = call_end(c, inst);                   // nothing is written to the caller's arrays on an error
@@ -1126,7 +1211,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
   if (c->precision == SWE_PREC_FP64) {
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
-    a.fused = all_fct(c);
+    a.fused = all_fct_rows(c);
     a.S = c->S;
     launch_stage_f64(a, c->stream);
   } else {
@@ -1435,11 +1520,9 @@ static int autotune(swe_ctx* c) {
   // resident blocks per SM (64 registers, a few spilled) where an SM has more
   // than three tiles, else three.
   if (c->tiles_ok && !(tenv && tenv[0] == '0')) {
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
     const int64_t n_tiles = (c->G.n_rows + c->tiles.tile_rows - 1) / c->tiles.tile_rows;
     KernelTune t;
-    t.cap_low = n_tiles > 3 * (int64_t)sms;
+    t.cap_low = n_tiles > 3 * (int64_t)c->sms;
     for (int k = 0; k < 5; k++) { t.block[k] = 256; t.tiled[k] = 1; }
     c->tune = t;
     c->tuned = true;
@@ -1460,7 +1543,7 @@ static int autotune(swe_ctx* c) {
   a.type1 = has_type1(c);
   KernelTune t = c->tune;
   for (int& k : t.tiled) k = 0;
-  launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, t, nullptr, s);   // populate every work array once
+  launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, t, nullptr, StepTurn{}, s);   // populate every work array once
   launch_stage_mix(a, s, nullptr, t);
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1489,7 +1572,7 @@ static int autotune(swe_ctx* c) {
             float tmin = 1e30f;
             for (int rep = 0; rep < 3; rep++) {
               cudaEventRecord(e0, s);
-              if (kind == 0) launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, v, nullptr, s);
+              if (kind == 0) launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, v, nullptr, StepTurn{}, s);
               else launch_kernel_mix(kind, a_low, v, s);
               cudaEventRecord(e1, s);
               CK(cudaEventSynchronize(e1));
@@ -1757,18 +1840,19 @@ static int enqueue_rk3_steps(swe_ctx* c, int nsteps) {
   CK(cudaEventRecord(c->t0, c->stream));
   // the mixed stage 1 takes alpha from k_dt_mix: one k_node launch fewer
   const long long per_step = 3LL * kLaunchesPerStage + kLaunchesPerStepExtra -
-                             (is_mixed(c) ? 1 : 0) + (c->n_gauges ? 1 : 0);
+                             (is_mixed(c) ? 1 : 0) + (turn_in_dt(c) ? 0 : 1) + (c->n_gauges ? 2 : 0);
+  const long long per_graph = c->n_gauges ? 0 : 1;   // k_step_end
   if (nsteps >= chunk && chunk > 1) {
     for (int k = 0; k + chunk <= nsteps; k += chunk) {
       CK(cudaGraphLaunch(c->gexec, c->stream));
-      launches += per_step * chunk;
+      launches += per_step * chunk + per_graph;
     }
   }
   const int rem = chunk > 1 ? nsteps % chunk : nsteps;
   if (rem && !c->gexec1 && (rc = capture_steps(c, 1, &c->gexec1))) return rc;
   for (int k = 0; k < rem; k++) {
     CK(cudaGraphLaunch(c->gexec1, c->stream));
-    launches += per_step;
+    launches += per_step + per_graph;
   }
   CK(cudaEventRecord(c->t1, c->stream));
   CK(cudaGetLastError());
@@ -1826,7 +1910,7 @@ SWE_API int swe_profile_kernels(swe_ctx* c, int nsteps, double* ms_out) {
   KernelEvents kev;
   for (int k = 0; k < 10; k++) CK(cudaEventCreate(&kev.ev[k]));
   double acc[SWE_NKERNELS] = {0, 0, 0, 0, 0};
-  for (int n = 0; n < nsteps; n++) enqueue_step(c, &kev, acc);
+  for (int n = 0; n < nsteps; n++) enqueue_step(c, false, true, &kev, acc);
   CK(cudaStreamSynchronize(c->stream));
   for (int k = 0; k < 10; k++) cudaEventDestroy(kev.ev[k]);
   ms_out[0] = acc[0] / nsteps;

@@ -40,6 +40,57 @@ __host__ __device__ inline void inst_set_dt(InstState& s, double dt) {
   s.inv_dtf = (float)s.inv_dt;
 }
 
+// The turn between two time steps: it closes the step before (end_prev: time
+// = to + dt, main.f90:91) and opens the next (DO WHILE(time < Tfinal), dt =
+// CFL / max, main.f90:61, 173; the fixed dt = 2.5e-2 of the Malpasset case,
+// main.f90:67-69).  The last block of k_dt runs it where k_dt is a few waves
+// (ticket not null: the count of its blocks that are done); the fence and the
+// ticket cost a block more than a launch of its own costs a large grid (2k
+// nodes: 46 -> 43 us per step; 4M nodes: k_dt 161 -> 192 us).
+struct StepTurn {
+  unsigned* ticket;
+  int n_inst, end_prev;
+};
+__device__ __forceinline__ void turn_instance(const StepTurn& t, const InstConst& c, InstState& s) {
+  if (s.done) return;
+  if (t.end_prev) {
+    s.time = s.time + s.dt;
+    s.steps += 1;
+  }
+  if (!(s.time < s.t_final)) {
+    s.done = 1;
+    return;
+  }
+  const double mx = __longlong_as_double((long long)__ldcg(&s.maxd_bits));   // other SMs' atomics: from L2
+  inst_set_dt(s, c.type_test == 9 ? 2.5e-2 : c.cfl * 1 / mx);
+  s.maxd_bits = 0ull;
+}
+__device__ __forceinline__ void step_turn(const StepTurn& t, const InstConst* C, InstState* St) {
+  if (!t.ticket) return;
+  __shared__ bool last;
+  __syncthreads();                               // this block's maxima ...
+  if (threadIdx.x == 0) {
+    __threadfence();                             // ... before its ticket
+    last = atomicAdd(t.ticket, 1u) == gridDim.x - 1;
+    if (last) __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int b = threadIdx.x; b < t.n_inst; b += blockDim.x) turn_instance(t, C[b], St[b]);
+  if (threadIdx.x == 0) *t.ticket = 0u;
+}
+
+// Programmatic dependent launch: a kernel launched so may start while the
+// previous kernel's last blocks still run; pdl_trigger lets its dependents
+// start, pdl_wait waits until the previous grid has completed and its writes
+// are visible.  Completion is transitive (every kernel waits before it can
+// exit), so outputs of any earlier kernel are visible after the wait.  Without
+// the launch attribute both do nothing.  What an earlier kernel writes is read
+// through pointers without __restrict__: a restrict pointer's loads may be moved
+// above the wait.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The SELL-32 edge graph (see swe_setup.hpp).  Entry k of row r is at
 // slice_ptr[r>>5] + 32*k + (r&31); entries are the off-diagonal CSR entries
 // in reference order, the diagonal (c_ii) is stored per row and belongs

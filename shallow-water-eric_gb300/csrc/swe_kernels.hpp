@@ -1,5 +1,7 @@
 // Declarations shared by the kernel translation units and the C-ABI layer.
 #pragma once
+#include <cstdlib>
+
 #include "swe_device.cuh"
 
 namespace swe {
@@ -64,7 +66,7 @@ struct StageArgs {
   unsigned* err;
   int block;
   int entropy = 0;   // some instance uses 'entropy_visc': launch k_entropy
-  int fused = 0;     // every instance runs 'fct' with the roundoff fix: the 'fct' row kernels
+  int fused = 0;     // every instance runs 'fct' or 'viscous' 'type2' with the roundoff fix: the 'fct' row kernels
   int S = 3;
   const double* dij_in = nullptr;   // stage 1: d_ij of k_dt on the same state (bit-identical)
   int skip_node = 0;                // stage 1: k_node already ran on this state (before k_dt)
@@ -108,12 +110,37 @@ struct KernelEvents {
   cudaEvent_t ev[10];
 };
 
+// Launch of a stage kernel with programmatic stream serialization (the
+// kernels wait for their predecessor themselves, pdl_wait); SWE_PDL=0 makes
+// it an ordinary launch.
+inline bool pdl_enabled() {
+  static const int on = [] {
+    const char* e = getenv("SWE_PDL");
+    return (e && e[0] == '0') ? 0 : 1;
+  }();
+  return on != 0;
+}
+template <typename... KArgs, typename... Args>
+static void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* kev = nullptr);
 // launch_node_f64: per-node arrays of the state a.u; launch_dt_f64 reads them (node)
 void launch_node_f64(const StageArgs& a, cudaStream_t s);
 void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
-                   double* d_out, double* dii_out, unsigned* err, int block, cudaStream_t s);
-void launch_step_begin(const InstConst* C, InstState* St, int n_inst, cudaStream_t s);
+                   double* d_out, double* dii_out, unsigned* err, int block, const StepTurn& turn, cudaStream_t s);
+void launch_step_turn(const StepTurn& t, const InstConst* C, InstState* St, cudaStream_t s);
 void launch_step_end(InstState* St, int n_inst, cudaStream_t s);
 void launch_reset_counters(InstState* St, int n_inst, cudaStream_t s);
 void launch_fct_positivity_f64(const Graph& G, const InstConst* C, const double* unext, const double* mat,
@@ -147,7 +174,7 @@ size_t tile_smem_max(const TileCtl& tc, bool d);
 void launch_kernel_mix(int kind, const StageArgsMix& a, const KernelTune& t, cudaStream_t s);
 bool kind_has_tiles(int kind);   // kernel kinds with a shared-memory tile variant
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,
-                   unsigned* err, const KernelTune& t, const TileCtl* tiles, cudaStream_t s);
+                   unsigned* err, const KernelTune& t, const TileCtl* tiles, const StepTurn& turn, cudaStream_t s);
 void launch_refresh_eta(const Graph& G, StateMix u, cudaStream_t s);
 
 // Diagnostics (swe_diag.cu): field index kFieldH32 selects h^(3/2)
@@ -165,6 +192,6 @@ void launch_norms(int field, int precision, const StateF64& a, const StateMix& m
 
 // kernels launched per stage / per step (for launch accounting)
 constexpr int kLaunchesPerStage = 4;
-constexpr int kLaunchesPerStepExtra = 3;   // k_dt, k_step_begin, k_step_end
+constexpr int kLaunchesPerStepExtra = 1;   // k_dt (and k_step_turn on large meshes; k_step_end ends a captured graph)
 
 }  // namespace swe

@@ -62,7 +62,7 @@ __device__ __forceinline__ void sgn_node_f64(const InstConst& c, double m, doubl
 // per entry: the flux products v u_q, h + z, 1/h, the SGN pressure and the
 // FP32 shadow of lambda_row.
 // ---------------------------------------------------------------------------
-__global__ void k_node_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
+__global__ void k_node_f64(Graph G, const InstConst* C, const InstState* St,
                            StateF64 u, NodeF64 nd) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -317,10 +317,10 @@ __device__ __forceinline__ void smb_rows_f64(const Graph& G, const InstConst& c,
 // (:202-210), smb_2 + entropy residual (:825-878).  Writes dL/muL per entry,
 // uL per row, res per row, fix_roundoff-free low-order h.
 // ---------------------------------------------------------------------------
-__global__ void k_low_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
+__global__ void k_low_f64(Graph G, const InstConst* C, const InstState* St,
                           StateF64 u, NodeF64 nd, double* __restrict__ dL, double* __restrict__ muL,
                           double* __restrict__ dLii, double* __restrict__ muLii, StateF64 uL,
-                          double* __restrict__ res, const double* __restrict__ dij_in, unsigned* __restrict__ err) {
+                          double* __restrict__ res, const double* dij_in, unsigned* __restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
   const int L = G.len[r];
@@ -473,9 +473,9 @@ __global__ void k_low_f64(Graph G, const InstConst* __restrict__ C, const InstSt
 // (compute_fct_matrix :721-748), check_hmin of the low-order state (:271) and
 // R^-_i of FCT_positivity (SOURCES/fct.f90:15-30).
 // ---------------------------------------------------------------------------
-__global__ void k_fct_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                          StateF64 u, const double* __restrict__ dL, const double* __restrict__ muL,
-                          StateF64 uL, const double* __restrict__ res, double* __restrict__ fct,
+__global__ void k_fct_f64(Graph G, const InstConst* C, const InstState* St,
+                          StateF64 u, const double* dL, const double* muL,
+                          StateF64 uL, const double* res, double* __restrict__ fct,
                           double* __restrict__ rminus, unsigned* __restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -565,10 +565,10 @@ __device__ __forceinline__ void finish_row_f64(const Graph& G, const InstConst& 
 //   rk_stage 2: out = (3 u0 + unext)/4, Dirichlet
 //   rk_stage 3: out = (u0 + 2 unext)/3, Dirichlet
 // ---------------------------------------------------------------------------
-__global__ void k_update_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                             StateF64 u, const double* __restrict__ dL, const double* __restrict__ muL,
-                             StateF64 uL, const double* __restrict__ res, const double* __restrict__ fct,
-                             const double* __restrict__ rminus, StateF64 u0, StateF64 out, int rk_stage,
+__global__ void k_update_f64(Graph G, const InstConst* C, const InstState* St,
+                             StateF64 u, const double* dL, const double* muL,
+                             StateF64 uL, const double* res, const double* fct,
+                             const double* rminus, StateF64 u0, StateF64 out, int rk_stage,
                              double* __restrict__ lij_out, unsigned* __restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -624,10 +624,10 @@ __global__ void k_update_f64(Graph G, const InstConst* __restrict__ C, const Ins
 // u = u(1 + dt fix/m) + dt rk/m, check_hmin (:285), then the RK combination
 // and bdy like k_update.
 // ---------------------------------------------------------------------------
-__global__ void k_entropy_f64(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                              StateF64 u, NodeF64 nd, const double* __restrict__ dL, const double* __restrict__ muL,
-                              const double* __restrict__ dLii, const double* __restrict__ muLii,
-                              const double* __restrict__ res, StateF64 u0, StateF64 out, int rk_stage,
+__global__ void k_entropy_f64(Graph G, const InstConst* C, const InstState* St,
+                              StateF64 u, NodeF64 nd, const double* dL, const double* muL,
+                              const double* dLii, const double* muLii,
+                              const double* res, StateF64 u0, StateF64 out, int rk_stage,
                               unsigned* __restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -660,8 +660,9 @@ __global__ void k_entropy_f64(Graph G, const InstConst* __restrict__ C, const In
 }
 
 // ---------------------------------------------------------------------------
-// The 'fct' row kernels (every instance of the context runs 'fct' with the
-// roundoff fix; others take the general kernels above).  The FP64 unit bounds
+// The 'fct' row kernels (every instance of the context runs 'fct' or 'viscous'
+// 'type2' with the roundoff fix; others take the general kernels above).  A
+// 'viscous' instance stops at the low-order state.  The FP64 unit bounds
 // them: an SM retires a warp's FP64 instruction in 16 cycles, so they spend
 // memory (idle at 1-3% of its rate in the general kernels) to form every
 // FP64 value once:
@@ -687,9 +688,9 @@ __device__ __forceinline__ double rat_f64(double H, double h, double rh) {
 
 template <int S>
 __global__ void __launch_bounds__(128, 4)
-k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St, StateF64 u, NodeF64 nd,
+k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 nd,
           double* __restrict__ dL, double* __restrict__ muL, double* __restrict__ dLii, double* __restrict__ muLii,
-          StateF64 uL, double* __restrict__ res, double* __restrict__ ab, const double* __restrict__ dij_in,
+          StateF64 uL, double* __restrict__ res, double* __restrict__ ab, const double* dij_in,
           int want_diag, int64_t n_entries, unsigned* __restrict__ err) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -708,6 +709,7 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
   const double zi = G.bath[r], etai = nd.eta[r], rhi = nd.rh[r], ai = nd.alpha[r];
   const double w1i = nd.v1[r], w2i = nd.w2[r], ghi = g * ui[0];
   const bool wet_i = !le_nn(ui[0], htiny);
+  const bool fct = c.visc == VISC_FCT;          // the right-hand side of smb_2 too, for the residual
   // the diagonal's terms: -c_ii.F_i and the topography residue
   double Dq[S], Dfix, tdx, tdy;
   {
@@ -730,11 +732,14 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
   for (int k = 0; k <= L; k++) {
     if (k == dp) {                              // the diagonal's place in the row
       fix = fix - Dfix;
-      rk2[0] = rk2[0] - Dq[0];
 #pragma unroll
-      for (int q = 1; q < S; q++) { rk[q] = rk[q] - Dq[q]; rk2[q] = rk2[q] - Dq[q]; }
+      for (int q = 1; q < S; q++) rk[q] = rk[q] - Dq[q];
       rk[1] = rk[1] - tdx; rk[2] = rk[2] - tdy;
-      rk2[1] = rk2[1] - tdx; rk2[2] = rk2[2] - tdy;
+      if (fct) {
+#pragma unroll
+        for (int q = 0; q < S; q++) rk2[q] = rk2[q] - Dq[q];
+        rk2[1] = rk2[1] - tdx; rk2[2] = rk2[2] - tdy;
+      }
     }
     if (k == L) break;
     const int64_t e = base + 32 * k;
@@ -787,6 +792,7 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
     const double pij = 1.0 - qij, pji = 1.0 - qji;
 #pragma unroll
     for (int q = 0; q < S; q++) {
+      if (q == 0 && !fct) continue;
       double x2 = cxe * nd.flux[(int64_t)(2 * q) * nr + j];
       if (S == 3) x2 = x2 + cye * nd.flux[(int64_t)(2 * q + 1) * nr + j];
       double A, B = 0.0, mB = 0.0;
@@ -798,10 +804,12 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
         mB = mu * B;
       }
       const double dA = d * A;
-      ab[(int64_t)(2 * q) * n_entries + e] = A;
-      ab[(int64_t)(2 * q + 1) * n_entries + e] = B;
-      rk2[q] = rk2[q] - x2 + dA;
-      if (!flat) rk2[q] = rk2[q] + mB;
+      if (fct) {
+        ab[(int64_t)(2 * q) * n_entries + e] = A;
+        ab[(int64_t)(2 * q + 1) * n_entries + e] = B;
+        rk2[q] = rk2[q] - x2 + dA;
+        if (!flat) rk2[q] = rk2[q] + mB;
+      }
       if (q > 0) {
         rk[q] = rk[q] - x2;
         if (wet) {
@@ -884,6 +892,7 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
   uL.h[r] = ul[0]; uL.q1[r] = ul[1]; uL.q2[r] = ul[2];
   if (S == 5) { uL.q3[r] = ul[3]; uL.q4[r] = ul[4]; }
   if (bad) atomicOr(err, ERRB_DELTA);
+  if (!fct) return;
   // entropy residual (update.f90:838-868); Entprime(4:5) are 0
   double rm[3], un_[3];
 #pragma unroll
@@ -909,9 +918,9 @@ k_low_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict_
 
 // f_ij and R^-_i from the stored differences: five FP64 instructions per
 // entry (the general k_fct_f64 forms the rats again: 42).
-__global__ void k_fct_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                          const double* __restrict__ dL, const double* __restrict__ muL, const double* __restrict__ hL,
-                          const double* __restrict__ res, const double* __restrict__ ab, double* __restrict__ fct,
+__global__ void k_fct_fct(Graph G, const InstConst* C, const InstState* St,
+                          const double* dL, const double* muL, const double* hL,
+                          const double* res, const double* ab, double* __restrict__ fct,
                           double* __restrict__ rminus, int64_t n_entries, unsigned* __restrict__ err) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
@@ -919,6 +928,7 @@ __global__ void k_fct_fct(Graph G, const InstConst* __restrict__ C, const InstSt
   if (L == 0) return;
   const int b = G.slice_inst[r >> 5];
   if (St[b].done) return;
+  if (C[b].visc != VISC_FCT) return;
   const int64_t base = entry_base(G, r);
   const double resi = res[r];
   double P = -1.e-15;
@@ -943,10 +953,10 @@ __global__ void k_fct_fct(Graph G, const InstConst* __restrict__ C, const InstSt
 // l_ij, the limited antidiffusion from the stored differences, and the end of
 // the stage (see k_update_f64 for rk_stage).
 template <int S>
-__global__ void k_update_fct(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                             const double* __restrict__ dL, const double* __restrict__ muL, StateF64 uL,
-                             const double* __restrict__ res, const double* __restrict__ fct,
-                             const double* __restrict__ rminus, const double* __restrict__ ab, StateF64 u0,
+__global__ void k_update_fct(Graph G, const InstConst* C, const InstState* St,
+                             const double* dL, const double* muL, StateF64 uL,
+                             const double* res, const double* fct,
+                             const double* rminus, const double* ab, StateF64 u0,
                              StateF64 out, int rk_stage, double* __restrict__ lij_out, int64_t n_entries,
                              unsigned* __restrict__ err) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -958,11 +968,12 @@ __global__ void k_update_fct(Graph G, const InstConst* __restrict__ C, const Ins
   if (st.done) return;
   const InstConst& c = C[b];
   const int64_t base = entry_base(G, r);
-  const double resi = res[r], Ri = rminus[r];
+  const bool fct_mode = c.visc == VISC_FCT;
+  const double resi = fct_mode ? res[r] : 0.0, Ri = fct_mode ? rminus[r] : 0.0;
   double xx[S];
 #pragma unroll
   for (int q = 0; q < S; q++) xx[q] = 0.0;
-  for (int k = 0; k < L; k++) {
+  for (int k = 0; k < (fct_mode ? L : 0); k++) {
     const int64_t e = base + 32 * k;
     const int j = G.col[e];
     const double l = (bits64(fct[e]) << 1) == 0 || bits64(fct[e]) > 0 ? rminus[j] : Ri;   // f >= 0
@@ -979,7 +990,7 @@ __global__ void k_update_fct(Graph G, const InstConst* __restrict__ C, const Ins
   double un[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int q = 0; q < S; q++) un[q] = comp_f64(uL, q, r) + dt * div_known(xx[q], m, im);
-  finish_row_f64(G, c, st, r, S, un, true, rk_stage, u0, out, err);
+  finish_row_f64(G, c, st, r, S, un, fct_mode, rk_stage, u0, out, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -987,8 +998,9 @@ __global__ void k_update_fct(Graph G, const InstConst* __restrict__ C, const Ins
 // max |d_ii|/m_i (main.f90:166-174), per instance.  d_out (nullable)
 // receives every d_ij.
 // ---------------------------------------------------------------------------
-__global__ void k_dt_f64(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St, StateF64 u, NodeF64 nd,
-                         double* __restrict__ d_out, double* __restrict__ dii_out, unsigned* __restrict__ err) {
+__global__ void k_dt_f64(Graph G, const InstConst* C, InstState* St, StateF64 u, NodeF64 nd,
+                         double* __restrict__ d_out, double* __restrict__ dii_out, unsigned* __restrict__ err,
+                         StepTurn turn) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double val = 0.0;
   if (r < G.n_rows && G.len[r] > 0 && !St[G.slice_inst[r >> 5]].done) {
@@ -1019,24 +1031,18 @@ __global__ void k_dt_f64(Graph G, const InstConst* __restrict__ C, InstState* __
     const int bw = G.slice_inst[r0 >> 5];
     if (!St[bw].done && val > 0.0) atomicMax(&St[bw].maxd_bits, (unsigned long long)__double_as_longlong(val));
   }
+  step_turn(turn, C, St);
 }
 
-// Start of a time step: DO WHILE(time < Tfinal) and dt = CFL/max (main.f90:61,
-// 173), or the fixed dt = 2.5e-2 of the Malpasset case (type 9, main.f90:67-69)
-__global__ void k_step_begin(const InstConst* __restrict__ C, InstState* __restrict__ St, int n_inst) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_inst) return;
-  InstState& s = St[b];
-  if (s.done) return;
-  if (!(s.time < s.t_final)) { s.done = 1; return; }
-  double mx = __longlong_as_double((long long)s.maxd_bits);
-  inst_set_dt(s, C[b].type_test == 9 ? 2.5e-2 : C[b].cfl * 1 / mx);
-  s.maxd_bits = 0ull;
+// The turn between two steps as a kernel of its own
+__global__ void k_step_turn(StepTurn t, const InstConst* C, InstState* St) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < t.n_inst) turn_instance(t, C[b], St[b]);
 }
 
 // Start of a swe_rk3_steps call: step counters and the lambda_max maximum
 // restart (the instances' time, dt and done flags carry over)
-__global__ void k_reset_counters(InstState* __restrict__ St, int n_inst) {
+__global__ void k_reset_counters(InstState* St, int n_inst) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_inst) return;
   St[b].steps = 0;
@@ -1044,7 +1050,7 @@ __global__ void k_reset_counters(InstState* __restrict__ St, int n_inst) {
 }
 
 // End of a time step: time = to + dt (main.f90:91)
-__global__ void k_step_end(InstState* __restrict__ St, int n_inst) {
+__global__ void k_step_end(InstState* St, int n_inst) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_inst) return;
   InstState& s = St[b];
@@ -1127,62 +1133,69 @@ static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) 
 #define EV_BEGIN(k) if (kev) cudaEventRecord(kev->ev[2 * (k)], s)
 #define EV_END(k) if (kev) cudaEventRecord(kev->ev[2 * (k) + 1], s)
 
+// Ordinary launches: with programmatic dependent launch the next kernel's
+// blocks are placed while this one's still hold their SMs, and the FP64 unit of
+// an SM that got two is the step's time (10k nodes: 357 us against 253).
+template <typename... KArgs, typename... Args>
+static void launch_full(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  kern<<<grid, block, smem, s>>>(static_cast<KArgs>(args)...);
+}
+
 void launch_node_f64(const StageArgs& a, cudaStream_t s) {
   const NodeF64 nd = node_of(a.w);
-  k_node_f64<<<nblk(a.G.n_rows, a.block), a.block, 0, s>>>(a.G, a.C, a.St, a.u, nd);
+  launch_full(k_node_f64, nblk(a.G.n_rows, a.block), a.block, 0, s, a.G, a.C, a.St, a.u, nd);
 }
 
 void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* kev) {
   const int bs = a.block;
   const NodeF64 nd = node_of(a.w);
   EV_BEGIN(1);
-  if (!a.skip_node) k_node_f64<<<nblk(a.G.n_rows, bs), bs, 0, s>>>(a.G, a.C, a.St, a.u, nd);
+  if (!a.skip_node) launch_full(k_node_f64, nblk(a.G.n_rows, bs), bs, 0, s, a.G, a.C, a.St, a.u, nd);
   EV_END(1); EV_BEGIN(2);
   const unsigned nb = nblk(a.G.n_rows, bs);
   if (a.fused) {
     const int64_t ne = a.w.n_entries;
     const int diag = a.rk_stage == 0;            // swe_euler_intermediates hands out the diagonals
     if (a.S == 5)
-      k_low_fct<5><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
+      launch_full(k_low_fct<5>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
                                      a.w.ab, a.dij_in, diag, ne, a.err);
     else
-      k_low_fct<3><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
+      launch_full(k_low_fct<3>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
                                      a.w.ab, a.dij_in, diag, ne, a.err);
     EV_END(2); EV_BEGIN(3);
-    k_fct_fct<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
+    launch_full(k_fct_fct, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
                                 a.err);
     EV_END(3); EV_BEGIN(4);
     if (a.S == 5)
-      k_update_fct<5><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
+      launch_full(k_update_fct<5>, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
                                         a.u0, a.out, a.rk_stage, a.lij_out, ne, a.err);
     else
-      k_update_fct<3><<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
+      launch_full(k_update_fct<3>, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
                                         a.u0, a.out, a.rk_stage, a.lij_out, ne, a.err);
     EV_END(4);
     return;
   }
-  k_low_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res, a.dij_in,
+  launch_full(k_low_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res, a.dij_in,
                               a.err);
   EV_END(2); EV_BEGIN(3);
-  k_fct_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.err);
+  launch_full(k_fct_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.err);
   EV_END(3); EV_BEGIN(4);
-  k_update_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.u0, a.out,
+  launch_full(k_update_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.u0, a.out,
                                  a.rk_stage, a.lij_out, a.err);
   if (a.entropy)
-    k_entropy_f64<<<nb, bs, 0, s>>>(a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.res, a.u0, a.out,
+    launch_full(k_entropy_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.res, a.u0, a.out,
                                     a.rk_stage, a.err);
   EV_END(4);
 }
 
 void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
-                   double* d_out, double* dii_out, unsigned* err, int block, cudaStream_t s) {
-  k_dt_f64<<<nblk(G.n_rows, block), block, 0, s>>>(G, C, St, u, node_of(node), d_out, dii_out, err);
+                   double* d_out, double* dii_out, unsigned* err, int block, const StepTurn& turn, cudaStream_t s) {
+  launch_full(k_dt_f64, nblk(G.n_rows, block), block, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
 }
 
-void launch_step_begin(const InstConst* C, InstState* St, int n_inst, cudaStream_t s) {
-  k_step_begin<<<nblk(n_inst, 128), 128, 0, s>>>(C, St, n_inst);
+void launch_step_turn(const StepTurn& t, const InstConst* C, InstState* St, cudaStream_t s) {
+  k_step_turn<<<nblk(t.n_inst, 128), 128, 0, s>>>(t, C, St);
 }
-
 void launch_step_end(InstState* St, int n_inst, cudaStream_t s) {
   k_step_end<<<nblk(n_inst, 128), 128, 0, s>>>(St, n_inst);
 }

@@ -49,18 +49,6 @@ namespace swe {
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
-// Programmatic dependent launch: the stage kernels are launched so that a
-// kernel's blocks may start while the previous kernel's last blocks still
-// run.  Each kernel lets its dependents launch at once (pdl_trigger), may
-// prefetch data no kernel writes (the graph), then waits in pdl_wait until
-// the previous grid has completed and its writes are visible, before it
-// reads anything a kernel produced or writes anything.  Completion is
-// transitive (every kernel waits before it can exit), so outputs of any
-// earlier kernel are visible after the wait.  Without the launch attribute
-// both instructions do nothing.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // c . v with an explicit rounding sequence.  The low-order mass flux
 // (mu_ij - c.v_j) h_j is non-negative only if mu_ij >= c.v_j holds bit for
 // bit, so c.v_j is formed once per entry with a fixed rounding.
@@ -520,8 +508,8 @@ __device__ __forceinline__ float alpha_from(float num, float denom) {
 
 // k_node_mix: alpha_i from the FP32 depth.
 template <int B, class Nb>
-__device__ __forceinline__ void node_row(int r, const RowHead& hd, const InstConst* __restrict__ C,
-                                         const InstState* __restrict__ St, float* __restrict__ alpha_out,
+__device__ __forceinline__ void node_row(int r, const RowHead& hd, const InstConst* C,
+                                         const InstState* St, float* __restrict__ alpha_out,
                                          const Nb& nb) {
   const int L = hd.L;
   if (L == 0) return;
@@ -553,8 +541,8 @@ __device__ __forceinline__ void node_row(int r, const RowHead& hd, const InstCon
 }
 
 template <int B>
-__global__ void __launch_bounds__(256) k_node_mix(Graph G, const InstConst* __restrict__ C,
-                                                  const InstState* __restrict__ St, StateMix u,
+__global__ void __launch_bounds__(256) k_node_mix(Graph G, const InstConst* C,
+                                                  const InstState* St, StateMix u,
                                                   float* __restrict__ alpha_out) {
   pdl_trigger();
   pdl_wait();
@@ -564,8 +552,8 @@ __global__ void __launch_bounds__(256) k_node_mix(Graph G, const InstConst* __re
 }
 
 template <int T>
-__global__ void __launch_bounds__(T) k_node_tile(Graph G, const InstConst* __restrict__ C,
-                                                 const InstState* __restrict__ St, StateMix u,
+__global__ void __launch_bounds__(T) k_node_tile(Graph G, const InstConst* C,
+                                                 const InstState* St, StateMix u,
                                                  float* __restrict__ alpha_out, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
@@ -598,8 +586,8 @@ __global__ void __launch_bounds__(T) k_node_tile(Graph G, const InstConst* __res
 // FCT: every instance runs 'fct' with the roundoff fix and alpha_limit (the
 // usual run), so the mode tests fall away.
 template <int B, bool LAMIN, bool D, bool FCT, class Nb>
-__device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
-                                        const InstState* __restrict__ St, const StateMix& u, float2* __restrict__ dmu,
+__device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G, const InstConst* C,
+                                        const InstState* St, const StateMix& u, float2* __restrict__ dmu,
                                         const WorkMix& w, float* __restrict__ res, unsigned* __restrict__ err,
                                         const Nb& nb) {
   const int L = hd.L;
@@ -818,9 +806,9 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
 }
 
 template <int B, bool LAMIN, int MINB, bool D>
-__global__ void __launch_bounds__(256, MINB) k_low_mix(Graph G, const InstConst* __restrict__ C,
-                                                       const InstState* __restrict__ St, StateMix u,
-                                                       const float* __restrict__ alpha, float2* __restrict__ dmu,
+__global__ void __launch_bounds__(256, MINB) k_low_mix(Graph G, const InstConst* C,
+                                                       const InstState* St, StateMix u,
+                                                       const float* alpha, float2* __restrict__ dmu,
                                                        WorkMix w, float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
@@ -830,9 +818,9 @@ __global__ void __launch_bounds__(256, MINB) k_low_mix(Graph G, const InstConst*
 }
 
 template <int T, int S, bool LAMIN, int MINB, bool D, bool FCT>
-__global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const InstConst* __restrict__ C,
-                                                                 const InstState* __restrict__ St, StateMix u,
-                                                                 const float* __restrict__ alpha,
+__global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const InstConst* C,
+                                                                 const InstState* St, StateMix u,
+                                                                 const float* alpha,
                                                                  float2* __restrict__ dmu, WorkMix w,
                                                                  float* __restrict__ res, unsigned* __restrict__ err,
                                                                  TileCtl tc) {
@@ -878,7 +866,7 @@ __global__ void __launch_bounds__(T, MINB* (256 / T)) k_low_tile(Graph G, const 
 // other instances of a batch run low_row.  3-component systems only.
 template <bool D>
 __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const InstConst& c, const InstState& st,
-                                              const StateMix& u, const float* __restrict__ alpha,
+                                              const StateMix& u, const float* alpha,
                                               float2* __restrict__ dmu, const WorkMix& w, unsigned* __restrict__ err) {
   const NbGlobal nb{G, u, u.nq, alpha, nullptr, nullptr};
   const int L = G.len[r];
@@ -946,9 +934,9 @@ __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const I
 }
 
 template <bool D>
-__global__ void __launch_bounds__(256) k_low_type1(Graph G, const InstConst* __restrict__ C,
-                                                   const InstState* __restrict__ St, StateMix u,
-                                                   const float* __restrict__ alpha, float2* __restrict__ dmu, WorkMix w,
+__global__ void __launch_bounds__(256) k_low_type1(Graph G, const InstConst* C,
+                                                   const InstState* St, StateMix u,
+                                                   const float* alpha, float2* __restrict__ dmu, WorkMix w,
                                                    float* __restrict__ res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
@@ -980,8 +968,8 @@ __device__ __forceinline__ float fct_entry(float d0, float m0, float rij, float 
 // k_fct_mix: f_ij and the limiter R^-_i (fct.f90:15-30): P^- = sum f^- - 1e-15,
 // Q^- = -m h^L/dt, R^- = min(Q^-/P^-, 1), 0 where m h^L/dt <= htiny.
 template <int B, bool D, class Nb>
-__device__ __forceinline__ void fct_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
-                                        const InstState* __restrict__ St, const float2* __restrict__ dmu,
+__device__ __forceinline__ void fct_row(int r, const RowHead& hd, const Graph& G, const InstConst* C,
+                                        const InstState* St, const float2* dmu,
                                         const WorkMix& w, unsigned* __restrict__ err, const Nb& nb) {
   const int L = hd.L;
   if (L == 0) return;
@@ -1049,9 +1037,9 @@ __device__ __forceinline__ void fct_row(int r, const RowHead& hd, const Graph& G
 }
 
 template <int B, bool D>
-__global__ void __launch_bounds__(256) k_fct_mix(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                                                 StateMix u, const float2* __restrict__ dmu, WorkMix w,
-                                                 const float* __restrict__ res, unsigned* __restrict__ err) {
+__global__ void __launch_bounds__(256) k_fct_mix(Graph G, const InstConst* C, const InstState* St,
+                                                 StateMix u, const float2* dmu, WorkMix w,
+                                                 const float* res, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
   const NbGlobal nb{G, u, u.nq, res, nullptr, nullptr};
@@ -1060,10 +1048,10 @@ __global__ void __launch_bounds__(256) k_fct_mix(Graph G, const InstConst* __res
 }
 
 template <int T, bool D>
-__global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* __restrict__ C,
-                                                const InstState* __restrict__ St, StateMix u,
-                                                const float2* __restrict__ dmu, WorkMix w,
-                                                const float* __restrict__ res, unsigned* __restrict__ err, TileCtl tc) {
+__global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* C,
+                                                const InstState* St, StateMix u,
+                                                const float2* dmu, WorkMix w,
+                                                const float* res, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
   const TileSmem sm = tile_smem<T, 3, 3, D, false>(tile_mem, tc);
@@ -1134,8 +1122,8 @@ __device__ __forceinline__ void finish_mix(const Graph& G, const InstConst& c, c
 // FCT: every instance runs 'fct'.
 template <int B, bool D, bool FCT, class Nb>
 __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph& G,
-                                           const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                                           const StateMix& u, const float2* __restrict__ dmu, const WorkMix& w,
+                                           const InstConst* C, const InstState* St,
+                                           const StateMix& u, const float2* dmu, const WorkMix& w,
                                            const StateMix& u0, const StateMix& out, int rk_stage,
                                            unsigned* __restrict__ err, const Nb& nb) {
   const int L = hd.L;
@@ -1238,9 +1226,9 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
 }
 
 template <int B, bool D>
-__global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* __restrict__ C, const InstState* __restrict__ St,
-                                                    StateMix u, const float2* __restrict__ dmu, WorkMix w,
-                                                    const float* __restrict__ res, StateMix u0, StateMix out,
+__global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* C, const InstState* St,
+                                                    StateMix u, const float2* dmu, WorkMix w,
+                                                    const float* res, StateMix u0, StateMix out,
                                                     int rk_stage, unsigned* __restrict__ err) {
   pdl_trigger();
   pdl_wait();
@@ -1250,10 +1238,10 @@ __global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* __
 }
 
 template <int T, int S, bool D, bool FCT>
-__global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* __restrict__ C,
-                                                   const InstState* __restrict__ St, StateMix u,
-                                                   const float2* __restrict__ dmu, WorkMix w,
-                                                   const float* __restrict__ res, StateMix u0, StateMix out,
+__global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* C,
+                                                   const InstState* St, StateMix u,
+                                                   const float2* dmu, WorkMix w,
+                                                   const float* res, StateMix u0, StateMix out,
                                                    int rk_stage, unsigned* __restrict__ err, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
@@ -1291,8 +1279,8 @@ __global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* __r
 // reused by stage 1's k_low_mix) and alpha_i (alpha_out, stage 1's
 // k_node_mix), when those are non-null.
 template <int B, class Nb>
-__device__ __forceinline__ float dt_row(int r, const RowHead& hd, const Graph& G, const InstConst* __restrict__ C,
-                                        const InstState* __restrict__ St, float* __restrict__ dlam,
+__device__ __forceinline__ float dt_row(int r, const RowHead& hd, const Graph& G, const InstConst* C,
+                                        const InstState* St, float* __restrict__ dlam,
                                         float* __restrict__ alpha_out, unsigned* __restrict__ err, const Nb& nb) {
   const int L = hd.L;
   if (L == 0) return 0.f;
@@ -1345,7 +1333,7 @@ __device__ __forceinline__ float dt_row(int r, const RowHead& hd, const Graph& G
 
 // Warp max of |d_ii| / m_i into the instance's maximum (the 32 rows of a warp
 // are one slice, so one instance).  A maximum does not depend on the order.
-__device__ __forceinline__ void dt_reduce(float val, int64_t r, const Graph& G, InstState* __restrict__ St) {
+__device__ __forceinline__ void dt_reduce(float val, int64_t r, const Graph& G, InstState* St) {
   for (int off = 16; off > 0; off >>= 1) val = fmaxf(val, __shfl_down_sync(0xffffffffu, val, off));
   const int64_t r0 = r & ~(int64_t)31;
   if ((threadIdx.x & 31) == 0 && r0 < G.n_rows) {
@@ -1357,8 +1345,8 @@ __device__ __forceinline__ void dt_reduce(float val, int64_t r, const Graph& G, 
 
 // k_dt_mix: FP32 lambda_max, max |d_ii|/m_i per instance (main.f90:166-174).
 template <int B>
-__global__ void __launch_bounds__(256) k_dt_mix(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St, StateMix u,
-                         float* __restrict__ dlam, float* __restrict__ alpha_out, unsigned* __restrict__ err) {
+__global__ void __launch_bounds__(256) k_dt_mix(Graph G, const InstConst* C, InstState* St, StateMix u,
+                         float* __restrict__ dlam, float* __restrict__ alpha_out, unsigned* __restrict__ err, StepTurn turn) {
   pdl_trigger();
   pdl_wait();
   // grid-stride over block-sized row ranges: every lane of a warp runs the
@@ -1368,12 +1356,13 @@ __global__ void __launch_bounds__(256) k_dt_mix(Graph G, const InstConst* __rest
     const int64_t r = rb + threadIdx.x;
     dt_reduce(r < G.n_rows ? dt_row<B>((int)r, row_head(G, r), G, C, St, dlam, alpha_out, err, nb) : 0.f, r, G, St);
   }
+  step_turn(turn, C, St);
 }
 
 template <int T>
-__global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* __restrict__ C, InstState* __restrict__ St,
+__global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* C, InstState* St,
                                                StateMix u, float* __restrict__ dlam, float* __restrict__ alpha_out,
-                                               unsigned* __restrict__ err, TileCtl tc) {
+                                               unsigned* __restrict__ err, StepTurn turn, TileCtl tc) {
   extern __shared__ float4 tile_mem[];
   const Tile t = tile_of<T>(G, tc);
   const TileSmem sm = tile_smem<T, 0, 3, false, false>(tile_mem, tc);
@@ -1392,6 +1381,7 @@ __global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* __restr
   __syncthreads();
   pdl_trigger();
   dt_reduce(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile<3>(t, sm)), t.r, G, St);
+  step_turn(turn, C, St);
 }
 
 // Free surface of the packed node records after a bathymetry change
@@ -1402,31 +1392,6 @@ __global__ void k_refresh_eta(Graph G, StateMix u) {
 }
 
 static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
-
-// Launch of a stage kernel with programmatic stream serialization (the
-// kernels wait for their predecessor themselves, pdl_wait); SWE_PDL=0 makes
-// it an ordinary launch.
-static bool pdl_enabled() {
-  static const int on = [] {
-    const char* e = getenv("SWE_PDL");
-    return (e && e[0] == '0') ? 0 : 1;
-  }();
-  return on != 0;
-}
-template <typename... KArgs, typename... Args>
-static void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
 
 // Grid of a row kernel: one thread per row (mode 0), or a resident grid of
 // mode x (blocks per SM at full occupancy) x SMs whose threads stride over
@@ -1587,11 +1552,11 @@ void launch_stage_mix(const StageArgsMix& a, cudaStream_t s, const KernelEvents*
 }
 
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,
-                   unsigned* err, const KernelTune& t, const TileCtl* tiles, cudaStream_t s) {
+                   unsigned* err, const KernelTune& t, const TileCtl* tiles, const StepTurn& turn, cudaStream_t s) {
   if (t.tiled[0] && tiles) {
-    SWE_TILE_T(*tiles, launch_tile(k_dt_tile<T>, *tiles, G.n_rows, 0, false, false, s, G, C, St, u, dlam, alpha, err));
+    SWE_TILE_T(*tiles, launch_tile(k_dt_tile<T>, *tiles, G.n_rows, 0, false, false, s, G, C, St, u, dlam, alpha, err, turn));
   } else {
-    SWE_DISPATCH_B(t.batch[0], k_dt_mix, G.n_rows, t.block[0], t.grid[0], G, C, St, u, dlam, alpha, err)
+    SWE_DISPATCH_B(t.batch[0], k_dt_mix, G.n_rows, t.block[0], t.grid[0], G, C, St, u, dlam, alpha, err, turn)
   }
 }
 
