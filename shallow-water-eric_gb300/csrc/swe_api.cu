@@ -277,14 +277,13 @@ static bool has_entropy(const swe_ctx* c) {
   return false;
 }
 
-// every instance runs 'fct', or 'viscous' 'type2', with the roundoff fix: the FP64 path's row kernels
+// every instance runs 'fct', 'viscous' 'type2' or 'entropy_visc' with the roundoff fix: the FP64 path's row kernels
 static bool all_fct_rows(const swe_ctx* c) {
   for (const swe_params& p : c->params)
-    if (!p.if_roundoff_fix || p.viscous_type != 2 ||
-        (p.viscosity_type != SWE_VISC_FCT && p.viscosity_type != SWE_VISC_VISCOUS))
-      return false;
+    if (!p.if_roundoff_fix || p.viscous_type != 2 || p.viscosity_type == SWE_VISC_GALERKIN) return false;
   return true;
 }
+// every instance runs 'fct' with the roundoff fix
 static bool all_fct(const swe_ctx* c) {
   for (const swe_params& p : c->params)
     if (p.viscosity_type != SWE_VISC_FCT || !p.if_roundoff_fix) return false;
@@ -823,6 +822,7 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
       StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, stage, nullptr, c->d_err, c->block};
       a.entropy = has_entropy(c);
       a.fused = all_fct_rows(c);
+      a.all_fct = all_fct(c);
       a.S = c->S;
       if (stage == 1) { a.dij_in = c->w.fct; a.skip_node = 1; }
       if (stage == 2) { a.u = c->B; a.out = c->Cs; }
@@ -1212,6 +1212,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
     a.fused = all_fct_rows(c);
+    a.all_fct = all_fct(c);
     a.S = c->S;
     launch_stage_f64(a, c->stream);
   } else {

@@ -324,6 +324,10 @@ __device__ __forceinline__ bool lambda_vacc(T hl, T qxl, T qyl, T ovhl, T sqghl,
 // can matter before they evaluate one in FP64.  Every result keeps the
 // reference's bits (the sign of a zero aside).
 __device__ __forceinline__ long long bits64(double x) { return __double_as_longlong(x); }
+// Marks a block that a warp skips when none of its lanes need it: without side
+// effects the compiler forms both sides of a short branch and selects, which
+// costs FP64 instructions.
+__device__ __forceinline__ void real_branch() { asm volatile("" ::); }
 // MAX(x, 0)
 __device__ __forceinline__ double pos_part(double x) { return bits64(x) > 0 ? x : 0.0; }
 // MAX, MIN of non-negative values
@@ -445,10 +449,12 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
   double f1 = 1.0, v2 = 0.0, ht = 0.0;
   const bool nt = !tr1 || (both && !triv_r);
   if (nt || both) {
+    real_branch();
     const double o2 = need_l ? r.ovh : l.ovh;
     v2 = __dmul_rn(__dadd_rn(__dmul_rn(need_l ? r.q1 : l.q1, nx), __dmul_rn(need_l ? r.q2 : l.q2, ny)), o2);
   }
   if (nt) {
+    real_branch();
     const double vl = need_l ? v1 : v2, vr = need_l ? v2 : v1;
     // ((vl - vr) + 2 sql) + 2 sqr, each product by 2 exact
     const double sd = pos_part(__fma_rn(2.0, r.sq, __fma_rn(2.0, l.sq, __dsub_rn(vl, vr))));
@@ -458,6 +464,7 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
       ht = tmin((t0 * t0) * tmin(l.h, r.h), ht);
     }
     if (!tr1) {
+      real_branch();
       const double x = pos_part(__dmul_rn(__dsub_rn(ht, h1), o1));
       f1 = sqrt(__dmul_rn(__fma_rn(x, 0.5, 1.0), __dadd_rn(1.0, x)));   // x/2 is exact
     }
@@ -465,6 +472,7 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
   double cf = tr1 ? c1 : __dmul_rn(c1, f1);
   double lam = fabs(need_l ? __dsub_rn(v1, cf) : __dadd_rn(v1, cf));
   if (both) {
+    real_branch();
     double f2 = f1;
     if (bits64(l.h) != bits64(r.h)) {                     // equal depths: equal factors
       f2 = 1.0;

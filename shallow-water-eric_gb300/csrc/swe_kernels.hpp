@@ -66,7 +66,8 @@ struct StageArgs {
   unsigned* err;
   int block;
   int entropy = 0;   // some instance uses 'entropy_visc': launch k_entropy
-  int fused = 0;     // every instance runs 'fct' or 'viscous' 'type2' with the roundoff fix: the 'fct' row kernels
+  int fused = 0;     // every instance runs 'fct', 'viscous' 'type2' or 'entropy_visc' with the roundoff fix: the 'fct' row kernels
+  int all_fct = 0;   // every instance runs 'fct' with the roundoff fix
   int S = 3;
   const double* dij_in = nullptr;   // stage 1: d_ij of k_dt on the same state (bit-identical)
   int skip_node = 0;                // stage 1: k_node already ran on this state (before k_dt)

@@ -660,9 +660,10 @@ __global__ void k_entropy_f64(Graph G, const InstConst* C, const InstState* St,
 }
 
 // ---------------------------------------------------------------------------
-// The 'fct' row kernels (every instance of the context runs 'fct' or 'viscous'
-// 'type2' with the roundoff fix; others take the general kernels above).  A
-// 'viscous' instance stops at the low-order state.  The FP64 unit bounds
+// The 'fct' row kernels (every instance of the context runs 'fct', 'viscous'
+// 'type2' or 'entropy_visc' with the roundoff fix; others take the general
+// kernels above).  A 'viscous' instance stops at the low-order state;
+// 'entropy_visc' walks its rows once more (k_entropy_rows).  The FP64 unit bounds
 // them: an SM retires a warp's FP64 instruction in 16 cycles, so they spend
 // memory (idle at 1-3% of its rate in the general kernels) to form every
 // FP64 value once:
@@ -686,12 +687,15 @@ __device__ __forceinline__ double rat_f64(double H, double h, double rh) {
   return bits64(H) == bits64(h) ? 1.0 : div_known(H, h, rh);
 }
 
-template <int S>
-__global__ void __launch_bounds__(128, 4)
-k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 nd,
-          double* __restrict__ dL, double* __restrict__ muL, double* __restrict__ dLii, double* __restrict__ muLii,
-          StateF64 uL, double* __restrict__ res, double* __restrict__ ab, const double* dij_in,
-          int want_diag, int64_t n_entries, unsigned* __restrict__ err) {
+// FCT: every instance runs 'fct' (no mode tests in the loop, which would cost
+// registers).
+template <int S, bool FCT, bool HIGH>
+__device__ __forceinline__ void fct_row_f64(const Graph& G, const InstConst* C, const InstState* St, const StateF64& u,
+                                            const NodeF64& nd, double* __restrict__ dL, double* __restrict__ muL,
+                                            double* __restrict__ dLii, double* __restrict__ muLii, const StateF64& uL,
+                                            double* res, double* __restrict__ ab, const double* dij_in, int want_diag,
+                                            int64_t n_entries, unsigned* err, const StateF64& u0, const StateF64& out,
+                                            int rk_stage) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= G.n_rows) return;
   const int L = G.len[r];
@@ -699,6 +703,7 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
   const int b = G.slice_inst[r >> 5];
   if (St[b].done) return;
   const InstConst& c = C[b];
+  if (HIGH && c.visc != VISC_ENTROPY) return;
   const int64_t base = entry_base(G, r), nr = G.n_rows;
   const int dp = G.dpos[r];
   const double g = c.g, htiny = c.htiny;
@@ -709,7 +714,9 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
   const double zi = G.bath[r], etai = nd.eta[r], rhi = nd.rh[r], ai = nd.alpha[r];
   const double w1i = nd.v1[r], w2i = nd.w2[r], ghi = g * ui[0];
   const bool wet_i = !le_nn(ui[0], htiny);
-  const bool fct = c.visc == VISC_FCT;          // the right-hand side of smb_2 too, for the residual
+  const bool fct = FCT || (!HIGH && c.visc == VISC_FCT);                    // keep the row differences
+  const bool full = fct || (!HIGH && c.visc == VISC_ENTROPY);     // the right-hand side of smb_2 too, for the residual
+  const double resi = HIGH ? res[r] : 0.0;
   // the diagonal's terms: -c_ii.F_i and the topography residue
   double Dq[S], Dfix, tdx, tdy;
   {
@@ -735,7 +742,7 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
 #pragma unroll
       for (int q = 1; q < S; q++) rk[q] = rk[q] - Dq[q];
       rk[1] = rk[1] - tdx; rk[2] = rk[2] - tdy;
-      if (fct) {
+      if (full) {
 #pragma unroll
         for (int q = 0; q < S; q++) rk2[q] = rk2[q] - Dq[q];
         rk2[1] = rk2[1] - tdx; rk2[2] = rk2[2] - tdy;
@@ -747,30 +754,39 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
     const double cxe = G.cx[e], cye = G.cy[e];
     const LamState lj = lam_state(u, nd, j);
     // d_ij, mu_ij (compute_dij, compute_muij, MAX, alpha_limit)
-    double d;
-    if (dij_in) {
-      d = dij_in[e];
-    } else {
-      double lam;
-      if (!lambda_row(li, lj, G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
-      d = G.cnorm[e] * lam;
+    double d, mu;
+    if (!HIGH) {
+      if (dij_in) {
+        d = dij_in[e];
+      } else {
+        double lam;
+        if (!lambda_row(li, lj, G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
+        d = G.cnorm[e] * lam;
+      }
     }
     const double w1j = nd.v1[j];
-    const double sl = cxe * w1i + cye * w2i;
     double sr = cxe * w1j, srf = sr;             // c.v_j: the viscosity's velocity, the flux's (type 13: v2 = 0)
     sr = sr + cye * nd.w2[j];
     if (S == 3) srf = sr;
-    double mu = max_nn(pos_part(-sl), pos_part(sr));
-    if (want_diag) { sd = sd + d; sm = sm + mu; }
-    d = max_nn(d, mu);
-    const double s = max_nn(ai, nd.alpha[j]);    // 1 without alpha_limit
-    d = d * s;
-    mu = mu * s;
-    dL[e] = d;
-    muL[e] = mu;
-    const double ej = nd.ent[j];
-    emax = max_any(emax, ej);
-    emin = min_any(emin, ej);
+    if (HIGH) {                                  // d^H = MIN(d, res_ij), mu^H = MIN(mu, res_ij) (update.f90:232-239)
+      const double rij = max_nn(resi, res[j]);
+      d = min_nn(dL[e], rij);
+      mu = min_nn(muL[e], rij);
+    } else {
+      mu = max_nn(pos_part(-(cxe * w1i + cye * w2i)), pos_part(sr));
+      if (want_diag) { sd = sd + d; sm = sm + mu; }
+      d = max_nn(d, mu);
+      const double s = max_nn(ai, nd.alpha[j]);  // 1 without alpha_limit
+      d = d * s;
+      mu = mu * s;
+      dL[e] = d;
+      muL[e] = mu;
+    }
+    if (full) {
+      const double ej = nd.ent[j];
+      emax = max_any(emax, ej);
+      emin = min_any(emin, ej);
+    }
     // hydrostatic reconstruction
     const double zj = G.bath[j], etaj = nd.eta[j];
     const double zmax = max_any(zi, zj);
@@ -792,13 +808,14 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
     const double pij = 1.0 - qij, pji = 1.0 - qji;
 #pragma unroll
     for (int q = 0; q < S; q++) {
-      if (q == 0 && !fct) continue;
+      if (q == 0 && !full) continue;
       double x2 = cxe * nd.flux[(int64_t)(2 * q) * nr + j];
       if (S == 3) x2 = x2 + cye * nd.flux[(int64_t)(2 * q + 1) * nr + j];
       double A, B = 0.0, mB = 0.0;
       if (flat) {
         A = uj[q] - ui[q];
       } else {
+        real_branch();
         A = uj[q] * qji - ui[q] * qij;
         B = uj[q] * pji - ui[q] * pij;
         mB = mu * B;
@@ -807,15 +824,18 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
       if (fct) {
         ab[(int64_t)(2 * q) * n_entries + e] = A;
         ab[(int64_t)(2 * q + 1) * n_entries + e] = B;
+      }
+      if (full) {
         rk2[q] = rk2[q] - x2 + dA;
-        if (!flat) rk2[q] = rk2[q] + mB;
+        if (!flat) { real_branch(); rk2[q] = rk2[q] + mB; }
       }
       if (q > 0) {
         rk[q] = rk[q] - x2;
         if (wet) {
           rk[q] = rk[q] + dA;
-          if (!flat) rk[q] = rk[q] + mB;
+          if (!flat) { real_branch(); rk[q] = rk[q] + mB; }
         } else {                                // rats are 0 where h <= htiny
+          real_branch();
           const double ti = wet_i ? qij : 0.0, tj = wet_j ? qji : 0.0;
           rk[q] = rk[q] + d * (uj[q] * tj - ui[q] * ti) + mu * (uj[q] * (1.0 - tj) - ui[q] * (1.0 - ti));
         }
@@ -824,7 +844,7 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
       if (q == 2) { rk[2] = rk[2] - ty; rk2[2] = rk2[2] - ty; }
     }
   }
-  if (want_diag) {   // the diagonals of the viscosities (update.f90:315-323, 782-798), as k_low_f64 forms them
+  if (!HIGH && want_diag) {   // the diagonals of the viscosities (update.f90:315-323, 782-798), as k_low_f64 forms them
     const double dii_raw = -sd, muii_raw = -sm;
     double dii = tmax(dii_raw, muii_raw), muii = muii_raw;
     if (c.alpha_limit) {
@@ -889,10 +909,17 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
   ul[0] = ui[0] * (1.0 + div_known(dt * fix, m, im)) + dt * div_known(rk[0], m, im);
 #pragma unroll
   for (int q = 1; q < S; q++) ul[q] = ui[q] + dt * div_known(rk[q], m, im);
+  if (HIGH) {        // 'entropy_visc': this is the stage's result
+    double un[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < S; q++) un[q] = ul[q];
+    finish_row_f64(G, c, St[b], r, S, un, true, rk_stage, u0, out, err);
+    return;
+  }
   uL.h[r] = ul[0]; uL.q1[r] = ul[1]; uL.q2[r] = ul[2];
   if (S == 5) { uL.q3[r] = ul[3]; uL.q4[r] = ul[4]; }
   if (bad) atomicOr(err, ERRB_DELTA);
-  if (!fct) return;
+  if (!full) return;
   // entropy residual (update.f90:838-868); Entprime(4:5) are 0
   double rm[3], un_[3];
 #pragma unroll
@@ -914,6 +941,25 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
   rsd = rsd - m * rm[2] * v2i;
   const double rescale = __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor);   // the product is exact
   res[r] = fabs(rsd) / rescale;
+}
+
+template <int S, bool FCT>
+__global__ void __launch_bounds__(128, 4)
+k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 nd, double* __restrict__ dL,
+          double* __restrict__ muL, double* __restrict__ dLii, double* __restrict__ muLii, StateF64 uL,
+          double* __restrict__ res, double* __restrict__ ab, const double* dij_in, int want_diag, int64_t n_entries,
+          unsigned* __restrict__ err) {
+  fct_row_f64<S, FCT, false>(G, C, St, u, nd, dL, muL, dLii, muLii, uL, res, ab, dij_in, want_diag, n_entries, err, u, u, 0);
+}
+
+// 'entropy_visc' (update.f90:225-262): the smb_2_roundoff rows again, with
+// d^H and mu^H, are the stage's result.
+template <int S>
+__global__ void __launch_bounds__(128, 4)
+k_entropy_rows(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 nd, double* dL, double* muL,
+               double* res, StateF64 u0, StateF64 out, int rk_stage, unsigned* err) {
+  fct_row_f64<S, false, true>(G, C, St, u, nd, dL, muL, nullptr, nullptr, u, res, nullptr, nullptr, 0, 0, err, u0, out,
+                       rk_stage);
 }
 
 // f_ij and R^-_i from the stored differences: five FP64 instructions per
@@ -967,6 +1013,7 @@ __global__ void k_update_fct(Graph G, const InstConst* C, const InstState* St,
   const InstState& st = St[b];
   if (st.done) return;
   const InstConst& c = C[b];
+  if (c.visc == VISC_ENTROPY) return;          // k_entropy_rows writes these rows
   const int64_t base = entry_base(G, r);
   const bool fct_mode = c.visc == VISC_FCT;
   const double resi = fct_mode ? res[r] : 0.0, Ri = fct_mode ? rminus[r] : 0.0;
@@ -1156,12 +1203,12 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
   if (a.fused) {
     const int64_t ne = a.w.n_entries;
     const int diag = a.rk_stage == 0;            // swe_euler_intermediates hands out the diagonals
-    if (a.S == 5)
-      launch_full(k_low_fct<5>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
-                                     a.w.ab, a.dij_in, diag, ne, a.err);
-    else
-      launch_full(k_low_fct<3>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res,
-                                     a.w.ab, a.dij_in, diag, ne, a.err);
+#define SWE_LOWF(S, F)                                                                                              \
+    launch_full(k_low_fct<S, F>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, \
+                a.w.res, a.w.ab, a.dij_in, diag, ne, a.err)
+    if (a.S == 5) { if (a.all_fct) SWE_LOWF(5, true); else SWE_LOWF(5, false); }
+    else { if (a.all_fct) SWE_LOWF(3, true); else SWE_LOWF(3, false); }
+#undef SWE_LOWF
     EV_END(2); EV_BEGIN(3);
     launch_full(k_fct_fct, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
                                 a.err);
@@ -1172,6 +1219,14 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
     else
       launch_full(k_update_fct<3>, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.w.ab,
                                         a.u0, a.out, a.rk_stage, a.lij_out, ne, a.err);
+    if (a.entropy) {
+      if (a.S == 5)
+        launch_full(k_entropy_rows<5>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.res, a.u0, a.out,
+                    a.rk_stage, a.err);
+      else
+        launch_full(k_entropy_rows<3>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.res, a.u0, a.out,
+                    a.rk_stage, a.err);
+    }
     EV_END(4);
     return;
   }

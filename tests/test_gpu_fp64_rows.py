@@ -120,6 +120,31 @@ def test_fct_stage_bit_exact(kind, type_test, alpha, bumpy):
         np.testing.assert_array_equal(got, ref[0])
 
 
+@pytest.mark.parametrize("visc", ["viscous", "entropy_visc"])
+@pytest.mark.parametrize("kind", STATES)
+def test_other_modes_bit_exact(kind, visc):
+    """The same row kernels without the limiter: one stage of 'viscous'
+    'type2' and of 'entropy_visc' over an uneven bottom."""
+    n = 15
+    rng = np.random.default_rng(200 + STATES.index(kind))
+    mesh = M.jittered_mesh(n, n, 0.0, 1.0, 0.0, 1.0, jitter=0.3, seed=6)
+    z = rng.uniform(-0.4, 0.4, n * n) * (rng.random(n * n) < 0.7)
+    p = C.Params(max_water_h=1.0, htiny=1e-4, viscosity_type=C.VISC[visc])
+    o, upd = _pair(mesh, z, p)
+    for _ in range(3):
+        u = _state(kind, n * n, p.htiny, rng)
+        try:
+            pd = replace(p, dt=o.compute_dij(u)[1])
+        except oracle.OracleError:
+            continue
+        o.set_params(oracle.Params(*pd.fields()))
+        upd.set_params(pd)
+        ref, got = _both(lambda: o.euler(u), lambda: upd.euler(u),
+                         (L.SWE_ERR_NEG_H, L.SWE_ERR_DELTA, L.SWE_ERR_NAN))
+        if ref is not None:
+            np.testing.assert_array_equal(got, ref)
+
+
 @pytest.mark.parametrize("nx,ny", [(2, 2), (33, 3), (65, 64)])
 @pytest.mark.parametrize("sgn", [0, 1])
 def test_fct_steps_bit_exact(sgn, nx, ny):
