@@ -952,6 +952,271 @@ k_low_fct(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 
   fct_row_f64<S, FCT, false>(G, C, St, u, nd, dL, muL, dLii, muLii, uL, res, ab, dij_in, want_diag, n_entries, err, u, u, 0);
 }
 
+// ---------------------------------------------------------------------------
+// Small meshes: four warps per 32 rows.  The FP64 unit of an SM quarter takes 64
+// cycles per warp instruction however few warps there are, so below about two
+// slices per SM a row's chain of instructions is the kernel's time and most
+// quarters idle.  Warp w forms the terms of entries w, w + 4, ... of the slice's
+// rows and leaves them in shared memory; the warps then add them up in the
+// reference's order, each its own sums (independent chains), and share the
+// tail the same way.  Same operations and order as fct_row_f64.
+// ---------------------------------------------------------------------------
+template <int S>
+struct SplitTerms {
+  enum { MU, F, A0, B0, E, TX, TY, DRAW, MRAW, Q, N = Q + 5 * S };   // Q + 5 q: x2, d A, mu B, and those of smb_2_roundoff
+};
+
+template <int S>
+__global__ void __launch_bounds__(128)
+k_low_split(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF64 nd, double* __restrict__ dL,
+            double* __restrict__ muL, double* __restrict__ dLii, double* __restrict__ muLii, StateF64 uL,
+            double* __restrict__ res, double* __restrict__ ab, const double* dij_in, int want_diag, int64_t n_entries,
+            unsigned* __restrict__ err) {
+  using T = SplitTerms<S>;
+  __shared__ double term[4][T::N][32];
+  __shared__ double tail[6][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r = (int64_t)blockIdx.x * 32 + lane;     // n_rows is a multiple of 32
+  const int b = G.slice_inst[blockIdx.x];
+  if (St[b].done) return;                               // the whole block
+  const InstConst& c = C[b];
+  const int L = G.len[r], width = (int)((G.slice_ptr[blockIdx.x + 1] - G.slice_ptr[blockIdx.x]) >> 5);
+  const int64_t base = entry_base(G, r), nr = G.n_rows;
+  const int dp = G.dpos[r];
+  const double g = c.g, htiny = c.htiny;
+  const LamState li = lam_state(u, nd, r);
+  double ui[S];
+  ui[0] = li.h; ui[1] = li.q1; ui[2] = li.q2;
+  if (S == 5) { ui[3] = u.q3[r]; ui[4] = u.q4[r]; }
+  const double zi = G.bath[r], etai = nd.eta[r], rhi = nd.rh[r], ai = nd.alpha[r];
+  const double w1i = nd.v1[r], w2i = nd.w2[r], ghi = g * ui[0];
+  const bool wet_i = !le_nn(ui[0], htiny);
+  // this warp's sums: warp 0 fix and rk[0], warp 1 rk2[0] and the entropy's
+  // maximum and minimum; the pair rk[p], rk2[p] of one momentum component each
+  const int p = w == 2 ? 1 : w == 3 ? 2 : (S == 5 ? (w == 0 ? 3 : 4) : 0);
+  const double cxd = G.cxii[r], cyd = G.cyii[r];
+  auto diag = [&](int q) {                              // c_ii.F_i
+    double x = cxd * nd.flux[(int64_t)(2 * q) * nr + r];
+    if (S == 3) x = x + cyd * nd.flux[(int64_t)(2 * q + 1) * nr + r];
+    return x;
+  };
+  const double Dp = p ? diag(p) : 0.0;
+  double D0 = 0.0, td = 0.0;
+  if (w == 0) {
+    D0 = cxd * w1i;
+    if (S == 3) D0 = D0 + cyd * w2i;
+  } else if (w == 1) {
+    D0 = diag(0);
+  } else {
+    td = ghi * (etai - ui[0] - zi) * (w == 2 ? cxd : cyd);
+  }
+  double s0 = 0.0, s1 = 0.0, rk = 0.0, rk2 = 0.0;       // warp 0: fix, rk[0]; warp 1: rk2[0]; the pair
+  double emax = nd.ent[r], emin = emax, sd = 0.0, sm = 0.0;
+  auto add_diag = [&]() {
+    if (w <= 1) s0 = s0 - D0;
+    if (p) { rk = rk - Dp; rk2 = rk2 - Dp; }
+    if (w >= 2) { rk = rk - td; rk2 = rk2 - td; }
+  };
+  bool bad = false;
+  for (int k0 = 0; k0 < width; k0 += 4) {
+    if (k0 + w < L) {
+      const int64_t e = base + 32 * (k0 + w);
+      const int j = G.col[e];
+      const double cxe = G.cx[e], cye = G.cy[e];
+      const LamState lj = lam_state(u, nd, j);
+      double d;
+      if (dij_in) {
+        d = dij_in[e];
+      } else {
+        double lam;
+        if (!lambda_row(li, lj, G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
+        d = G.cnorm[e] * lam;
+      }
+      double sr = cxe * nd.v1[j], srf = sr;
+      sr = sr + cye * nd.w2[j];
+      if (S == 3) srf = sr;
+      double mu = max_nn(pos_part(-(cxe * w1i + cye * w2i)), pos_part(sr));
+      term[w][T::DRAW][lane] = d;
+      term[w][T::MRAW][lane] = mu;
+      d = max_nn(d, mu);
+      const double s = max_nn(ai, nd.alpha[j]);
+      d = d * s;
+      mu = mu * s;
+      dL[e] = d;
+      muL[e] = mu;
+      term[w][T::E][lane] = nd.ent[j];
+      const double zj = G.bath[j], etaj = nd.eta[j], zmax = max_any(zi, zj);
+      const double Hij = pos_part(etai - zmax), Hji = pos_part(etaj - zmax);
+      const double qij = rat_f64(Hij, ui[0], rhi), qji = rat_f64(Hji, lj.h, nd.rh[j]);
+      const bool wet_j = !le_nn(lj.h, htiny);
+      const double dmu = d - mu;
+      term[w][T::MU][lane] = mu;
+      term[w][T::F][lane] = wet_i ? dmu * qij : 0.0;
+      term[w][T::A0][lane] = (mu - srf) * lj.h;
+      term[w][T::B0][lane] = pos_part(dmu * Hji);
+      const double tp = ghi * (etaj - ui[0] - zi);
+      term[w][T::TX][lane] = tp * cxe;
+      term[w][T::TY][lane] = tp * cye;
+      double uj[S];
+      uj[0] = lj.h; uj[1] = lj.q1; uj[2] = lj.q2;
+      if (S == 5) { uj[3] = u.q3[j]; uj[4] = u.q4[j]; }
+      const bool flat = bits64(qij) == 0x3ff0000000000000ll && bits64(qji) == 0x3ff0000000000000ll;
+      const double pij = 1.0 - qij, pji = 1.0 - qji;
+      const double ti = wet_i ? qij : 0.0, tj = wet_j ? qji : 0.0;
+#pragma unroll
+      for (int q = 0; q < S; q++) {
+        double x2 = cxe * nd.flux[(int64_t)(2 * q) * nr + j];
+        if (S == 3) x2 = x2 + cye * nd.flux[(int64_t)(2 * q + 1) * nr + j];
+        double A, B = 0.0, mB = 0.0;
+        if (flat) {
+          A = uj[q] - ui[q];
+        } else {
+          real_branch();
+          A = uj[q] * qji - ui[q] * qij;
+          B = uj[q] * pji - ui[q] * pij;
+          mB = mu * B;
+        }
+        const double dA = d * A;
+        ab[(int64_t)(2 * q) * n_entries + e] = A;
+        ab[(int64_t)(2 * q + 1) * n_entries + e] = B;
+        term[w][T::Q + 5 * q][lane] = x2;
+        term[w][T::Q + 5 * q + 1][lane] = dA;
+        term[w][T::Q + 5 * q + 2][lane] = mB;
+        if (q > 0) {
+          double dAr = dA, mBr = mB;
+          if (!(wet_i && wet_j)) {
+            real_branch();
+            dAr = d * (uj[q] * tj - ui[q] * ti);
+            mBr = mu * (uj[q] * (1.0 - tj) - ui[q] * (1.0 - ti));
+          }
+          term[w][T::Q + 5 * q + 3][lane] = dAr;
+          term[w][T::Q + 5 * q + 4][lane] = mBr;
+        }
+      }
+    }
+    __syncthreads();
+    for (int k = k0; k < k0 + 4; k++) {
+      if (k == dp && k < L) add_diag();
+      if (k >= L) continue;
+      const auto& t = term[k - k0];
+      if (w == 0) {
+        s0 = s0 - t[T::MU][lane] - t[T::F][lane];
+        s1 = s1 + t[T::A0][lane] + t[T::B0][lane];
+      } else if (w == 1) {
+        s0 = s0 - t[T::Q][lane] + t[T::Q + 1][lane];
+        s0 = s0 + t[T::Q + 2][lane];
+        emax = max_any(emax, t[T::E][lane]);
+        emin = min_any(emin, t[T::E][lane]);
+        if (want_diag) { sd = sd + t[T::DRAW][lane]; sm = sm + t[T::MRAW][lane]; }
+      }
+      if (p) {
+        const double x2 = t[T::Q + 5 * p][lane];
+        rk = rk - x2 + t[T::Q + 5 * p + 3][lane] + t[T::Q + 5 * p + 4][lane];
+        rk2 = rk2 - x2 + t[T::Q + 5 * p + 1][lane] + t[T::Q + 5 * p + 2][lane];
+      }
+      if (w >= 2) {
+        const double tp = t[w == 2 ? T::TX : T::TY][lane];
+        rk = rk - tp;
+        rk2 = rk2 - tp;
+      }
+    }
+    __syncthreads();
+  }
+  if (dp == L) add_diag();
+  const double m = G.lumped[r], im = G.inv_lumped[r], dt = St[b].dt;
+  const double v1i = w1i, v2i = nd.v2[r];
+  if (want_diag && w == 1 && L > 0) {    // as in fct_row_f64
+    const double dii_raw = -sd, muii_raw = -sm;
+    double dii = tmax(dii_raw, muii_raw), muii = muii_raw;
+    if (c.alpha_limit) {
+      sd = sm = 0.0;
+      for (int kk = 0; kk <= L; kk++) {
+        if (kk == dp) { sm = sm + muii; continue; }
+        const int64_t e = base + 32 * (kk - (kk > dp ? 1 : 0));
+        sd = sd + dL[e];
+        sm = sm + muL[e];
+      }
+      dii = -sd;
+      muii = -sm;
+    }
+    dLii[r] = dii;
+    muLii[r] = muii;
+  }
+  // source terms (:425-551)
+  if (S == 5) {
+    double p_i, s_i;
+    sgn_node_f64(c, m, ui[0], ui[3], &p_i, &s_i);
+    if (w >= 2) {
+      const double pd = p_i * (w == 2 ? cxd : cyd);
+      for (int k = 0; k <= L; k++) {
+        if (k == dp) { rk = rk - pd; rk2 = rk2 - pd; }
+        if (k == L) break;
+        const int64_t e = base + 32 * k;
+        const double px = nd.pt[G.col[e]] * (w == 2 ? G.cx[e] : G.cy[e]);
+        rk = rk - px;
+        rk2 = rk2 - px;
+      }
+    } else if (w == 0) {
+      const double x = m * ui[S - 1];
+      rk = rk + x; rk2 = rk2 + x;
+    } else {
+      const double x = m * s_i;
+      rk = rk - x; rk2 = rk2 - x;
+    }
+  } else if (w >= 2) {
+    const double up = w == 2 ? ui[1] : ui[2];
+    if (c.type_test == 9 || c.type_test == 10) {
+      const double fric = c.g * c.mannings * c.mannings;
+      const double hstar = pow_43(max_any(ui[0], htiny));
+      const double vel = fric * sqrt(v1i * v1i + v2i * v2i);
+      const double den = hstar + max_nn(hstar, vel * dt);
+      const double x = m * up * vel * 2.0 / den;
+      rk = rk - x; rk2 = rk2 - x;
+    } else if (c.type_test == 11) {
+      const double kappa = 0.2, x = m * kappa * up;
+      rk = rk - x; rk2 = rk2 - x;
+    } else if (c.type_test == 12) {
+      const double f = 2.0, x = m * f * (w == 2 ? ui[2] : ui[1]);
+      rk = w == 2 ? rk + x : rk - x;
+      rk2 = w == 2 ? rk2 + x : rk2 - x;
+    }
+  }
+  // divide_by_lumped (:801-808), the low-order state (:202-215), and what the
+  // residual takes of the smb_2 rows
+  if (w == 0 && L > 0) uL.h[r] = ui[0] * (1.0 + div_known(dt * s0, m, im)) + dt * div_known(s1, m, im);
+  if (p) {
+    const double up = p == 1 ? ui[1] : p == 2 ? ui[2] : p == 3 ? ui[S - 2] : ui[S - 1];
+    const double ul = up + dt * div_known(rk, m, im);
+    if (L > 0) store_f64(uL, p, r, ul);
+    if (w >= 2) {
+      const double rm = div_known(rk2, m, im);
+      tail[2 * p][lane] = rm;
+      tail[2 * p + 1][lane] = up + dt * rm;
+    }
+  }
+  if (w == 1) {
+    const double rm = div_known(s0, m, im);
+    tail[0][lane] = rm;
+    tail[1][lane] = ui[0] + dt * rm;
+  }
+  if (bad) atomicOr(err, ERRB_DELTA);
+  __syncthreads();
+  if (w != 1 || L == 0) return;
+  // entropy residual (update.f90:838-868)
+  const double un0 = tail[1][lane], un1 = tail[3][lane], un2 = tail[5][lane];
+  const double on = one_over_h(un0, htiny);
+  double En = g * (un0 * un0);
+  En = En + un1 * on * un1;
+  En = En + un2 * on * un2;
+  En = 0.5 * En;
+  const double Ep0 = ghi - 0.5 * (v1i * v1i) - 0.5 * (v2i * v2i);
+  double rsd = div_known(m * (En - nd.ent[r]), dt, St[b].inv_dt);
+  rsd = rsd - m * tail[0][lane] * Ep0;
+  rsd = rsd - m * tail[2][lane] * v1i;
+  rsd = rsd - m * tail[4][lane] * v2i;
+  res[r] = fabs(rsd) / __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor);
+}
+
 // 'entropy_visc' (update.f90:225-262): the smb_2_roundoff rows again, with
 // d^H and mu^H, are the stage's result.
 template <int S>
@@ -1081,6 +1346,49 @@ __global__ void k_dt_f64(Graph G, const InstConst* C, InstState* St, StateF64 u,
   step_turn(turn, C, St);
 }
 
+// k_dt for small meshes, four warps per 32 rows (see k_low_split)
+__global__ void __launch_bounds__(128) k_dt_split(Graph G, const InstConst* C, InstState* St, StateF64 u, NodeF64 nd,
+                                                  double* __restrict__ d_out, double* __restrict__ dii_out,
+                                                  unsigned* __restrict__ err, StepTurn turn) {
+  __shared__ double dk[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r = (int64_t)blockIdx.x * 32 + lane;
+  const int b = G.slice_inst[blockIdx.x];
+  if (!St[b].done) {                                    // the whole block
+    const InstConst& c = C[b];
+    const int L = G.len[r], width = (int)((G.slice_ptr[blockIdx.x + 1] - G.slice_ptr[blockIdx.x]) >> 5);
+    const int64_t base = entry_base(G, r);
+    const LamState li = lam_state(u, nd, r);
+    double s = 0.0;
+    bool bad = false;
+    for (int k0 = 0; k0 < width; k0 += 8) {
+      for (int q = w; q < 8 && k0 + q < L; q += 4) {
+        const int64_t e = base + 32 * (k0 + q);
+        double lam;
+        if (!lambda_row(li, lam_state(u, nd, G.col[e]), G.cnx[e], G.cny[e], G.cnf[e], c, &lam)) bad = true;
+        const double d = G.cnorm[e] * lam;
+        if (d_out) d_out[e] = d;
+        dk[q][lane] = d;
+      }
+      __syncthreads();
+      if (w == 0)
+        for (int q = 0; q < 8 && k0 + q < L; q++) s = s + dk[q][lane];
+      __syncthreads();
+    }
+    if (bad) atomicOr(err, ERRB_DELTA);
+    if (w == 0) {
+      double val = 0.0;
+      if (L > 0) {
+        if (dii_out) dii_out[r] = -s;
+        val = div_known(s, G.lumped[r], G.inv_lumped[r]);
+      }
+      for (int off = 16; off > 0; off >>= 1) val = fmax(val, __shfl_down_sync(0xffffffffu, val, off));
+      if (lane == 0 && val > 0.0) atomicMax(&St[b].maxd_bits, (unsigned long long)__double_as_longlong(val));
+    }
+  }
+  step_turn(turn, C, St);
+}
+
 // The turn between two steps as a kernel of its own
 __global__ void k_step_turn(StepTurn t, const InstConst* C, InstState* St) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1188,6 +1496,20 @@ static void launch_full(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
   kern<<<grid, block, smem, s>>>(static_cast<KArgs>(args)...);
 }
 
+// Where the four-warp kernels run: up to one wave of their blocks, 4 slices per
+// SM (registers), 2.5 for 5-component systems.  Per step, four warps against
+// one: 2k nodes 153 against 244 us, 10k 179 / 248, 16k 244 / 250, 20k 268 /
+// 332, 29k 360 / 346; SGN 2k 171 / 248, 12k 231 / 249, 16k 299 / 256.
+static bool split_rows(int64_t n_rows, int S) {
+  static const int64_t sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return (int64_t)n;
+  }();
+  return n_rows <= (S == 5 ? 80 : 128) * sms;
+}
+
 void launch_node_f64(const StageArgs& a, cudaStream_t s) {
   const NodeF64 nd = node_of(a.w);
   launch_full(k_node_f64, nblk(a.G.n_rows, a.block), a.block, 0, s, a.G, a.C, a.St, a.u, nd);
@@ -1203,6 +1525,15 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
   if (a.fused) {
     const int64_t ne = a.w.n_entries;
     const int diag = a.rk_stage == 0;            // swe_euler_intermediates hands out the diagonals
+    if (a.all_fct && split_rows(a.G.n_rows, a.S)) {
+      const unsigned ns = (unsigned)(a.G.n_rows / 32);
+      if (a.S == 5)
+        launch_full(k_low_split<5>, ns, 128, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL,
+                    a.w.res, a.w.ab, a.dij_in, diag, ne, a.err);
+      else
+        launch_full(k_low_split<3>, ns, 128, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL,
+                    a.w.res, a.w.ab, a.dij_in, diag, ne, a.err);
+    } else
 #define SWE_LOWF(S, F)                                                                                              \
     launch_full(k_low_fct<S, F>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, \
                 a.w.res, a.w.ab, a.dij_in, diag, ne, a.err)
@@ -1245,6 +1576,10 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
 
 void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
                    double* d_out, double* dii_out, unsigned* err, int block, const StepTurn& turn, cudaStream_t s) {
+  if (split_rows(G.n_rows, u.q3 ? 5 : 3)) {
+    launch_full(k_dt_split, (unsigned)(G.n_rows / 32), 128, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
+    return;
+  }
   launch_full(k_dt_f64, nblk(G.n_rows, block), block, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
 }
 

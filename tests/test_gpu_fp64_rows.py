@@ -145,11 +145,11 @@ def test_other_modes_bit_exact(kind, visc):
             np.testing.assert_array_equal(got, ref)
 
 
-@pytest.mark.parametrize("nx,ny", [(2, 2), (33, 3), (65, 64)])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (33, 3), (65, 64), (161, 160)])
 @pytest.mark.parametrize("sgn", [0, 1])
 def test_fct_steps_bit_exact(sgn, nx, ny):
-    """RK3 steps of both system sizes at row counts about a warp, a block and
-    several, against the oracle."""
+    """RK3 steps of both system sizes at row counts about a warp, a block,
+    several, and above the four-warp kernels' range, against the oracle."""
     if sgn:
         case = C.sgn_case(nx=max(nx, 3), ny=ny, Lx=0.01 * nx, Ly=0.01 * ny, x0=0.005 * nx, cfl=5e-4)
     else:
