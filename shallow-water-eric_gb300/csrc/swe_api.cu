@@ -28,10 +28,11 @@ using namespace swe;
 namespace {
 
 // Zeroed device arrays, 256-byte aligned, freed together.  Small ones share
-// slabs of 1 MB: a context has some fifty, and an allocation and a memset each
+// slabs of 4 MB: a context has some fifty, and an allocation and a memset each
 // were most of the set-up time of a small mesh.
 struct DevBuf {
-  static constexpr size_t kSlab = 1 << 20;
+  static constexpr size_t kSlab = 4 << 20;
+  bool in_use = false;   // the context works on its own stream: the memset has to be waited for
   std::vector<void*> ptrs;
   char* slab = nullptr;
   size_t left = 0;
@@ -46,7 +47,7 @@ struct DevBuf {
       if (st != cudaSuccess) return nullptr;
       ptrs.push_back(p);
       st = cudaMemset(p, 0, take);
-      if (st == cudaSuccess) st = cudaStreamSynchronize(0);   // contexts run on their own non-blocking streams
+      if (st == cudaSuccess && in_use) st = cudaStreamSynchronize(0);
       if (st != cudaSuccess) return nullptr;
       if (!shared) return static_cast<T*>(p);
       slab = static_cast<char*>(p);
@@ -346,6 +347,22 @@ static float2 bath_df(double z) {
   return make_float2(hi, (float)(z - (double)hi));
 }
 
+// compute_dij's norm = SQRT(c.c) and normal c/norm per entry (update.f90:309-312;
+// padding entries, never read: 0/0), and the normal in FP32
+__global__ void k_edge_normals(const double* __restrict__ cx, const double* __restrict__ cy, int64_t n,
+                               double* __restrict__ nrm, double* __restrict__ nx, double* __restrict__ ny,
+                               float2* __restrict__ nf) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const double x = cx[e], y = cy[e];
+    const double q = __dsqrt_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)));
+    const double a = __ddiv_rn(x, q), b = __ddiv_rn(y, q);
+    nrm[e] = q;
+    nx[e] = a;
+    ny[e] = b;
+    nf[e] = make_float2((float)a, (float)b);
+  }
+}
+
 static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& baths) {
   c->L = build_layout(c->meshes, baths);
   const Layout& L = c->L;
@@ -371,23 +388,19 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
   if (c->precision == SWE_PREC_FP64) {
     G.cx = upload_vec(c, L.cx, st);
     G.cy = upload_vec(c, L.cy, st);
-    {   // compute_dij's norm = SQRT(c.c) and normal c/norm per entry (update.f90:309-312),
-        // the same IEEE operations as a kernel would do per use
-      std::vector<double> nrm(L.n_entries), nx(L.n_entries), ny(L.n_entries);
-      std::vector<float2> nf(L.n_entries);
-      for (int64_t e = 0; e < L.n_entries; e++) {
-        const double cx = L.cx[e], cy = L.cy[e];
-        const double cc = cx * cx + cy * cy;
-        nrm[e] = std::sqrt(cc);
-        nx[e] = cx / nrm[e];                       // padding entries (never read): 0/0
-        ny[e] = cy / nrm[e];
-        nf[e] = make_float2((float)nx[e], (float)ny[e]);
-      }
-      G.cnf = upload_vec(c, nf, st);
-      G.cnorm = upload_vec(c, nrm, st);
-      G.cnx = upload_vec(c, nx, st);
-      G.cny = upload_vec(c, ny, st);
+    double* nrm = c->buf.alloc<double>(L.n_entries, st);
+    double* nx = c->buf.alloc<double>(L.n_entries, st);
+    double* ny = c->buf.alloc<double>(L.n_entries, st);
+    float2* nf = c->buf.alloc<float2>(L.n_entries, st);
+    if (st == cudaSuccess && L.n_entries > 0) {
+      k_edge_normals<<<(unsigned)std::min<int64_t>((L.n_entries + 255) / 256, 1 << 20), 256>>>(G.cx, G.cy, L.n_entries,
+                                                                                          nrm, nx, ny, nf);
+      st = cudaGetLastError();
     }
+    G.cnorm = nrm;
+    G.cnx = nx;
+    G.cny = ny;
+    G.cnf = nf;
     G.cxii = upload_vec(c, L.cxii, st);
     G.cyii = upload_vec(c, L.cyii, st);
   } else {
@@ -925,6 +938,7 @@ static int create_common(swe_ctx** out, int n_inst, const int* np, const int* me
   if (cuda_check(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate")) return SWE_ERR_CUDA;
   int rc = build_device(c, baths);
   if (rc) return rc;
+  c->buf.in_use = true;
   return cuda_check(c, cudaDeviceSynchronize(), "setup");
 }
 
