@@ -184,8 +184,10 @@ __device__ __forceinline__ bool lambda_f(float hl, float hr, float vl, float vr,
     }
   }
   const float tl = (ht - hl) * ovhl, tr = (ht - hr) * ovhr;
-  const float lbdl = fma_(-sql, sqrtf((1.f + fmaxf(tl * 0.5f, 0.f)) * (1.f + fmaxf(tl, 0.f))), vl);
-  const float lbdr = fma_(sqr, sqrtf((1.f + fmaxf(tr * 0.5f, 0.f)) * (1.f + fmaxf(tr, 0.f))), vr);
+  // (1 + max(t/2, 0)) (1 + max(t, 0)); halving is exact
+  const float xl = fmaxf(tl, 0.f), xr = fmaxf(tr, 0.f);
+  const float lbdl = fma_(-sql, sqrtf(fma_(xl, 0.5f, 1.f) * (1.f + xl)), vl);
+  const float lbdr = fma_(sqr, sqrtf(fma_(xr, 0.5f, 1.f) * (1.f + xr)), vr);
   *lambda = fmaxf(fabsf(lbdl), fabsf(lbdr));
   return ok;
 }
@@ -323,11 +325,11 @@ template <int S>
 struct NbTile {
   static constexpr bool kGlobal = false;
   static constexpr int kS = S;
-  const float4* a;            // k_low (h, q1, q2, eta); k_dt (h, v1, v2, sq); k_fct (h, eta, res); k_update as k_low
+  const float4* a;            // k_low and k_update (h, q1, q2, eta); k_dt (h, v1, v2, sq)
   const float4* b;            // k_low (ovh, v1, v2, sq); k_update (res, R, inv, one)
   const float4* c;            // k_low (inv, one, E, alpha)
-  const float* o;             // k_dt: ovh; k_node: h
-  const float2* q;            // h eta, h w (5-component systems)
+  const float* o;             // k_dt: ovh; k_node: h; k_fct: res
+  const float2* q;            // h eta, h w (5-component systems); k_fct: h, eta
   const float* p;             // k_low: SGN pressure
   const double* R64_;
   const int16_t* loc;         // this row's positions, c_ij or (d, mu), |c_ij| lambda
@@ -350,8 +352,8 @@ struct NbTile {
     return NodeL{x.x, x.y, x.z, x.w, o[j]};
   }
   __device__ __forceinline__ NodeC fct(const Raw&, int j) const {
-    const float4 x = a[j];
-    return NodeC{x.x, x.y, x.z};
+    const float2 x = q[j];
+    return NodeC{x.x, x.y, o[j]};
   }
   __device__ __forceinline__ NodeU upd(const Raw&, int j) const {
     const float4 x = a[j], y = b[j];
@@ -369,14 +371,14 @@ struct TileParts {
   int a, b, c, q, r64, e8, e4, o, p;   // bytes per position / entry
 };
 __host__ __device__ constexpr TileParts tile_parts(int kind, int S, bool d, bool lamin) {
-  return TileParts{kind == 1 ? 0 : 16,
+  return TileParts{kind == 1 || kind == 3 ? 0 : 16,
                    kind == 2 || kind == 4 ? 16 : 0,
                    kind == 2 ? 16 : 0,
-                   S == 5 && (kind == 2 || kind == 4) ? 8 : 0,
+                   kind == 3 || (S == 5 && (kind == 2 || kind == 4)) ? 8 : 0,
                    kind == 4 && d ? 8 : 0,
                    kind == 1 ? 0 : 8,
                    kind == 2 && lamin ? 4 : 0,
-                   kind <= 1 ? 4 : 0,
+                   kind <= 1 || kind == 3 ? 4 : 0,
                    S == 5 && kind == 2 ? 4 : 0};
 }
 struct TileSmem {
@@ -674,7 +676,7 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
     } else if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, ni.sq, nj.sq, lk, &dlam)) {
       delta_bad = true;
     }
-    float mu = fmaxf(fmaxf(-cvi, 0.f), fmaxf(cvj, 0.f));
+    float mu = fmaxf(fmaxf(-cvi, cvj), 0.f);
     float d = fmaxf(dlam, mu);
     const float s = galerkin ? 0.f : (limit ? fmaxf(ni.al, nj.al) : 1.f);
     d *= s;
@@ -895,7 +897,7 @@ __device__ __forceinline__ void low_row_type1(int64_t r, const Graph& G, const I
     float dlam;
     if (!dlam_f(cxe, cye, cvi, cvj, ni.h, nj.h, ni.ovh, nj.ovh, ni.sq, nj.sq, lk, &dlam))
       delta_bad = true;
-    float mu = fmaxf(fmaxf(-cvi, 0.f), fmaxf(cvj, 0.f));
+    float mu = fmaxf(fmaxf(-cvi, cvj), 0.f);
     float d = fmaxf(dlam, mu);
     const float s = c.alpha_limit ? fmaxf(ni.al, nj.al) : 1.f;
     d *= s;
@@ -1061,7 +1063,10 @@ __global__ void __launch_bounds__(T) k_fct_tile(Graph G, const InstConst* C,
   row_prefetch<T>(G, RowPrefetch{{G.lumpedf, D ? (const void*)w.hL64 : (const void*)w.hL}, {4, 8}});
   struct Node { float4 n; float res; };
   stage_nodes<T>(tc, t, [&](int row) { return Node{u.nq[row], res[row]}; },
-                 [&](int i, int, const Node& x) { sm.a[i] = make_float4(x.n.x, x.n.w, x.res, 0.f); });
+                 [&](int i, int, const Node& x) {
+                   sm.q[i] = make_float2(x.n.x, x.n.w);
+                   sm.o[i] = x.res;
+                 });
   cp_wait();
   __syncthreads();
   pdl_trigger();
@@ -1237,8 +1242,9 @@ __global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* C,
     update_row<B, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, u0, out, rk_stage, err, nb);
 }
 
+// six resident blocks of 256 (40 registers): 141 -> 136 us at 4M nodes
 template <int T, int S, bool D, bool FCT>
-__global__ void __launch_bounds__(T) k_update_tile(Graph G, const InstConst* C,
+__global__ void __launch_bounds__(T, S == 3 ? 6 * (256 / T) : 4) k_update_tile(Graph G, const InstConst* C,
                                                    const InstState* St, StateMix u,
                                                    const float2* dmu, WorkMix w,
                                                    const float* res, StateMix u0, StateMix out,
@@ -1332,14 +1338,48 @@ __device__ __forceinline__ float dt_row(int r, const RowHead& hd, const Graph& G
 }
 
 // Warp max of |d_ii| / m_i into the instance's maximum (the 32 rows of a warp
-// are one slice, so one instance).  A maximum does not depend on the order.
+// are one slice, so one instance).  A maximum does not depend on the order;
+// the values are not negative (NaN counts as 0), so their bits compare as
+// integers.
+__device__ __forceinline__ unsigned dt_warp_max(float val) {
+  return __reduce_max_sync(0xffffffffu, val > 0.f ? __float_as_uint(val) : 0u);
+}
+__device__ __forceinline__ void dt_atomic(unsigned bits, InstState* st) {
+  // a maximum that is already there (or an older, smaller one) saves the atomic: all go to one address
+  const unsigned long long v = (unsigned long long)__double_as_longlong((double)__uint_as_float(bits));
+  if (bits && v > __ldcg(&st->maxd_bits)) atomicMax(&st->maxd_bits, v);
+}
 __device__ __forceinline__ void dt_reduce(float val, int64_t r, const Graph& G, InstState* St) {
-  for (int off = 16; off > 0; off >>= 1) val = fmaxf(val, __shfl_down_sync(0xffffffffu, val, off));
+  const unsigned m = dt_warp_max(val);
   const int64_t r0 = r & ~(int64_t)31;
   if ((threadIdx.x & 31) == 0 && r0 < G.n_rows) {
     const int bw = G.slice_inst[r0 >> 5];
-    if (!St[bw].done && val > 0.f)
-      atomicMax(&St[bw].maxd_bits, (unsigned long long)__double_as_longlong((double)val));
+    if (!St[bw].done) dt_atomic(m, &St[bw]);
+  }
+}
+// The same for a tile: one atomic per block where its slices are of one
+// instance (one per warp cost 4M nodes 125,000 atomics on one address).
+template <int T>
+__device__ __forceinline__ void dt_reduce_tile(float val, const Tile& t, InstState* St) {
+  __shared__ unsigned wm[T / 32];
+  __shared__ int wb[T / 32];
+  const unsigned m = dt_warp_max(val);
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    wm[w] = m;
+    wb[w] = t.live ? t.hd.b : -1;               // rows exist by whole slices
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned best = 0;
+    for (int k = 0; k < T / 32; k++) {
+      best = wm[k] > best ? wm[k] : best;
+      const int b = wb[k];
+      if (k == T / 32 - 1 || wb[k + 1] != b) {   // the end of an instance's slices
+        if (b >= 0 && !St[b].done) dt_atomic(best, &St[b]);
+        best = 0;
+      }
+    }
   }
 }
 
@@ -1380,7 +1420,7 @@ __global__ void __launch_bounds__(T) k_dt_tile(Graph G, const InstConst* C, Inst
   cp_wait();
   __syncthreads();
   pdl_trigger();
-  dt_reduce(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile<3>(t, sm)), t.r, G, St);
+  dt_reduce_tile<T>(dt_row<1>(t.r, t.hd, G, C, St, dlam, alpha_out, err, nb_tile<3>(t, sm)), t, St);
   step_turn(turn, C, St);
 }
 
