@@ -1253,11 +1253,16 @@ __global__ void k_fct_fct(Graph G, const InstConst* C, const InstState* St,
     if (bits64(f) < 0) P = P + f;                 // -0 adds nothing
   }
   const double h = hL[r];
-  if (h < 0.0) atomicOr(err, ERRB_NEG_H);
+  if (__double2hiint(h) < 0 && h < 0.0) atomicOr(err, ERRB_NEG_H);
   const double scaled = div_known(G.lumped[r], St[b].dt, St[b].inv_dt) * h;
-  const double Q = 0.0 - scaled;
-  double R = tmin(Q / P, 1.0);
-  if (scaled <= C[b].htiny) R = 0.0;
+  double R = 0.0;
+  if (!le_nn(scaled, C[b].htiny)) {
+    R = 1.0;                                      // Q^-/P^- >= 1: most rows
+    if (bits64(scaled) < bits64(-P)) {
+      real_branch();
+      R = scaled / -P;
+    }
+  }
   rminus[r] = R;
 }
 

@@ -46,6 +46,20 @@
 
 namespace swe {
 
+// (double)f without the FP64 unit, which bounds the precision split's limiter
+// and update: the exponent rebiased, the mantissa moved; subnormals are 0 as
+// everywhere in this file.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+  const bool zero = m < 0x00800000u;
+  const unsigned hi = (m >> 3) + (m >= 0x7f800000u ? 0x70000000u : 0x38000000u);
+  return __hiloint2double((int)((b & 0x80000000u) | (zero ? 0u : hi)), (int)(zero ? 0u : m << 29));
+}
+__device__ __forceinline__ float2 df_split(double v) {   // df_from_double
+  const float hi = __double2float_rn(v);
+  return make_float2(hi, __double2float_rn(v - widen(hi)));
+}
+
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
@@ -772,12 +786,12 @@ __device__ __forceinline__ void low_row(int r, const RowHead& hd, const Graph& G
   // k_update adds the high-order correction before MAX(., 0))
   const bool clip = FCT || c.visc != VISC_ENTROPY;
   if (D) {
-    const double hd = df_to_double(h), ad = st.dt * G.inv_lumped[r];
+    const double hd = widen(h.x) + widen(h.y), ad = st.dt * G.inv_lumped[r];
     double hL;
     if (roundoff) {
-      hL = fma(ad, fma(-(double)cvd, (double)ni.h, (double)P - (double)N), hd);
+      hL = fma(ad, fma(-widen(cvd), widen(ni.h), widen(P) - widen(N)), hd);
     } else {
-      hL = fma(ad, (double)g0, hd);
+      hL = fma(ad, widen(g0), hd);
       if (clip && hL < 0.0) hL = 0.0;
     }
     w.hL64[r] = hL;
@@ -1011,13 +1025,18 @@ __device__ __forceinline__ void fct_row(int r, const RowHead& hd, const Graph& G
     }
   }
   if (D) {   // precision split: Q^-, P^-, R^- and the dry test in FP64, as the reference
+    // (the FP64 unit bounds this kernel: compares and conversions on integers)
     const double hL = w.hL64[r];
-    if (hL < 0.0) atomicOr(err, ERRB_NEG_H);
-    const double scaled = (G.lumped[r] / st.dt) * hL;                           // (lumped/dt) h^L
+    if (__double2hiint(hL) < 0 && hL < 0.0) atomicOr(err, ERRB_NEG_H);
+    const double scaled = div_known(G.lumped[r], st.dt, st.inv_dt) * hL;        // (lumped/dt) h^L
     double R = 0.0;
-    if (!(scaled <= c.htiny)) {
-      const double Pm = -1.e-15 + (double)neg;
-      R = fmin((0.0 - scaled) / Pm, 1.0);
+    if (!le_nn(scaled, c.htiny)) {
+      const double mP = 1.e-15 - widen(neg);                                    // -P^- > 0
+      R = 1.0;                                                                   // Q^-/P^- >= 1: most rows
+      if (bits64(scaled) < bits64(mP)) {
+        real_branch();
+        R = scaled / mP;
+      }
     }
     w.rminus64[r] = R;
     w.rminus[r] = (float)R;
@@ -1098,7 +1117,7 @@ __device__ __forceinline__ void finish_mix(const Graph& G, const InstConst& c, c
   if (rk_stage >= 1 && G.dir_mask) {
     const unsigned msk = G.dir_mask[r];
     if (msk) {
-      if (msk & 1u) hn = df_from_double(dirichlet_value(G, c, st, rk_stage, 0, r));
+      if (msk & 1u) hn = df_split(dirichlet_value(G, c, st, rk_stage, 0, r));
       if (msk & 2u) q1 = (float)dirichlet_value(G, c, st, rk_stage, 1, r);
       if (msk & 4u) q2 = (float)dirichlet_value(G, c, st, rk_stage, 2, r);
       if (S == 5 && (msk & 8u)) q3 = (float)G.dir_val[3 * G.n_rows + r];
@@ -1141,7 +1160,7 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
   const bool ent = !FCT && c.visc == VISC_ENTROPY;
   if (!FCT && c.visc != VISC_FCT && !ent) {             // 'galerkin' / 'viscous': u^L is the result
     const float2 qL = w.qL[r];
-    finish_mix(G, c, st, r, S, D ? df_from_double(w.hL64[r]) : w.hL[r], qL.x, qL.y, S == 5 ? w.q3L[r] : 0.f,
+    finish_mix(G, c, st, r, S, D ? df_split(w.hL64[r]) : w.hL[r], qL.x, qL.y, S == 5 ? w.q3L[r] : 0.f,
                S == 5 ? w.q4L[r] : 0.f, rk_stage, u0, out, err);
     return;
   }
@@ -1192,7 +1211,7 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
     float lf = Ri;
     if (f >= 0.f) {
       lf = ent ? 1.f : nj.R;
-      if (D && !ent) pos64 = fma(nb.r64(jb[q]), (double)f, pos64);
+      if (D && !ent) pos64 = fma(nb.r64(jb[q]), widen(f), pos64);
       else pos = __fmaf_rn(lf, f, pos);
     } else {
       neg = __fadd_rn(neg, f);
@@ -1212,10 +1231,10 @@ __device__ __forceinline__ void update_row(int r, const RowHead& hd, const Graph
   const float invm = G.inv_lumpedf[r], dtf = st.dtf;
   float2 hn;
   if (D) {       // u^L + dt/m sum l_ij f_ij for the depth, in FP64
-    const double sh = ent ? (double)__fadd_rn(neg, pos) : fma(nb.r64(me), (double)neg, pos64);
+    const double sh = ent ? (double)__fadd_rn(neg, pos) : fma(nb.r64(me), widen(neg), pos64);
     double h64 = fma(st.dt * G.inv_lumped[r], sh, w.hL64[r]);
     if (ent && !c.roundoff_fix && h64 < 0.0) h64 = 0.0;       // smb_2: MAX(h + dt rk, 0)
-    hn = df_from_double(h64);
+    hn = df_split(h64);
   } else {
     const float sh = __fadd_rn(__fmul_rn(Ri, neg), pos);
     hn = df_add_f(w.hL[r], __fmul_rn(__fmul_rn(dtf, invm), sh));
