@@ -272,6 +272,12 @@ static bool has_type1(const swe_ctx* c) {
   return false;
 }
 
+static bool has_fct(const swe_ctx* c) {
+  for (const swe_params& p : c->params)
+    if (p.viscosity_type == SWE_VISC_FCT) return true;
+  return false;
+}
+
 static bool has_entropy(const swe_ctx* c) {
   for (const swe_params& p : c->params)
     if (p.viscosity_type == SWE_VISC_ENTROPY) return true;
@@ -295,6 +301,13 @@ static bool all_fct_limited(const swe_ctx* c) {
   for (const swe_params& p : c->params)
     if (!p.if_alpha_limit) return false;
   return all_fct(c);
+}
+
+// The mixed stage's mode flags (see StageArgsMix)
+static void set_modes(const swe_ctx* c, StageArgsMix& a) {
+  a.fct = all_fct_limited(c);
+  a.any_fct = has_fct(c);
+  a.any_high = a.any_fct || has_entropy(c);
 }
 
 static int check_params(swe_ctx* c, const swe_params& p) {
@@ -834,6 +847,7 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
     if (c->precision == SWE_PREC_FP64) {
       StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, stage, nullptr, c->d_err, c->block};
       a.entropy = has_entropy(c);
+      a.any_fct = has_fct(c);
       a.fused = all_fct_rows(c);
       a.all_fct = all_fct(c);
       a.S = c->S;
@@ -846,8 +860,8 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
       a.tiles = c->tiles_ok ? &c->tiles : nullptr;
       a.f64 = is_split(c);
       a.type1 = has_type1(c);
-      a.fct = all_fct_limited(c);
-      if (stage == 2) { a.u = c->mB; a.out = c->mC; }
+      set_modes(c, a);
+            if (stage == 2) { a.u = c->mB; a.out = c->mC; }
       if (stage == 3) { a.u = c->mC; a.out = c->mA; }
       launch_stage_mix(a, s, kev, c->tune);
     }
@@ -1225,6 +1239,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
   if (c->precision == SWE_PREC_FP64) {
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
+    a.any_fct = has_fct(c);
     a.fused = all_fct_rows(c);
     a.all_fct = all_fct(c);
     a.S = c->S;
@@ -1234,8 +1249,8 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
     a.tiles = c->tiles_ok ? &c->tiles : nullptr;
     a.f64 = is_split(c);
     a.type1 = has_type1(c);
-    a.fct = all_fct_limited(c);
-    launch_stage_mix(a, c->stream, nullptr, c->tune);
+    set_modes(c, a);
+        launch_stage_mix(a, c->stream, nullptr, c->tune);
   }
   if ((rc = cuda_check(c, cudaGetLastError(), "euler")) ||
       (rc = from_device_state(c, unext, false, c->node_off[inst], c->node_off[inst + 1],
@@ -1556,6 +1571,7 @@ static int autotune(swe_ctx* c) {
   StageArgsMix a{c->G, c->d_C, c->d_St, c->mA, c->mA, c->mB, c->wm, 1, c->d_err, c->block};
   a.f64 = is_split(c);
   a.type1 = has_type1(c);
+  set_modes(c, a);
   KernelTune t = c->tune;
   for (int& k : t.tiled) k = 0;
   launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, t, nullptr, StepTurn{}, s);   // populate every work array once
@@ -1855,7 +1871,7 @@ static int enqueue_rk3_steps(swe_ctx* c, int nsteps) {
   CK(cudaEventRecord(c->t0, c->stream));
   // the mixed stage 1 takes alpha from k_dt_mix: one k_node launch fewer
   const long long per_step = 3LL * kLaunchesPerStage + kLaunchesPerStepExtra -
-                             (is_mixed(c) ? 1 : 0) + (turn_in_dt(c) ? 0 : 1) + (c->n_gauges ? 2 : 0);
+                             (is_mixed(c) ? 1 : 0) - (has_fct(c) ? 0 : 3) + (turn_in_dt(c) ? 0 : 1) + (c->n_gauges ? 2 : 0);
   const long long per_graph = c->n_gauges ? 0 : 1;   // k_step_end
   if (nsteps >= chunk && chunk > 1) {
     for (int k = 0; k + chunk <= nsteps; k += chunk) {

@@ -66,6 +66,7 @@ struct StageArgs {
   unsigned* err;
   int block;
   int entropy = 0;   // some instance uses 'entropy_visc': launch k_entropy
+  int any_fct = 1;   // some instance uses 'fct': launch k_fct
   int fused = 0;     // every instance runs 'fct', 'viscous' 'type2' or 'entropy_visc' with the roundoff fix: the 'fct' row kernels
   int all_fct = 0;   // every instance runs 'fct' with the roundoff fix
   int S = 3;
@@ -103,6 +104,8 @@ struct StageArgsMix {
   bool f64 = false;                 // precision split: h^L, R^- and the depth's limited sum in FP64
   bool type1 = false;               // some instance runs 'viscous' with viscous_type 'type1'
   bool fct = false;                 // every instance runs 'fct' with the roundoff fix and alpha_limit
+  bool any_fct = true;              // some instance runs 'fct': k_fct
+  bool any_high = true;             // some instance runs 'fct' or 'entropy_visc': k_update walks the entries
 };
 
 // Optional per-kernel event timing: when non-null, ev[2k], ev[2k+1] bracket

@@ -1546,7 +1546,8 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
     else { if (a.all_fct) SWE_LOWF(3, true); else SWE_LOWF(3, false); }
 #undef SWE_LOWF
     EV_END(2); EV_BEGIN(3);
-    launch_full(k_fct_fct, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
+    if (a.any_fct)
+      launch_full(k_fct_fct, nb, bs, 0, s, a.G, a.C, a.St, a.w.dL, a.w.muL, a.w.uL.h, a.w.res, a.w.ab, a.w.fct, a.w.rminus, ne,
                                 a.err);
     EV_END(3); EV_BEGIN(4);
     if (a.S == 5)
@@ -1569,7 +1570,8 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
   launch_full(k_low_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res, a.dij_in,
                               a.err);
   EV_END(2); EV_BEGIN(3);
-  launch_full(k_fct_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.err);
+  if (a.any_fct)
+    launch_full(k_fct_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.err);
   EV_END(3); EV_BEGIN(4);
   launch_full(k_update_f64, nb, bs, 0, s, a.G, a.C, a.St, a.u, a.w.dL, a.w.muL, a.w.uL, a.w.res, a.w.fct, a.w.rminus, a.u0, a.out,
                                  a.rk_stage, a.lij_out, a.err);

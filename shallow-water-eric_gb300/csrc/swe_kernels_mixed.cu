@@ -1570,7 +1570,8 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
             else
               launch_low<false, D>(a, t.batch[2], t.cap_low, t.grid[2], t.block[2], t.tiled[2], s);
             break;
-    case 3: if (t.tiled[3] && a.tiles) {
+    case 3: if (!a.any_fct) break;
+            if (t.tiled[3] && a.tiles) {
               SWE_TILE_T(*a.tiles, launch_tile(k_fct_tile<T, D>, *a.tiles, n, 3, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu,
                                                a.w, a.w.res, a.err));
             } else {
@@ -1578,7 +1579,8 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
                               a.w.res, a.err)
             }
             break;
-    case 4: if (t.tiled[4] && a.tiles) {
+    case 4: if (t.tiled[4] && a.tiles && a.any_high) {   // else rows only: nothing to stage
+
 #define SWE_UPDT(TT, SS, F)                                                                                        \
               launch_tile(k_update_tile<TT, SS, D, F>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu,   \
                           a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err)
