@@ -15,6 +15,9 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/swe_gpu.h"
@@ -660,6 +663,30 @@ static int to_device(swe_ctx* c, const double* un, bool device_src, int64_t node
   return SWE_OK;
 }
 
+// Maps the pages of a caller's pageable array that the kernel has not mapped
+// yet (a fresh numpy array's), while the GPU works: a copy into unmapped pages
+// waits for every one of them (24 MB: about 1 ms).  A page's first byte is
+// written back unchanged; mapped pages and page-locked memory are left alone.
+static void prefault(void* p, size_t bytes) {
+  if (!p || bytes < (64 << 10)) return;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  char* b = reinterpret_cast<char*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)(page - 1));
+  char* e = static_cast<char*>(p) + bytes;
+  std::vector<unsigned char> in((size_t)(e - b + page - 1) / page);
+  if (mincore(b, e - b, in.data()) != 0) return;
+  for (size_t k = 0; k < in.size(); k++)
+    if (!(in[k] & 1)) {
+      volatile char* q = k ? b + k * page : static_cast<char*>(p);
+      *q = *q;
+    }
+}
+
 static int from_device_state(swe_ctx* c, double* un, bool device_dst, int64_t node_begin, int64_t node_end,
                              const StateF64* sf, const StateMix* sm, bool low_mix = false) {
   const int64_t nn = node_end - node_begin;
@@ -1178,7 +1205,8 @@ static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, con
     cudaError_t st = cudaSuccess;
     c->d_ref_pos = upload_vec(c, L.ref_pos, st);
     c->d_ref_pos_diag = upload_vec(c, L.ref_pos_diag, st);
-    double* csr = c->buf.alloc<double>(most, st);
+    // FP64: the row differences are free between calls
+    double* csr = c->w.ab ? c->w.ab : c->buf.alloc<double>(most, st);
     if (st != cudaSuccess) return cuda_check(c, st, "device allocation");
     c->d_csr = csr;
   }
@@ -1215,6 +1243,7 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
     launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, StepTurn{}, c->stream);
     rc = cuda_check(c, cudaGetLastError(), "compute_dij");
   }
+  if (!rc && dij) prefault(dij, c->meshes[inst].ja.size() * sizeof(double));
   if (!rc) rc = call_end(c, inst);                   // nothing is written to the caller's arrays on an error
   if (rc) { drain(c); return rc; }
   if (dij) {
@@ -1252,6 +1281,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
     set_modes(c, a);
         launch_stage_mix(a, c->stream, nullptr, c->tune);
   }
+  prefault(unext, sizeof(double) * c->S * (size_t)c->meshes[inst].np);
   if ((rc = cuda_check(c, cudaGetLastError(), "euler")) ||
       (rc = from_device_state(c, unext, false, c->node_off[inst], c->node_off[inst + 1],
                               c->precision == SWE_PREC_FP64 ? &c->B : nullptr,
@@ -1423,6 +1453,7 @@ SWE_API int swe_upload(swe_ctx* c, const double* un) {
 SWE_API int swe_download(swe_ctx* c, double* un) {
   NvtxRange nvtx("swe_download");
   if (!c || !un) return fail(c, SWE_ERR_ARG, "bad arguments");
+  prefault(un, sizeof(double) * c->S * (size_t)c->node_off[c->n_inst]);
   int rc = from_device_state(c, un, false, 0, c->node_off[c->n_inst], c->precision == SWE_PREC_FP64 ? &c->A : nullptr,
                              c->precision == SWE_PREC_FP64 ? nullptr : &c->mA);
   if (rc) { drain(c); return rc; }
@@ -1925,9 +1956,13 @@ SWE_API int swe_rk3_steps_host(swe_ctx* c, const double* un, double* unext, int 
   if (!c || nsteps < 0) return fail(c, SWE_ERR_ARG, "bad arguments");
   const int64_t nn = c->node_off[c->n_inst];
   int rc;
-  if ((un && (rc = to_device(c, un, false, 0, nn))) || (rc = enqueue_rk3_steps(c, nsteps)) ||
-      (unext && (rc = from_device_state(c, unext, false, 0, nn, c->precision == SWE_PREC_FP64 ? &c->A : nullptr,
-                                        c->precision == SWE_PREC_FP64 ? nullptr : &c->mA)))) {
+  if ((un && (rc = to_device(c, un, false, 0, nn))) || (rc = enqueue_rk3_steps(c, nsteps))) {
+    drain(c);
+    return rc;
+  }
+  if (unext) prefault(unext, sizeof(double) * c->S * (size_t)nn);
+  if (unext && (rc = from_device_state(c, unext, false, 0, nn, c->precision == SWE_PREC_FP64 ? &c->A : nullptr,
+                                       c->precision == SWE_PREC_FP64 ? nullptr : &c->mA))) {
     drain(c);
     return rc;
   }
