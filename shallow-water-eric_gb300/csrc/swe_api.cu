@@ -1565,7 +1565,7 @@ static int apply_tuning(swe_ctx* c, const char* spec, const char* what) {
 }
 
 // Launch configuration of the mixed kernels: the tile variants where the mesh
-// has tiles; else (5-component systems, tiles too large for shared memory)
+// has tiles; else (tiles too large for shared memory, or left out)
 // every (block size, entry batch, grid) variant of each kernel is timed on the
 // current state and the fastest kept.  All variants give the same bits, and
 // every timed kernel is idempotent on its inputs (it only rewrites its own

@@ -158,7 +158,7 @@ void launch_fct_generic_f64(const Graph& G, double* unext, const double* maxn, c
 // rows, or one block per tile of rows with shared-memory neighbours), and for
 // low a register cap (cap_low 0, 1, 2: at least 3, 4 or 5 resident blocks of
 // 256 threads per SM, i.e. at most 85, 64 or 51 registers; the tightest
-// spills a little).  Chosen by the autotuner in swe_api.cu.  Every choice
+// spills a little).  Chosen by autotune() in swe_api.cu.  Every choice
 // performs the same IEEE operations in the same entry order (the mixed
 // kernels are built without FMA contraction and spell out every fused
 // multiply-add), so every choice gives bit-identical results.
@@ -176,7 +176,6 @@ constexpr int kTileSmemMax = 100 * 1024;
 // dynamic shared memory of a tile block, the most over the kernel kinds (d: with the FP64 R^- of the precision split)
 size_t tile_smem_max(const TileCtl& tc, bool d);
 void launch_kernel_mix(int kind, const StageArgsMix& a, const KernelTune& t, cudaStream_t s);
-bool kind_has_tiles(int kind);   // kernel kinds with a shared-memory tile variant
 void launch_dt_mix(const Graph& G, const InstConst* C, InstState* St, const StateMix& u, float* dlam, float* alpha,
                    unsigned* err, const KernelTune& t, const TileCtl* tiles, const StepTurn& turn, cudaStream_t s);
 void launch_refresh_eta(const Graph& G, StateMix u, cudaStream_t s);

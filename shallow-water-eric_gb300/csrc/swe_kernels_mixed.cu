@@ -1550,8 +1550,6 @@ static void launch_low(const StageArgsMix& a, int batch, int cap, int mode, int 
 #undef SWE_LOW
 }
 
-bool kind_has_tiles(int kind) { return kind >= 0 && kind <= 4; }
-
 template <bool D>
 static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTune& t, cudaStream_t s) {
   const int64_t n = a.G.n_rows;
@@ -1580,7 +1578,6 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
             }
             break;
     case 4: if (t.tiled[4] && a.tiles && a.any_high) {   // else rows only: nothing to stage
-
 #define SWE_UPDT(TT, SS, F)                                                                                        \
               launch_tile(k_update_tile<TT, SS, D, F>, *a.tiles, n, 4, D, false, s, a.G, a.C, a.St, a.u, a.w.dmu,   \
                           a.w, a.w.res, a.u0, a.out, a.rk_stage, a.err)
