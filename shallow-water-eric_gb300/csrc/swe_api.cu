@@ -306,6 +306,9 @@ static bool all_fct_limited(const swe_ctx* c) {
   return all_fct(c);
 }
 
+// more than four 256-row blocks per SM
+static bool large_mesh(const swe_ctx* c) { return c->G.n_rows > 4 * 256 * (int64_t)c->sms; }
+
 // The mixed stage's mode flags (see StageArgsMix)
 static void set_modes(const swe_ctx* c, StageArgsMix& a) {
   a.fct = all_fct_limited(c);
@@ -498,7 +501,6 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     w.alpha = c->buf.alloc<float>(n, st); w.res = c->buf.alloc<float>(n, st);
     w.rminus = c->buf.alloc<float>(n, st);
     w.dmu = c->buf.alloc<float2>(ne, st);
-    w.dlam = c->buf.alloc<float>(ne, st);
     w.hL = c->buf.alloc<float2>(n, st);
     if (is_split(c)) {     // FP64 low-order depth in hL's 8 bytes per row, FP64 R^-
       w.hL64 = reinterpret_cast<double*>(w.hL);
@@ -537,6 +539,12 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
       c->tiles.halo_rows = upload_vec(c, halo, st);
       c->tiles_ok = true;
     }
+    // Stage 1 reads |c_ij| lambda_max from k_dt while the entries stay in L2
+    // or the latency of a small mesh counts (10k nodes 44.4 us a step against
+    // 44.8, 103k 77.2 / 78.3, 260k equal); with tiles on a larger mesh it forms
+    // them again: 48 bytes per node less (708k nodes 326.8 -> 319.0 us, 1M 397.1 ->
+    // 394.5, 4M 1394 -> 1389, 2M of a 5-component system 929 -> 923).
+    if (!c->tiles_ok || !large_mesh(c)) w.dlam = c->buf.alloc<float>(ne, st);
   }
   if (st != cudaSuccess) return fail(c, SWE_ERR_CUDA, std::string("device allocation: ") + cudaGetErrorString(st));
   return SWE_OK;
@@ -831,7 +839,7 @@ static int save_state(swe_ctx* c, std::vector<InstState>& saved) {
 }
 
 // k_dt's last block runs the turn between steps: up to four 256-row blocks per SM
-static bool turn_in_dt(const swe_ctx* c) { return c->G.n_rows <= 4 * 256 * (int64_t)c->sms; }
+static bool turn_in_dt(const swe_ctx* c) { return !large_mesh(c); }
 
 // One time step of a sequence.  k_dt's last block closes the step before
 // (open: it is still open) and opens this one; the last step of a sequence

@@ -47,7 +47,7 @@ struct WorkMix {
   float *alpha, *res;                    // per row
   float* rminus;                         // per row: R^-_i
   float2* dmu;                           // per entry: (d_ij, mu_ij), one 8-byte load
-  float* dlam;                           // per entry: |c_ij| lambda_max from k_dt_mix (stage 1)
+  float* dlam;                           // per entry: |c_ij| lambda_max from k_dt_mix (stage 1), or null
   float2* hL;                            // low-order depth (double-float)
   double* hL64;                          // precision split: the FP64 low-order depth (hL's storage), or null
   double* rminus64;                      // precision split: FP64 R^-_i, or null

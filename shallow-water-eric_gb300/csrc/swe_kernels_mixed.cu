@@ -1563,7 +1563,7 @@ static void launch_kernel_mix_d(int kind, const StageArgsMix& a, const KernelTun
     case 2: if (a.type1)                       // some instance runs 'viscous' with 'type1'
               launch_k(k_low_type1<D>, nblk(n, 128), 128, 0, s, a.G, a.C, a.St, a.u, a.w.alpha, a.w.dmu, a.w, a.w.res,
                        a.err);
-            else if (a.rk_stage == 1 && a.w.dlam)   // stage 1 follows k_dt_mix on the same state
+            else if (a.rk_stage == 1 && a.w.dlam)   // k_dt_mix on the same state kept them
               launch_low<true, D>(a, t.batch[2], t.cap_low, t.grid[2], t.block[2], t.tiled[2], s);
             else
               launch_low<false, D>(a, t.batch[2], t.cap_low, t.grid[2], t.block[2], t.tiled[2], s);
@@ -1604,7 +1604,7 @@ void launch_stage_mix(const StageArgsMix& a, cudaStream_t s, const KernelEvents*
   for (int kind = 1; kind <= 4; kind++) {
     EV_BEGIN(kind);
     // stage 1 follows k_dt_mix on the same state, which already stored alpha
-    if (!(kind == 1 && a.rk_stage == 1 && a.w.dlam)) launch_kernel_mix(kind, a, t, s);
+    if (!(kind == 1 && a.rk_stage == 1)) launch_kernel_mix(kind, a, t, s);
     EV_END(kind);
   }
 }

@@ -94,3 +94,29 @@ def test_tiles_straddling_instances(monkeypatch, prec):
     instances, each with its own depth scale, friction and dt."""
     items = C.batch_instances(n_inst=7, nmin=20, nmax=900, seed=5, precision=prec)
     _same(monkeypatch, items, np.hstack([c.u0 for c in items]))
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("kind", ["basin", "sgn"])
+def test_batch_above_the_size_rules(kind, prec):
+    """Meshes above four 256-row blocks per SM take another turn between steps,
+    and their stage 1 forms the wave speeds k_dt keeps on smaller ones: a batch
+    above that size equals its instances, each below it, bit for bit."""
+    c = _case(kind, 300, 290, prec, "fct")
+    one = Update(c.mesh, c.bath, c.params)
+    one.upload(c.u0)
+    one.set_time(0.0, 1e30)
+    _, dt1, _ = one.rk3_steps(3)
+    u1 = one.download()
+    one.close()
+    both = Update(batch=[(c.mesh, c.bath, c.params)] * 2)
+    both.upload(np.hstack([c.u0, c.u0]))
+    both.set_time(0.0, 1e30)
+    _, dt2, _ = both.rk3_steps(3)
+    u2 = both.download()
+    both.close()
+    n = u1.shape[1]
+    assert n < 4 * 256 * 152 < 2 * n
+    for b in (0, 1):
+        np.testing.assert_array_equal(u2[:, b * n:(b + 1) * n], u1)
+        assert dt2[b] == dt1[0]
