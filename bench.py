@@ -139,12 +139,14 @@ def design_bytes(n, nnz):
     """Bytes per node that each mixed stage kernel reads and writes once per
     launch in the four-sweep design (3-component systems), with e the
     off-diagonal entries per row (16-bit position, c_ij or (d, mu), |c|lambda
-    per entry): k_dt 25 + 14e; k_low 65 + 18e, plus 4e in stage 1 (it reads
-    k_dt's |c|lambda); k_fct 37 + 10e; k_update 78 + 10e, plus 24 in stages 2
-    and 3 (u0); k_node 21 + 4e in stages 2 and 3.  Averaged per stage like
-    swe_profile_kernels' times."""
+    per entry): k_dt 25 + 10e; k_low 65 + 18e; k_fct 37 + 10e; k_update
+    78 + 10e, plus 24 in stages 2 and 3 (u0); k_node 21 + 4e in stages 2 and
+    3.  Meshes of up to four 256-row blocks per SM keep k_dt's |c|lambda for
+    stage 1: 4e more written by k_dt and read by k_low.  Averaged per stage
+    like swe_profile_kernels' times."""
     e = (nnz - n) / n
-    return {"dt": 25 + 14 * e, "node": (21 + 4 * e) * 2 / 3, "low": 65 + 18 * e + 4 * e / 3,
+    kept = 4 * e if n <= 4 * 256 * 152 else 0.0
+    return {"dt": 25 + 10 * e + kept, "node": (21 + 4 * e) * 2 / 3, "low": 65 + 18 * e + kept / 3,
             "fct": 37 + 10 * e, "update": 78 + 10 * e + 16}
 
 
