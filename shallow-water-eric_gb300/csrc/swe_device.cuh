@@ -433,7 +433,8 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
   const float s = (lv - rv) + 2.f * (l.f.y + r.f.y);
   const float i16g = 0.0625f / c.gf;
   const float su = fmaxf(s + tol, 0.f), sm = fmaxf(s, 0.f);
-  const float hup = su * su * i16g * 1.000002f, hst = sm * sm * i16g;   // ht <= hup
+  const float hup = su * su * i16g * 1.000002f;                         // ht <= hup
+  const float hst = fminf(sm * sm * i16g, 3.3431458f * hmin);
   const bool triv_l = hup <= l.f.x * 0.999998f, triv_r = hup <= r.f.x * 0.999998f;
   const float xl = fmaxf((hst - l.f.x) * one_over_h_f(l.f.x, c.htinyf), 0.f);
   const float xr = fmaxf((hst - r.f.x) * one_over_h_f(r.f.x, c.htinyf), 0.f);

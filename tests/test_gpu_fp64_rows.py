@@ -89,6 +89,65 @@ def test_dij_bit_exact(kind, n):
 DUMPS = ("dij_low", "muij_low", "alpha", "u_low", "res", "fctmat", "rminus", "lij")
 
 
+def _normals(mesh):
+    """{(i, j): c_ij / |c_ij|} of the edges, c_ij the integral of phi_i grad phi_j."""
+    c = {}
+    for tri in mesh["jj"].T - 1:
+        a, b, d = mesh["rr"][:, tri].T
+        two_area = (b[0] - a[0]) * (d[1] - a[1]) - (b[1] - a[1]) * (d[0] - a[0])
+        s = np.sign(two_area)
+        for k in range(3):
+            p, q = mesh["rr"][:, tri[(k + 1) % 3]], mesh["rr"][:, tri[(k + 2) % 3]]
+            grad = s * np.array([p[1] - q[1], q[0] - p[0]]) / 6.0         # area/3 grad phi_k
+            for m in range(3):
+                if m != k:
+                    c[tri[m], tri[k]] = c.get((tri[m], tri[k]), 0.0) + grad
+    return {e: v / np.hypot(*v) for e, v in c.items()}
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_dij_where_the_depth_limit_decides(seed):
+    """Pairs of nodes whose two-rarefaction depth is cut off at x0 hmin, and
+    whose larger speed is the other one without the cut."""
+    rng = np.random.default_rng(seed)
+    g, n = 9.81, 400_000
+    x0 = (2 * np.sqrt(2.0) - 1) ** 2
+    cmin = np.sqrt(g)
+    ratio = rng.uniform(3.05, 3.34, n)
+    swap = rng.random(n) < 0.5
+    hl, hr = np.where(swap, 1.0, ratio), np.where(swap, ratio, 1.0)
+    dv, mid = rng.uniform(1.75, 1.887, n) * cmin, rng.uniform(-1, 1, n) * cmin
+    vl, vr = mid + dv / 2, mid - dv / 2
+    hs = (dv + 2 * np.sqrt(g * hl) + 2 * np.sqrt(g * hr)) ** 2 / 16 / g
+
+    def speeds(h):
+        xl, xr = np.maximum((h - hl) / hl, 0), np.maximum((h - hr) / hr, 0)
+        return (np.abs(vl - np.sqrt(g * hl) * np.sqrt((1 + xl / 2) * (1 + xl))),
+                np.abs(vr + np.sqrt(g * hr) * np.sqrt((1 + xr / 2) * (1 + xr))))
+
+    (al, ar), (tl, tr) = speeds(hs), speeds(np.minimum(x0, hs))
+    pick = np.nonzero((al > 1.001 * ar) & (tr > 1.001 * tl) | (ar > 1.001 * al) & (tl > 1.001 * tr))[0]
+    assert len(pick) > 50
+    mesh = M.jittered_mesh(21, 21, 0.0, 10.0, 0.0, 10.0, jitter=0.3, seed=7)
+    p = C.Params(max_water_h=4.0, precision=0)
+    nn = mesh["rr"].shape[1]
+    u = np.zeros((3, nn), order="F")
+    u[0] = 1.0
+    used, k = set(), 0
+    for (i, j), nv in _normals(mesh).items():
+        if i in used or j in used:
+            continue
+        used |= {i, j}
+        q = pick[k % len(pick)]
+        k += 1
+        u[:, i] = np.r_[hl[q], hl[q] * vl[q] * nv]
+        u[:, j] = np.r_[hr[q], hr[q] * vr[q] * nv]
+    o, upd = _pair(mesh, np.zeros(nn), p)
+    ref, got = o.compute_dij(u), upd.compute_dij(u)
+    np.testing.assert_array_equal(got[0], ref[0])
+    assert got[1] == ref[1]
+
+
 @pytest.mark.parametrize("type_test,alpha,bumpy", [(4, 1, 0), (4, 1, 1), (4, 0, 1), (11, 1, 1), (12, 1, 0)])
 @pytest.mark.parametrize("kind", STATES)
 def test_fct_stage_bit_exact(kind, type_test, alpha, bumpy):
