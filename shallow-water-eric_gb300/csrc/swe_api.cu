@@ -871,7 +871,7 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
   }
   if (kev) cudaEventRecord(kev->ev[0], s);
   if (c->precision == SWE_PREC_FP64)
-    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.fct, nullptr, c->d_err, c->block, turn, s);
+    launch_dt_f64(c->G, c->d_C, c->d_St, c->A, c->w, c->w.fct, nullptr, c->d_err, turn, s);
   else launch_dt_mix(c->G, c->d_C, c->d_St, c->mA, c->wm.dlam, c->wm.alpha, c->d_err, c->tune,
                    c->tiles_ok ? &c->tiles : nullptr, turn, s);
   if (kev) cudaEventRecord(kev->ev[1], s);
@@ -1248,7 +1248,7 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
     a.w.alpha = nullptr;                             // the last euler call's alpha stays readable
     launch_node_f64(a, c->stream);
-    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, c->block, StepTurn{}, c->stream);
+    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, StepTurn{}, c->stream);
     rc = cuda_check(c, cudaGetLastError(), "compute_dij");
   }
   if (!rc && dij) prefault(dij, c->meshes[inst].ja.size() * sizeof(double));

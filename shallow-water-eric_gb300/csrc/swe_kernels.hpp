@@ -143,7 +143,7 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
 // launch_node_f64: per-node arrays of the state a.u; launch_dt_f64 reads them (node)
 void launch_node_f64(const StageArgs& a, cudaStream_t s);
 void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
-                   double* d_out, double* dii_out, unsigned* err, int block, const StepTurn& turn, cudaStream_t s);
+                   double* d_out, double* dii_out, unsigned* err, const StepTurn& turn, cudaStream_t s);
 void launch_step_turn(const StepTurn& t, const InstConst* C, InstState* St, cudaStream_t s);
 void launch_step_end(InstState* St, int n_inst, cudaStream_t s);
 void launch_reset_counters(InstState* St, int n_inst, cudaStream_t s);

@@ -1310,6 +1310,17 @@ __global__ void k_update_fct(Graph G, const InstConst* C, const InstState* St,
   finish_row_f64(G, c, st, r, S, un, fct_mode, rk_stage, u0, out, err);
 }
 
+// Maximum over a warp of values >= 0 (NaN counts as 0, as in fmax), lane 0:
+// compared as integers, off the FP64 unit.
+__device__ __forceinline__ double warp_max(double v) {
+  long long m = bits64(v) <= 0x7ff0000000000000ll ? bits64(v) : 0;
+  for (int off = 16; off > 0; off >>= 1) {
+    const long long o = __shfl_down_sync(0xffffffffu, m, off);
+    m = o > m ? o : m;
+  }
+  return __longlong_as_double(m);
+}
+
 // ---------------------------------------------------------------------------
 // k_dt: compute_dij (update.f90:291-326) diagonal and COMPUTE_DT's
 // max |d_ii|/m_i (main.f90:166-174), per instance.  d_out (nullable)
@@ -1341,8 +1352,7 @@ __global__ void k_dt_f64(Graph G, const InstConst* C, InstState* St, StateF64 u,
   }
   // warp-level max per instance: a warp covers one 32-row slice and a slice
   // never straddles two instances
-  const unsigned full = 0xffffffffu;
-  for (int off = 16; off > 0; off >>= 1) val = fmax(val, __shfl_down_sync(full, val, off));
+  val = warp_max(val);
   const int64_t r0 = r & ~(int64_t)31;
   if ((threadIdx.x & 31) == 0 && r0 < G.n_rows) {
     const int bw = G.slice_inst[r0 >> 5];
@@ -1387,7 +1397,7 @@ __global__ void __launch_bounds__(128) k_dt_split(Graph G, const InstConst* C, I
         if (dii_out) dii_out[r] = -s;
         val = div_known(s, G.lumped[r], G.inv_lumped[r]);
       }
-      for (int off = 16; off > 0; off >>= 1) val = fmax(val, __shfl_down_sync(0xffffffffu, val, off));
+      val = warp_max(val);
       if (lane == 0 && val > 0.0) atomicMax(&St[b].maxd_bits, (unsigned long long)__double_as_longlong(val));
     }
   }
@@ -1501,19 +1511,33 @@ static void launch_full(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
   kern<<<grid, block, smem, s>>>(static_cast<KArgs>(args)...);
 }
 
-// Where the four-warp kernels run: up to one wave of their blocks, 4 slices per
-// SM (registers), 2.5 for 5-component systems.  Per step, four warps against
-// one: 2k nodes 153 against 244 us, 10k 179 / 248, 16k 244 / 250, 20k 268 /
-// 332, 29k 360 / 346; SGN 2k 171 / 248, 12k 231 / 249, 16k 299 / 256.
-static bool split_rows(int64_t n_rows, int S) {
+static int64_t sm_count() {
   static const int64_t sms = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     return (int64_t)n;
   }();
-  return n_rows <= (S == 5 ? 80 : 128) * sms;
+  return sms;
 }
+
+// Where k_low runs four warps per slice: up to one wave of its blocks, 4 slices per
+// SM (registers), 2.5 for 5-component systems.  Per step, four warps against
+// one: 2k nodes 153 against 244 us, 10k 179 / 248, 16k 244 / 250, 20k 268 /
+// 332, 29k 360 / 346; SGN 2k 171 / 248, 12k 231 / 249, 16k 299 / 256.
+static bool split_rows(int64_t n_rows, int S) { return n_rows <= (S == 5 ? 80 : 128) * sm_count(); }
+// k_dt adds one sum per row, so its four warps cost nothing in throughput, and
+// they shorten the slices along a shoreline, whose general evaluations are its
+// time on meshes of ordinary size: wet/dry basin of 20k / 50k / 102k / 200k / 1M
+// nodes 65 / 76 / 93 / 134 / 499 us, one warp 103 / 115 / 130 / 187 / 499; dam
+// break of 102k / 200k / 1M 75 / 114 / 450 against 91 / 136 / 424; SGN of 36k /
+// 102k / 200k 33 / 59 / 93 against 27 / 57 / 89.
+static bool split_dt(int64_t n_rows, int S) { return n_rows <= (S == 5 ? 80 : 1400) * sm_count(); }
+// One slice per block in k_dt and k_low: neighbouring slices are alike, and four
+// expensive ones (a shoreline) in one block wait for one SM.  k_dt 512 -> 499
+// and k_low 1840 -> 1832 us on the basin of 1M nodes, 122 -> 115 and 192 -> 185
+// at 50k, SGN of 20k nodes k_low 82 -> 62.
+constexpr int kRowBlock = 32;
 
 void launch_node_f64(const StageArgs& a, cudaStream_t s) {
   const NodeF64 nd = node_of(a.w);
@@ -1540,8 +1564,8 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
                     a.w.res, a.w.ab, a.dij_in, diag, ne, a.err);
     } else
 #define SWE_LOWF(S, F)                                                                                              \
-    launch_full(k_low_fct<S, F>, nb, bs, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL, a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, \
-                a.w.res, a.w.ab, a.dij_in, diag, ne, a.err)
+    launch_full(k_low_fct<S, F>, nblk(a.G.n_rows, kRowBlock), kRowBlock, 0, s, a.G, a.C, a.St, a.u, nd, a.w.dL,       \
+                a.w.muL, a.w.dLii, a.w.muLii, a.w.uL, a.w.res, a.w.ab, a.dij_in, diag, ne, a.err)
     if (a.S == 5) { if (a.all_fct) SWE_LOWF(5, true); else SWE_LOWF(5, false); }
     else { if (a.all_fct) SWE_LOWF(3, true); else SWE_LOWF(3, false); }
 #undef SWE_LOWF
@@ -1582,12 +1606,12 @@ void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* ke
 }
 
 void launch_dt_f64(const Graph& G, const InstConst* C, InstState* St, const StateF64& u, const WorkF64& node,
-                   double* d_out, double* dii_out, unsigned* err, int block, const StepTurn& turn, cudaStream_t s) {
-  if (split_rows(G.n_rows, u.q3 ? 5 : 3)) {
+                   double* d_out, double* dii_out, unsigned* err, const StepTurn& turn, cudaStream_t s) {
+  if (split_dt(G.n_rows, u.q3 ? 5 : 3)) {
     launch_full(k_dt_split, (unsigned)(G.n_rows / 32), 128, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
     return;
   }
-  launch_full(k_dt_f64, nblk(G.n_rows, block), block, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
+  launch_full(k_dt_f64, nblk(G.n_rows, kRowBlock), kRowBlock, 0, s, G, C, St, u, node_of(node), d_out, dii_out, err, turn);
 }
 
 void launch_step_turn(const StepTurn& t, const InstConst* C, InstState* St, cudaStream_t s) {

@@ -100,9 +100,11 @@ def test_tiles_straddling_instances(monkeypatch, prec):
 @pytest.mark.parametrize("kind", ["basin", "sgn"])
 def test_batch_above_the_size_rules(kind, prec):
     """Meshes above four 256-row blocks per SM take another turn between steps,
-    and their stage 1 forms the wave speeds k_dt keeps on smaller ones: a batch
-    above that size equals its instances, each below it, bit for bit."""
-    c = _case(kind, 300, 290, prec, "fct")
+    and their stage 1 forms the wave speeds k_dt keeps on smaller ones; above
+    1400 rows per SM the FP64 k_dt gives a slice one warp instead of four.  A
+    batch above those sizes equals its instances, each below them, bit for
+    bit."""
+    c = _case(kind, 340, 330, prec, "fct")
     one = Update(c.mesh, c.bath, c.params)
     one.upload(c.u0)
     one.set_time(0.0, 1e30)
@@ -116,7 +118,7 @@ def test_batch_above_the_size_rules(kind, prec):
     u2 = both.download()
     both.close()
     n = u1.shape[1]
-    assert n < 4 * 256 * 152 < 2 * n
+    assert n < 4 * 256 * 152 < 1400 * 152 < 2 * n
     for b in (0, 1):
         np.testing.assert_array_equal(u2[:, b * n:(b + 1) * n], u1)
         assert dt2[b] == dt1[0]
