@@ -391,6 +391,18 @@ __device__ __forceinline__ float one_over_h_f(float h, float htiny) {
   return __fdividef(2.f * h, h * h + m * m);
 }
 
+// phi(x0 hmin) >= 0 for certain, from phi in FP32 (within 2e-6 M): a dam front
+// or a bank, where the depths differ by more than x0
+__device__ __forceinline__ bool rarefactions_f(const LamState& l, const LamState& r, float lv, float rv, float hmin,
+                                               float hmax, float M, const InstConst& c) {
+  const float hx = 3.3431458f * hmin, ox = one_over_h_f(hx, c.htinyf), cx = sqrt_approx(c.gf * hx), hg = 0.5f * c.gf;
+  const float fl = hx > l.f.x ? (hx - l.f.x) * sqrt_approx(hg * (ox + one_over_h_f(l.f.x, c.htinyf)))
+                              : 2.f * (cx - l.f.y);
+  const float fr = hx > r.f.x ? (hx - r.f.x) * sqrt_approx(hg * (ox + one_over_h_f(r.f.x, c.htinyf)))
+                              : 2.f * (cx - r.f.y);
+  return fl + fr + (rv - lv) > 1e-5f * M && hmin > 1e-18f && hmax < 1e18f && bits64(l.h) > 0 && bits64(r.h) > 0;
+}
+
 // compute_lambda_vacc (SOURCES/condlim.f90:879-957) with the same bits and
 // about a third of the FP64 instructions (the bound of k_dt_f64 and
 // k_low_fct).  With c = sqrt(g h):
@@ -402,6 +414,8 @@ __device__ __forceinline__ float one_over_h_f(float h, float htiny) {
 //    1.8884 c_min for hmin >= htiny, at least (x0 - 1) / sqrt(2 x0) c_min =
 //    0.9061 c_min where only x0 hmin >= htiny.  phi's square roots and
 //    division are not formed.
+//    Else FP32 forms phi(x0 hmin) itself (rarefactions_f): dam break of 10k
+//    nodes, first steps, k_dt 32 -> 17 and k_low 46 -> 38 us.
 //  * sqrt((1 + max(x/2, 0)) (1 + max(x, 0))) is 1 exactly where ht <= h.
 //  * only the larger of |lambda_l| and |lambda_r| is formed where FP32 tells
 //    them apart.
@@ -418,7 +432,8 @@ __device__ __forceinline__ bool lambda_row(const LamState& l, const LamState& r,
   const float hmin = fminf(l.f.x, r.f.x), hmax = fmaxf(l.f.x, r.f.x);
   const float kmin = hmin > 1.00001f * c.htinyf ? 1.888f : (3.3431f * hmin > 1.00001f * c.htinyf ? 0.906f : 0.f);
   if (!(3.3431f * hmin > hmax && (lv - rv) + 2e-6f * V <= kmin * fminf(l.f.y, r.f.y) && hmin > 1e-18f &&
-        hmax < 1e18f)) {
+        hmax < 1e18f) &&
+      !rarefactions_f(l, r, lv, rv, hmin, hmax, M, c)) {
     const bool dry_l = (bits64(l.h) << 1) == 0, dry_r = (bits64(r.h) << 1) == 0;
     if ((dry_l || dry_r) && bits64(l.h) >= 0 && bits64(r.h) >= 0 && bits64(c.htiny) > 0 && V < 1e30f) {
       const double qx = dry_l ? r.q1 : l.q1, qy = dry_l ? r.q2 : l.q2, o = dry_l ? r.ovh : l.ovh;

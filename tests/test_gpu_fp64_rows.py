@@ -17,7 +17,8 @@ from swe.update import Update
 
 pytestmark = pytest.mark.gpu
 
-STATES = ["rest", "equal", "near_equal", "ratio", "film", "dry", "compress", "expand", "fast", "mixed", "tiny", "huge"]
+STATES = ["rest", "equal", "near_equal", "ratio", "film", "dry", "compress", "expand", "fast", "mixed", "tiny", "huge",
+          "cliff"]
 
 
 def _state(kind, n, htiny, rng):
@@ -46,6 +47,9 @@ def _state(kind, n, htiny, rng):
         v *= np.where(h < 10 * htiny, 0.01, 1.0)
     elif kind == "tiny":
         h = np.where(rng.random(n) < 0.5, h, 10.0 ** rng.uniform(-300, -20, n))
+    elif kind == "cliff":                        # depth ratios of 10 to 100, phi(x0 hmin) of both signs
+        h = rng.choice([0.02, 0.2, 1.0, 2.0], n) * rng.uniform(0.9, 1.1, n)
+        v *= 5.0
     elif kind == "huge":
         h = h * 1e30
         v *= 1e14
