@@ -1584,8 +1584,8 @@ static int autotune(swe_ctx* c) {
   int rc;
   const char* tenv = getenv("SWE_TILED");   // 0 leaves the tile variants out
   // A mesh with row tiles runs them, without timing: per RK3 step they take
-  // 44 / 46 / 72 / 105 / 1470 us at 2k / 20k / 100k / 200k / 4M nodes, the best
-  // of the global-gather variants 60 / 68 / 87 / 128 / 1780 us.  k_low runs four
+  // 42 / 45 / 70 / 96 / 1389 us at 2k / 20k / 100k / 200k / 4M nodes, the
+  // global-gather variants 64 / 70 / 81 / 123 / 2142 us.  k_low runs four
   // resident blocks per SM (64 registers, a few spilled) where an SM has more
   // than three tiles, else three.
   if (c->tiles_ok && !(tenv && tenv[0] == '0')) {

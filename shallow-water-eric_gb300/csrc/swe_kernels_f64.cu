@@ -679,6 +679,10 @@ __global__ void k_entropy_f64(Graph G, const InstConst* C, const InstState* St,
 //   * the diagonals of d and mu enter nothing ('fct' multiplies them by
 //     u_i rat_ii - u_i rat_ii = 0): only swe_euler, which hands them out, forms
 //     them.
+// Wet/dry basin of 250k nodes, general kernels -> row kernels with lambda_row:
+// k_low 942 -> 436 us (stage 1, d_ij from k_dt) and 576 (stages 2, 3), 836 and
+// 1007 FP64 instructions per 32 rows, the unit 82-83% busy; k_fct 191 -> 37;
+// k_update 258 -> 78 (75% busy).
 // ---------------------------------------------------------------------------
 
 // H / h for H >= 0, h > 0 (rh = 1/h): 1 where they are equal
@@ -1324,7 +1328,9 @@ __device__ __forceinline__ double warp_max(double v) {
 // ---------------------------------------------------------------------------
 // k_dt: compute_dij (update.f90:291-326) diagonal and COMPUTE_DT's
 // max |d_ii|/m_i (main.f90:166-174), per instance.  d_out (nullable)
-// receives every d_ij.
+// receives every d_ij.  The FP64 unit (67% busy at 250k nodes, the slices along
+// the shoreline end last): 554 -> 159 us with lambda_row, 182 FP64 instructions
+// per 32 rows.
 // ---------------------------------------------------------------------------
 __global__ void k_dt_f64(Graph G, const InstConst* C, InstState* St, StateF64 u, NodeF64 nd,
                          double* __restrict__ d_out, double* __restrict__ dii_out, unsigned* __restrict__ err,
@@ -1361,7 +1367,7 @@ __global__ void k_dt_f64(Graph G, const InstConst* C, InstState* St, StateF64 u,
   step_turn(turn, C, St);
 }
 
-// k_dt for small meshes, four warps per 32 rows (see k_low_split)
+// k_dt, four warps per 32 rows (see k_low_split; measured at split_dt)
 __global__ void __launch_bounds__(128) k_dt_split(Graph G, const InstConst* C, InstState* St, StateF64 u, NodeF64 nd,
                                                   double* __restrict__ d_out, double* __restrict__ dii_out,
                                                   unsigned* __restrict__ err, StepTurn turn) {
