@@ -35,7 +35,7 @@ namespace {
 // were most of the set-up time of a small mesh.
 struct DevBuf {
   static constexpr size_t kSlab = 4 << 20;
-  bool in_use = false;   // the context works on its own stream: the memset has to be waited for
+  bool in_use = false;   // the context works on its own stream: what the null stream does here has to be waited for
   std::vector<void*> ptrs;
   char* slab = nullptr;
   size_t left = 0;
@@ -60,6 +60,14 @@ struct DevBuf {
     slab += bytes;
     left -= bytes;
     return reinterpret_cast<T*>(p);
+  }
+  // Host to device on the null stream.  A copy from pageable memory may return
+  // before its data are on the device, and the context's stream is not ordered
+  // after the null stream.
+  cudaError_t upload(void* d, const void* src, size_t bytes) {
+    cudaError_t st = cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice);
+    if (st == cudaSuccess && in_use) st = cudaStreamSynchronize(0);
+    return st;
   }
   void release() { for (void* p : ptrs) cudaFree(p); ptrs.clear(); slab = nullptr; left = 0; }
 };
@@ -355,7 +363,7 @@ static int alloc_state_mix(swe_ctx* c, StateMix& s, cudaError_t& st) {
 template <typename T>
 static T* upload_vec(swe_ctx* c, const std::vector<T>& v, cudaError_t& st) {
   T* d = c->buf.alloc<T>(v.size(), st);
-  if (st == cudaSuccess && !v.empty()) st = cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  if (st == cudaSuccess && !v.empty()) st = c->buf.upload(d, v.data(), v.size() * sizeof(T));
   return d;
 }
 
@@ -1420,10 +1428,8 @@ SWE_API int swe_norms(swe_ctx* c, int inst, int field, const double* f_anal, dou
     gauss_points(m, rj.data(), nullptr);
     c->d_jj_inst[inst] = c->buf.alloc<int>(m.jj.size(), st);
     c->d_rj_inst[inst] = c->buf.alloc<double>(rj.size(), st);
-    if (st == cudaSuccess) st = cudaMemcpy(c->d_jj_inst[inst], m.jj.data(), m.jj.size() * sizeof(int),
-                                           cudaMemcpyHostToDevice);
-    if (st == cudaSuccess) st = cudaMemcpy(c->d_rj_inst[inst], rj.data(), rj.size() * sizeof(double),
-                                           cudaMemcpyHostToDevice);
+    if (st == cudaSuccess) st = c->buf.upload(c->d_jj_inst[inst], m.jj.data(), m.jj.size() * sizeof(int));
+    if (st == cudaSuccess) st = c->buf.upload(c->d_rj_inst[inst], rj.data(), rj.size() * sizeof(double));
   }
   if (f_anal && c->fanal_cap < (size_t)3 * m.me) {
     c->d_fanal = c->buf.alloc<double>((size_t)3 * m.me, st);
@@ -1858,6 +1864,7 @@ SWE_API int swe_gauges_set(swe_ctx* c, int n, const int* inst, const double* rr,
   if (st == cudaSuccess) st = cudaMalloc(&c->d_gauge_rec, sizeof(double) * 3 * n * (size_t)swe_ctx::kGaugeRing);
   if (st == cudaSuccess) st = cudaMalloc(&c->d_gauge_count, sizeof(unsigned long long));
   if (st == cudaSuccess) st = cudaMemset(c->d_gauge_count, 0, sizeof(unsigned long long));
+  if (st == cudaSuccess) st = cudaStreamSynchronize(0);   // the steps run on the context's stream
   if (st != cudaSuccess) { free_gauges(c); return cuda_check(c, st, "gauges"); }
   c->n_gauges = n;
   return SWE_OK;
