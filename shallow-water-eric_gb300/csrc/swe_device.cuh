@@ -333,6 +333,19 @@ __device__ __forceinline__ double pos_part(double x) { return bits64(x) > 0 ? x 
 // MAX, MIN of non-negative values
 __device__ __forceinline__ double max_nn(double a, double b) { return bits64(a) > bits64(b) ? a : b; }
 __device__ __forceinline__ double min_nn(double a, double b) { return bits64(a) < bits64(b) ? a : b; }
+// Entropy residuals, not negative or NaN (0/0 at rest with max_water_h = 0).  A
+// NaN is kept with its sign bit set: above every residual as an unsigned
+// integer and below as a signed one, so that MAX(res_i, res_j) and MIN(d, res_ij)
+// in the general kernels' comparisons (a > b ? a : b, a < b ? a : b) pass on a
+// NaN of the neighbour at no instruction per entry.  own_res: the row's own, whose
+// NaN the comparison drops.
+__device__ __forceinline__ double keep_res(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) > 0x7ff00000u ? __longlong_as_double(0xfff8000000000000ll) : x;
+}
+__device__ __forceinline__ double own_res(double res) { return bits64(res) < 0 ? 0.0 : res; }
+__device__ __forceinline__ double max_res(double own, double res) {
+  return (unsigned long long)bits64(own) > (unsigned long long)bits64(res) ? own : res;
+}
 // h <= t for t >= 0 and any h
 __device__ __forceinline__ bool le_nn(double h, double t) { return bits64(h) <= bits64(t); }
 // integers in the order of the doubles

@@ -720,7 +720,7 @@ __device__ __forceinline__ void fct_row_f64(const Graph& G, const InstConst* C, 
   const bool wet_i = !le_nn(ui[0], htiny);
   const bool fct = FCT || (!HIGH && c.visc == VISC_FCT);                    // keep the row differences
   const bool full = fct || (!HIGH && c.visc == VISC_ENTROPY);     // the right-hand side of smb_2 too, for the residual
-  const double resi = HIGH ? res[r] : 0.0;
+  const double resi = HIGH ? own_res(res[r]) : 0.0;
   // the diagonal's terms: -c_ii.F_i and the topography residue
   double Dq[S], Dfix, tdx, tdy;
   {
@@ -734,6 +734,10 @@ __device__ __forceinline__ void fct_row_f64(const Graph& G, const InstConst* C, 
     }
     Dfix = cxd * w1i;
     if (S == 3) Dfix = Dfix + cyd * w2i;
+    if (HIGH && bits64(res[r]) < 0) {            // a NaN residual: d_ii, which multiplies a zero, is one too
+#pragma unroll
+      for (int q = 1; q < S; q++) Dq[q] = res[r];
+    }
   }
   double fix = 0.0, rk[S], rk2[S];
 #pragma unroll
@@ -773,7 +777,7 @@ __device__ __forceinline__ void fct_row_f64(const Graph& G, const InstConst* C, 
     sr = sr + cye * nd.w2[j];
     if (S == 3) srf = sr;
     if (HIGH) {                                  // d^H = MIN(d, res_ij), mu^H = MIN(mu, res_ij) (update.f90:232-239)
-      const double rij = max_nn(resi, res[j]);
+      const double rij = max_res(resi, res[j]);
       d = min_nn(dL[e], rij);
       mu = min_nn(muL[e], rij);
     } else {
@@ -944,7 +948,7 @@ __device__ __forceinline__ void fct_row_f64(const Graph& G, const InstConst* C, 
   rsd = rsd - m * rm[1] * v1i;
   rsd = rsd - m * rm[2] * v2i;
   const double rescale = __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor);   // the product is exact
-  res[r] = fabs(rsd) / rescale;
+  res[r] = keep_res(fabs(rsd) / rescale);
 }
 
 template <int S, bool FCT>
@@ -1218,7 +1222,7 @@ k_low_split(Graph G, const InstConst* C, const InstState* St, StateF64 u, NodeF6
   rsd = rsd - m * tail[0][lane] * Ep0;
   rsd = rsd - m * tail[2][lane] * v1i;
   rsd = rsd - m * tail[4][lane] * v2i;
-  res[r] = fabs(rsd) / __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor);
+  res[r] = keep_res(fabs(rsd) / __fma_rn(fabs(emax - emin), 0.5, c.rescale_floor));
 }
 
 // 'entropy_visc' (update.f90:225-262): the smb_2_roundoff rows again, with
@@ -1245,16 +1249,16 @@ __global__ void k_fct_fct(Graph G, const InstConst* C, const InstState* St,
   if (St[b].done) return;
   if (C[b].visc != VISC_FCT) return;
   const int64_t base = entry_base(G, r);
-  const double resi = res[r];
+  const double resi = own_res(res[r]);
   double P = -1.e-15;
 #pragma unroll 2
   for (int k = 0; k < L; k++) {
     const int64_t e = base + 32 * k;
-    const double rij = max_nn(resi, res[G.col[e]]);
+    const double rij = max_res(resi, res[G.col[e]]);
     const double d0 = dL[e], m0 = muL[e];
     const double f = (min_nn(d0, rij) - d0) * ab[e] + (min_nn(m0, rij) - m0) * ab[n_entries + e];
     fct[e] = f;
-    if (bits64(f) < 0) P = P + f;                 // -0 adds nothing
+    if (__double2hiint(f) <= (int)0xfff00000) P = P + f;   // f < 0 and not NaN; -0 adds nothing
   }
   const double h = hL[r];
   if (__double2hiint(h) < 0 && h < 0.0) atomicOr(err, ERRB_NEG_H);
@@ -1290,7 +1294,7 @@ __global__ void k_update_fct(Graph G, const InstConst* C, const InstState* St,
   if (c.visc == VISC_ENTROPY) return;          // k_entropy_rows writes these rows
   const int64_t base = entry_base(G, r);
   const bool fct_mode = c.visc == VISC_FCT;
-  const double resi = fct_mode ? res[r] : 0.0, Ri = fct_mode ? rminus[r] : 0.0;
+  const double resi = fct_mode ? own_res(res[r]) : 0.0, Ri = fct_mode ? rminus[r] : 0.0;
   double xx[S];
 #pragma unroll
   for (int q = 0; q < S; q++) xx[q] = 0.0;
@@ -1299,7 +1303,7 @@ __global__ void k_update_fct(Graph G, const InstConst* C, const InstState* St,
     const int j = G.col[e];
     const double l = (bits64(fct[e]) << 1) == 0 || bits64(fct[e]) > 0 ? rminus[j] : Ri;   // f >= 0
     if (lij_out) lij_out[e] = l;
-    const double rij = max_nn(resi, res[j]);
+    const double rij = max_res(resi, res[j]);
     const double d0 = dL[e], m0 = muL[e];
     const double dd = (min_nn(d0, rij) - d0) * l;
     const double dm = (min_nn(m0, rij) - m0) * l;
