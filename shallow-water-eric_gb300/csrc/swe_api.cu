@@ -918,14 +918,20 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
 }
 
 static int capture_steps(swe_ctx* c, int steps, cudaGraphExec_t* exec) {
-  cudaGraph_t g;
+  cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < steps; k++) enqueue_step(c, k > 0 && !c->n_gauges, k == steps - 1);
-  CK(cudaStreamEndCapture(c->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  CK(e);
-  return SWE_OK;
+  // a refused launch must not leave a sequence without it
+  cudaError_t e = cudaGetLastError();
+  const cudaError_t ended = cudaStreamEndCapture(c->stream, &g);
+  if (e == cudaSuccess) e = ended;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+  if (ended == cudaSuccess) cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    *exec = nullptr;
+    cudaGetLastError();
+  }
+  return cuda_check(c, e, "capture of the steps");
 }
 
 static int build_graph(swe_ctx* c, int steps) {
@@ -1992,8 +1998,10 @@ SWE_API int swe_profile_kernels(swe_ctx* c, int nsteps, double* ms_out) {
   for (int k = 0; k < 10; k++) CK(cudaEventCreate(&kev.ev[k]));
   double acc[SWE_NKERNELS] = {0, 0, 0, 0, 0};
   for (int n = 0; n < nsteps; n++) enqueue_step(c, false, true, &kev, acc);
+  const cudaError_t launched = cudaGetLastError();
   CK(cudaStreamSynchronize(c->stream));
   for (int k = 0; k < 10; k++) cudaEventDestroy(kev.ev[k]);
+  CK(launched);
   ms_out[0] = acc[0] / nsteps;
   for (int k = 1; k < SWE_NKERNELS; k++) ms_out[k] = acc[k] / (3.0 * nsteps);
   return read_errors(c);

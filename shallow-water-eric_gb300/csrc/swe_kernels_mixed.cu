@@ -1523,7 +1523,9 @@ template <typename... KArgs, typename... Args>
 static void launch_tile(void (*kern)(KArgs...), const TileCtl& tc, int64_t n_rows, int kind, bool d, bool lamin,
                         cudaStream_t s, Args... args) {
   const size_t sm = tile_smem_bytes(tc, kind, d, lamin);
-  if (sm > 48 * 1024)    // above the default limit; the attribute only ever grows a kernel's allowance
+  // above the default limit of 48 KB, which counts a kernel's static arrays too (k_dt_tile: under 128 bytes); the
+  // attribute only ever grows a kernel's allowance
+  if (sm + 128 > 48 * 1024)
     cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
   launch_k(kern, (unsigned)((n_rows + tc.tile_rows - 1) / tc.tile_rows), tc.tile_rows, sm, s, args..., tc);
 }
