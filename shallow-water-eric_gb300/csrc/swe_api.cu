@@ -164,6 +164,7 @@ struct swe_ctx {
   int* d_ref_pos = nullptr;              // per entry / per row: CSR position in its instance or -1 (on first use)
   int* d_ref_pos_diag = nullptr;
   double* d_csr = nullptr;               // one instance's entries in CSR order
+  double* d_dij = nullptr;               // swe_compute_dij: d_ij per entry, d_ii per row (on first use)
   // mixed path
   StateMix mA{}, mB{}, mC{};
   WorkMix wm{};
@@ -1217,18 +1218,23 @@ __global__ void k_entries_to_csr(const T* __restrict__ ent, const U* __restrict_
   }
 }
 
+// CSR entries of the largest instance
+static size_t csr_size(const swe_ctx* c) {
+  size_t most = 0;
+  for (const HostMesh& m : c->meshes) most = std::max(most, m.ja.size());
+  return most;
+}
+
 template <typename T, typename U = T>
 static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, const U* d_diag_rows = nullptr,
                           int comp = 0) {
   const Layout& L = c->L;
   if (!c->d_csr) {                                   // on first use
-    size_t most = 0;
-    for (const HostMesh& m : c->meshes) most = std::max(most, m.ja.size());
     cudaError_t st = cudaSuccess;
     c->d_ref_pos = upload_vec(c, L.ref_pos, st);
     c->d_ref_pos_diag = upload_vec(c, L.ref_pos_diag, st);
     // FP64: the row differences are free between calls
-    double* csr = c->w.ab ? c->w.ab : c->buf.alloc<double>(most, st);
+    double* csr = c->w.ab ? c->w.ab : c->buf.alloc<double>(csr_size(c), st);
     if (st != cudaSuccess) return cuda_check(c, st, "device allocation");
     c->d_csr = csr;
   }
@@ -1253,23 +1259,42 @@ static int rows_to_nodes(swe_ctx* c, int inst, const T* d_arr, double* out) {
   return SWE_OK;
 }
 
+// Where swe_compute_dij leaves d_ij and d_ii: not in dL and dLii, which
+// swe_euler_intermediates hands out.  Behind the CSR order in the row
+// differences, which are free between calls, else an array of its own.
+static int dij_buffers(swe_ctx* c, double** ent, double** diag) {
+  const size_t ne = c->L.n_entries, n = c->L.n_rows, csr = csr_size(c);
+  if (c->w.ab && csr + ne + n <= 2 * (size_t)c->S * ne) {
+    *ent = c->w.ab + csr;
+  } else {
+    cudaError_t st = cudaSuccess;
+    if (!c->d_dij) c->d_dij = c->buf.alloc<double>(ne + n, st);
+    if (st != cudaSuccess) return cuda_check(c, st, "device allocation");
+    *ent = c->d_dij;
+  }
+  *diag = *ent + ne;
+  return SWE_OK;
+}
+
 SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij, double* dt_out) {
   if (!c || inst < 0 || inst >= c->n_inst || !un) return fail(c, SWE_ERR_ARG, "bad arguments");
   if (c->precision != SWE_PREC_FP64) return fail(c, SWE_ERR_ARG, "swe_compute_dij is an FP64 operator");
   int rc = to_device(c, un, false, c->node_off[inst], c->node_off[inst + 1]);
   if (!rc) rc = call_begin(c, inst, c->params[inst].dt > 0 ? c->params[inst].dt : 1.0);
+  double *d = nullptr, *dii = nullptr;
+  if (!rc) rc = dij_buffers(c, &d, &dii);
   if (!rc) {
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, nullptr, c->d_err, c->block};
     a.w.alpha = nullptr;                             // the last euler call's alpha stays readable
     launch_node_f64(a, c->stream);
-    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, c->w.dL, c->w.dLii, c->d_err, StepTurn{}, c->stream);
+    launch_dt_f64(c->G, c->d_C, c->d_St_call, c->A, c->w, d, dii, c->d_err, StepTurn{}, c->stream);
     rc = cuda_check(c, cudaGetLastError(), "compute_dij");
   }
   if (!rc && dij) prefault(dij, c->meshes[inst].ja.size() * sizeof(double));
   if (!rc) rc = call_end(c, inst);                   // nothing is written to the caller's arrays on an error
   if (rc) { drain(c); return rc; }
   if (dij) {
-    if ((rc = entries_to_csr(c, inst, c->w.dL, dij, c->w.dLii))) { drain(c); return rc; }
+    if ((rc = entries_to_csr(c, inst, d, dij, dii))) { drain(c); return rc; }
     CK(cudaStreamSynchronize(c->stream));
   }
   if (dt_out) {                                      // COMPUTE_DT: CFL / max |d_ii| / m_i, the maximum from k_dt

@@ -65,3 +65,22 @@ def test_first_norms_and_gauges(n, prec):
         tri = case.mesh["jj"][:, 0] - 1
         assert abs(h[0, 0] - upd.download()[0, tri].mean()) <= 1e-12 * max(1.0, abs(h[0, 0]))
         upd.close()
+
+
+@pytest.mark.parametrize("visc", ["galerkin", "viscous", "entropy_visc", "fct"])
+@pytest.mark.parametrize("n", [9, 65])
+def test_dij_leaves_the_intermediates_alone(n, visc):
+    """euler's intermediates are those of the last euler call also after
+    compute_dij on another state."""
+    case, upd = _context(n, 0, 0)
+    upd.set_params(replace(case.params, dt=1e-4, viscosity_type=C.VISC[visc]))
+    upd.euler(case.u0)
+    a = upd.euler_intermediates()
+    other = case.u0.copy(order="F")
+    other[0] += 0.3
+    first = upd.compute_dij(other)[0]
+    b = upd.euler_intermediates()
+    for k in a:
+        np.testing.assert_array_equal(b[k], a[k], err_msg=k)
+    np.testing.assert_array_equal(upd.compute_dij(other)[0], first)
+    upd.close()
