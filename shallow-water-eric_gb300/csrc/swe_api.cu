@@ -153,6 +153,7 @@ struct swe_ctx {
   // FP64 path
   StateF64 A{}, B{}, Cs{};
   WorkF64 w{};
+  bool rows_refused = false;             // no memory for the row kernels' arrays (rows_setup)
   double* d_lij = nullptr;
   // per-call operators (swe_euler, swe_compute_dij): their own instance state,
   // so that the time loop's is neither saved nor restored
@@ -391,6 +392,35 @@ __global__ void k_edge_normals(const double* __restrict__ cx, const double* __re
   }
 }
 
+// The arrays that only the FP64 row kernels use, once every instance runs a
+// mode of theirs: 373 bytes per node beside 830 (5 components: 590 beside 957),
+// so a mesh that fills the memory without them keeps the general kernels (the
+// same bits).  Half as much again stays free for what is allocated on first use
+// (CSR positions and element lists 110 bytes per node, frames, analytic boundary
+// data).
+static void rows_setup(swe_ctx* c) {
+  WorkF64& w = c->w;
+  if (c->precision != SWE_PREC_FP64 || w.ab || c->rows_refused || !all_fct_rows(c)) return;
+  const size_t n = c->L.n_rows, ab = (size_t)2 * c->S * c->L.n_entries, flux = (size_t)2 * c->S * n;
+  const size_t need = sizeof(double) * (ab + flux + 3 * n);
+  size_t avail = 0, total = 0;
+  cudaError_t st = cudaMemGetInfo(&avail, &total);
+  if (st == cudaSuccess && need + need / 2 <= avail) {
+    w.w2 = c->buf.alloc<double>(n, st);
+    w.eta = c->buf.alloc<double>(n, st);
+    w.rh = c->buf.alloc<double>(n, st);
+    w.flux = c->buf.alloc<double>(flux, st);
+    w.ab = c->buf.alloc<double>(ab, st);
+  }
+  if (!w.ab) {
+    w.flux = nullptr;
+    c->rows_refused = true;
+    cudaGetLastError();
+  }
+}
+// the FP64 stage runs the row kernels
+static bool fct_rows(const swe_ctx* c) { return c->w.ab && all_fct_rows(c); }
+
 static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& baths) {
   c->L = build_layout(c->meshes, baths);
   const Layout& L = c->L;
@@ -493,11 +523,8 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     w.ovh = c->buf.alloc<double>(n, st); w.v1 = c->buf.alloc<double>(n, st); w.v2 = c->buf.alloc<double>(n, st);
     w.ent = c->buf.alloc<double>(n, st); w.alpha = c->buf.alloc<double>(n, st);
     w.sqgh = c->buf.alloc<double>(n, st);
-    w.w2 = c->buf.alloc<double>(n, st); w.eta = c->buf.alloc<double>(n, st); w.rh = c->buf.alloc<double>(n, st);
-    w.flux = c->buf.alloc<double>((size_t)2 * c->S * n, st);
     w.nf = c->buf.alloc<float4>(n, st);
     if (c->S == 5) w.pt = c->buf.alloc<double>(n, st);
-    w.ab = c->buf.alloc<double>((size_t)2 * c->S * ne, st);
     w.n_entries = (int64_t)ne;
     w.dL = c->buf.alloc<double>(ne, st); w.muL = c->buf.alloc<double>(ne, st); w.fct = c->buf.alloc<double>(ne, st);
     w.dLii = c->buf.alloc<double>(n, st); w.muLii = c->buf.alloc<double>(n, st);
@@ -556,6 +583,7 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
     if (!c->tiles_ok || !large_mesh(c)) w.dlam = c->buf.alloc<float>(ne, st);
   }
   if (st != cudaSuccess) return fail(c, SWE_ERR_CUDA, std::string("device allocation: ") + cudaGetErrorString(st));
+  rows_setup(c);
   return SWE_OK;
 }
 
@@ -892,7 +920,7 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
       StageArgs a{c->G, c->d_C, c->d_St, c->A, c->A, c->B, c->w, stage, nullptr, c->d_err, c->block};
       a.entropy = has_entropy(c);
       a.any_fct = has_fct(c);
-      a.fused = all_fct_rows(c);
+      a.fused = fct_rows(c);
       a.all_fct = all_fct(c);
       a.S = c->S;
       if (stage == 1) { a.dij_in = c->w.fct; a.skip_node = 1; }
@@ -1312,11 +1340,12 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
   int rc = to_device(c, un, false, c->node_off[inst], c->node_off[inst + 1]);
   if (!rc) rc = call_begin(c, inst, c->params[inst].dt);
   if (rc) { drain(c); return rc; }
+  rows_setup(c);
   if (c->precision == SWE_PREC_FP64) {
     StageArgs a{c->G, c->d_C, c->d_St_call, c->A, c->A, c->B, c->w, 0, c->d_lij, c->d_err, c->block};
     a.entropy = has_entropy(c);
     a.any_fct = has_fct(c);
-    a.fused = all_fct_rows(c);
+    a.fused = fct_rows(c);
     a.all_fct = all_fct(c);
     a.S = c->S;
     launch_stage_f64(a, c->stream);
@@ -1940,6 +1969,7 @@ static int enqueue_rk3_steps(swe_ctx* c, int nsteps) {
     if (env && env[0] == '0') c->tuned = true;
     else if ((rc = autotune(c))) return rc;
   }
+  rows_setup(c);
   launch_reset_counters(c->d_St, c->n_inst, c->stream);
   const int chunk = nsteps >= 8 ? 8 : 1;
   long long launches = 0;
@@ -2022,6 +2052,7 @@ SWE_API int swe_profile_kernels(swe_ctx* c, int nsteps, double* ms_out) {
   KernelEvents kev;
   for (int k = 0; k < 10; k++) CK(cudaEventCreate(&kev.ev[k]));
   double acc[SWE_NKERNELS] = {0, 0, 0, 0, 0};
+  rows_setup(c);
   for (int n = 0; n < nsteps; n++) enqueue_step(c, false, true, &kev, acc);
   const cudaError_t launched = cudaGetLastError();
   CK(cudaStreamSynchronize(c->stream));

@@ -31,7 +31,7 @@ struct WorkF64 {
   double *ovh, *v1, *v2, *ent, *alpha;   // per row
   double* sqgh;                          // per row: sqrt(g |h|)
   double* w2;                            // per row: qy one_over_h (v2 is 0 for type 13)
-  double *eta, *rh;                      // per row: h + z, 1/h
+  double *eta, *rh;                      // per row: h + z, 1/h (w2, eta, rh, flux, ab: null until the row kernels run)
   double* flux;                          // per row: v1 u_q, v2 u_q (component q at 2 q n_rows, (2 q + 1) n_rows)
   double* pt;                            // per row: the SGN pressure pTilde (type 13)
   float4* nf;                            // per row, FP32: h, sqrt(g |h|), q one_over_h

@@ -26,7 +26,7 @@ struct NodeF64 {        // per-row arrays of the FP64 path
   double* alpha;        // or null: no alpha_i (swe_compute_dij)
   double* sqgh;         // sqrt(g |h|), the sql / sqr of compute_lambda_vacc
   double* w2;           // qy one_over_h (v2 unless type 13)
-  double* eta;          // h + z
+  double* eta;          // h + z (w2, eta, rh and flux: null without the row kernels)
   double* rh;           // 1/h
   double* flux;         // v1 u_q and v2 u_q: (2 q + a) n_rows + r
   double* pt;           // SGN pressure (type 13)
@@ -60,8 +60,9 @@ __device__ __forceinline__ void sgn_node_f64(const InstConst& c, double m, doubl
 // smoothness indicator alpha_i of alpha_limit (update.f90:758-781), and every
 // other quantity of one node that the entry loops would otherwise form once
 // per entry: the flux products v u_q, h + z, 1/h, the SGN pressure and the
-// FP32 shadow of lambda_row.
+// FP32 shadow of lambda_row.  ROWS: with what only the row kernels read.
 // ---------------------------------------------------------------------------
+template <bool ROWS>
 __global__ void k_node_f64(Graph G, const InstConst* C, const InstState* St,
                            StateF64 u, NodeF64 nd) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -81,22 +82,28 @@ __global__ void k_node_f64(Graph G, const InstConst* C, const InstState* St,
   nd.ovh[r] = o;
   nd.v1[r] = v1;
   nd.v2[r] = v2;
-  nd.w2[r] = w2;
+  if (ROWS) nd.w2[r] = w2;
   nd.sqgh[r] = sq;
-  nd.eta[r] = h + G.bath[r];
-  nd.rh[r] = 1.0 / h;
+  if (ROWS) {
+    nd.eta[r] = h + G.bath[r];
+    nd.rh[r] = 1.0 / h;
+  }
   nd.nf[r] = make_float4((float)h, (float)sq, (float)v1, (float)w2);
-  const double f10 = v1 * h, f11 = v1 * qx, f22 = v2 * qy;
-  nd.flux[r] = f10;
-  nd.flux[2 * n + r] = f11;
-  nd.flux[4 * n + r] = v1 * qy;
+  const double f11 = v1 * qx, f22 = v2 * qy;
+  if (ROWS) {
+    nd.flux[r] = v1 * h;
+    nd.flux[2 * n + r] = f11;
+    nd.flux[4 * n + r] = v1 * qy;
+  }
   if (c.type_test == 13) {           // v2 = 0
     const double heta = u.q3[r];
-    nd.flux[6 * n + r] = v1 * heta;
-    nd.flux[8 * n + r] = v1 * u.q4[r];
+    if (ROWS) {
+      nd.flux[6 * n + r] = v1 * heta;
+      nd.flux[8 * n + r] = v1 * u.q4[r];
+    }
     double s;
     sgn_node_f64(c, G.lumped[r], h, heta, &nd.pt[r], &s);
-  } else {
+  } else if (ROWS) {
     nd.flux[n + r] = v2 * h;
     nd.flux[3 * n + r] = v2 * qx;
     nd.flux[5 * n + r] = f22;
@@ -1551,14 +1558,16 @@ constexpr int kRowBlock = 32;
 
 void launch_node_f64(const StageArgs& a, cudaStream_t s) {
   const NodeF64 nd = node_of(a.w);
-  launch_full(k_node_f64, nblk(a.G.n_rows, a.block), a.block, 0, s, a.G, a.C, a.St, a.u, nd);
+  const unsigned nb = nblk(a.G.n_rows, a.block);
+  if (nd.flux) launch_full(k_node_f64<true>, nb, a.block, 0, s, a.G, a.C, a.St, a.u, nd);
+  else launch_full(k_node_f64<false>, nb, a.block, 0, s, a.G, a.C, a.St, a.u, nd);
 }
 
 void launch_stage_f64(const StageArgs& a, cudaStream_t s, const KernelEvents* kev) {
   const int bs = a.block;
   const NodeF64 nd = node_of(a.w);
   EV_BEGIN(1);
-  if (!a.skip_node) launch_full(k_node_f64, nblk(a.G.n_rows, bs), bs, 0, s, a.G, a.C, a.St, a.u, nd);
+  if (!a.skip_node) launch_node_f64(a, s);
   EV_END(1); EV_BEGIN(2);
   const unsigned nb = nblk(a.G.n_rows, bs);
   if (a.fused) {
