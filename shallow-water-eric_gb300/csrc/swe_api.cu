@@ -319,6 +319,24 @@ static bool all_fct_limited(const swe_ctx* c) {
 // more than four 256-row blocks per SM
 static bool large_mesh(const swe_ctx* c) { return c->G.n_rows > 4 * 256 * (int64_t)c->sms; }
 
+// Tiles whose halos are so large that the global gathers are the faster ones.
+// Halo rows per row (mean over the tiles) of meshes numbered ever more loosely,
+// us per RK3 step of the tiles against the global gathers:
+//   23k nodes   2.9 65 / 82, 4.3 74 / 85: one tile per SM, always
+//   102k nodes  2.9 90 / 103, 3.6 100 / 107, 3.7 112 / 102, 4.4 119 / 102; split 3.6 112 / 121, 3.7 125 / 124
+//   1M nodes    2.0 557 / 620, 2.9 624 / 654, 3.0 644 / 647, 3.6 749 / 681, 4.4 855 / 714; split 2.9 733 / 719,
+//               3.0 754 / 711, 3.6 875 / 742
+// (5 components 1M nodes 2.9 732 / 733, 3.6 831 / 799).  A single such tile costs all blocks the
+// shared memory of its halo: 1M nodes with 0.4 halo rows per row and one tile of
+// 3.8 577 / 600, of 4.7 689 / 602.
+static bool tiles_pay(const swe_ctx* c, const RowTiles& F) {
+  const int64_t n_tiles = (int64_t)F.halo_ptr.size() - 1;
+  const double mean = (double)F.halo_ptr.back() / (double)(n_tiles * F.tile);
+  if (c->G.n_rows <= 256 * (int64_t)c->sms) return true;
+  if (!large_mesh(c)) return mean <= 3.65;
+  return mean <= 2.9 && F.halo_cap <= 4 * F.tile;
+}
+
 // The mixed stage's mode flags (see StageArgsMix)
 static void set_modes(const swe_ctx* c, StageArgsMix& a) {
   a.fct = all_fct_limited(c);
@@ -559,7 +577,7 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
       probe.ent_cap = F.ent_cap;
       c->tiles_named = 32 * (F.tile + F.halo_cap) + F.tile / 4 + F.tile <= 48 * 1024;
     }
-    if (c->tiles_named && tile_smem_max(probe, is_split(c)) <= (size_t)kTileSmemMax) {
+    if (c->tiles_named && tile_smem_max(probe, is_split(c)) <= (size_t)kTileSmemMax && tiles_pay(c, F)) {
       c->tiles = probe;
       c->tiles.loc = upload_vec(c, F.loc, st);
       std::vector<int4> head(F.halo_ptr.size() - 1);

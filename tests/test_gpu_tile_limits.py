@@ -7,7 +7,8 @@ more."""
 import numpy as np
 import pytest
 
-from swe import cases as C
+from swe import cases as C, mesh as M
+from swe.update import Update
 from test_gpu_tiles import _fan, _same
 
 pytestmark = pytest.mark.gpu
@@ -24,3 +25,34 @@ def test_tile_just_below_48_kb(monkeypatch, k, total, prec):
         items.append(C.Case("fan", _fan(f), C.Params(max_water_h=1.0, precision=prec), rng.uniform(0.0, 0.3, n),
                             np.asfortranarray(u), 1e30))
     _same(monkeypatch, items, np.hstack([c.u0 for c in items]))
+
+
+def _scattered(nx, ny, lines):
+    """A lattice numbered line by line, each node moved by up to `lines` lines, and one node so far away that the
+    others share a cell of the Z-order's grid, which then keeps their numbering."""
+    rng = np.random.default_rng(0)
+    mesh = M.jittered_mesh(nx, ny, 0.0, 1.0, 0.0, ny / nx, jitter=0.2, seed=2)
+    i = np.arange(nx * ny)
+    at = np.argsort(np.round(mesh["rr"][1] * (nx - 1)) + rng.uniform(0.0, lines, nx * ny), kind="stable")
+    new = np.empty_like(i)
+    new[at] = i
+    rr = mesh["rr"][:, at].copy()
+    rr[:, rr.sum(axis=0).argmax()] += 1e6
+    return dict(jj=np.asfortranarray(new[mesh["jj"] - 1] + 1, np.int32), rr=np.asfortranarray(rr))
+
+
+@pytest.mark.parametrize("nx,ny,lines,tiled", [(330, 70, 4.0, True), (330, 310, 3.0, True), (330, 310, 6.0, False),
+                                               (330, 560, 1e-3, True), (330, 560, 4.0, False)])
+def test_tiles_only_where_they_are_faster(nx, ny, lines, tiled):
+    """Halos of 0.4 rows per row are the rule; meshes whose numbering is loose have up to 4.5.  Small meshes take the
+    tiles all the same, larger ones the global gathers above 3.65, large ones above 2.9 (sizes for 152 SMs)."""
+    mesh = _scattered(nx, ny, lines)
+    n = mesh["rr"].shape[1]
+    rng = np.random.default_rng(1)
+    u = np.asfortranarray(np.vstack([rng.uniform(0.5, 1.0, n), rng.normal(0, 0.1, (2, n))]))
+    upd = Update(mesh, np.zeros(n), C.Params(max_water_h=1.0, precision=1))
+    upd.upload(u)
+    upd.set_time(0.0, 1e30)
+    upd.rk3_steps(1)
+    assert ("/tiled" in upd.tuning) == tiled, upd.tuning
+    upd.close()
