@@ -726,10 +726,12 @@ static int to_device(swe_ctx* c, const double* un, bool device_src, int64_t node
   return SWE_OK;
 }
 
-// Maps the pages of a caller's pageable array that the kernel has not mapped
-// yet (a fresh numpy array's), while the GPU works: a copy into unmapped pages
-// waits for every one of them (24 MB: about 1 ms).  A page's first byte is
-// written back unchanged; mapped pages and page-locked memory are left alone.
+// Maps the pages of a caller's pageable array that are not mapped yet (a fresh
+// numpy array's), while the GPU works: a copy into unmapped pages faults on every
+// one of them.  24 MB take 0.72 ms to map and 0.16 to copy, 0.99 ms unmapped
+// (touching each page from here takes 7.5: a read maps the zero page, the write
+// then copies it).  The bytes stay as they are.  Three pages tell a fresh array
+// from one in use, whose call costs 15 us; page-locked memory is left alone.
 static void prefault(void* p, size_t bytes) {
   if (!p || bytes < (64 << 10)) return;
   cudaPointerAttributes at{};
@@ -738,16 +740,17 @@ static void prefault(void* p, size_t bytes) {
     return;
   }
   if (at.type != cudaMemoryTypeUnregistered) return;
-  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  char* b = reinterpret_cast<char*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)(page - 1));
-  char* e = static_cast<char*>(p) + bytes;
-  std::vector<unsigned char> in((size_t)(e - b + page - 1) / page);
-  if (mincore(b, e - b, in.data()) != 0) return;
-  for (size_t k = 0; k < in.size(); k++)
-    if (!(in[k] & 1)) {
-      volatile char* q = k ? b + k * page : static_cast<char*>(p);
-      *q = *q;
-    }
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), mask = ~(page - 1);
+  const uintptr_t b = reinterpret_cast<uintptr_t>(p), e = b + bytes;
+  for (const uintptr_t q : {e - 1, b + bytes / 2, b}) {
+    unsigned char in = 0;
+    if (mincore(reinterpret_cast<void*>(q & mask), 1, &in) != 0) return;
+    if (in & 1) continue;
+#ifdef MADV_POPULATE_WRITE
+    madvise(reinterpret_cast<void*>(b & mask), e - (b & mask), MADV_POPULATE_WRITE);   // Linux 5.14; else not done
+#endif
+    return;
+  }
 }
 
 static int from_device_state(swe_ctx* c, double* un, bool device_dst, int64_t node_begin, int64_t node_end,
@@ -1290,6 +1293,7 @@ static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, con
   k_entries_to_csr<T, U><<<(unsigned)nb, 256, 0, c->stream>>>(d_arr, d_diag_rows, c->d_ref_pos, c->d_ref_pos_diag, e0, e1,
                                                               r0, r1, comp, c->d_csr);
   CK(cudaGetLastError());
+  prefault(out, c->meshes[inst].ja.size() * sizeof(double));
   CK(cudaMemcpyAsync(out, c->d_csr, c->meshes[inst].ja.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   return SWE_OK;
 }
@@ -1393,6 +1397,7 @@ SWE_API int swe_euler_intermediates(swe_ctx* c, int inst, double* dij_low, doubl
   if (!c || inst < 0 || inst >= c->n_inst) return fail(c, SWE_ERR_ARG, "bad instance");
   if (!c->euler_done || c->euler_inst != inst) return fail(c, SWE_ERR_ARG, "call swe_euler on this instance first");
   int rc;
+  if (u_low) prefault(u_low, sizeof(double) * c->S * (size_t)c->meshes[inst].np);
   if (c->precision == SWE_PREC_FP64) {
     if (dij_low && (rc = entries_to_csr(c, inst, c->w.dL, dij_low, c->w.dLii))) return rc;
     if (muij_low && (rc = entries_to_csr(c, inst, c->w.muL, muij_low, c->w.muLii))) return rc;

@@ -2,6 +2,7 @@
 8-byte offset, already written, page-locked), and the page-locked slots that
 contexts read their status back through."""
 import mmap
+import time
 
 import numpy as np
 import pytest
@@ -24,7 +25,7 @@ def test_fresh_and_written_targets_get_the_same(prec, shift):
     ref = upd.download().ravel(order="F")
     n = ref.size
     total = n + shift + 1024
-    fresh = np.frombuffer(mmap.mmap(-1, 8 * total), np.float64)
+    fresh = np.frombuffer(mmap.mmap(-1, 8 * total, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.float64)
     written = np.full(total, -3.0)
     pinned = torch.full((total,), -3.0, dtype=torch.float64).pin_memory().numpy()
     for buf, about in ((fresh, 0.0), (written, -3.0), (pinned, -3.0)):
@@ -33,6 +34,28 @@ def test_fresh_and_written_targets_get_the_same(prec, shift):
         assert (buf[:shift] == about).all() and (buf[shift + n:] == about).all()
         upd.rk3_steps_host_ptr(0, buf.ctypes.data + 8 * shift, 0)
         np.testing.assert_array_equal(buf[shift:shift + n], ref)
+    upd.close()
+
+
+def test_fresh_target_costs_no_more_than_mapping_it():
+    """A download into a fresh array of 48 MB against filling a fresh one on
+    the host, which is the mapping of its pages (both about 2 ms; one page at a
+    time by reading and writing it back took 15)."""
+    case = C.dam_break_case(n=1420, tfinal=1.0)
+    upd = Update(case.mesh, case.bath, case.params)
+    upd.upload(case.u0)
+    size = case.u0.nbytes
+    fill, down = [], []
+    for _ in range(9):
+        m = np.frombuffer(mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.uint8)
+        t = time.perf_counter()
+        m[:] = 1
+        fill.append(time.perf_counter() - t)
+        m = np.frombuffer(mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.uint8)
+        t = time.perf_counter()
+        upd.download_ptr(m.ctypes.data)
+        down.append(time.perf_counter() - t)
+    assert min(down) < 4.0 * min(fill), (min(down), min(fill))
     upd.close()
 
 
