@@ -730,7 +730,7 @@ static int to_device(swe_ctx* c, const double* un, bool device_src, int64_t node
 // numpy array's), while the GPU works: a copy into unmapped pages faults on every
 // one of them.  24 MB take 0.72 ms to map and 0.16 to copy, 0.99 ms unmapped
 // (touching each page from here takes 7.5: a read maps the zero page, the write
-// then copies it).  The bytes stay as they are.  Three pages tell a fresh array
+// then copies it).  The bytes stay as they are.  Two pages tell a fresh array
 // from one in use, whose call costs 15 us; page-locked memory is left alone.
 static void prefault(void* p, size_t bytes) {
   if (!p || bytes < (64 << 10)) return;
@@ -742,7 +742,7 @@ static void prefault(void* p, size_t bytes) {
   if (at.type != cudaMemoryTypeUnregistered) return;
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), mask = ~(page - 1);
   const uintptr_t b = reinterpret_cast<uintptr_t>(p), e = b + bytes;
-  for (const uintptr_t q : {e - 1, b + bytes / 2, b}) {
+  for (const uintptr_t q : {e - 1, b + bytes / 2}) {
     unsigned char in = 0;
     if (mincore(reinterpret_cast<void*>(q & mask), 1, &in) != 0) return;
     if (in & 1) continue;
