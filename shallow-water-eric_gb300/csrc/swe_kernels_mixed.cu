@@ -432,6 +432,13 @@ __device__ __forceinline__ void cp_range(void* dst, const void* src, int bytes) 
 }
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Entry k of this block's halo list.  Unsigned: a large mesh has up to four halo
+// rows per row, so the index passes 2^31 from 540M rows on; 2^32 would take 1.07
+// billion, which no memory holds.
+__device__ __forceinline__ int halo_row(const TileCtl& tc, unsigned k) {
+  return tc.halo_rows[blockIdx.x * (unsigned)tc.halo_cap + k];
+}
+
 // A block's tile and this thread's row.  All loads are independent of each
 // other, so one memory latency covers them.
 struct Tile {
@@ -448,7 +455,7 @@ __device__ __forceinline__ Tile tile_of(const Graph& G, const TileCtl& tc) {
   Tile t;
   t.r = (int)blockIdx.x * T + (int)threadIdx.x;
   t.live = t.r < (int)G.n_rows;
-  t.hr = (int)threadIdx.x < tc.halo_cap ? tc.halo_rows[(int)blockIdx.x * tc.halo_cap + (int)threadIdx.x] : -1;
+  t.hr = (int)threadIdx.x < tc.halo_cap ? halo_row(tc, threadIdx.x) : -1;
   t.hd = RowHead{0, 0, 0};
   if (t.live) t.hd = row_head(G, t.r);
   t.e0 = (int64_t)(((unsigned long long)(unsigned)h.y << 32) | (unsigned)h.x);
@@ -466,7 +473,7 @@ __device__ __forceinline__ void stage_nodes(const TileCtl& tc, const Tile& t, Lo
   if (t.live) put(i, ro, x);
   if (t.hr >= 0) put(T + i, rh, y);
   for (int k = i + T; k < tc.halo_cap; k += T) {       // halos above T rows
-    const int row = tc.halo_rows[(int)blockIdx.x * tc.halo_cap + k];
+    const int row = halo_row(tc, k);
     if (row >= 0) put(T + k, row, load(row));
   }
 }
