@@ -135,7 +135,7 @@ def b_alg(n, nnz, precision, S=3):
     return n * (3 * 8 * S + 8 + 8 + 4) + nnz * (4 + 2 * 8)
 
 
-def design_bytes(n, nnz):
+def design_bytes(n, nnz, sms):
     """Bytes per node that each mixed stage kernel reads and writes once per
     launch in the four-sweep design (3-component systems), with e the
     off-diagonal entries per row (16-bit position, c_ij or (d, mu), |c|lambda
@@ -145,7 +145,7 @@ def design_bytes(n, nnz):
     stage 1: 4e more written by k_dt and read by k_low.  Averaged per stage
     like swe_profile_kernels' times."""
     e = (nnz - n) / n
-    kept = 4 * e if n <= 4 * 256 * 152 else 0.0
+    kept = 4 * e if n <= 4 * 256 * sms else 0.0
     return {"dt": 25 + 10 * e + kept, "node": (21 + 4 * e) * 2 / 3, "low": 65 + 18 * e + kept / 3,
             "fct": 37 + 10 * e, "update": 78 + 10 * e + 16}
 
@@ -378,7 +378,8 @@ def run_ours(args, rank, world, dist):
     achieved = balg / (stage_ms / 1e3) / 1e9
     kernel_bw = {k: {"ms": round(prof[k], 4), "design_bytes_per_node": round(b, 1),
                      "gbs": round(b * N / (prof[k] / 1e3) / 1e9, 1)}
-                 for k, b in design_bytes(N, nnz).items() if prof.get(k)}
+                 for k, b in design_bytes(N, nnz, torch.cuda.get_device_properties(dev).multi_processor_count).items()
+                 if prof.get(k)}
     traffic = None
     tf = ROOT / "profiles" / "traffic_per_node_stage.json"
     if tf.exists():

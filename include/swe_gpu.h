@@ -227,11 +227,14 @@ enum { SWE_NKERNELS = 5 };
 int swe_profile_kernels(swe_ctx* ctx, int nsteps, double* ms_out);
 
 /* Launch configuration of the mixed kernels: the shared-memory row-tile
- * variants where the mesh has tiles (3-component systems, unless SWE_TILED=0),
- * else the fastest block-size / entry-batch / grid variant of each kernel,
- * timed on the current state (every variant gives the same bits).
+ * variants, by rule and without timing, where the mesh has tiles (both system
+ * sizes; not where a larger mesh is numbered so loosely that a tile reads some
+ * three rows outside it per row of its own, nor with SWE_TILED=0), else the fastest block-size / entry-batch /
+ * grid variant of each kernel, timed on the current state (every variant gives
+ * the same bits).
  * swe_rk3_steps runs it on its first call unless the environment sets
- * SWE_AUTOTUNE=0.  swe_tuning names the chosen configuration; setting
+ * SWE_AUTOTUNE=0.  swe_tuning names the chosen configuration ("autotuned ..."
+ * also where the rule chose it); setting
  * SWE_TUNE to that description (the text after "autotuned ") makes a later
  * context launch exactly those variants without timing (a malformed value
  * -> SWE_ERR_ARG). */

@@ -171,7 +171,10 @@ struct swe_ctx {
   WorkMix wm{};
   TileCtl tiles{};                       // row tiles of the shared-memory variants
   bool tiles_ok = false;
-  bool tiles_named = false;              // a tuning description may name tile variants (without tiles they run as the others)
+  // a tuning description may name tile variants: halos of up to 1270 rows, also
+  // where the mesh runs without tiles (the names then mean the gathers), so that
+  // a stored description stays valid
+  bool tiles_named = false;
   double* d_mass_acc = nullptr;
   double* d_mass_part = nullptr;         // per-slice partial sums of swe_mass
   int64_t* d_inst_slice = nullptr;       // n_inst + 1 slice offsets
@@ -954,7 +957,7 @@ static void enqueue_step(swe_ctx* c, bool open, bool close, const KernelEvents* 
       a.f64 = is_split(c);
       a.type1 = has_type1(c);
       set_modes(c, a);
-            if (stage == 2) { a.u = c->mB; a.out = c->mC; }
+      if (stage == 2) { a.u = c->mB; a.out = c->mC; }
       if (stage == 3) { a.u = c->mC; a.out = c->mA; }
       launch_stage_mix(a, s, kev, c->tune);
     }
@@ -1289,11 +1292,10 @@ static int entries_to_csr(swe_ctx* c, int inst, const T* d_arr, double* out, con
   }
   const int64_t s0 = L.row_off[inst] / 32, s1 = L.row_off[inst + 1] / 32;
   const int64_t e0 = L.slice_ptr[s0], e1 = L.slice_ptr[s1], r0 = L.row_off[inst], r1 = L.row_off[inst + 1];
-  const int64_t nb = std::min<int64_t>(((e1 - e0) + (r1 - r0) + 255) / 256, 152 * 16);
+  const int64_t nb = std::min<int64_t>(((e1 - e0) + (r1 - r0) + 255) / 256, 16 * c->sms);
   k_entries_to_csr<T, U><<<(unsigned)nb, 256, 0, c->stream>>>(d_arr, d_diag_rows, c->d_ref_pos, c->d_ref_pos_diag, e0, e1,
                                                               r0, r1, comp, c->d_csr);
   CK(cudaGetLastError());
-  prefault(out, c->meshes[inst].ja.size() * sizeof(double));
   CK(cudaMemcpyAsync(out, c->d_csr, c->meshes[inst].ja.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   return SWE_OK;
 }
@@ -1377,7 +1379,7 @@ SWE_API int swe_euler(swe_ctx* c, int inst, const double* un, double* unext) {
     a.f64 = is_split(c);
     a.type1 = has_type1(c);
     set_modes(c, a);
-        launch_stage_mix(a, c->stream, nullptr, c->tune);
+    launch_stage_mix(a, c->stream, nullptr, c->tune);
   }
   prefault(unext, sizeof(double) * c->S * (size_t)c->meshes[inst].np);
   if ((rc = cuda_check(c, cudaGetLastError(), "euler")) ||
@@ -1397,7 +1399,8 @@ SWE_API int swe_euler_intermediates(swe_ctx* c, int inst, double* dij_low, doubl
   if (!c || inst < 0 || inst >= c->n_inst) return fail(c, SWE_ERR_ARG, "bad instance");
   if (!c->euler_done || c->euler_inst != inst) return fail(c, SWE_ERR_ARG, "call swe_euler on this instance first");
   int rc;
-  if (u_low) prefault(u_low, sizeof(double) * c->S * (size_t)c->meshes[inst].np);
+  prefault(u_low, sizeof(double) * c->S * (size_t)c->meshes[inst].np);
+  for (double* entries : {dij_low, muij_low, fctmat, lij}) prefault(entries, sizeof(double) * c->meshes[inst].ja.size());
   if (c->precision == SWE_PREC_FP64) {
     if (dij_low && (rc = entries_to_csr(c, inst, c->w.dL, dij_low, c->w.dLii))) return rc;
     if (muij_low && (rc = entries_to_csr(c, inst, c->w.muL, muij_low, c->w.muLii))) return rc;
@@ -1672,7 +1675,7 @@ static int autotune(swe_ctx* c) {
   if (const char* spec = getenv("SWE_TUNE")) return apply_tuning(c, spec, "SWE_TUNE");
   int rc;
   const char* tenv = getenv("SWE_TILED");   // 0 leaves the tile variants out
-  // A mesh with row tiles runs them, without timing: per RK3 step they take
+  // A mesh with row tiles (see tiles_pay) runs them, without timing: per RK3 step they take
   // 42 / 45 / 70 / 96 / 1389 us at 2k / 20k / 100k / 200k / 4M nodes, the
   // global-gather variants 64 / 70 / 81 / 123 / 2142 us.  k_low runs four
   // resident blocks per SM (64 registers, a few spilled) where an SM has more

@@ -4,7 +4,7 @@
 // order, so every sum is formed in the same order as the Fortran loops.  This
 // translation unit is compiled with -fmad=false (no FMA contraction) and uses
 // IEEE sqrt/div: the result equals the FP64 CPU restatement bit for bit (the
-// Manning friction's pow() aside).  It is the parity path and the "plain FP64
+// Manning friction's x**(4/3) aside).  It is the parity path and the "plain FP64
 // GPU step" of the measurements.
 //
 // Per stage (SOURCES/update.f90 euler, :134-289, 'fct' + 'type2'):
