@@ -1275,7 +1275,7 @@ __global__ void __launch_bounds__(256) k_update_mix(Graph G, const InstConst* C,
     update_row<B, D, false>((int)r, row_head(G, r), G, C, St, u, dmu, w, u0, out, rk_stage, err, nb);
 }
 
-// HBM: 139-163 bytes per node at 4.4-4.8 TB/s, 4M nodes 159 -> 134 us; six
+// HBM: 139-163 bytes per node at 4.4-4.8 TB/s, 4M nodes 159 -> 131 us; six
 // resident blocks of 256 (40 registers) 141 -> 136 of it.
 template <int T, int S, bool D, bool FCT>
 __global__ void __launch_bounds__(T, S == 3 ? 6 * (256 / T) : 4) k_update_tile(Graph G, const InstConst* C,
