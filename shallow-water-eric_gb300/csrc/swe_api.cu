@@ -158,8 +158,9 @@ struct swe_ctx {
   // per-call operators (swe_euler, swe_compute_dij): their own instance state,
   // so that the time loop's is neither saved nor restored
   InstState* d_St_call = nullptr;
-  // page-locked: the instance states and the error word that a call reads back
+  // page-locked: the instance states, one d_ii and the error word that a call reads back
   InstState* h_St = nullptr;
+  double* h_dii = nullptr;
   unsigned* h_err = nullptr;
   double* d_times = nullptr;             // swe_set_time: time and t_final per instance
   int* d_ref_pos = nullptr;              // per entry / per row: CSR position in its instance or -1 (on first use)
@@ -515,10 +516,11 @@ static int build_device(swe_ctx* c, const std::vector<std::vector<double>>& bath
   c->d_St_call = upload_vec(c, hs, st);
   c->d_times = c->buf.alloc<double>(2 * (size_t)c->n_inst, st);
   if (st == cudaSuccess) {
-    void* h = g_pinned.take(sizeof(InstState) * c->n_inst + sizeof(unsigned));
+    void* h = g_pinned.take(sizeof(InstState) * c->n_inst + sizeof(double) + sizeof(unsigned));
     if (!h) return fail(c, SWE_ERR_CUDA, "page-locked allocation");
     c->h_St = static_cast<InstState*>(h);
-    c->h_err = reinterpret_cast<unsigned*>(c->h_St + c->n_inst);
+    c->h_dii = reinterpret_cast<double*>(c->h_St + c->n_inst);
+    c->h_err = reinterpret_cast<unsigned*>(c->h_dii + 1);
   }
   c->d_err = c->buf.alloc<unsigned>(1, st);
   c->d_ticket = c->buf.alloc<unsigned>(1, st);
@@ -1343,6 +1345,9 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
     rc = cuda_check(c, cudaGetLastError(), "compute_dij");
   }
   if (!rc && dij) prefault(dij, c->meshes[inst].ja.size() * sizeof(double));
+  if (!rc && dt_out && !dij)
+    rc = cuda_check(c, cudaMemcpyAsync(c->h_dii, dii + c->L.new_of_old[inst][0], sizeof(double), cudaMemcpyDeviceToHost,
+                                       c->stream), "compute_dij");
   if (!rc) rc = call_end(c, inst);                   // nothing is written to the caller's arrays on an error
   if (rc) { drain(c); return rc; }
   if (dij) {
@@ -1352,6 +1357,9 @@ SWE_API int swe_compute_dij(swe_ctx* c, int inst, const double* un, double* dij,
   if (dt_out) {                                      // COMPUTE_DT: CFL / max |d_ii| / m_i, the maximum from k_dt
     double mx;
     std::memcpy(&mx, &c->h_St[inst].maxd_bits, sizeof mx);
+    // the maximum over the nodes in order, which starts with node 0 and passes over a later NaN
+    const double d0 = dij ? dij[c->meshes[inst].diag[0]] : *c->h_dii;
+    if (d0 != d0) mx = d0;
     *dt_out = c->params[inst].cfl * 1 / mx;
   }
   return SWE_OK;

@@ -2,6 +2,8 @@
 where the rescaling of update.f90:866 is 0) reaches the state of the rows that
 take it from a neighbour and ends the call, in the FP64 row kernels as in the
 general ones, which a batch with a 'galerkin' instance runs."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -59,3 +61,27 @@ def test_nan_residual(visc, kind, sgn, nx, ny):
         o.set_params(oracle.Params(*p.fields()))
         o.set_bath(z)
         assert not np.isfinite(o.euler(u)).all()
+
+
+@pytest.mark.parametrize("dry", ["first", "other"])
+def test_dt_of_a_nan_wave_speed(dry):
+    """htiny = 0 and a dry node: 1/h is 0/0 there, and so is d_ii of its wet
+    neighbours.  The dt is a NaN where node 1, with which the maximum begins, is
+    one of them, and passes over the others."""
+    mesh, u = _scene("rest", 0, 9, 11)
+    z = np.zeros(u.shape[1])
+    tri = mesh["jj"][:, (mesh["jj"] == 1).any(axis=0)][:, 0]
+    u[0, tri[tri != 1][0] - 1 if dry == "first" else u.shape[1] // 2] = 0.0
+    p = C.Params(max_water_h=1.0, htiny=0.0)
+    o = oracle.Oracle(mesh["jj"], mesh["rr"])
+    o.set_params(oracle.Params(*p.fields()))
+    o.set_bath(z)
+    ref = o.compute_dij(u)
+    assert np.isnan(ref[1]) == (dry == "first")
+    upd = Update(mesh, z, p)
+    dij, dt = upd.compute_dij(u)
+    np.testing.assert_array_equal(dij, ref[0])
+    np.testing.assert_array_equal(dt, ref[1])
+    only = ctypes.c_double()
+    assert upd._L.swe_compute_dij(upd.h, 0, L.dp(np.asfortranarray(u)), None, ctypes.byref(only)) == L.SWE_OK
+    np.testing.assert_array_equal(only.value, ref[1])
